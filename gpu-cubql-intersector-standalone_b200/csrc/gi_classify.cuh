@@ -183,23 +183,47 @@ __device__ __forceinline__ int lone_index(const int s[3])
     return 2;
 }
 
-// Endpoint pattern of a pair that the first stage found intersecting: in
-// general position the intersection is the segment between two of the four
-// edge-plane crossings X0, X1 (P's edges from its lone vertex o1, in vertex
-// order, through plane(Q)) and Y0, Y1 (Q's edges from o2 through plane(P));
-// xin / yin mark the crossings that lie inside the other interval.  The exact
-// classification gives the same points in the same order (X's, then Y's), so a
-// consumer can construct them without evaluating any sign again.
-//   bit 0 valid, bits 1-2 o1, bits 3-4 o2, bits 5-6 xin, bits 7-8 yin
-constexpr unsigned kPatValid = 1u;
-__device__ __forceinline__ unsigned make_pattern(int o1, int o2, unsigned xin, unsigned yin)
+// Construction code of a result: what its segments are made of, in one word, so
+// that whoever builds them evaluates no sign again (22 bits used):
+//   bits 0-1  kind: 0 no segment, 1 one point, 2 one segment, 3 a triangle's three edges
+//   bits 2-3  axis dropped by the line-line crossings
+//   bits 4 + 6k ..  point k (k < kind):
+//     0 .. 5     vertex v (0-2 of P, 3-5 of Q)
+//     6 .. 17    6 + 2 e + r: edge e through the other triangle's plane; edge e
+//                (0-2 of P, 3-5 of Q) runs from vertex e % 3 to the next one, r = 1 backwards
+//     18 .. 53   18 + 4 (3 e1 + e2) + 2 w + r: edge e1 of P crossing edge e2 of Q
+//                in the projection; the point lies on P's edge, with w = 1 on
+//                Q's, r = 1 backwards
+// The edges keep the direction they are constructed in, so a point is the same
+// whichever stage found it.
+constexpr unsigned kCodePlane = 6u, kCodeLine = 18u;
+__device__ __forceinline__ unsigned edge_code(unsigned i, unsigned j)  // 2 e + r of edge i -> j (vertices 0..2)
 {
-    return kPatValid | ((unsigned)o1 << 1) | ((unsigned)o2 << 3) | (xin << 5) | (yin << 7);
+    const unsigned e = i + j == 1u ? 0u : (i + j == 3u ? 1u : 2u);
+    return 2u * e + (i == e ? 0u : 1u);
+}
+__device__ __forceinline__ unsigned make_code(unsigned kind, unsigned drop, unsigned p0, unsigned p1, unsigned p2)
+{
+    return kind | (drop << 2) | (p0 << 4) | (p1 << 10) | (p2 << 16);
+}
+// General position: the segment between the two of the four edge-plane crossings
+// X0, X1 (P's edges from its lone vertex o1, in vertex order, through plane(Q))
+// and Y0, Y1 (Q's edges from o2 through plane(P)) that lie inside the other
+// interval (bits of xin, yin), in the order X's, then Y's.
+__device__ __forceinline__ unsigned crossing_code(int o1, int o2, unsigned xin, unsigned yin)
+{
+    unsigned m = xin | (yin << 2);
+    const unsigned s0 = __ffs(m) - 1;
+    m &= m - 1u;
+    const unsigned s1 = m ? __ffs(m) - 1 : s0;
+    auto pt = [&](unsigned s) {
+        const unsigned lone = s < 2u ? o1 : o2;
+        const unsigned other = (s & 1u) == 0u ? (lone == 0u ? 1u : 0u) : (lone == 2u ? 1u : 2u);
+        return kCodePlane + (s < 2u ? 0u : 6u) + edge_code(lone, other);
+    };
+    return make_code(2u, 0u, pt(s0), pt(s1), 0u);
 }
 
-// First stage: decides the general-position case (every vertex strictly off the
-// other triangle's plane) with filtered signs; everything else escalates.  For
-// an intersecting pair, *pat receives its endpoint pattern (make_pattern).
 // The vertex of three that `i` names (0, 1, 2), by selects (no indexed array).
 __device__ __forceinline__ double3 sel3(int i, const double3& a, const double3& b, const double3& c)
 {
@@ -216,11 +240,11 @@ __device__ __forceinline__ int lone3(int s0, int s1, int s2)
 
 // First stage: decides the general-position case (every vertex strictly off the
 // other triangle's plane) with filtered signs; everything else escalates.  For
-// an intersecting pair, *pat receives its endpoint pattern (make_pattern).
+// an intersecting pair, *code receives its construction code (crossing_code).
 // Inlined, on values only (the vertex choices are selects), so that nothing of
 // it lives in local memory.
 template <class T>
-__device__ __forceinline__ int classify_fast(const double3* P, const double3* Q, unsigned* pat = nullptr)
+__device__ __forceinline__ int classify_fast(const double3* P, const double3* Q, unsigned* code = nullptr)
 {
     const double3 P0 = P[0], P1 = P[1], P2 = P[2], Q0 = Q[0], Q1 = Q[1], Q2 = Q[2];
     const Plane<T> pp = make_plane<T>(vdiff<T>(P1, P0), vdiff<T>(P2, P0));
@@ -256,7 +280,7 @@ __device__ __forceinline__ int classify_fast(const double3* P, const double3* Q,
     const unsigned xin = (c00 * c01 < 0 ? 1u : 0u) | (c10 * c11 < 0 ? 2u : 0u);
     const unsigned yin = (c00 * c10 < 0 ? 1u : 0u) | (c01 * c11 < 0 ? 2u : 0u);
     if (!(xin | yin)) return DEC_NO;
-    if (pat) *pat = make_pattern(o1, o2, xin, yin);
+    if (code) *code = crossing_code(o1, o2, xin, yin);
     return DEC_YES;
 }
 
@@ -1059,26 +1083,68 @@ static __device__ __noinline__ bool construct_point(const double3* pts, const Sy
     return construct_exact(pts, s, out);
 }
 
-// Symbolic result of a pair from its endpoint pattern (make_pattern): the same
-// points, in the same order, as classify_exact gives for it.
-__device__ __forceinline__ void pattern_result(unsigned pat, TTRes& r)
+// Construction code of an exact classification.
+__device__ __forceinline__ unsigned symbolic_code(const SymPt& s)
 {
-    const int o1 = (pat >> 1) & 3, o2 = (pat >> 3) & 3;
-    const unsigned xin = (pat >> 5) & 3, yin = (pat >> 7) & 3;
-    r.n = 0;
-    int k = 0;
-    for (int i = 0; i < 3; i++) {
-        if (i == o1) continue;
-        if ((xin >> k) & 1u) r.pt[r.n++] = sp_plane(o1, i, 3, 4, 5);
-        k++;
+    if (s.kind == PK_VERTEX) return s.a;
+    const unsigned side = s.a >= 3 ? 1u : 0u;
+    const unsigned er = edge_code(s.a - 3u * side, s.b - 3u * side);
+    if (s.kind == PK_PLANE) return kCodePlane + 6u * side + er;
+    const unsigned o = 3u * (1u - side), eo = edge_code(s.p - o, s.q - o) >> 1;
+    return kCodeLine + 4u * (side ? 3u * eo + (er >> 1) : 3u * (er >> 1) + eo) + 2u * side + (er & 1u);
+}
+__device__ __forceinline__ unsigned result_code(const TTRes& r)
+{
+    if (r.kind != KIND_POINT && r.kind != KIND_SEGMENT && r.kind != KIND_TRIANGLE) return 0u;
+    unsigned c = (unsigned)r.kind, drop = 0u;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        if (k >= r.kind) break;
+        c |= symbolic_code(r.pt[k]) << (4 + 6 * k);
+        if (r.pt[k].kind == PK_LINE2) drop = r.pt[k].drop;
     }
-    k = 0;
-    for (int j = 0; j < 3; j++) {
-        if (j == o2) continue;
-        if ((yin >> k) & 1u) r.pt[r.n++] = sp_plane(3 + o2, 3 + j, 0, 1, 2);
-        k++;
+    return c | (drop << 2);
+}
+
+// The point of code `c`, exact path included, from the six vertices in memory
+// (called when the fast constructions below could not round it).
+static __device__ __noinline__ bool code_point_exact(const double3* pts, unsigned c, unsigned drop, double3& out,
+                                                     unsigned long long* nexact)
+{
+    SymPt s;
+    if (c < kCodePlane) {
+        s = sp_vertex((int)c);
+    } else if (c < kCodeLine) {
+        const unsigned e = (c - kCodePlane) >> 1, r = c & 1u, base = e < 3u ? 0u : 3u;
+        const int i = (int)e, j = (int)(base + (e - base + 1u) % 3u), o = 3 - (int)base;
+        s = r ? sp_plane(j, i, o, o + 1, o + 2) : sp_plane(i, j, o, o + 1, o + 2);
+    } else {
+        const unsigned q = (c - kCodeLine) >> 2, w = (c - kCodeLine) & 2u, r = (c - kCodeLine) & 1u;
+        const int e1 = (int)(q / 3u), e2 = (int)(q % 3u);
+        const int p0 = e1, p1 = (e1 + 1) % 3, q0 = 3 + e2, q1 = 3 + (e2 + 1) % 3;
+        if (w) s = r ? sp_line2(q1, q0, p0, p1, (int)drop) : sp_line2(q0, q1, p0, p1, (int)drop);
+        else s = r ? sp_line2(p1, p0, q0, q1, (int)drop) : sp_line2(p0, p1, q0, q1, (int)drop);
     }
-    r.kind = r.n == 1 ? KIND_POINT : KIND_SEGMENT;
+    return construct_point(pts, s, out, nexact);
+}
+
+// Crossing of edge (a, b) with the line (p, q) in the projection dropping an
+// axis, fast path only, on values in registers: the coordinates to use are
+// chosen by selects.
+__device__ __forceinline__ bool construct_line_fast(const double3& p, const double3& q, const double3& a,
+                                                    const double3& b, unsigned drop, double3& out)
+{
+    auto U = [&](const double3& v) { return drop == 0u ? v.y : (drop == 1u ? v.z : v.x); };
+    auto V = [&](const double3& v) { return drop == 0u ? v.z : (drop == 1u ? v.x : v.y); };
+    auto side = [&](const double3& x, double* perm) {
+        const dd l = dd_mul(two_diff_dd(U(p), U(x)), two_diff_dd(V(q), V(x)));
+        const dd r = dd_mul(two_diff_dd(V(p), V(x)), two_diff_dd(U(q), U(x)));
+        *perm = fabs(l.hi) + fabs(r.hi);
+        return dd_add(l, dd_neg(r));
+    };
+    double pa, pb;
+    const dd sa = side(a, &pa), sb = side(b, &pb);
+    return construct_fast(a, b, sa, sb, 32.0 * 0x1p-106 * pa, 32.0 * 0x1p-106 * pb, out);
 }
 
 }  // namespace gi
