@@ -1106,6 +1106,26 @@ __device__ __forceinline__ unsigned result_code(const TTRes& r)
     return c | (drop << 2);
 }
 
+// Decides a pair that the first stage escalated; *code receives the construction
+// code of an intersecting one.  After the FP32 form (fp32) the FP64 form of the
+// same filter is asked first: its bound is 2^29 times tighter, so of pairs in
+// general position it leaves none to the integers, whose out-of-line code and
+// local memory take 8 us for a single pair (two 1.3M-triangle meshes with 3
+// escalated pairs: exact phase of the finish 9.0 -> 4.8 us; 1.2 M pairs
+// classified, a few escalated: 59.8 -> 58.9 us).  Pairs that are not in general
+// position pay for it: 2.4 M on coplanar grids, 3.2 -> 3.5 ms.
+__device__ __forceinline__ bool decide_escalated(const double3* pts, bool fp32, unsigned* code, ExactSigns& S)
+{
+    if (fp32) {
+        const int dec = classify_fast<double>(pts, pts + 3, code);
+        if (dec != DEC_ESC) return dec == DEC_YES;
+    }
+    TTRes r;
+    classify_exact(pts, r, S);
+    *code = result_code(r);
+    return r.kind != KIND_NONE;
+}
+
 // The point of code `c`, exact path included, from the six vertices in memory
 // (called when the fast constructions below could not round it).
 static __device__ __noinline__ bool code_point_exact(const double3* pts, unsigned c, unsigned drop, double3& out,

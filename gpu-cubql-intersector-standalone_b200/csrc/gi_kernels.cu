@@ -2183,10 +2183,7 @@ __device__ __forceinline__ void exact_stage(const Bufs& B, unsigned gtid, unsign
             load_tri<false>(J.A, J.pa, c.y, pts, &ta);
             load_tri<false>(J.B, J.pb, c.z, pts + 3, &tb);
             ExactSigns S{&C->err, 0ull};
-            TTRes r;
-            classify_exact(pts, r, S);
-            yes = r.kind != KIND_NONE;
-            code = result_code(r);
+            yes = decide_escalated(pts, B.precision == 0, &code, S);
             nexact += S.nexact;
         }
         unsigned pr = warp_append(yes, &C->res);

@@ -66,7 +66,8 @@ __global__ void __launch_bounds__(256) k_pairs_filter(JobDev J, const int32_t* _
 }
 
 __global__ void __launch_bounds__(128) k_pairs_exact(JobDev J, const int32_t* __restrict__ pairs,
-                                                     uint8_t* __restrict__ out, unsigned* __restrict__ scratch)
+                                                     uint8_t* __restrict__ out, unsigned* __restrict__ scratch,
+                                                     bool fp32)
 {
     const unsigned nesc = __ldcg(&scratch[0]);
     for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < nesc; k += gridDim.x * blockDim.x) {
@@ -75,9 +76,8 @@ __global__ void __launch_bounds__(128) k_pairs_exact(JobDev J, const int32_t* __
         pairs_load_tri(J.A, J.pa, (uint32_t)pairs[2 * (size_t)i], pts);
         pairs_load_tri(J.B, J.pb, (uint32_t)pairs[2 * (size_t)i + 1], pts + 3);
         ExactSigns S{&scratch[1], 0ull};
-        TTRes r;
-        classify_exact(pts, r, S);
-        out[i] = r.kind != KIND_NONE ? 1 : 0;
+        unsigned code;
+        out[i] = decide_escalated(pts, fp32, &code, S) ? 1 : 0;
     }
 }
 
@@ -94,7 +94,7 @@ static cudaError_t run_pairs(const JobDev& J, const int32_t* d_pairs, uint32_t n
         if (blocks > maxb) blocks = maxb;
         if (precision == GI_PREC_FP64) k_pairs_filter<true><<<blocks, 256, 0, st>>>(J, d_pairs, n, d_out, scratch);
         else k_pairs_filter<false><<<blocks, 256, 0, st>>>(J, d_pairs, n, d_out, scratch);
-        k_pairs_exact<<<sms * 4, 128, 0, st>>>(J, d_pairs, d_out, scratch);
+        k_pairs_exact<<<sms * 4, 128, 0, st>>>(J, d_pairs, d_out, scratch, precision != GI_PREC_FP64);
         note_launches(2);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
