@@ -4,7 +4,7 @@
 // src/GPUIntersector/KernelBVHController.cu:603-699 in the reference, whose chunk
 // loop syncs and copies to the host several times per chunk and calls CGAL on
 // the CPU for undecided pairs):
-//   counters reset -> frontier init -> k_traverse (cooperative) -> k_exact
+//   counters reset -> k_traverse_blocks (cooperative) -> k_exact
 //   -> one counters read-back (capacity check; buffers grow x4 and the call is
 //      re-run on overflow) -> k_segments -> ordering -> copies to the host.
 // No CPU fallback exists: every pair is decided on the device.
@@ -84,7 +84,7 @@ extern "C" gi_status gi_create(const gi_options* opts, gi_ctx** out)
     c->device = opts ? opts->device : 0;
     c->budget = opts ? opts->hbm_budget_bytes : 0;
     c->flags = opts ? opts->flags : 0;
-    if (c->flags & GI_FLAG_FIXED_SHAPE) c->fixed_shape = (int)((c->flags >> 9) & 7u);
+    if (c->flags & GI_FLAG_FIXED_SHAPE) c->shape = (int)((c->flags >> 9) & 7u);
     if (c->device < 0 || c->device >= ndev) {
         delete c;
         return GI_ERR_INVALID_ARG;
@@ -128,7 +128,7 @@ extern "C" gi_status gi_destroy(gi_ctx* c)
     c->copy_pool.reset();
     if (c->d_cnt) cudaFree(c->d_cnt);
     if (c->d_jobs) cudaFree(c->d_jobs);
-    void* pooled[] = {c->queue, c->qflag,     c->cand,         c->cflag,   c->res,
+    void* pooled[] = {c->queue, c->qflag,     c->res,
                       c->esc,   c->segs,      c->nseg,         c->pairs_out, c->job_out,
                       c->segs_out, c->segpair_out, c->order_scratch};
     for (void* p : pooled)
@@ -480,10 +480,10 @@ DevPose make_dev_pose(const gi_pose& p)
         double m = fabs(d.C[r]) + fabs(d.T[r]) + fabs(d.R[3 * r]) * fabs(d.C[0]) +
                    fabs(d.R[3 * r + 1]) * fabs(d.C[1]) + fabs(d.R[3 * r + 2]) * fabs(d.C[2]);
         d.padm64[r] = m * (1.0 + 0x1p-40);
-        d.bf[r] = (float)d.b64[r];
-        d.padm[r] = nextafterf((float)d.padm64[r], INFINITY);
+        d.fw.row[r] = make_float4((float)d.R[3 * r], (float)d.R[3 * r + 1], (float)d.R[3 * r + 2], (float)d.b64[r]);
+        d.fw.padm[r] = nextafterf((float)d.padm64[r], INFINITY);
     }
-    for (int i = 0; i < 9; i++) d.Rf[i] = (float)d.R[i];
+    d.fw.use = d.identity ? 0 : 1;
     // inverse map, used to test boxes in this mesh's own frame as well
     if (!d.identity) {
         double eta = 0.0;
@@ -505,10 +505,10 @@ DevPose make_dev_pose(const gi_pose& p)
             }
             d.bi64[r] = d.C[r] - acc;
             d.padmi64[r] = m * (1.0 + 0x1p-40);
-            d.bif[r] = (float)d.bi64[r];
-            d.padmi[r] = nextafterf((float)d.padmi64[r], INFINITY);
+            d.inv.row[r] = make_float4((float)d.Ri64[3 * r], (float)d.Ri64[3 * r + 1], (float)d.Ri64[3 * r + 2], (float)d.bi64[r]);
+            d.inv.padm[r] = nextafterf((float)d.padmi64[r], INFINITY);
         }
-        for (int i = 0; i < 9; i++) d.Rif[i] = (float)d.Ri64[i];
+        d.inv.use = d.inv_ok;
     }
     return d;
 }
@@ -616,12 +616,11 @@ static gi_status run_jobs(gi_ctx* c, const std::vector<JobDev>& jobs, const gi_i
     memcpy(c->h_jobs, jobs.data(), sizeof(JobDev) * nj);
     CK(c, cudaMemcpyAsync(c->d_jobs, c->h_jobs, sizeof(JobDev) * nj, cudaMemcpyHostToDevice, c->st), "jobs copy");
     const bool tiny = (c->flags & GI_FLAG_TINY_BUFFERS) != 0;
-    uint32_t need_front =
-        std::max<uint32_t>(c->cap_front, tiny ? 64u : (uint32_t)std::min<uint64_t>(std::max<uint64_t>(1u << 21, sumT), 1u << 26));
-    uint32_t need_cand =
-        std::max<uint32_t>(c->cap_cand, tiny ? 64u : (uint32_t)std::min<uint64_t>(sumT * 2 + 4096, 1u << 22));
-    uint32_t need_res = std::max<uint32_t>(c->cap_res, tiny ? 64u : std::max<uint32_t>(need_cand / 4, 1u << 16));
-    uint32_t need_esc = std::max<uint32_t>(c->cap_esc, tiny ? 64u : std::max<uint32_t>(need_cand / 4, 1u << 16));
+    // pool of handed-over node pairs: a few slots per resident block at every size
+    uint32_t need_front = std::max<uint32_t>(c->cap_front, tiny ? 64u : 1u << 21);
+    const uint32_t guess = (uint32_t)std::min<uint64_t>(sumT * 2 + 4096, 1u << 22);
+    uint32_t need_res = std::max<uint32_t>(c->cap_res, tiny ? 64u : std::max<uint32_t>(guess / 4, 1u << 16));
+    uint32_t need_esc = std::max<uint32_t>(c->cap_esc, tiny ? 64u : std::max<uint32_t>(guess / 4, 1u << 16));
     const unsigned long long launches0 = launch_count();
     Counters& H = *c->h_cnt;
     int retries = 0;
@@ -650,19 +649,13 @@ static gi_status run_jobs(gi_ctx* c, const std::vector<JobDev>& jobs, const gi_i
     if (c->fin_backoff) c->fin_backoff--;
     const int kbits = ba + bb + bj;
     const int fin_shift = kbits > kFinPartBits ? kbits - kFinPartBits : 0;
-    const uint32_t tune_key = TravTuner::key(prec, nj, sumT);
-    const int shape = c->fixed_shape >= 0 ? c->fixed_shape : c->tuner.pick(tune_key);
+    const int shape = c->shape;
     for (;;) {
         CK(c, grow(c->queue, c->cap_front, need_front, c->pool, c->st), "node queue");
         if (c->cap_qflag < c->cap_front) {
             // fresh tag words must not match any call's tag: zero them
             CK(c, grow(c->qflag, c->cap_qflag, c->cap_front, c->pool, c->st), "node queue");
             CK(c, cudaMemsetAsync(c->qflag, 0, sizeof(unsigned) * c->cap_qflag, c->st), "node queue");
-        }
-        CK(c, grow(c->cand, c->cap_cand, need_cand, c->pool, c->st), "candidates");
-        if (c->cap_cflag < c->cap_cand) {
-            CK(c, grow(c->cflag, c->cap_cflag, c->cap_cand, c->pool, c->st), "candidates");
-            CK(c, cudaMemsetAsync(c->cflag, 0, sizeof(unsigned) * c->cap_cflag, c->st), "candidates");
         }
         CK(c, grow(c->res, c->cap_res, need_res, c->pool, c->st), "results");
         CK(c, grow(c->esc, c->cap_esc, need_esc, c->pool, c->st), "escalations");
@@ -696,13 +689,9 @@ static gi_status run_jobs(gi_ctx* c, const std::vector<JobDev>& jobs, const gi_i
         b.queue = c->queue;
         b.qflag = c->qflag;
         b.cap_queue = std::min(c->cap_front, c->cap_qflag);
-        b.cand = c->cand;
-        b.cflag = c->cflag;
-        b.cap_cand = std::min(c->cap_cand, c->cap_cflag);
         if (++c->tag == 0) {
             // after 2^32 calls the tags wrap: clear the tag words once
             CK(c, cudaMemsetAsync(c->qflag, 0, sizeof(unsigned) * c->cap_qflag, c->st), "node queue");
-            CK(c, cudaMemsetAsync(c->cflag, 0, sizeof(unsigned) * c->cap_cflag, c->st), "candidates");
             c->tag = 1;
         }
         b.tag = c->tag;
@@ -713,13 +702,8 @@ static gi_status run_jobs(gi_ctx* c, const std::vector<JobDev>& jobs, const gi_i
         b.cnt = c->d_cnt;
         b.precision = prec;
         b.two_frame = nj > 1 ? 1 : 0;
-        // one pair: skip the narrowest level by seeding from the depth-4 cuts
-        // (up to 256 x 256 seed tests); a batch keeps the depth-3 cuts, whose
-        // seed tests grow with the number of jobs
-        b.deep_seed = nj == 1 ? 1 : 0;
-        b.quad_below = 0u;   // set by the launcher of the level-synchronous traversal
-        b.cand_blocks = 0u;
-        b.publish = 0u;
+        b.keep = 0u;  // set by the launcher
+        b.job0 = jobs[0];
         CK(c, cudaMemsetAsync(c->d_cnt, 0, sizeof(Counters), c->st), "counters");
         CK(c, cudaEventRecord(c->ev[0], c->st), "event");
         CK(c, launch_traverse(b, c->cfg, prec, trav_shape(shape), c->st), "traverse");
@@ -804,10 +788,10 @@ static gi_status run_jobs(gi_ctx* c, const std::vector<JobDev>& jobs, const gi_i
                 uint64_t v = std::max<uint64_t>((uint64_t)cur * 4, (uint64_t)seen + seen / 2 + 1024);
                 return (uint32_t)std::min<uint64_t>(v, 0x7fffffffu);
             };
-            if (H.overflow & kOvfFrontier) need_front = g4(c->cap_front, H.q_tail);
-            if (H.overflow & kOvfCand) need_cand = g4(c->cap_cand, (uint32_t)(H.work_cand >> 32));
-            if (H.overflow & (kOvfRes | kOvfCand)) need_res = g4(c->cap_res, H.res);
-            if (H.overflow & (kOvfEsc | kOvfCand)) need_esc = g4(c->cap_esc, H.esc);
+            // (a pool that was too small starves the later stages: they may grow too)
+            if (H.overflow & kOvfFrontier) need_front = g4(c->cap_front, (uint32_t)std::min<uint64_t>((H.pool & 0xffffffffull) * 64, 0x7fffffffu));
+            if (H.overflow & kOvfRes) need_res = g4(c->cap_res, H.res);
+            if (H.overflow & kOvfEsc) need_esc = g4(c->cap_esc, H.esc);
             continue;
         }
         if (H.order_redo) {
@@ -871,7 +855,6 @@ static gi_status run_jobs(gi_ctx* c, const std::vector<JobDev>& jobs, const gi_i
         cudaEventElapsedTime(&ms_seg, c->ev[2], c->ev[3]);
         cudaEventElapsedTime(&ms_sort, c->ev[3], c->ev[4]);
     }
-    if (c->fixed_shape < 0) c->tuner.report(tune_key, shape, ms_trav);
     // split per job (sorted by job first)
     std::vector<uint32_t> job_start(nj + 1, 0);
     if (nj == 1) {
@@ -938,18 +921,10 @@ static gi_status run_jobs(gi_ctx* c, const std::vector<JobDev>& jobs, const gi_i
         s2.ms_segments = ms_seg;
         s2.ms_sort = ms_sort;
         s2.ms_total = ms_total;
-        static_assert(sizeof(s2.level_end_ms) / sizeof(double) == (size_t)kLevelTimes, "level time slots");
         if (fin && H.fin_ns[0] && H.fin_ns[4] >= H.fin_ns[0]) {
             for (int k = 0; k < 4; k++)
                 s2.finish_ms[k] = H.fin_ns[k + 1] >= H.fin_ns[0] ? 1e-6 * double(H.fin_ns[k + 1] - H.fin_ns[0]) : 0.0;
             s2.finish_phases = 4;
-        }
-        if (trav_shape(shape).levels && H.t_start) {
-            const uint32_t nl = std::min<uint32_t>(H.levels + 1u, (uint32_t)kLevelTimes);
-            for (uint32_t l = 0; l < nl && H.level_ns[l] >= H.t_start; l++) {
-                s2.level_end_ms[l] = 1e-6 * double(H.level_ns[l] - H.t_start);
-                s2.level_times = l + 1;
-            }
         }
     }
     buf = nullptr;  // now held by the results

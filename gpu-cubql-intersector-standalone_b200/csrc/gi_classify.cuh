@@ -250,33 +250,32 @@ __device__ __forceinline__ int classify_fast(const double3* P, const double3* Q,
     const Plane<T> pp = make_plane<T>(vdiff<T>(P1, P0), vdiff<T>(P2, P0));
     if (!pp.proper) return DEC_ESC;
     // orient3d(P0,P1,P2,X) = (P0 - X) . nP
-    const int s20 = filt_dot<T>(pp, vdiff<T>(P0, Q0)), s21 = filt_dot<T>(pp, vdiff<T>(P0, Q1)),
-              s22 = filt_dot<T>(pp, vdiff<T>(P0, Q2));
+    const V3<T> f0 = vdiff<T>(P0, Q0);
+    const int s20 = filt_dot<T>(pp, f0), s21 = filt_dot<T>(pp, vdiff<T>(P0, Q1)), s22 = filt_dot<T>(pp, vdiff<T>(P0, Q2));
     if ((s20 == 1 && s21 == 1 && s22 == 1) || (s20 == -1 && s21 == -1 && s22 == -1)) return DEC_NO;
     const Plane<T> pq = make_plane<T>(vdiff<T>(Q1, Q0), vdiff<T>(Q2, Q0));
     if (!pq.proper) return DEC_ESC;
-    const int s10 = filt_dot<T>(pq, vdiff<T>(Q0, P0)), s11 = filt_dot<T>(pq, vdiff<T>(Q0, P1)),
+    const int s10 = filt_dot<T>(pq, V3<T>{-f0.x, -f0.y, -f0.z}), s11 = filt_dot<T>(pq, vdiff<T>(Q0, P1)),
               s12 = filt_dot<T>(pq, vdiff<T>(Q0, P2));
     if ((s10 == 1 && s11 == 1 && s12 == 1) || (s10 == -1 && s11 == -1 && s12 == -1)) return DEC_NO;
     if (s10 == kUnsure || s11 == kUnsure || s12 == kUnsure || s20 == kUnsure || s21 == kUnsure || s22 == kUnsure)
         return DEC_ESC;
-    // both intervals consist of two edge crossings from the lone vertex; the
-    // edges in vertex order of their other end, each from its negative end
+    // both intervals consist of two edge crossings from the lone vertex (L), X_i
+    // on P's edge to its i-th other vertex (A, B), Y_j on Q's.  Position of Y_j
+    // against X_i along the line of the planes: the sign of det[L1 - L2, X - L2,
+    // Y - L2], up to one factor of the pair, which the products below square.
+    // With L2 as the common origin the four signs share five differences and two
+    // cross products (each sign by itself took three and one: 36 FP64
+    // differences and conversions instead of 15).
     const int o1 = lone3(s10, s11, s12), o2 = lone3(s20, s21, s22);
-    const bool neg1 = (o1 == 0 ? s10 : (o1 == 1 ? s11 : s12)) < 0;
-    const bool neg2 = (o2 == 0 ? s20 : (o2 == 1 ? s21 : s22)) < 0;
     const double3 L1 = sel3(o1, P0, P1, P2), A1 = o1 == 0 ? P1 : P0, B1 = o1 == 2 ? P1 : P2;
     const double3 L2 = sel3(o2, Q0, Q1, Q2), A2 = o2 == 0 ? Q1 : Q0, B2 = o2 == 2 ? Q1 : Q2;
-    const double3 xn0 = neg1 ? L1 : A1, xp0 = neg1 ? A1 : L1, xn1 = neg1 ? L1 : B1, xp1 = neg1 ? B1 : L1;
-    const double3 yn0 = neg2 ? L2 : A2, yp0 = neg2 ? A2 : L2, yn1 = neg2 ? L2 : B2, yp1 = neg2 ? B2 : L2;
-    const int c00 = filt_o3<T>(xn0, xp0, yn0, yp0);
-    if (c00 == kUnsure) return DEC_ESC;
-    const int c01 = filt_o3<T>(xn0, xp0, yn1, yp1);
-    if (c01 == kUnsure) return DEC_ESC;
-    const int c10 = filt_o3<T>(xn1, xp1, yn0, yp0);
-    if (c10 == kUnsure) return DEC_ESC;
-    const int c11 = filt_o3<T>(xn1, xp1, yn1, yp1);
-    if (c11 == kUnsure) return DEC_ESC;
+    const V3<T> l = vdiff<T>(L1, L2), ya = vdiff<T>(A2, L2), yb = vdiff<T>(B2, L2);
+    const Plane<T> na = make_plane<T>(l, vdiff<T>(A1, L2));
+    const int c00 = filt_dot<T>(na, ya), c01 = filt_dot<T>(na, yb);
+    const Plane<T> nb = make_plane<T>(l, vdiff<T>(B1, L2));
+    const int c10 = filt_dot<T>(nb, ya), c11 = filt_dot<T>(nb, yb);
+    if (c00 == kUnsure || c01 == kUnsure || c10 == kUnsure || c11 == kUnsure) return DEC_ESC;
     const unsigned xin = (c00 * c01 < 0 ? 1u : 0u) | (c10 * c11 < 0 ? 2u : 0u);
     const unsigned yin = (c00 * c10 < 0 ? 1u : 0u) | (c01 * c11 < 0 ? 2u : 0u);
     if (!(xin | yin)) return DEC_NO;

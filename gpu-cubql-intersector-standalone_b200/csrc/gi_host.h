@@ -263,59 +263,6 @@ struct gi_result {
     gi_stats stats;
 };
 
-// Traversal autotuner: per workload class (precision, number of jobs, total
-// triangles in factors of 4), each traversal shape is timed on the context's
-// own calls (the best of kTries traversals, CUDA events on the context's
-// stream); a shape whose first time is over 1.3x the best so far is not tried
-// again.  After that the fastest shape is used.  Every shape gives the same
-// result.
-struct TravTuner {
-    static constexpr int kTries = 2;
-    struct Entry {
-        float best[gi::kTravShapes];
-        int tries[gi::kTravShapes];
-        int choice = -1;
-        Entry()
-        {
-            for (int k = 0; k < gi::kTravShapes; k++) {
-                best[k] = 3.0e38f;
-                tries[k] = 0;
-            }
-        }
-    };
-    std::map<uint32_t, Entry> table;
-    static uint32_t key(int precision, uint32_t njobs, uint64_t tris)
-    {
-        const uint32_t jc = njobs <= 1 ? 0u : njobs < 16 ? 1u : njobs < 256 ? 2u : 3u;
-        uint32_t lg = 0;
-        while (lg < 20 && (4ull << (2 * lg)) <= tris) lg++;
-        return (uint32_t)(precision & 1) | (jc << 1) | (lg << 3);
-    }
-    int pick(uint32_t k)
-    {
-        Entry& e = table[k];
-        if (e.choice >= 0) return e.choice;
-        for (int s = 0; s < gi::kTravShapes; s++)
-            if (e.tries[s] < kTries) return s;
-        int b = 0;
-        for (int s = 1; s < gi::kTravShapes; s++)
-            if (e.best[s] < e.best[b]) b = s;
-        e.choice = b;
-        return b;
-    }
-    void report(uint32_t k, int s, float ms)
-    {
-        Entry& e = table[k];
-        if (e.choice >= 0 || s < 0 || s >= gi::kTravShapes) return;
-        e.tries[s]++;
-        if (ms < e.best[s]) e.best[s] = ms;
-        float lead = 3.0e38f;
-        for (int q = 0; q < gi::kTravShapes; q++)
-            if (q != s && e.tries[q] > 0) lead = lead < e.best[q] ? lead : e.best[q];
-        if (e.tries[s] == 1 && ms > 1.3f * lead) e.tries[s] = kTries;  // clearly slower: one try is enough
-    }
-};
-
 struct gi_ctx {
     int device = 0;
     cudaStream_t st = nullptr;
@@ -339,11 +286,7 @@ struct gi_ctx {
     uint4* queue = nullptr;
     unsigned* qflag = nullptr;
     uint32_t cap_front = 0, cap_qflag = 0;
-    unsigned* cflag = nullptr;
-    uint32_t cap_cflag = 0;
     unsigned tag = 0;
-    uint4* cand = nullptr;
-    uint32_t cap_cand = 0;
     uint4* res = nullptr;
     uint32_t cap_res = 0;
     uint4* esc = nullptr;
@@ -362,8 +305,7 @@ struct gi_ctx {
     size_t order_scratch_bytes = 0;
     // pinned blocks the results are copied into
     std::shared_ptr<PinnedPool> pinned = std::make_shared<PinnedPool>();
-    TravTuner tuner;
-    int fixed_shape = -1;  // >= 0: traversal shape forced (tests), else tuned
+    int shape = gi::kDefaultShape;  // traversal shape (GI_FLAG_FIXED_SHAPE sets another)
     cudaEvent_t ev[8] = {};
 };
 

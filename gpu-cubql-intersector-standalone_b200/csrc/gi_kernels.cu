@@ -10,10 +10,10 @@
 //
 // Intersect (replaces crossCheck.cu, DualTreeStep.cu, rapidDescendKernel.cu and the
 // chunk loop of SingleTreeBatchIntersector.cu:170-455 in the reference):
-//   k_traverse  one persistent launch: seeding from the cut pairs, BVH4 x BVH4
-//               traversal through warp stacks and a device work queue (16 child
-//               pairs per node pair; no grid barrier), and the first filter
-//               stage on the leaf pairs, run by warps without node pairs.
+//   k_traverse_blocks  one persistent launch: seeding from the cut pairs, BVH4 x
+//               BVH4 traversal in the blocks' shared memory (16 child pairs per
+//               node pair), a pool through which loaded blocks hand node pairs to
+//               idle ones, and the first filter stage on the leaf pairs.
 //   k_exact     FP64 filter + exact integer signs for the escalated pairs.
 //   k_segments  intersection sets and correctly rounded endpoints.
 //   ordering    radix sort by (job, a, b) and gathers.
@@ -91,6 +91,22 @@ __device__ __forceinline__ void store_box(S* p, const S b[6])
     q[0] = V{b[0], b[1]};
     q[1] = V{b[2], b[3]};
     q[2] = V{b[4], b[5]};
+}
+
+// One child slot of a wide node, as whole 16-byte vectors.
+__device__ __forceinline__ void store_kid(WKid* kd, const float b[6], uint32_t ref)
+{
+    float4* q = reinterpret_cast<float4*>(kd);
+    q[0] = make_float4(b[0], b[1], b[2], __uint_as_float(ref));
+    q[1] = make_float4(b[3], b[4], b[5], 0.0f);
+}
+__device__ __forceinline__ void store_kid(WKid64* kd, const double b[6], uint32_t ref)
+{
+    double2* q = reinterpret_cast<double2*>(kd);
+    q[0] = make_double2(b[0], b[1]);
+    q[1] = make_double2(b[2], b[3]);
+    q[2] = make_double2(b[4], b[5]);
+    *reinterpret_cast<uint4*>(q + 3) = make_uint4(ref, 0u, 0u, 0u);
 }
 
 // FP32 boxes rounded outward (so every exact triangle lies inside its box) and
@@ -447,8 +463,8 @@ __global__ void k_collapse(int n, const uint4* __restrict__ child, const uint32_
         num[b + 1] = g.w;
         ns++;
     }
-    NodeT out;
     uint32_t kids = 0, leaves = 0;
+#pragma unroll
     for (int k = 0; k < 4; k++) {
         uint32_t r = k < ns ? slot[k] : kEmpty;
         if (r != kEmpty && !(r & kLeaf) && (!wide[r] || widx[r] >= nw)) {
@@ -456,51 +472,56 @@ __global__ void k_collapse(int n, const uint4* __restrict__ child, const uint32_
             r = kEmpty;
         }
         S bx[6] = {(S)INFINITY, (S)INFINITY, (S)INFINITY, (S)-INFINITY, (S)-INFINITY, (S)-INFINITY};
+        uint32_t ref = kEmpty;
         if (r == kEmpty) {
-            out.child[k] = kEmpty;
         } else if (r & kLeaf) {
             load_box_cg(leafBox + 6 * (size_t)(r & ~kLeaf), bx);
-            out.child[k] = r;
+            ref = r;
             kids++;
             leaves++;
         } else {
-            const uint32_t cw = widx[r];
-            out.child[k] = cw;
-            nodeUp[cw] = make_uint2(wi, (uint32_t)k);
+            ref = widx[r];
+            nodeUp[ref] = make_uint2(wi, (uint32_t)k);
             kids++;
         }
-        out.lox[k] = bx[0];
-        out.loy[k] = bx[1];
-        out.loz[k] = bx[2];
-        out.hix[k] = bx[3];
-        out.hiy[k] = bx[4];
-        out.hiz[k] = bx[5];
+        store_kid(&nodes[wi].kid[k], bx, ref);
     }
-    for (int k = 0; k < (int)(sizeof(out.pad) / sizeof(out.pad[0])); k++) out.pad[k] = 0;
     nkids[wi] = kids | (leaves << 8);
     arrive[wi] = leaves;
-    nodes[wi] = out;
 }
 
-// The six child-box fields of a wide node, read through L2 (other threads of
-// the same launch wrote them): the union of its slots (empty slots hold
-// +inf / -inf and change nothing).
+// The child boxes of a wide node, read through L2 (other threads of the same
+// launch wrote them): the union of its slots (empty slots hold +inf / -inf and
+// change nothing).
 __device__ __forceinline__ void node_union_cg(const WNode* nd, float b[6])
 {
     const float4* q = reinterpret_cast<const float4*>(nd);
+    float4 lo[4], hi[4];
 #pragma unroll
-    for (int f = 0; f < 6; f++) {
-        const float4 v = __ldcg(q + f);
-        b[f] = f < 3 ? fminf(fminf(v.x, v.y), fminf(v.z, v.w)) : fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w));
+    for (int k = 0; k < 4; k++) {
+        lo[k] = __ldcg(q + 2 * k);
+        hi[k] = __ldcg(q + 2 * k + 1);
     }
+    b[0] = fminf(fminf(lo[0].x, lo[1].x), fminf(lo[2].x, lo[3].x));
+    b[1] = fminf(fminf(lo[0].y, lo[1].y), fminf(lo[2].y, lo[3].y));
+    b[2] = fminf(fminf(lo[0].z, lo[1].z), fminf(lo[2].z, lo[3].z));
+    b[3] = fmaxf(fmaxf(hi[0].x, hi[1].x), fmaxf(hi[2].x, hi[3].x));
+    b[4] = fmaxf(fmaxf(hi[0].y, hi[1].y), fmaxf(hi[2].y, hi[3].y));
+    b[5] = fmaxf(fmaxf(hi[0].z, hi[1].z), fmaxf(hi[2].z, hi[3].z));
 }
 __device__ __forceinline__ void node_union_cg(const WNode64* nd, double b[6])
 {
-    const double2* q = reinterpret_cast<const double2*>(nd);
+    for (int f = 0; f < 6; f++) b[f] = f < 3 ? (double)INFINITY : (double)-INFINITY;
 #pragma unroll
-    for (int f = 0; f < 6; f++) {
-        const double2 v = __ldcg(q + 2 * f), w = __ldcg(q + 2 * f + 1);
-        b[f] = f < 3 ? fmin(fmin(v.x, v.y), fmin(w.x, w.y)) : fmax(fmax(v.x, v.y), fmax(w.x, w.y));
+    for (int k = 0; k < 4; k++) {
+        const double2* q = reinterpret_cast<const double2*>(&nd->kid[k]);
+        const double2 u = __ldcg(q), v = __ldcg(q + 1), w = __ldcg(q + 2);
+        b[0] = fmin(b[0], u.x);
+        b[1] = fmin(b[1], u.y);
+        b[2] = fmin(b[2], v.x);
+        b[3] = fmax(b[3], v.y);
+        b[4] = fmax(b[4], w.x);
+        b[5] = fmax(b[5], w.y);
     }
 }
 
@@ -524,6 +545,7 @@ __global__ void k_refit_wide(uint32_t nw, const uint2* __restrict__ nodeUp, cons
     S b[6];
     node_union_cg(nodes + w0, b);
     uint2 up = nodeUp[w0];
+    uint32_t self = w0;  // the slot holds this node
     for (uint32_t guard = 0; guard < nw; guard++) {
         if (up.x == kEmpty) return;  // the root is complete
         const uint32_t w = up.x, k = up.y & 3u;
@@ -532,18 +554,14 @@ __global__ void k_refit_wide(uint32_t nw, const uint2* __restrict__ nodeUp, cons
             return;
         }
         NodeT* nd = nodes + w;
-        nd->lox[k] = b[0];
-        nd->loy[k] = b[1];
-        nd->loz[k] = b[2];
-        nd->hix[k] = b[3];
-        nd->hiy[k] = b[4];
-        nd->hiz[k] = b[5];
+        store_kid(&nd->kid[k], b, self);
         const uint2 upn = nodeUp[w];
         const uint32_t need = nkids[w] & 0xffu;
         // release: this slot's stores before the arrival; acquire: the other slots' after it
         if (arrive_acq_rel(&arrive[w]) + 1u != need) return;
         node_union_cg(nd, b);
         up = upn;
+        self = w;
     }
 }
 
@@ -587,7 +605,7 @@ __global__ void __launch_bounds__(kCutThreads) k_cut(const NodeT* __restrict__ n
         if (tid < n) {
             if (!node) cnt = 1;
             else
-                for (int c = 0; c < 4; c++) cnt += nodes[ref].child[c] != kEmpty;
+                for (int c = 0; c < 4; c++) cnt += nodes[ref].kid[c].ref != kEmpty;
         }
         unsigned tot;
         const unsigned ex = block_exclusive_scan(cnt, sw, &tot);
@@ -600,14 +618,13 @@ __global__ void __launch_bounds__(kCutThreads) k_cut(const NodeT* __restrict__ n
                 const NodeT& nd = nodes[ref];
                 unsigned m = ex;
                 for (int c = 0; c < 4; c++) {
-                    if (nd.child[c] == kEmpty) continue;
-                    r[nx][m] = nd.child[c];
-                    b[nx][m][0] = nd.lox[c];
-                    b[nx][m][1] = nd.loy[c];
-                    b[nx][m][2] = nd.loz[c];
-                    b[nx][m][3] = nd.hix[c];
-                    b[nx][m][4] = nd.hiy[c];
-                    b[nx][m][5] = nd.hiz[c];
+                    const auto& kid = nd.kid[c];
+                    if (kid.ref == kEmpty) continue;
+                    r[nx][m] = kid.ref;
+                    for (int q = 0; q < 3; q++) {
+                        b[nx][m][q] = kid.lo[q];
+                        b[nx][m][3 + q] = kid.hi[q];
+                    }
                     m++;
                 }
             }
@@ -794,22 +811,24 @@ struct Box {
 //   centre' = Rf c + bf, half' = |Rf| h, padded by rho (|Rf|(|c| + h) + padm) + tau.
 // rho = 2^-19 (FP32) / 2^-48 (FP64) covers, with a margin of >= 3x, the rounding of
 // Rf and bf, of the box arithmetic, of c and h, and of the FP64 posed vertices.
-__device__ __forceinline__ void world_box(const DevPose& P, Box<float>& b)
+// The map's rows are read as 16-byte vectors (from the constant bank for a single
+// pair, four loads from a batch's job in memory).
+__device__ __forceinline__ void map_box(const BoxMap& P, Box<float>& b)
 {
-    float c[3], h[3];
+    float c[3], h[3], s[3];
+#pragma unroll
     for (int k = 0; k < 3; k++) {
         c[k] = 0.5f * b.lo[k] + 0.5f * b.hi[k];
         h[k] = 0.5f * b.hi[k] - 0.5f * b.lo[k];
+        s[k] = fabsf(c[k]) + h[k];
     }
+#pragma unroll
     for (int r = 0; r < 3; r++) {
-        float wc = P.bf[r], wh = 0.0f, mag = P.padm[r];
-        for (int k = 0; k < 3; k++) {
-            float a = P.Rf[3 * r + k];
-            wc = fmaf(a, c[k], wc);
-            wh = fmaf(fabsf(a), h[k], wh);
-            mag = fmaf(fabsf(a), fabsf(c[k]) + h[k], mag);
-        }
-        float pad = fmaf(0x1p-19f, mag, 0x1p-120f);
+        const float4 w = P.row[r];
+        const float wc = fmaf(w.z, c[2], fmaf(w.y, c[1], fmaf(w.x, c[0], w.w)));
+        const float wh = fmaf(fabsf(w.z), h[2], fmaf(fabsf(w.y), h[1], fabsf(w.x) * h[0]));
+        const float mag = fmaf(fabsf(w.z), s[2], fmaf(fabsf(w.y), s[1], fmaf(fabsf(w.x), s[0], P.padm[r])));
+        const float pad = fmaf(0x1p-19f, mag, 0x1p-120f);
         b.lo[r] = wc - wh - pad;
         b.hi[r] = wc + wh + pad;
     }
@@ -839,26 +858,6 @@ __device__ __forceinline__ void world_box(const DevPose& P, Box<double>& b)
 // local = Ri*w + bi, Ri = R^T).  Same construction and bound as world_box; the
 // pad also covers the error of R^T as the inverse (inv_eta <= 2^-30) and the
 // FP64 rounding of the posed vertices.
-__device__ __forceinline__ void local_box(const DevPose& P, Box<float>& b)
-{
-    float c[3], h[3];
-    for (int k = 0; k < 3; k++) {
-        c[k] = 0.5f * b.lo[k] + 0.5f * b.hi[k];
-        h[k] = 0.5f * b.hi[k] - 0.5f * b.lo[k];
-    }
-    for (int r = 0; r < 3; r++) {
-        float wc = P.bif[r], wh = 0.0f, mag = P.padmi[r];
-        for (int k = 0; k < 3; k++) {
-            float a = P.Rif[3 * r + k];
-            wc = fmaf(a, c[k], wc);
-            wh = fmaf(fabsf(a), h[k], wh);
-            mag = fmaf(fabsf(a), fabsf(c[k]) + h[k], mag);
-        }
-        float pad = fmaf(0x1p-19f, mag, 0x1p-120f);
-        b.lo[r] = wc - wh - pad;
-        b.hi[r] = wc + wh + pad;
-    }
-}
 __device__ __forceinline__ void local_box(const DevPose& P, Box<double>& b)
 {
     double c[3], h[3];
@@ -880,6 +879,10 @@ __device__ __forceinline__ void local_box(const DevPose& P, Box<double>& b)
         b.hi[r] = wc + wh + pad;
     }
 }
+__device__ __forceinline__ void world_box(const DevPose& P, Box<float>& b)
+{
+    map_box(P.fw, b);
+}
 
 template <bool F64>
 struct Prec;
@@ -897,113 +900,6 @@ struct Prec<true> {
     static __device__ __forceinline__ const Node* nodes(const MeshDev& M) { return M.nodes64; }
     static __device__ __forceinline__ const S* leafBox(const MeshDev& M) { return M.leafBox64; }
 };
-
-// Children of a node reference in the mesh-local frame, structure of arrays
-// (slot i of every array is child i).  A wide node gives up to four (one
-// 128-byte line loaded as seven 16-byte vectors, or two lines for FP64); a
-// leaf reference stands for itself in slot 0.  Every array is indexed by
-// constants only, so the whole set lives in registers.
-template <class S>
-struct Kids {
-    S lx[4], ly[4], lz[4], hx[4], hy[4], hz[4];
-    uint32_t c[4];
-};
-
-__device__ __forceinline__ void put4(float (&d)[4], const float4& v)
-{
-    d[0] = v.x;
-    d[1] = v.y;
-    d[2] = v.z;
-    d[3] = v.w;
-}
-__device__ __forceinline__ void put4(double (&d)[4], const double2& a, const double2& b)
-{
-    d[0] = a.x;
-    d[1] = a.y;
-    d[2] = b.x;
-    d[3] = b.y;
-}
-
-__device__ __forceinline__ void load_kids(const MeshDev& M, uint32_t ref, Kids<float>& k)
-{
-    if (ref & kLeaf) {
-        const float2* lb = reinterpret_cast<const float2*>(M.leafBox + 6 * (size_t)(ref & ~kLeaf));
-        const float2 a = __ldg(lb), b = __ldg(lb + 1), c = __ldg(lb + 2);
-        put4(k.lx, make_float4(a.x, 0.f, 0.f, 0.f));
-        put4(k.ly, make_float4(a.y, 0.f, 0.f, 0.f));
-        put4(k.lz, make_float4(b.x, 0.f, 0.f, 0.f));
-        put4(k.hx, make_float4(b.y, 0.f, 0.f, 0.f));
-        put4(k.hy, make_float4(c.x, 0.f, 0.f, 0.f));
-        put4(k.hz, make_float4(c.y, 0.f, 0.f, 0.f));
-        k.c[0] = ref;
-        k.c[1] = k.c[2] = k.c[3] = kEmpty;
-        return;
-    }
-    const float4* p = reinterpret_cast<const float4*>(M.nodes + ref);
-    put4(k.lx, __ldg(p));
-    put4(k.ly, __ldg(p + 1));
-    put4(k.lz, __ldg(p + 2));
-    put4(k.hx, __ldg(p + 3));
-    put4(k.hy, __ldg(p + 4));
-    put4(k.hz, __ldg(p + 5));
-    const uint4 ch = __ldg(reinterpret_cast<const uint4*>(p + 6));
-    k.c[0] = ch.x;
-    k.c[1] = ch.y;
-    k.c[2] = ch.z;
-    k.c[3] = ch.w;
-}
-__device__ __forceinline__ void load_kids(const MeshDev& M, uint32_t ref, Kids<double>& k)
-{
-    if (ref & kLeaf) {
-        const double2* lb = reinterpret_cast<const double2*>(M.leafBox64 + 6 * (size_t)(ref & ~kLeaf));
-        const double2 a = __ldg(lb), b = __ldg(lb + 1), c = __ldg(lb + 2);
-        const double2 z = make_double2(0.0, 0.0);
-        put4(k.lx, make_double2(a.x, 0.0), z);
-        put4(k.ly, make_double2(a.y, 0.0), z);
-        put4(k.lz, make_double2(b.x, 0.0), z);
-        put4(k.hx, make_double2(b.y, 0.0), z);
-        put4(k.hy, make_double2(c.x, 0.0), z);
-        put4(k.hz, make_double2(c.y, 0.0), z);
-        k.c[0] = ref;
-        k.c[1] = k.c[2] = k.c[3] = kEmpty;
-        return;
-    }
-    const double2* p = reinterpret_cast<const double2*>(M.nodes64 + ref);
-    put4(k.lx, __ldg(p), __ldg(p + 1));
-    put4(k.ly, __ldg(p + 2), __ldg(p + 3));
-    put4(k.lz, __ldg(p + 4), __ldg(p + 5));
-    put4(k.hx, __ldg(p + 6), __ldg(p + 7));
-    put4(k.hy, __ldg(p + 8), __ldg(p + 9));
-    put4(k.hz, __ldg(p + 10), __ldg(p + 11));
-    const uint4 ch = __ldg(reinterpret_cast<const uint4*>(p + 12));
-    k.c[0] = ch.x;
-    k.c[1] = ch.y;
-    k.c[2] = ch.z;
-    k.c[3] = ch.w;
-}
-
-// Maps the four child boxes to the world frame (same bound as world_box).
-template <class S>
-__device__ __forceinline__ void world_kids(const DevPose& P, Kids<S>& k)
-{
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        Box<S> b;
-        b.lo[0] = k.lx[i];
-        b.lo[1] = k.ly[i];
-        b.lo[2] = k.lz[i];
-        b.hi[0] = k.hx[i];
-        b.hi[1] = k.hy[i];
-        b.hi[2] = k.hz[i];
-        world_box(P, b);
-        k.lx[i] = b.lo[0];
-        k.ly[i] = b.lo[1];
-        k.lz[i] = b.lo[2];
-        k.hx[i] = b.hi[0];
-        k.hy[i] = b.hi[1];
-        k.hz[i] = b.hi[2];
-    }
-}
 
 template <class S>
 __device__ __forceinline__ bool overlap(const Box<S>& a, const Box<S>& b)
@@ -1040,250 +936,55 @@ __device__ __forceinline__ void load_tri(const MeshDev& M, const DevPose& P, uin
     *tri_id = t.w;
 }
 
-// Maps the four child boxes (world frame) into the local frame of pose P.
-template <class S>
-__device__ __forceinline__ void local_kids(const DevPose& P, Kids<S>& k)
+// The job of an entry: one job travels in the kernel's parameters (constant
+// bank), a batch's in memory.
+template <bool MULTI>
+__device__ __forceinline__ const JobDev& job_at(const Bufs& B, uint32_t j)
 {
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        Box<S> b;
-        b.lo[0] = k.lx[i];
-        b.lo[1] = k.ly[i];
-        b.lo[2] = k.lz[i];
-        b.hi[0] = k.hx[i];
-        b.hi[1] = k.hy[i];
-        b.hi[2] = k.hz[i];
-        local_box(P, b);
-        k.lx[i] = b.lo[0];
-        k.ly[i] = b.lo[1];
-        k.lz[i] = b.lo[2];
-        k.hx[i] = b.hi[0];
-        k.hy[i] = b.hi[1];
-        k.hz[i] = b.hi[2];
-    }
+    if constexpr (MULTI) return B.jobs[j];
+    else return B.job0;
 }
 
-// 16-bit mask of the overlapping child pairs (bit 4i+j: a's child i, b's child j).
-template <class S>
-__device__ __forceinline__ unsigned overlap_mask(const Kids<S>& a, const Kids<S>& b)
-{
-    unsigned m = 0;
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const bool ov = (a.lx[i] <= b.hx[j]) & (b.lx[j] <= a.hx[i]) & (a.ly[i] <= b.hy[j]) &
-                            (b.ly[j] <= a.hy[i]) & (a.lz[i] <= b.hz[j]) & (b.lz[j] <= a.hz[i]);
-            m |= (ov ? 1u : 0u) << (4 * i + j);
-        }
-    return m;
-}
-
-// Bit i of `x` (i < 4) spread over nibble i: the child pairs (i, *).
-__device__ __forceinline__ unsigned rows4(unsigned x)
-{
-    return ((x & 1u) ? 0x000Fu : 0u) | ((x & 2u) ? 0x00F0u : 0u) | ((x & 4u) ? 0x0F00u : 0u) |
-           ((x & 8u) ? 0xF000u : 0u);
-}
-
-
-// One node pair: load both nodes, map the child boxes to the world frame and
-// test the 4 x 4 child pairs without branches.  fm / cm: bit 4i+j set when
-// child pair (i, j) overlaps and leads to a node pair / a leaf pair.
-template <bool F64>
-__device__ __forceinline__ void expand_pair(const Bufs& B, const uint4& ent, unsigned& fm, unsigned& cm,
-                                            uint32_t (&ca)[4], uint32_t (&cb)[4])
-{
-    using S = typename Prec<F64>::S;
-    const JobDev& J = B.jobs[ent.x];
-    Kids<S> a, b;
-    load_kids(J.A, ent.y, a);
-    load_kids(J.B, ent.z, b);
-    if (!J.pa.identity) world_kids(J.pa, a);
-    // a posed B can also be tested in its own frame (A's world boxes mapped
-    // back through B's pose against B's stored boxes): the world box of a
-    // rotated box is wider than the box, and each test alone is conservative.
-    // It removes about a quarter of the pairs for about a third more work per
-    // pair, which pays where the traversal is bound by work (batches), not by
-    // the latency of its levels (one pair).
-    unsigned m = 0xFFFFu;
-    if (B.two_frame && J.pb.inv_ok) {
-        Kids<S> al = a;
-        local_kids(J.pb, al);
-        m = overlap_mask(al, b);
-    }
-    if (!J.pb.identity) world_kids(J.pb, b);
-    m &= overlap_mask(a, b);
-    unsigned va = 0, vb = 0, la = 0, lb = 0;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        ca[i] = a.c[i];
-        cb[i] = b.c[i];
-        va |= (a.c[i] != kEmpty ? 1u : 0u) << i;
-        vb |= (b.c[i] != kEmpty ? 1u : 0u) << i;
-        la |= ((a.c[i] & kLeaf) && a.c[i] != kEmpty ? 1u : 0u) << i;
-        lb |= ((b.c[i] & kLeaf) && b.c[i] != kEmpty ? 1u : 0u) << i;
-    }
-    m &= rows4(va) & (vb * 0x1111u);
-    const unsigned leafpair = rows4(la) & (lb * 0x1111u);
-    cm = m & leafpair;
-    fm = m & ~leafpair;
-}
-
-// ---------------------------------------------------------------------------
-// Quad-cooperative expansion: the four lanes of a quad share one node pair and
-// lane k (= lane & 3) owns child k of both nodes.  Each lane loads one child
-// slot of each node (the four lanes of a quad read one 16-byte segment per
-// field of the structure-of-arrays node), maps its own boxes to the world
-// frame, receives B's four child boxes from its quad by width-4 shuffles and
-// tests its A child against them: four tests instead of sixteen, one box
-// transform instead of four, so the dependent chain of one expansion is a
-// fraction of the one-lane form's.
-// ---------------------------------------------------------------------------
+// Child k of a node reference: a wide node's slot, or the leaf itself (k = 0; the
+// other three are empty).  The four lanes of a quad read one node's line.
 __device__ __forceinline__ void load_kid(const MeshDev& M, uint32_t ref, unsigned k, Box<float>& b, uint32_t& c)
 {
     if (ref & kLeaf) {
+        c = kEmpty;
         if (k == 0u) {
-            const float* lb = M.leafBox + 6 * (size_t)(ref & ~kLeaf);
-            for (int q = 0; q < 3; q++) {
-                b.lo[q] = __ldg(lb + q);
-                b.hi[q] = __ldg(lb + 3 + q);
-            }
+            const float2* lb = reinterpret_cast<const float2*>(M.leafBox + 6 * (size_t)(ref & ~kLeaf));
+            const float2 u = __ldg(lb), v = __ldg(lb + 1), w = __ldg(lb + 2);
+            b.lo[0] = u.x, b.lo[1] = u.y, b.lo[2] = v.x;
+            b.hi[0] = v.y, b.hi[1] = w.x, b.hi[2] = w.y;
             c = ref;
-        } else {
-            for (int q = 0; q < 3; q++) b.lo[q] = b.hi[q] = 0.0f;
-            c = kEmpty;
         }
         return;
     }
-    const float* p = reinterpret_cast<const float*>(M.nodes + ref);
-    for (int q = 0; q < 3; q++) {
-        b.lo[q] = __ldg(p + 4 * q + k);
-        b.hi[q] = __ldg(p + 12 + 4 * q + k);
-    }
-    c = __ldg(reinterpret_cast<const uint32_t*>(p + 24) + k);
+    const float4* p = reinterpret_cast<const float4*>(&M.nodes[ref].kid[k]);
+    const float4 u = __ldg(p), v = __ldg(p + 1);
+    b.lo[0] = u.x, b.lo[1] = u.y, b.lo[2] = u.z;
+    b.hi[0] = v.x, b.hi[1] = v.y, b.hi[2] = v.z;
+    c = __float_as_uint(u.w);
 }
 __device__ __forceinline__ void load_kid(const MeshDev& M, uint32_t ref, unsigned k, Box<double>& b, uint32_t& c)
 {
+    const double2* p;
+    c = kEmpty;
     if (ref & kLeaf) {
-        if (k == 0u) {
-            const double* lb = M.leafBox64 + 6 * (size_t)(ref & ~kLeaf);
-            for (int q = 0; q < 3; q++) {
-                b.lo[q] = __ldg(lb + q);
-                b.hi[q] = __ldg(lb + 3 + q);
-            }
-            c = ref;
-        } else {
-            for (int q = 0; q < 3; q++) b.lo[q] = b.hi[q] = 0.0;
-            c = kEmpty;
-        }
-        return;
+        if (k != 0u) return;
+        p = reinterpret_cast<const double2*>(M.leafBox64 + 6 * (size_t)(ref & ~kLeaf));
+        c = ref;
+    } else {
+        p = reinterpret_cast<const double2*>(&M.nodes64[ref].kid[k]);
+        c = __ldg(reinterpret_cast<const uint32_t*>(p + 3));
     }
-    const double* p = reinterpret_cast<const double*>(M.nodes64 + ref);
-    for (int q = 0; q < 3; q++) {
-        b.lo[q] = __ldg(p + 4 * q + k);
-        b.hi[q] = __ldg(p + 12 + 4 * q + k);
-    }
-    c = __ldg(reinterpret_cast<const uint32_t*>(p + 24) + k);
+    const double2 u = __ldg(p), v = __ldg(p + 1), w = __ldg(p + 2);
+    b.lo[0] = u.x, b.lo[1] = u.y, b.lo[2] = v.x;
+    b.hi[0] = v.y, b.hi[1] = w.x, b.hi[2] = w.y;
 }
 
-template <class S>
-__device__ __forceinline__ void shfl_box(const Box<S>& src, Box<S>& dst, unsigned j)
-{
-#pragma unroll
-    for (int q = 0; q < 3; q++) {
-        dst.lo[q] = __shfl_sync(0xffffffffu, src.lo[q], (int)j, 4);
-        dst.hi[q] = __shfl_sync(0xffffffffu, src.hi[q], (int)j, 4);
-    }
-}
-
-// Called by all 32 lanes (the shuffles need them); lanes of a quad without a
-// node pair pass have = false and get no children.  fm / cm: bit j set when
-// (own A child, B child j) overlap and lead to a node pair / a leaf pair;
-// cb[j] receives B's child refs.
-template <bool F64>
-__device__ __forceinline__ void expand_quad(const Bufs& B, const uint4& ent, bool have, unsigned sub, unsigned& fm,
-                                            unsigned& cm, uint32_t& ca, uint32_t (&cb)[4])
-{
-    using S = typename Prec<F64>::S;
-    const JobDev& J = B.jobs[have ? ent.x : 0u];
-    Box<S> a, b;
-    uint32_t mb = kEmpty;
-    ca = kEmpty;
-    for (int q = 0; q < 3; q++) a.lo[q] = a.hi[q] = b.lo[q] = b.hi[q] = S(0);
-    if (have) {
-        load_kid(J.A, ent.y, sub, a, ca);
-        load_kid(J.B, ent.z, sub, b, mb);
-        if (ca != kEmpty && !J.pa.identity) world_box(J.pa, a);
-    }
-    // optional second test in B's own frame (see expand_pair)
-    unsigned m2 = 0xFu;
-    if (B.two_frame) {  // uniform over the launch
-        const bool twof = have && J.pb.inv_ok;
-        Box<S> al = a;
-        if (twof && ca != kEmpty) local_box(J.pb, al);
-        m2 = 0u;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            Box<S> bl;
-            shfl_box(b, bl, (unsigned)j);
-            if (!twof || overlap(al, bl)) m2 |= 1u << j;
-        }
-    }
-    if (have && mb != kEmpty && !J.pb.identity) world_box(J.pb, b);
-    fm = cm = 0u;
-    const bool leafa = (ca & kLeaf) && ca != kEmpty;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-        Box<S> bj;
-        shfl_box(b, bj, (unsigned)j);
-        cb[j] = __shfl_sync(0xffffffffu, mb, j, 4);
-        const bool ov = ca != kEmpty && cb[j] != kEmpty && ((m2 >> j) & 1u) && overlap(a, bj);
-        const bool leafb = (cb[j] & kLeaf) != 0u;
-        if (ov) {
-            if (leafa && leafb) cm |= 1u << j;
-            else fm |= 1u << j;
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Persistent BVH4 x BVH4 traversal: a small warp stack in front of a device
-// work queue (no grid barrier).
-//
-// Each warp expands up to 32 node pairs per iteration (one per lane).  It
-// keeps up to 32 of their children on its own shared-memory stack for its next
-// iteration, with no global round trip, and publishes the rest to the global
-// queue; leaf pairs (candidates) always go to the global candidate list, so
-// the first filter stage runs on warps that have no node pair at hand.  The
-// launch first seeds the queue: every overlapping pair of the two meshes'
-// cut entries (depth 4 for a single pair, depth 3 for a batch) becomes a node
-// pair (a leaf pair, a candidate).
-//
-// Slot protocol (queue and candidate list): producers reserve slots with one
-// atomic per warp, write the entries and, after a release fence, store the
-// call's tag in each slot's flag word.  A warp takes a ticket of 32
-// consecutive slots (one atomicAdd on the head counter), polls their 32 tag
-// words with acquire loads (one 128-byte line, so polling has no hot spot;
-// a ready tag orders the entry's load after it) and keeps the ticket
-// until all 32 slots are processed.  Only warps with empty stacks take node
-// tickets, and ready queue slots come before stack entries, so queued work
-// never waits behind a warp that is busy with its own.
-//
-// Termination: the low half of `work_cand` is the number of node pairs that
-// exist, its high half the candidate slots reserved.  Seeds add to both
-// before the seed count completes; an expansion adds (children - expanded
-// pairs) and its candidates in one atomic, before any child is published, so
-// the node-pair count never passes through zero while a node pair exists, and
-// the load that reads it at zero reads the final candidate count.  Reading
-// seed_done == all seed tests and then a zero node-pair count proves the
-// traversal is over.  Every wait is bounded; overflow or a spent wait raises the abort
-// flag.
-// ---------------------------------------------------------------------------
+constexpr unsigned kBlkThreads = 256, kBlkWarps = kBlkThreads / 32;
 constexpr unsigned kIdleSpins = 1u << 22;     // consecutive idle polls of one warp (~1 s)
-constexpr unsigned kWarpStack = 32;           // stack capacity of a warp (both expansion forms)
-constexpr int kTravThreads = 256;
-constexpr int kTravWarps = kTravThreads / 32;
 
 __device__ __forceinline__ unsigned ld_vol(const unsigned* p)
 {
@@ -1315,141 +1016,6 @@ __device__ __forceinline__ void wait_prior_grid()
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-__device__ __forceinline__ void fence_acq_rel()
-{
-    asm volatile("fence.acq_rel.gpu;" ::: "memory");
-}
-
-__device__ __forceinline__ unsigned take_ticket(unsigned* head)
-{
-    unsigned b = 0;
-    if ((threadIdx.x & 31) == 0) b = atomicAdd(head, 32u);
-    return __shfl_sync(0xffffffffu, b, 0);
-}
-
-// Seed tests per job: every pair of the two meshes' cut entries.
-__device__ __forceinline__ unsigned seed_tests_per_job(const Bufs& B)
-{
-    return B.deep_seed ? (unsigned)kCut4Max * kCut4Max : (unsigned)kCutMax * kCutMax;
-}
-
-// Seeds the queue: pair (i, j) of the depth-3 (or depth-4) cut entries of every job.  Warps
-// claim chunks of 32 seed tests with one atomic, so only warps that run do the
-// work (nothing waits for a block that never becomes resident); seed_done
-// counts finished tests after their node pairs are counted in `work`.
-template <bool F64>
-__device__ __forceinline__ void seed_cut_pairs(const Bufs& B, unsigned total)
-{
-    using S = typename Prec<F64>::S;
-    Counters* C = B.cnt;
-    const unsigned lane = threadIdx.x & 31;
-    const unsigned per_job = seed_tests_per_job(B);
-    const unsigned coff = B.deep_seed ? (unsigned)kCutMax : 0u;  // the cut's first entry
-    for (;;) {
-        unsigned base = 0;
-        if (lane == 0) base = atomicAdd(&C->seed_head, 32u);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= total) break;
-        const unsigned g = base + lane;
-        bool front = false, cand = false;
-        uint32_t ra = 0, rb = 0, job = 0;
-        if (g < total) {
-            job = g / per_job;
-            const unsigned t = g % per_job;
-            const JobDev& J = B.jobs[job];
-            const bool both = J.A.nt && J.B.nt;  // an empty mesh has no cut (null sizes)
-            const unsigned nA = both ? __ldg(J.A.ncuts + (B.deep_seed ? 1 : 0)) : 0u;
-            const unsigned nB = both ? __ldg(J.B.ncuts + (B.deep_seed ? 1 : 0)) : 0u;
-            if (t < nA * nB) {
-                const unsigned i = coff + t / nB, j = coff + t % nB;
-                const S* ba_ = F64 ? (const S*)J.A.cutBox64 : (const S*)J.A.cutBox;
-                const S* bb_ = F64 ? (const S*)J.B.cutBox64 : (const S*)J.B.cutBox;
-                Box<S> ba, bb;
-                for (int k = 0; k < 3; k++) {
-                    ba.lo[k] = ba_[6 * i + k];
-                    ba.hi[k] = ba_[6 * i + 3 + k];
-                    bb.lo[k] = bb_[6 * j + k];
-                    bb.hi[k] = bb_[6 * j + 3 + k];
-                }
-                if (!J.pa.identity) world_box(J.pa, ba);
-                if (!J.pb.identity) world_box(J.pb, bb);
-                if (overlap(ba, bb)) {
-                    ra = J.A.cutRef[i];
-                    rb = J.B.cutRef[j];
-                    cand = (ra & kLeaf) && (rb & kLeaf);
-                    front = !cand;
-                }
-            }
-        }
-        const unsigned nfront = __popc(__ballot_sync(0xffffffffu, front));
-        unsigned pf = warp_append(front, &C->q_tail);
-        if (front) {
-            if (pf < B.cap_queue) B.queue[pf] = make_uint4(job, ra, rb, 0u);
-            else {
-                atomicOr(&C->overflow, kOvfFrontier);
-                atomicExch(&C->abort_, 1u);
-            }
-        }
-        // candidate slots and node pairs counted in one atomic, before any seed is published
-        const unsigned cm = __ballot_sync(0xffffffffu, cand);
-        unsigned long long old = 0;
-        if (lane == 0 && (cm || nfront))
-            old = atomicAdd(&C->work_cand, ((unsigned long long)__popc(cm) << 32) + nfront);
-        const unsigned pc = (unsigned)(__shfl_sync(0xffffffffu, old, 0) >> 32) + __popc(cm & ((1u << lane) - 1u));
-        if (cand) {
-            if (pc < B.cap_cand) B.cand[pc] = make_uint4(job, ra & ~kLeaf, rb & ~kLeaf, 0u);
-            else {
-                atomicOr(&C->overflow, kOvfCand);
-                atomicExch(&C->abort_, 1u);
-            }
-        }
-        __syncwarp();
-        fence_acq_rel();
-        if (front && pf < B.cap_queue) *(volatile unsigned*)(B.qflag + pf) = B.tag;
-        if (cand && pc < B.cap_cand) *(volatile unsigned*)(B.cflag + pc) = B.tag;
-        __syncwarp();
-        if (lane == 0) {
-            fence_acq_rel();
-            atomicAdd(&C->seed_done, min(32u, total - base));
-        }
-    }
-}
-
-// First filter stage on one candidate per lane (have = lane holds one):
-// intersecting pairs go to the result list, undecided ones to the escalation
-// list (one atomic per list per warp).
-template <bool F64>
-__device__ __forceinline__ void filter_candidates(const Bufs& B, bool have, const uint4& c,
-                                                  unsigned long long& decided, unsigned long long& tested)
-{
-    Counters* C = B.cnt;
-    int dec = DEC_NO;
-    uint32_t ta = 0, tb = 0;
-    unsigned pat = 0;
-    if (have) {
-        tested++;
-        const JobDev& J = B.jobs[c.x];
-        double3 P[3], Q[3];
-        load_tri<F64>(J.A, J.pa, c.y, P, &ta);
-        load_tri<F64>(J.B, J.pb, c.z, Q, &tb);
-        if constexpr (F64) dec = classify_fast<double>(P, Q, &pat);
-        else dec = classify_fast<float>(P, Q, &pat);
-        decided += (dec != DEC_ESC);
-    }
-    const bool yes = have && dec == DEC_YES;
-    const bool esc = have && dec == DEC_ESC;
-    const unsigned pr = warp_append(yes, &C->res);
-    if (yes) {
-        if (pr < B.cap_res) B.res[pr] = make_uint4(c.x, ta, tb, pat);
-        else atomicOr(&C->overflow, kOvfRes);
-    }
-    const unsigned pe = warp_append(esc, &C->esc);
-    if (esc) {
-        if (pe < B.cap_esc) B.esc[pe] = make_uint4(c.x, c.y, c.z, 0u);
-        else atomicOr(&C->overflow, kOvfEsc);
-    }
-}
-
 // A traversal block's counts at its end: summed over its warps in shared
 // memory, then one atomic per counter for the block (every warp's own atomics
 // on the same three words queued up at the end of the launch).  Every thread
@@ -1457,7 +1023,7 @@ __device__ __forceinline__ void filter_candidates(const Bufs& B, bool have, cons
 __device__ __forceinline__ void block_stats(Counters* C, unsigned long long visited, unsigned long long decided,
                                             unsigned long long tested, unsigned levels = 0u)
 {
-    __shared__ unsigned long long s_stats[4][kTravWarps];
+    __shared__ unsigned long long s_stats[4][kBlkWarps];
     for (int o = 16; o > 0; o >>= 1) {
         visited += __shfl_xor_sync(0xffffffffu, visited, o);
         decided += __shfl_xor_sync(0xffffffffu, decided, o);
@@ -1474,8 +1040,7 @@ __device__ __forceinline__ void block_stats(Counters* C, unsigned long long visi
     __syncthreads();
     if (threadIdx.x < 4u) {
         unsigned long long t = 0;
-#pragma unroll
-        for (int w = 0; w < kTravWarps; w++)
+        for (unsigned w = 0; w < kBlkWarps; w++)
             t = threadIdx.x == 3u ? max(t, s_stats[3][w]) : t + s_stats[threadIdx.x][w];
         if (threadIdx.x == 3u) {
             if (t) atomicMax(&C->levels, (unsigned)t);
@@ -1485,253 +1050,44 @@ __device__ __forceinline__ void block_stats(Counters* C, unsigned long long visi
     }
 }
 
-// QUAD selects the expansion form: one node pair per lane (32 per warp
-// iteration, the form for work-bound launches) or one per quad (8 per
-// iteration with a quarter of the dependent chain, the form for launches bound
-// by the latency of the traversal's levels).  The host picks it per workload.
-template <bool F64, bool QUAD>
-__global__ void __launch_bounds__(kTravThreads, 2) k_traverse(Bufs B)
-{
-    constexpr unsigned kSlots = QUAD ? 8u : 32u;  // node-queue slots per ticket: one per work unit
-    constexpr unsigned kStack = QUAD ? 8u : 32u;  // node pairs kept for the next iteration
-    __shared__ uint4 stk[kTravWarps][kWarpStack];
-    allow_dependent_launch();
-    Counters* C = B.cnt;
-    const unsigned lane = threadIdx.x & 31;
-    uint4* S = stk[threadIdx.x >> 5];
-    const unsigned seed_total = B.njobs * seed_tests_per_job(B);
-    seed_cut_pairs<F64>(B, seed_total);
-    unsigned long long visited = 0, decided = 0, tested = 0;
-    unsigned maxlev = 0, idle = 0, backoff = 32;
-    unsigned sn = 0;         // node pairs on this warp's stack (warp-uniform, <= kWarpStack)
-    bool ticket = false;     // holds a node-queue ticket
-    unsigned nbase = 0, npend = 0;
-    unsigned cbase = take_ticket(&C->c_head);
-    unsigned cpend = 0xffffffffu;  // lanes whose candidate slot is still to be processed
-    unsigned iter = 0;
-    for (;;) {
-        ++iter;
-        if (!ticket && sn == 0u) {
-            unsigned b0 = 0;
-            if (lane == 0) b0 = atomicAdd(&C->q_head, kSlots);
-            nbase = __shfl_sync(0xffffffffu, b0, 0);
-            npend = kSlots == 32u ? 0xffffffffu : (1u << kSlots) - 1u;
-            ticket = true;
-        }
-        const unsigned unit = QUAD ? (lane >> 2) : lane;  // work unit: a quad or a lane
-        const unsigned sub = QUAD ? (lane & 3u) : 0u;
-        const unsigned ubit = QUAD ? 4u * unit : unit;     // the unit's first lane
-        const unsigned ns = nbase + unit;  // one queue slot per unit
-        const unsigned i = cbase + lane;   // one candidate slot per lane
-        const bool nslot = ticket && ((npend >> unit) & 1u) && ns < B.cap_queue;
-        const bool cslot = ((cpend >> lane) & 1u) && i < B.cap_cand;
-        // everything this pass polls, issued together.  The abort flag is one
-        // line that every warp reads, so it is read every 8th pass only; its
-        // round trip overlaps the node loads of a warp that works from its stack.
-        unsigned ab = 0;
-        if (lane == 0 && (iter & 7u) == 0u) ab = ld_vol(&C->abort_);
-        const unsigned ntag = nslot ? ld_acq(B.qflag + ns) : 0u;
-        const unsigned ctag = cslot ? ld_acq(B.cflag + i) : 0u;
-        const bool from_queue = nslot && ntag == B.tag;  // the same in every lane of a unit
-        const unsigned qball = __ballot_sync(0xffffffffu, from_queue && sub == 0u);  // a unit's first lane: ready
-        if (sn != 0u || qball != 0u) {
-            idle = 0;
-            backoff = 32;
-            // ready queue slots first (queued work is what idle warps wait
-            // for), the other units pop the stack
-            const unsigned take = min(sn, kSlots - (unsigned)__popc(qball));
-            const unsigned rank = unit - (unsigned)__popc(qball & ((1u << ubit) - 1u));
-            const bool from_stack = !from_queue && rank < take;
-            uint4 ent = make_uint4(0u, kEmpty, kEmpty, 0u);
-            if (from_stack) {
-                ent = S[sn - 1u - rank];
-            } else if (from_queue) {
-                ent = __ldcg(B.queue + ns);  // ordered after the tag's acquire load
-            }
-            sn -= take;
-            __syncwarp();  // popped entries are read before the pushes below reuse their slots
-            const bool have = from_stack || from_queue;
-            if (have && sub == 0u) {
-                visited++;
-                maxlev = max(maxlev, ent.w);
-            }
-            unsigned fm = 0, cm = 0;
-            uint32_t ca[4], cb[4];
-            if constexpr (QUAD) {
-                expand_quad<F64>(B, ent, have, sub, fm, cm, ca[0], cb);
-            } else {
-                if (have) expand_pair<F64>(B, ent, fm, cm, ca, cb);
-            }
-            // children: node pairs onto the stack (up to keep), the rest to the
-            // queue; candidates to the global candidate list
-            const unsigned nf = __popc(fm), nc = __popc(cm);
-            unsigned incf = nf, incc = nc;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned yf = __shfl_up_sync(0xffffffffu, incf, o);
-                const unsigned yc = __shfl_up_sync(0xffffffffu, incc, o);
-                if (lane >= (unsigned)o) {
-                    incf += yf;
-                    incc += yc;
-                }
-            }
-            const unsigned kf = __shfl_sync(0xffffffffu, incf, 31);
-            const unsigned kc = __shfl_sync(0xffffffffu, incc, 31);
-            const unsigned done = __popc(__ballot_sync(0xffffffffu, have && sub == 0u));
-            const unsigned keep = min(kf, kStack - sn);
-            unsigned qb = 0, cg = 0;
-            if (lane == 31) {
-                if (kf > keep) qb = atomicAdd(&C->q_tail, kf - keep);
-                // candidate slots and node pairs made minus expanded in one
-                // atomic, before any child is published: the node-pair count
-                // reaches zero in the same update that reserves the last
-                // expansion's candidate slots
-                if (kc || kf != done) {
-                    const unsigned long long old = atomicAdd(
-                        &C->work_cand, ((unsigned long long)kc << 32) + (unsigned long long)(long long)(int)(kf - done));
-                    cg = (unsigned)(old >> 32);
-                }
-            }
-            qb = __shfl_sync(0xffffffffu, qb, 31);
-            cg = __shfl_sync(0xffffffffu, cg, 31);
-            const unsigned f0 = incf - nf;  // this lane's first node child in the warp's order
-            const unsigned c0 = cg + incc - nc;  // this lane's first candidate slot
-            {
-                // child slot q: the pair (A child q / 4, B child q % 4) in the lane
-                // form, (own A child, B child q) in the quad form; the unrolled
-                // loop indexes the registers with constants and has no
-                // data-dependent trip count
-                constexpr int kQ = QUAD ? 4 : 16;
-                unsigned g = f0, h = c0;
-#pragma unroll
-                for (int q = 0; q < kQ; q++) {
-                    const uint32_t ra = QUAD ? ca[0] : ca[q >> 2], rb = QUAD ? cb[q] : cb[q & 3];
-                    if ((fm >> q) & 1u) {
-                        const uint4 e = make_uint4(ent.x, ra, rb, ent.w + 1u);
-                        if (g < keep) {
-                            S[sn + g] = e;
-                        } else {
-                            const unsigned sl = qb + (g - keep);
-                            if (sl < B.cap_queue) B.queue[sl] = e;
-                        }
-                        g++;
-                    }
-                    if ((cm >> q) & 1u) {
-                        if (h < B.cap_cand) B.cand[h] = make_uint4(ent.x, ra & ~kLeaf, rb & ~kLeaf, 0u);
-                        h++;
-                    }
-                }
-            }
-            __syncwarp();  // the work count above precedes every tag store below
-            const unsigned qx0 = max(f0, keep), qx1 = f0 + nf;
-            if (qx0 < qx1 || nc != 0u) {
-                fence_acq_rel();
-                for (unsigned x = qx0; x < qx1; x++) {
-                    const unsigned sl = qb + (x - keep);
-                    if (sl < B.cap_queue) {
-                        *(volatile unsigned*)(B.qflag + sl) = B.tag;
-                    } else {
-                        atomicOr(&C->overflow, kOvfFrontier);
-                        atomicExch(&C->abort_, 1u);
-                    }
-                }
-                for (unsigned x = c0; x < c0 + nc; x++) {
-                    if (x < B.cap_cand) {
-                        *(volatile unsigned*)(B.cflag + x) = B.tag;
-                    } else {
-                        atomicOr(&C->overflow, kOvfCand);
-                        atomicExch(&C->abort_, 1u);
-                    }
-                }
-            }
-            __syncwarp();  // stack pushes visible to the whole warp
-            sn += keep;
-            if (ticket) {
-                unsigned qm = qball;
-                if constexpr (QUAD) {
-                    qm = 0;
-#pragma unroll
-                    for (int q = 0; q < 8; q++) qm |= ((qball >> (4 * q)) & 1u) << q;
-                }
-                npend &= ~qm;
-                if (npend == 0u) ticket = false;
-            }
-            if (__any_sync(0xffffffffu, ab != 0u)) break;
-            continue;
-        }
-        if (__any_sync(0xffffffffu, ab != 0u)) break;
-        // ---- no node pair: candidates of the candidate ticket ----
-        const bool cready = cslot && ctag == B.tag;
-        const unsigned cavail = __ballot_sync(0xffffffffu, cready);
-        if (cavail) {
-            idle = 0;
-            backoff = 32;
-            uint4 c = make_uint4(0u, 0u, 0u, 0u);
-            if (cready) {
-                c = __ldcg(B.cand + i);  // ordered after the tag's acquire load
-            }
-            filter_candidates<F64>(B, cready, c, decided, tested);
-            cpend &= ~cavail;
-            if (cpend == 0u) {
-                cbase = take_ticket(&C->c_head);
-                cpend = 0xffffffffu;
-            }
-            continue;
-        }
-        // ---- nothing ready: over, or wait.  Over (all seed tests done, then
-        // work == 0, read in that order) means no node pair exists any more and
-        // no slot will be published: the warp is done once none of its pending
-        // candidate slots lies below the final candidate count.
-        if ((idle & 3u) == 3u) {
-            unsigned over = 0, ncand = 0;
-            if (lane == 0) {
-                const unsigned sd = ld_vol(&C->seed_done);
-                fence_acq_rel();
-                const unsigned long long wc = *(const volatile unsigned long long*)&C->work_cand;
-                over = sd == seed_total && (unsigned)wc == 0u;
-                ncand = min((unsigned)(wc >> 32), B.cap_cand);
-            }
-            over = __shfl_sync(0xffffffffu, over, 0);
-            ncand = __shfl_sync(0xffffffffu, ncand, 0);
-            if (over && !__any_sync(0xffffffffu, ((cpend >> lane) & 1u) && i < ncand)) break;
-        }
-        if (++idle > kIdleSpins) {
-            if (lane == 0) {
-                atomicOr(&C->err, kErrTimeout);
-                atomicExch(&C->abort_, 1u);
-            }
-            break;
-        }
-        __nanosleep(backoff);
-        backoff = min(backoff * 2u, 256u);
-    }
-    block_stats(C, visited, decided, tested, maxlev + 1u);
-}
-
 // ---------------------------------------------------------------------------
-// Level-synchronous BVH4 x BVH4 traversal (one cooperative launch).
+// Block traversal (BVH4 x BVH4, one cooperative launch): the blocks work alone
+// on their own node pairs, in shared memory, and hand over what they cannot
+// expand at once to blocks that have run out.
 //
-// In the queue traversal above, the levels' end times advance by 12-15 us while
-// one warp iteration takes about 3 us: most of a level is the hand-off of node
-// pairs between warps through tagged queue slots.  Here the grid moves level by
-// level instead.  All node pairs of a level, and the leaf pairs the previous
-// level made, are split among all warps in static chunks (warp w takes chunks
-// w, w + warps, ...); the children form the next level's list; one grid barrier
-// (about a microsecond) separates the levels, so a level costs one or a few warp
-// iterations plus the barrier.  A level of at most `quad_below` node pairs is
-// expanded in the quad form (a quarter of the dependent chain, 8 node pairs per
-// warp), a wider one in the lane form (32 per warp).
+// A block holds a ring of node pairs and a list of leaf pairs (candidates) in
+// shared memory.  An iteration pops up to 64 of the newest node pairs, one per
+// quad of lanes, and pushes the overlapping children; 256 candidates are
+// filtered at a time, one per thread, as soon as there are so many; results
+// wait in shared memory and are appended to the result list in one piece.  A
+// block starts from its share of the seed tests (the pairs of the two meshes'
+// cut entries).
 //
-// Level l appends its node children (low half) and its leaf pairs (high half)
-// to the 64-bit counter lvl[l % 3], one atomic per warp and chunk.  The last
-// block to arrive at the barrier that ends level l decides whether the
-// traversal is over (no pair made, or the abort flag set: the same decision
-// for every block), clears lvl[(l + 2) % 3] (last read before level l began)
-// and stamps the level's end time.  Node pairs of level l live in half l % 2 of
-// the queue buffer; leaf pairs are appended to the candidate list in level
-// order, so level l + 1 filters candidates [snap_l, snap_l + count) with snap
-// summed from the counters in every block alike.  Every barrier wait is
-// bounded; a spent wait sets kErrTimeout and the abort flag and the block ends.
+// Sharing out: a block without node pairs takes a ticket (q_head) and polls
+// that slot of the pool.  Every iteration a block looks, with loads that its
+// node loads hide, how many tickets are ahead of the slots given out (q_tail);
+// if some are, what it holds beyond one iteration's 64 node pairs goes to them
+// from the oldest end (the largest subtrees), up to 64 a slot.  Slots are
+// published by the call's tag in their flag word (release; a poll acquires it),
+// so nothing is cleared between calls.
+//
+// Termination: the high half of `pool` counts blocks that work plus slots given
+// out and not yet taken, less the grid's blocks.  A hand-over raises it in the
+// same atomic that reserves its slots, a block lowers it when it runs out, and
+// a taken slot's count becomes its taker's; so it reaches -blocks when, and
+// only when, no node pair is left.  Every wait is bounded; a spent wait sets
+// kErrTimeout and the block ends.
+//
+// What bounds it is latency: an iteration is a chain of a shared-memory pop, a
+// node load, a box transform, the tests and two block barriers, 1.2-2 us with
+// three blocks per SM.  The forms it replaces handed every generation of node
+// pairs to other SMs through L2, level by level with a grid barrier (5 us a
+// level, 11 levels for two meshes of 1.3 M triangles) or through a queue of
+// tagged slots.  Traversal with the filter, launch included, the better of those
+// and this one: two UV spheres of 1,216 triangles 38 -> 21 us, of 20,224 57 -> 31,
+// two spheres of 200 k 97 -> 53, of 1.3 M 96 -> 52 (FP64 form 100 -> 56), 48
+// pairs of 10 k to 100 k in a batch 156 -> 134, coplanar 512 x 512 grids 216 ->
+// 202; 256 pairs of 1 k to 200 k 484 -> 519.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ unsigned long long globaltimer_ns()
 {
@@ -1744,417 +1100,485 @@ __device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v)
 {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-__device__ __forceinline__ void st_relaxed_u32(unsigned* p, unsigned v)
-{
-    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
 
-// Grid barrier ending level `lev` of the level-synchronous traversal, among
-// `nblocks` blocks.  Returns false when the block's wait ran out (the block must
-// leave the kernel).  The last block to arrive decides for every block whether
-// the traversal is over, clears the counter slot that level lev + 2 will use,
-// stamps the level's end time and publishes the level's candidates to the
-// candidate blocks (split form); they are all written once every node block has
-// arrived.  Its loads go out together and its stores are released by one
-// release store of the generation word, so the barrier costs few round trips
-// to L2 on its critical path.
-__device__ __forceinline__ bool level_barrier(const Bufs& B, unsigned& gen, unsigned lev, unsigned nblocks,
-                                              unsigned long long& v_out, bool& stop_out)
-{
-    __shared__ unsigned s_ok, s_stop;
-    __shared__ unsigned long long s_v;
-    Counters* C = B.cnt;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        s_ok = 1u;
-        // the arrival is an acquire-release atomic: it releases this block's
-        // writes of the level (ordered before it by the block barrier) and, for
-        // the last arriver, acquires every other block's
-        const unsigned arrived = arrive_acq_rel(&C->bar_count) + 1u;
-        if (arrived == nblocks) {
-            // every block has arrived: the counts of this level are final
-            const unsigned long long v = __ldcg(&C->lvl[lev % 3u]);
-            const unsigned ab = __ldcg(&C->abort_);
-            const unsigned prev = __ldcg(&C->cand_total);
-            // with published candidates the levels stop when no node pair is left
-            // (the filtering warps finish the candidates); otherwise when the
-            // level made nothing
-            const bool stop = ab != 0u || (B.publish ? (unsigned)v == 0u : v == 0ull);
-            const unsigned tot = prev + (unsigned)(v >> 32);
-            C->bar_count = 0u;
-            C->bstop = stop ? 1u : 0u;
-            C->bpub[0] = v;
-            C->bpub[1] = stop ? 1ull : 0ull;
-            s_v = v;
-            s_stop = stop ? 1u : 0u;
-            C->lvl[(lev + 2u) % 3u] = 0ull;
-            C->cand_total = tot;
-            atomicMax(&C->q_tail, 2u * (unsigned)v);  // both halves of the queue buffer must hold the widest level
-            if (lev < (unsigned)kLevelTimes) C->level_ns[lev] = globaltimer_ns();
-            if (B.publish) {
-                st_relaxed_u32(&C->cand_ready, tot);
-                // cand_ready is visible before the final flag
-                if (stop) st_release_u32(&C->cand_final, 1u);
-            }
-            st_release_u32(&C->bar_gen, gen + 1u);  // releases every store above
-        } else {
-            unsigned spins = 0;
-            while (ld_acq(&C->bar_gen) == gen) {
-                if (++spins > kIdleSpins) {
-                    atomicOr(&C->err, kErrTimeout);
-                    atomicExch(&C->abort_, 1u);
-                    s_ok = 0u;
-                    break;
-                }
-                __nanosleep(32);
-            }
-            // the level's counts and the decision, published before the release
-            const ulonglong2 pub = __ldcg(reinterpret_cast<const ulonglong2*>(C->bpub));
-            s_v = pub.x;
-            s_stop = pub.y != 0ull ? 1u : 0u;
-        }
-        gen++;
-    }
-    __syncthreads();
-    v_out = s_v;
-    stop_out = s_stop != 0u;
-    return s_ok != 0u;
-}
+// resident blocks per SM that the registers are cut for, [batch].  A single pair
+// is bound by latency: a fourth block's tighter registers cost small meshes 1 us;
+// a batch is bound by work (256 pairs: 564 us of traversal with three, 519 with four).
+constexpr int kBlkPerSm[2] = {3, 4};
+constexpr unsigned kBlkUnits = kBlkThreads / 4;  // node pairs per iteration, and per slot of the pool
+constexpr unsigned kBlkRing = 32 * kBlkUnits;               // node pairs a block holds (an iteration pushes at most 16 per unit)
+constexpr unsigned kBlkHigh = kBlkRing - 16 * kBlkUnits;      // ... and may hold when an iteration begins
+constexpr unsigned kBlkCand = kBlkThreads + 16 * kBlkUnits;  // candidates: less than a filter pass, and an iteration's
+constexpr unsigned kBlkRes = 2 * kBlkThreads;    // results a block holds (a filter pass makes at most one per thread)
+static_assert((kBlkRing & (kBlkRing - 1u)) == 0u, "ring index by mask");
+static_assert(kBlkUnits + kBlkThreads <= kBlkHigh, "seeds are taken below one iteration's node pairs");
 
-// Level 0: every pair of the two meshes' cut entries; overlapping pairs become
-// the first level's node pairs or candidates.
-template <bool F64>
-__device__ __forceinline__ void seed_levels(const Bufs& B, unsigned gw, unsigned nw, uint4* front, uint32_t capL)
-{
-    using S = typename Prec<F64>::S;
-    Counters* C = B.cnt;
-    const unsigned lane = threadIdx.x & 31;
-    const unsigned per_job = seed_tests_per_job(B);
-    const unsigned total = B.njobs * per_job;
-    const unsigned coff = B.deep_seed ? (unsigned)kCutMax : 0u;
-    for (unsigned base = gw * 32u; base < total; base += nw * 32u) {
-        const unsigned g = base + lane;
-        bool fr = false, cand = false;
-        uint32_t ra = 0, rb = 0, job = 0;
-        if (g < total) {
-            job = g / per_job;
-            const unsigned t = g % per_job;
-            const JobDev& J = B.jobs[job];
-            const bool both = J.A.nt && J.B.nt;
-            const unsigned nA = both ? __ldg(J.A.ncuts + (B.deep_seed ? 1 : 0)) : 0u;
-            const unsigned nB = both ? __ldg(J.B.ncuts + (B.deep_seed ? 1 : 0)) : 0u;
-            if (t < nA * nB) {
-                const unsigned i = coff + t / nB, j = coff + t % nB;
-                const S* ba_ = F64 ? (const S*)J.A.cutBox64 : (const S*)J.A.cutBox;
-                const S* bb_ = F64 ? (const S*)J.B.cutBox64 : (const S*)J.B.cutBox;
-                Box<S> ba, bb;
-                for (int k = 0; k < 3; k++) {
-                    ba.lo[k] = ba_[6 * i + k];
-                    ba.hi[k] = ba_[6 * i + 3 + k];
-                    bb.lo[k] = bb_[6 * j + k];
-                    bb.hi[k] = bb_[6 * j + 3 + k];
-                }
-                if (!J.pa.identity) world_box(J.pa, ba);
-                if (!J.pb.identity) world_box(J.pb, bb);
-                if (overlap(ba, bb)) {
-                    ra = J.A.cutRef[i];
-                    rb = J.B.cutRef[j];
-                    cand = (ra & kLeaf) && (rb & kLeaf);
-                    fr = !cand;
-                }
-            }
-        }
-        const unsigned fb = __ballot_sync(0xffffffffu, fr), cb = __ballot_sync(0xffffffffu, cand);
-        if (!(fb | cb)) continue;
-        unsigned long long old = 0;
-        if (lane == 0) old = atomicAdd(&C->lvl[0], ((unsigned long long)__popc(cb) << 32) + __popc(fb));
-        old = __shfl_sync(0xffffffffu, old, 0);
-        const unsigned lt = (1u << lane) - 1u;
-        if (fr) {
-            const unsigned pf = (unsigned)old + __popc(fb & lt);
-            if (pf < capL) {
-                front[pf] = make_uint4(job, ra, rb, 0u);
-            } else {
-                atomicOr(&C->overflow, kOvfFrontier);
-                atomicExch(&C->abort_, 1u);
-            }
-        }
-        if (cand) {
-            const unsigned pc = (unsigned)(old >> 32) + __popc(cb & lt);
-            if (pc < B.cap_cand) {
-                B.cand[pc] = make_uint4(job, ra & ~kLeaf, rb & ~kLeaf, 0u);
-            } else {
-                atomicOr(&C->overflow, kOvfCand);
-                atomicExch(&C->abort_, 1u);
-            }
-        }
-    }
-}
-
-// Reserves the warp's children in one atomic: node pairs of the next level and
-// candidates of this level.  nf / nc: this lane's counts.  Returns this lane's
-// first node-pair slot (f) and first candidate slot (c).
-__device__ __forceinline__ void level_reserve(const Bufs& B, unsigned lev, unsigned snap, unsigned nf, unsigned nc,
-                                              unsigned& f, unsigned& c)
-{
-    const unsigned lane = threadIdx.x & 31;
-    unsigned incf = nf, incc = nc;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned yf = __shfl_up_sync(0xffffffffu, incf, o);
-        const unsigned yc = __shfl_up_sync(0xffffffffu, incc, o);
-        if (lane >= (unsigned)o) {
-            incf += yf;
-            incc += yc;
-        }
-    }
-    unsigned long long old = 0;
-    if (lane == 31 && (incf | incc))
-        old = atomicAdd(&B.cnt->lvl[lev % 3u], ((unsigned long long)incc << 32) + incf);
-    old = __shfl_sync(0xffffffffu, old, 31);
-    f = (unsigned)old + incf - nf;
-    c = snap + (unsigned)(old >> 32) + incc - nc;
-}
-
-// Published candidates (split form).  A warp takes chunks of 32 candidates
-// with one atomic and filters each once the node blocks have published it
-// (every level's candidates are published by the barrier that ends it).  The
-// loop is software-pipelined: the next chunk is claimed before the current one
-// is filtered, and when it is already published, its candidate records and
-// triangle records are loaded before the current chunk's vertices, so these
-// two dependent round trips overlap the current chunk's work.  A warp leaves
-// when its chunk starts at or beyond the final count.
-constexpr unsigned kGone = 0xffffffffu;
-
-// Lane 0 waits (bounded) until the chunk at `base` is published in full or no
-// more candidates will come; returns the published count, or kGone.
-__device__ __forceinline__ unsigned wait_published(Counters* C, unsigned base)
-{
-    unsigned ready = 0, spins = 0;
-    for (;;) {
-        ready = ld_acq(&C->cand_ready);
-        if (ready >= base + 32u) return ready;
-        if (ld_acq(&C->cand_final)) return ld_acq(&C->cand_ready);  // written before the final flag
-        if (ld_vol(&C->abort_)) return kGone;
-        if (++spins > kIdleSpins) {
-            atomicOr(&C->err, kErrTimeout);
-            atomicExch(&C->abort_, 1u);
-            return kGone;
-        }
-        __nanosleep(64);
-    }
-}
-
-struct PubChunk {
-    uint4 c;       // candidate: job, leaf position in A, leaf position in B
-    uint4 ta, tb;  // the two leaves' records: vertex indices and original triangle id
-    bool have;
+// a warp's child boxes of B, field by field, four children of a quad together
+template <class S>
+struct QuadBoxes {
+    S f[6][32];
+    uint32_t ref[32];
+};
+template <bool F64, bool MULTI>
+struct BlockShared {
+    QuadBoxes<typename Prec<F64>::S> x[kBlkThreads / 32];
+    uint2 ring[kBlkRing];
+    uint2 cand[kBlkCand];
+    uint4 res[kBlkRes];
+    uint32_t ring_job[MULTI ? kBlkRing : 1];
+    uint32_t cand_job[MULTI ? kBlkCand : 1];
+    unsigned push[2];  // pushed by the iteration: node pairs (low half), candidates (high half)
+    unsigned nres, base, hungry, room, ticket, state;
 };
 
-__device__ __forceinline__ PubChunk load_published(const Bufs& B, unsigned base, unsigned ready)
+// Results held by the block to the global list (all threads; nres is uniform).
+template <bool F64, bool MULTI>
+__device__ __forceinline__ void block_flush(const Bufs& B, BlockShared<F64, MULTI>& s, unsigned nres)
 {
-    PubChunk k;
-    const unsigned i = base + (threadIdx.x & 31u);
-    k.have = i < min(ready, B.cap_cand);
-    k.c = k.have ? __ldcg(B.cand + i) : make_uint4(0u, 0u, 0u, 0u);
-    k.ta = k.tb = make_uint4(0u, 0u, 0u, 0u);
-    if (k.have) {
-        const JobDev& J = B.jobs[k.c.x];
-        k.ta = __ldg(J.A.leafTri + k.c.y);
-        k.tb = __ldg(J.B.leafTri + k.c.z);
+    __syncthreads();
+    if (nres == 0u) return;
+    if (threadIdx.x == 0) s.base = atomicAdd(&B.cnt->res, nres);
+    __syncthreads();
+    const unsigned base = s.base;
+    for (unsigned k = threadIdx.x; k < nres; k += kBlkThreads) {
+        if (base + k < B.cap_res) B.res[base + k] = s.res[k];
+        else atomicOr(&B.cnt->overflow, kOvfRes);
     }
-    return k;
+    if (threadIdx.x == 0) s.nres = 0u;
+    __syncthreads();
 }
 
-template <bool F64>
-__device__ __forceinline__ void filter_loaded(const Bufs& B, const PubChunk& k, unsigned long long& decided,
-                                              unsigned long long& tested)
+// First filter stage on the block's last `m` candidates (m <= 256), one per
+// thread; every thread of the block calls it.
+template <bool F64, bool MULTI>
+__device__ __forceinline__ void block_filter(const Bufs& B, BlockShared<F64, MULTI>& s, unsigned cn, unsigned m,
+                                             unsigned long long& decided, unsigned long long& tested)
 {
     Counters* C = B.cnt;
+    const unsigned tid = threadIdx.x;
+    const bool have = tid < m;
     int dec = DEC_NO;
-    unsigned pat = 0;
-    if (k.have) {
+    uint4 r = make_uint4(0u, 0u, 0u, 0u);
+    uint2 c = make_uint2(0u, 0u);
+    if (have) {
+        c = s.cand[cn - 1u - tid];
+        if constexpr (MULTI) r.x = s.cand_job[cn - 1u - tid];
         tested++;
-        const JobDev& J = B.jobs[k.c.x];
+        const JobDev& J = job_at<MULTI>(B, r.x);
+        const uint4 ta = __ldg(J.A.leafTri + c.x), tb = __ldg(J.B.leafTri + c.y);
         double3 P[3], Q[3];
-        P[0] = world_vertex(J.A.verts, k.ta.x, J.pa);
-        P[1] = world_vertex(J.A.verts, k.ta.y, J.pa);
-        P[2] = world_vertex(J.A.verts, k.ta.z, J.pa);
-        Q[0] = world_vertex(J.B.verts, k.tb.x, J.pb);
-        Q[1] = world_vertex(J.B.verts, k.tb.y, J.pb);
-        Q[2] = world_vertex(J.B.verts, k.tb.z, J.pb);
-        if constexpr (F64) dec = classify_fast<double>(P, Q, &pat);
-        else dec = classify_fast<float>(P, Q, &pat);
+        P[0] = world_vertex(J.A.verts, ta.x, J.pa);
+        P[1] = world_vertex(J.A.verts, ta.y, J.pa);
+        P[2] = world_vertex(J.A.verts, ta.z, J.pa);
+        Q[0] = world_vertex(J.B.verts, tb.x, J.pb);
+        Q[1] = world_vertex(J.B.verts, tb.y, J.pb);
+        Q[2] = world_vertex(J.B.verts, tb.z, J.pb);
+        if constexpr (F64) dec = classify_fast<double>(P, Q, &r.w);
+        else dec = classify_fast<float>(P, Q, &r.w);
         decided += (dec != DEC_ESC);
+        r.y = ta.w;
+        r.z = tb.w;
     }
-    const bool yes = k.have && dec == DEC_YES;
-    const bool esc = k.have && dec == DEC_ESC;
-    const unsigned pr = warp_append(yes, &C->res);
-    if (yes) {
-        if (pr < B.cap_res) B.res[pr] = make_uint4(k.c.x, k.ta.w, k.tb.w, pat);
-        else atomicOr(&C->overflow, kOvfRes);
-    }
+    const unsigned at = warp_append(have && dec == DEC_YES, &s.nres);
+    if (have && dec == DEC_YES) s.res[at] = r;
+    const bool esc = have && dec == DEC_ESC;
     const unsigned pe = warp_append(esc, &C->esc);
     if (esc) {
-        if (pe < B.cap_esc) B.esc[pe] = make_uint4(k.c.x, k.c.y, k.c.z, 0u);
+        if (pe < B.cap_esc) B.esc[pe] = make_uint4(r.x, c.x, c.y, 0u);
         else atomicOr(&C->overflow, kOvfEsc);
     }
+    __syncthreads();
+    const unsigned nres = s.nres;
+    __syncthreads();  // read alike by all before the next pass adds to it
+    if (nres > kBlkRes - kBlkThreads) block_flush<F64, MULTI>(B, s, nres);
 }
 
-template <bool F64>
-__device__ __forceinline__ void filter_published(const Bufs& B, unsigned long long& decided,
-                                                 unsigned long long& tested)
+// Seed test t: the pair of cut entries it names, if their world boxes overlap.
+// A batch has kCutMax x kCutMax tests per job on the depth-3 cuts, one pair the
+// nA x nB tests of its depth-4 cuts.
+template <bool F64, bool MULTI>
+__device__ __forceinline__ bool seed_test(const Bufs& B, unsigned t, unsigned nA, unsigned nB, uint32_t& job, uint2& ab)
+{
+    using S = typename Prec<F64>::S;
+    unsigned coff = (unsigned)kCutMax;
+    job = 0;
+    if constexpr (MULTI) {
+        coff = 0u;
+        job = t / (unsigned)(kCutMax * kCutMax);
+        t %= (unsigned)(kCutMax * kCutMax);
+    }
+    const JobDev& J = job_at<MULTI>(B, job);
+    if constexpr (MULTI) {
+        if (!J.A.nt || !J.B.nt) return false;  // an empty mesh has no cut (null sizes)
+        nA = __ldg(J.A.ncuts);
+        nB = __ldg(J.B.ncuts);
+    }
+    if (t >= nA * nB) return false;
+    const unsigned i = coff + t / nB, j = coff + t % nB;
+    const S* ba_ = F64 ? (const S*)J.A.cutBox64 : (const S*)J.A.cutBox;
+    const S* bb_ = F64 ? (const S*)J.B.cutBox64 : (const S*)J.B.cutBox;
+    Box<S> ba, bb;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        ba.lo[k] = __ldg(ba_ + 6 * i + k);
+        ba.hi[k] = __ldg(ba_ + 6 * i + 3 + k);
+        bb.lo[k] = __ldg(bb_ + 6 * j + k);
+        bb.hi[k] = __ldg(bb_ + 6 * j + 3 + k);
+    }
+    ab = make_uint2(__ldg(J.A.cutRef + i), __ldg(J.B.cutRef + j));
+    if (!J.pa.identity) world_box(J.pa, ba);
+    if (!J.pb.identity) world_box(J.pb, bb);
+    return overlap(ba, bb);
+}
+
+// One node pair per quad of lanes, lane `sub` owning child `sub` of both nodes:
+// it maps its own child boxes to the world frame, the quad exchanges B's four
+// through shared memory (x holds a warp's 8 quads; a 16-byte read gives one
+// field of all four), and the lane tests its A child against them.  Called by
+// all 32 lanes; lanes without a node pair (have = false) get no children.
+// fm / cm: bit j set when (own A child, B child j) overlap and lead to a node
+// pair / a leaf pair; B's child refs stay in x.ref (until the warp's next call).
+//
+// A batch also tests B's boxes in B's own frame (A's world boxes mapped back
+// through B's pose): the world box of a rotated box is wider than the box, and
+// each test alone is conservative.  That removes a quarter of its node pairs
+// for about a third more work per pair (256 pairs of 1 k to 200 k triangles:
+// 649 us of traversal without, 559 with), which pays where the traversal is
+// bound by work, not for one pair, which is bound by latency.
+template <class S>
+struct Vec4 {
+    S v[4];
+};
+__device__ __forceinline__ Vec4<float> lds4(const float* p)
+{
+    const float4 q = *reinterpret_cast<const float4*>(p);
+    return {q.x, q.y, q.z, q.w};
+}
+__device__ __forceinline__ Vec4<double> lds4(const double* p)
+{
+    const double2 a = *reinterpret_cast<const double2*>(p), b = *reinterpret_cast<const double2*>(p + 2);
+    return {a.x, a.y, b.x, b.y};
+}
+template <class S>
+__device__ __forceinline__ void quad_put(QuadBoxes<S>& x, const Box<S>& b)
+{
+    const unsigned lane = threadIdx.x & 31u;
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+        x.f[q][lane] = b.lo[q];
+        x.f[3 + q][lane] = b.hi[q];
+    }
+}
+// bit j: box a meets box j of the quad
+template <class S>
+__device__ __forceinline__ unsigned quad_meets(const QuadBoxes<S>& x, const Box<S>& a)
+{
+    const unsigned q4 = threadIdx.x & 28u;
+    bool ov[4] = {true, true, true, true};
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+        const Vec4<S> lo = lds4(&x.f[q][q4]), hi = lds4(&x.f[3 + q][q4]);
+#pragma unroll
+        for (int j = 0; j < 4; j++) ov[j] = ov[j] & (a.lo[q] <= hi.v[j]) & (lo.v[j] <= a.hi[q]);
+    }
+    return (ov[0] ? 1u : 0u) | (ov[1] ? 2u : 0u) | (ov[2] ? 4u : 0u) | (ov[3] ? 8u : 0u);
+}
+template <bool F64, bool MULTI>
+__device__ __forceinline__ void block_expand(const Bufs& B, QuadBoxes<typename Prec<F64>::S>& x, const uint4& ent,
+                                             bool have, unsigned sub, unsigned& fm, unsigned& cm, uint32_t& ca)
+{
+    using S = typename Prec<F64>::S;
+    const JobDev& J = job_at<MULTI>(B, have ? ent.x : 0u);
+    const unsigned lane = threadIdx.x & 31u, q4 = lane & 28u;
+    Box<S> a, b;
+    uint32_t mb = kEmpty;
+    ca = kEmpty;
+#pragma unroll
+    for (int q = 0; q < 3; q++) a.lo[q] = a.hi[q] = b.lo[q] = b.hi[q] = S(0);
+    unsigned m = 0xFu;
+    if constexpr (MULTI && !F64) {
+        if (have) {
+            load_kid(J.A, ent.y, sub, a, ca);
+            load_kid(J.B, ent.z, sub, b, mb);
+            if (J.pa.fw.use) map_box(J.pa.fw, a);
+        }
+        if (B.two_frame) {  // uniform over the launch
+            quad_put(x, b);
+            __syncwarp();
+            if (have && J.pb.inv.use) {
+                Box<S> al = a;
+                map_box(J.pb.inv, al);
+                m = quad_meets(x, al);
+            }
+            __syncwarp();
+        }
+        if (have && J.pb.fw.use) map_box(J.pb.fw, b);
+    } else {
+        if (have) {
+            load_kid(J.A, ent.y, sub, a, ca);
+            load_kid(J.B, ent.z, sub, b, mb);
+            if (!J.pa.identity) world_box(J.pa, a);
+        }
+        if (MULTI && B.two_frame) {
+            quad_put(x, b);
+            __syncwarp();
+            if (have && J.pb.inv_ok) {
+                Box<S> al = a;
+                if constexpr (F64) local_box(J.pb, al);
+                m = quad_meets(x, al);
+            }
+            __syncwarp();
+        }
+        if (have && !J.pb.identity) world_box(J.pb, b);
+    }
+    quad_put(x, b);
+    x.ref[lane] = mb;
+    __syncwarp();
+    const uint4 r4 = *reinterpret_cast<const uint4*>(&x.ref[q4]);
+    const uint32_t cb[4] = {r4.x, r4.y, r4.z, r4.w};
+    m &= quad_meets(x, a);
+    unsigned there = 0, leaf = 0;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        there |= (cb[j] != kEmpty ? 1u : 0u) << j;
+        leaf |= (cb[j] >> 31) << j;
+    }
+    m = ca != kEmpty ? m & there : 0u;
+    cm = (ca & kLeaf) ? m & leaf : 0u;
+    fm = m & ~cm;
+}
+
+// Hands the block's `m` oldest node pairs (ring positions rb ..) to `d` slots of
+// the pool (m <= 64 d), as evenly as whole entries allow; all threads call it.
+// Slots past the pool's end are dropped and flagged (the call reruns with a
+// larger pool); they count as taken.
+template <bool F64, bool MULTI>
+__device__ __forceinline__ void block_give(const Bufs& B, BlockShared<F64, MULTI>& s, unsigned rb, unsigned m, unsigned d)
 {
     Counters* C = B.cnt;
-    const unsigned lane = threadIdx.x & 31;
-    unsigned base = 0, ready = 0;
-    if (lane == 0) {
-        base = atomicAdd(&C->c_head, 32u);
-        ready = wait_published(C, base);
+    const unsigned nslots = B.cap_queue / kBlkUnits, tid = threadIdx.x;
+    if (tid == 0) s.base = (unsigned)atomicAdd(&C->pool, ((unsigned long long)d << 32) + d);
+    __syncthreads();
+    const unsigned base = s.base, q = (m + d - 1u) / d;
+    for (unsigned k = tid; k < m; k += kBlkThreads) {
+        const unsigned c = k / q, at = (rb + k) & (kBlkRing - 1u);
+        const uint2 ab = s.ring[at];
+        uint32_t job = 0;
+        if constexpr (MULTI) job = s.ring_job[at];
+        if (base + c < nslots) B.queue[(size_t)(base + c) * kBlkUnits + (k - c * q)] = make_uint4(job, ab.x, ab.y, min(q, m - c * q));
     }
-    base = __shfl_sync(0xffffffffu, base, 0);
-    ready = __shfl_sync(0xffffffffu, ready, 0);
-    if (ready == kGone || base >= ready) return;
-    PubChunk cur = load_published(B, base, ready);
-    for (;;) {
-        // the next chunk: claimed now, its records loaded now if it is published
-        unsigned nbase = 0, nready = 0;
-        if (lane == 0) {
-            nbase = atomicAdd(&C->c_head, 32u);
-            nready = ld_acq(&C->cand_ready);
+    __syncthreads();
+    if (tid < d) {
+        if (base + tid < nslots) {
+            // an empty slot (the entries did not divide) is published with no entries
+            if (tid * q >= m) B.queue[(size_t)(base + tid) * kBlkUnits] = make_uint4(0u, kEmpty, kEmpty, 0u);
+            st_release_u32(B.qflag + base + tid, B.tag);
+        } else {
+            atomicOr(&C->overflow, kOvfFrontier);
+            atomicAdd(&C->pool, ~0ull << 32);
         }
-        nbase = __shfl_sync(0xffffffffu, nbase, 0);
-        nready = __shfl_sync(0xffffffffu, nready, 0);
-        const bool early = nready >= nbase + 32u;
-        PubChunk nxt;
-        if (early) nxt = load_published(B, nbase, nready);
-        filter_loaded<F64>(B, cur, decided, tested);
-        if (!early) {
-            if (lane == 0) nready = wait_published(C, nbase);
-            nready = __shfl_sync(0xffffffffu, nready, 0);
-            if (nready == kGone || nbase >= nready) return;
-            nxt = load_published(B, nbase, nready);
-        }
-        cur = nxt;
     }
 }
 
-template <bool F64>
-__global__ void __launch_bounds__(kTravThreads, 2) k_traverse_levels(Bufs B)
+template <bool F64, bool MULTI>
+__global__ void __launch_bounds__(kBlkThreads, kBlkPerSm[MULTI ? 1 : 0]) k_traverse_blocks(const __grid_constant__ Bufs B)
 {
+    extern __shared__ __align__(16) unsigned char blk_dyn[];
+    BlockShared<F64, MULTI>& s = *reinterpret_cast<BlockShared<F64, MULTI>*>(blk_dyn);
     Counters* C = B.cnt;
-    const unsigned lane = threadIdx.x & 31;
-    // blocks [0, nblocks) expand node pairs; in the split form the others filter candidates
-    const unsigned nblocks = gridDim.x - B.cand_blocks;
-    const bool node_block = blockIdx.x < nblocks;
-    const unsigned gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const unsigned nw = (nblocks * blockDim.x) >> 5;
-    const uint32_t capL = B.cap_queue / 2u;
-    uint4* const front0 = B.queue;
-    uint4* const front1 = B.queue + capL;
+    const unsigned tid = threadIdx.x, lane = tid & 31u, unit = tid >> 2, sub = tid & 3u;
+    const unsigned G = gridDim.x, b = blockIdx.x;
+    const unsigned nslots = B.cap_queue / kBlkUnits;
+    const unsigned lt = (1u << lane) - 1u;
     allow_dependent_launch();
-    if (blockIdx.x == 0 && threadIdx.x == 0) C->t_start = globaltimer_ns();
+    if (tid == 0) {
+        s.push[0] = s.push[1] = 0u;
+        s.nres = 0u;
+    }
+    // the block's share of the seed tests: one pair's with the grid's stride (its
+    // overlapping cut entries cluster), a batch's in runs of one block's threads
+    // (lanes then share a job)
+    unsigned nA = 0, nB = 0, total;
+    if constexpr (MULTI) {
+        total = B.njobs * (unsigned)(kCutMax * kCutMax);
+    } else {
+        if (B.job0.A.nt && B.job0.B.nt) {  // an empty mesh has no cut (null sizes)
+            nA = __ldg(B.job0.A.ncuts + 1);
+            nB = __ldg(B.job0.B.ncuts + 1);
+        }
+        total = nA * nB;
+    }
+    const unsigned deal = MULTI ? (total + kBlkThreads - 1u) / kBlkThreads : total;  // dealt to the blocks in turn
+    const unsigned share = deal > b ? (deal - b + G - 1u) / G : 0u;
+    const unsigned chunks = MULTI ? share : (share + kBlkThreads - 1u) / kBlkThreads;
+    unsigned taken = 0;
     unsigned long long visited = 0, decided = 0, tested = 0;
-    unsigned gen = 0, snap = 0, lev = 0;
-    bool ovf_f = false, ovf_c = false;
-    // the node blocks seed; the candidate blocks filter from the start
-    if (node_block) seed_levels<F64>(B, gw, nw, front0, capL);
-    else filter_published<F64>(B, decided, tested);
-    for (; node_block;) {
-        unsigned long long v;
-        bool stop;
-        if (!level_barrier(B, gen, lev, nblocks, v, stop)) return;
-        if (stop) break;
-        // v: the pairs made by level `lev`, expanded and filtered by level lev + 1
-        const unsigned n = min((unsigned)v, capL);
-        const unsigned cbase = snap, cend = min(snap + (unsigned)(v >> 32), B.cap_cand);
-        snap += (unsigned)(v >> 32);
-        ++lev;
-        const uint4* cur = (lev & 1u) ? front0 : front1;
-        uint4* nxt = (lev & 1u) ? front1 : front0;
-        const bool quad = n <= B.quad_below;
-        const unsigned per = quad ? 8u : 32u;
-        const unsigned node_chunks = (n + per - 1u) / per;
-        // published candidates are left to the filtering warps
-        const unsigned chunks = node_chunks + (!B.publish && cend > cbase ? (cend - cbase + 31u) / 32u : 0u);
-        for (unsigned k = gw; k < chunks; k += nw) {
-            if (k < node_chunks) {
-                if (quad) {
-                    const unsigned unit = lane >> 2, sub = lane & 3u;
-                    const unsigned idx = k * 8u + unit;
-                    const bool have = idx < n;
-                    const uint4 ent = have ? __ldcg(cur + idx) : make_uint4(0u, kEmpty, kEmpty, 0u);
-                    visited += (have && sub == 0u) ? 1u : 0u;
-                    unsigned fm = 0, cm = 0;
-                    uint32_t ca = kEmpty, cb[4];
-                    expand_quad<F64>(B, ent, have, sub, fm, cm, ca, cb);
-                    unsigned f, c;
-                    level_reserve(B, lev, snap, __popc(fm), __popc(cm), f, c);
-#pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        if ((fm >> j) & 1u) {
-                            if (f < capL) nxt[f] = make_uint4(ent.x, ca, cb[j], 0u);
-                            else ovf_f = true;
-                            f++;
+    // node pairs at ring positions rb .. rb + sn - 1, candidates 0 .. cn - 1 (alike in all threads)
+    unsigned rb = 0, sn = 0, cn = 0, it = 0;
+    __syncthreads();
+    for (;;) {
+        if (cn >= kBlkThreads) {
+            block_filter<F64, MULTI>(B, s, cn, kBlkThreads, decided, tested);
+            cn -= kBlkThreads;
+            continue;
+        }
+        if (sn > kBlkHigh) {  // too many for another iteration
+            const unsigned m = kBlkHigh / 2u;
+            block_give<F64, MULTI>(B, s, rb, m, m / kBlkUnits);
+            rb += m;
+            sn -= m;
+            continue;
+        }
+        if (taken < chunks && sn < kBlkUnits) {
+            const unsigned c = taken++;
+            __syncthreads();
+            if (tid == 0) s.push[(it & 1u) ^ 1u] = 0u;  // read by all before this barrier
+            const unsigned t = MULTI ? (c * G + b) * kBlkThreads + tid : (c * kBlkThreads + tid) * G + b;
+            uint32_t job = 0;
+            uint2 ab = make_uint2(kLeaf, kLeaf);
+            const bool ov = t < total && seed_test<F64, MULTI>(B, t, nA, nB, job, ab);
+            const bool cand = ov && (ab.x & kLeaf) && (ab.y & kLeaf), node = ov && !cand;
+            const unsigned bn = __ballot_sync(0xffffffffu, node), bc = __ballot_sync(0xffffffffu, cand);
+            unsigned old = 0;
+            if (lane == 0 && (bn | bc)) old = atomicAdd(&s.push[it & 1u], __popc(bn) + (__popc(bc) << 16));
+            old = __shfl_sync(0xffffffffu, old, 0);
+            if (node) {
+                const unsigned at = (rb + sn + (old & 0xffffu) + __popc(bn & lt)) & (kBlkRing - 1u);
+                s.ring[at] = ab;
+                if constexpr (MULTI) s.ring_job[at] = job;
+            }
+            if (cand) {
+                const unsigned at = cn + (old >> 16) + __popc(bc & lt);
+                s.cand[at] = make_uint2(ab.x & ~kLeaf, ab.y & ~kLeaf);
+                if constexpr (MULTI) s.cand_job[at] = job;
+            }
+            __syncthreads();
+            const unsigned p = s.push[it & 1u];
+            sn += p & 0xffffu;
+            cn += p >> 16;
+            it++;
+            continue;
+        }
+        if (sn == 0u) {
+            // out of node pairs: a ticket, and while its slot is not there the candidates left
+            if (tid == 0) {
+                s.ticket = atomicAdd(&C->q_head, 1u);
+                atomicAdd(&C->pool, ~0ull << 32);
+            }
+            unsigned state = 0;
+            for (;;) {
+                if (tid == 0) {
+                    const unsigned t = s.ticket, patience = cn ? 1u : kIdleSpins;
+                    unsigned st = 0;
+                    for (unsigned spins = 0; spins < patience; spins++) {
+                        if (t < nslots && ld_acq(B.qflag + t) == B.tag) {
+                            st = 1u;
+                            break;
                         }
-                        if ((cm >> j) & 1u) {
-                            if (c < B.cap_cand) B.cand[c] = make_uint4(ent.x, ca & ~kLeaf, cb[j] & ~kLeaf, 0u);
-                            else ovf_c = true;
-                            c++;
+                        if ((unsigned)(*(volatile unsigned long long*)&C->pool >> 32) == 0u - G) {
+                            st = 2u;
+                            break;
                         }
+                        if (spins) __nanosleep(64);
                     }
-                } else {
-                    const unsigned idx = k * 32u + lane;
-                    const bool have = idx < n;
-                    uint4 ent = make_uint4(0u, kEmpty, kEmpty, 0u);
-                    unsigned fm = 0, cm = 0;
-                    uint32_t ca[4], cb[4];
-                    if (have) {
-                        ent = __ldcg(cur + idx);
-                        visited++;
-                        expand_pair<F64>(B, ent, fm, cm, ca, cb);
+                    if (!st && !cn) {
+                        atomicOr(&C->err, kErrTimeout);
+                        st = 2u;
                     }
-                    unsigned f, c;
-                    level_reserve(B, lev, snap, __popc(fm), __popc(cm), f, c);
-                    // child slot q = 4i + j is the pair (A child i, B child j); the
-                    // unrolled loop indexes the registers with constants
-#pragma unroll
-                    for (int q = 0; q < 16; q++) {
-                        if ((fm >> q) & 1u) {
-                            if (f < capL) nxt[f] = make_uint4(ent.x, ca[q >> 2], cb[q & 3], 0u);
-                            else ovf_f = true;
-                            f++;
-                        }
-                        if ((cm >> q) & 1u) {
-                            if (c < B.cap_cand)
-                                B.cand[c] = make_uint4(ent.x, ca[q >> 2] & ~kLeaf, cb[q & 3] & ~kLeaf, 0u);
-                            else ovf_c = true;
-                            c++;
-                        }
-                    }
+                    s.state = st;
                 }
-            } else {
-                const unsigned i = cbase + (k - node_chunks) * 32u + lane;
-                const bool have = i < cend;
-                const uint4 cnd = have ? __ldcg(B.cand + i) : make_uint4(0u, 0u, 0u, 0u);
-                filter_candidates<F64>(B, have, cnd, decided, tested);
+                __syncthreads();
+                state = s.state;
+                if (state == 1u || !cn) break;
+                while (cn) {
+                    const unsigned m = min(cn, kBlkThreads);
+                    block_filter<F64, MULTI>(B, s, cn, m, decided, tested);
+                    cn -= m;
+                }
+                if (state == 2u) break;
+            }
+            if (state == 2u) break;
+            const uint4* const slot = B.queue + (size_t)s.ticket * kBlkUnits;
+            const unsigned m = min(__ldcg(slot).w, kBlkUnits);
+            if (tid < m) {
+                const uint4 e = __ldcg(slot + tid);
+                s.ring[tid] = make_uint2(e.y, e.z);
+                if constexpr (MULTI) s.ring_job[tid] = e.x;
+            }
+            rb = 0;
+            sn = m;
+            __syncthreads();
+            continue;
+        }
+        const unsigned take = min(sn, kBlkUnits);
+        const bool have = unit < take;
+        uint4 ent = make_uint4(0u, kEmpty, kEmpty, 0u);
+        if (have) {
+            const unsigned at = (rb + sn - 1u - unit) & (kBlkRing - 1u);
+            const uint2 ab = s.ring[at];
+            ent.y = ab.x;
+            ent.z = ab.y;
+            if constexpr (MULTI) ent.x = s.ring_job[at];
+            visited += sub == 0u ? 1u : 0u;
+        }
+        sn -= take;
+        // tickets and slots, looked at while the nodes load
+        unsigned head = 0, tail = 0;
+        if (tid == 0) {
+            head = ld_vol(&C->q_head);
+            tail = ld_vol(reinterpret_cast<const unsigned*>(&C->pool));
+        }
+        __syncthreads();  // the popped entries are read before the pushes reuse their places
+        if (tid == 0) s.push[(it & 1u) ^ 1u] = 0u;  // read by all before this barrier
+        unsigned fm = 0, cm = 0;
+        uint32_t ca = kEmpty;
+        if (__any_sync(0xffffffffu, have)) {
+            block_expand<F64, MULTI>(B, s.x[tid >> 5], ent, have, sub, fm, cm, ca);
+            // places of the lane's children: a warp scan of both counts in one word
+            const unsigned mine = __popc(fm) + (__popc(cm) << 16);
+            unsigned inc = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned y = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= (unsigned)o) inc += y;
+            }
+            unsigned old = 0;
+            if (lane == 31u && inc) old = atomicAdd(&s.push[it & 1u], inc);
+            old = __shfl_sync(0xffffffffu, old, 31) + inc - mine;
+            unsigned f = rb + sn + (old & 0xffffu), c = cn + (old >> 16);
+            for (unsigned left = fm | cm; left; left &= left - 1u) {  // two children at most, mostly
+                const unsigned j = __ffs(left) - 1u;
+                const uint32_t rB = s.x[tid >> 5].ref[(lane & 28u) + j];
+                if ((cm >> j) & 1u) {
+                    s.cand[c] = make_uint2(ca & ~kLeaf, rB & ~kLeaf);
+                    if constexpr (MULTI) s.cand_job[c] = ent.x;
+                    c++;
+                } else {
+                    s.ring[f & (kBlkRing - 1u)] = make_uint2(ca, rB);
+                    if constexpr (MULTI) s.ring_job[f & (kBlkRing - 1u)] = ent.x;
+                    f++;
+                }
             }
         }
-        if (ovf_f || ovf_c) {
-            if (ovf_f) atomicOr(&C->overflow, kOvfFrontier);
-            if (ovf_c) atomicOr(&C->overflow, kOvfCand);
-            atomicExch(&C->abort_, 1u);
-            ovf_f = ovf_c = false;
+        if (tid == 0) {
+            // tickets waiting; none where the pool is nearly full (every block may give 16 slots at once)
+            s.hungry = tail + 16u * G < nslots && (int)(head - tail) > 0 ? head - tail : 0u;
+        }
+        __syncthreads();
+        const unsigned p = s.push[it & 1u], hungry = s.hungry;
+        sn += p & 0xffffu;
+        cn += p >> 16;
+        it++;
+        if (hungry && sn > B.keep) {
+            const unsigned m0 = sn - B.keep, d = min(min(hungry, 16u), (m0 + kBlkUnits - 1u) / kBlkUnits);
+            const unsigned m = min(m0, d * kBlkUnits);
+            block_give<F64, MULTI>(B, s, rb, m, d);
+            rb += m;
+            sn -= m;
         }
     }
-    // published candidates: the node blocks are done (the last barrier published
-    // every candidate and the final flag) and filter what is left
-    if (node_block && B.publish) filter_published<F64>(B, decided, tested);
-    block_stats(C, visited, decided, tested);
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        C->levels = lev;
-        C->work_cand = (unsigned long long)snap << 32;  // candidates made, for the host's retry sizing
-    }
+    block_flush<F64, MULTI>(B, s, s.nres);
+    block_stats(C, visited, decided, tested, it);
 }
 
 // ===========================================================================
@@ -3258,54 +2682,38 @@ cudaError_t query_launch(int device, LaunchCfg* cfg)
     cudaDeviceProp prop;
     GI_TRY(cudaGetDeviceProperties(&prop, device));
     cfg->sms = prop.multiProcessorCount;
-    int n[2][2] = {}, nl[2] = {};
-    GI_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nl[0], k_traverse_levels<false>, kTravThreads, 0));
-    GI_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nl[1], k_traverse_levels<true>, kTravThreads, 0));
-    for (int a = 0; a < 2; a++) cfg->levels_per_sm[a] = nl[a] < 1 ? 1 : (nl[a] > 2 ? 2 : nl[a]);
+    int nr[2][2] = {};
+    cfg->blk_dyn[0][0] = sizeof(BlockShared<false, false>);
+    cfg->blk_dyn[0][1] = sizeof(BlockShared<false, true>);
+    cfg->blk_dyn[1][0] = sizeof(BlockShared<true, false>);
+    cfg->blk_dyn[1][1] = sizeof(BlockShared<true, true>);
+    const void* const kb[2][2] = {{(const void*)k_traverse_blocks<false, false>, (const void*)k_traverse_blocks<false, true>},
+                                  {(const void*)k_traverse_blocks<true, false>, (const void*)k_traverse_blocks<true, true>}};
+    for (int a = 0; a < 2; a++)
+        for (int m = 0; m < 2; m++) {
+            GI_TRY(cudaFuncSetAttribute(kb[a][m], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cfg->blk_dyn[a][m]));
+            GI_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nr[a][m], kb[a][m], kBlkThreads, cfg->blk_dyn[a][m]));
+        }
+    for (int a = 0; a < 2; a++)
+        for (int m = 0; m < 2; m++) cfg->blocks_per_sm[a][m] = nr[a][m] < 1 ? 1 : nr[a][m];
     int nf = 0;
     GI_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nf, k_finish, kFinThreads, kFinDyn));
     cfg->fin_per_sm = nf < 1 ? 1 : (nf > 2 ? 2 : nf);
-    GI_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n[0][0], k_traverse<false, false>, kTravThreads, 0));
-    GI_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n[0][1], k_traverse<false, true>, kTravThreads, 0));
-    GI_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n[1][0], k_traverse<true, false>, kTravThreads, 0));
-    GI_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n[1][1], k_traverse<true, true>, kTravThreads, 0));
-    for (int a = 0; a < 2; a++)
-        for (int q = 0; q < 2; q++) cfg->trav_per_sm[a][q] = n[a][q] < 1 ? 1 : n[a][q];
-    cfg->trav_threads = kTravThreads;
     return cudaSuccess;
 }
 
-// The persistent traversal needs no co-residency (nothing waits on a block
-// that has not started); the grid is at most the resident block count so
-// that every warp is live from the start.
 cudaError_t launch_traverse(const Bufs& b, const LaunchCfg& cfg, int precision, TravShape shape, cudaStream_t st)
 {
     note_launches(1);
-    const int f64 = precision == 1 ? 1 : 0, q = shape.quad ? 1 : 0;
-    if (shape.levels) {
-        // cooperative: the grid barriers need every block resident.  Bit 0 of the
-        // shape selects the split form: a quarter of the blocks filter candidates
-        // while the other three quarters expand the levels' node pairs (pose
-        // stream of two 1.3M-triangle meshes on B200: 0.1065 ms of traversal against 0.1072 with a third,
-        // 0.1075-0.1083 with a fifth, more with a half)
-        const int grid = cfg.levels_per_sm[f64] * cfg.sms;
-        Bufs bb = b;
-        bb.cand_blocks = shape.one_per_sm ? (unsigned)(grid / 4) : 0u;
-        bb.publish = shape.one_per_sm ? 1u : 0u;
-        bb.quad_below = shape.quad ? (unsigned)((grid - (int)bb.cand_blocks) * (kTravThreads / 32) * 8) : 0u;
-        void* args[] = {&bb};
-        return cudaLaunchCooperativeKernel(f64 ? (const void*)k_traverse_levels<true> : (const void*)k_traverse_levels<false>,
-                                           dim3(grid), dim3(kTravThreads), args, 0, st);
-    }
-    const int grid = (shape.one_per_sm ? 1 : cfg.trav_per_sm[f64][q]) * cfg.sms;
-    if (f64) {
-        if (q) k_traverse<true, true><<<grid, kTravThreads, 0, st>>>(b);
-        else k_traverse<true, false><<<grid, kTravThreads, 0, st>>>(b);
-    } else {
-        if (q) k_traverse<false, true><<<grid, kTravThreads, 0, st>>>(b);
-        else k_traverse<false, false><<<grid, kTravThreads, 0, st>>>(b);
-    }
-    return cudaGetLastError();
+    const int f64 = precision == 1 ? 1 : 0, m = b.njobs > 1 ? 1 : 0;
+    // cooperative: a block that waits needs every other resident
+    const int grid = (shape.one_per_sm ? 1 : cfg.blocks_per_sm[f64][m]) * cfg.sms;
+    Bufs bb = b;
+    bb.keep = shape.give_half ? kBlkUnits / 2u : kBlkUnits;
+    void* args[] = {&bb};
+    const void* kern = f64 ? (m ? (const void*)k_traverse_blocks<true, true> : (const void*)k_traverse_blocks<true, false>)
+                           : (m ? (const void*)k_traverse_blocks<false, true> : (const void*)k_traverse_blocks<false, false>);
+    return cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(kBlkThreads), args, cfg.blk_dyn[f64][m], st);
 }
 
 cudaError_t launch_exact(const Bufs& b, const LaunchCfg& cfg, cudaStream_t st)

@@ -48,35 +48,32 @@ cudaError_t build_bvh(MeshBuffers& m, bool fp64, unsigned* d_err, cudaMemPool_t 
 // Intersect launch configuration.
 struct LaunchCfg {
     int sms = 0;
-    int trav_per_sm[2][2] = {};  // resident traversal blocks per SM, [FP64][quad form]
-    int levels_per_sm[2] = {};   // resident blocks of the level-synchronous traversal (at most 2), [FP64]
-    int fin_per_sm = 1;          // resident blocks of the post-traversal launch (at most 2)
-    int trav_threads = 256;
+    int blocks_per_sm[2][2] = {};  // resident blocks of the block traversal, [FP64][batch]
+    size_t blk_dyn[2][2] = {};     // ... and their shared memory
+    int fin_per_sm = 1;            // resident blocks of the post-traversal launch (at most 2)
 };
 
-// Traversal shapes the tuner chooses from: the work-queue traversal or the
-// level-synchronous one (bit 2); expansion form (bit 1: one node pair per quad
-// of lanes; for the level-synchronous traversal, the quad form on levels of at
-// most 8 node pairs per warp); bit 0: the work-queue traversal with one block
-// per SM (else all resident), the level-synchronous one in its split form
-// (a quarter of the blocks only filter candidates).
+// Traversal shapes (GI_FLAG_SHAPE; every shape gives the same results): bit 0
+// one block per SM instead of all resident ones, bit 1 blocks hand over what
+// they hold beyond half an iteration's node pairs instead of beyond a whole
+// one's.  The default has neither: the other forms measured slower or equal at
+// every size (two 1.3 M-triangle meshes: 55 us of traversal against 60 with
+// bit 1 and 78 with bit 0).
 struct TravShape {
-    bool quad = false;
     bool one_per_sm = false;
-    bool levels = false;
+    bool give_half = false;
 };
-constexpr int kTravShapes = 8;
+constexpr int kDefaultShape = 4;
 inline TravShape trav_shape(int k)
 {
     TravShape t;
-    t.quad = (k & 2) != 0;
     t.one_per_sm = (k & 1) != 0;
-    t.levels = (k & 4) != 0;
+    t.give_half = (k & 2) != 0;
     return t;
 }
 cudaError_t query_launch(int device, LaunchCfg* cfg);
 
-// Traversal + first filter stage (persistent, work queue), then the exact stage.
+// Traversal + first filter stage (persistent), then the exact stage.
 cudaError_t launch_traverse(const Bufs& b, const LaunchCfg& cfg, int precision, TravShape shape, cudaStream_t st);
 cudaError_t launch_exact(const Bufs& b, const LaunchCfg& cfg, cudaStream_t st);
 // Segments of every result (count from the device counters):

@@ -87,14 +87,11 @@ typedef struct gi_server gi_server;
 /* gi_options.flags */
 #define GI_FLAG_TINY_BUFFERS 1u /* start every intersect buffer at 64 entries: exercises the
                                    capacity-overflow / retry path (host-side fault injection) */
-/* The traversal shape is autotuned per workload class on the context's own
- * calls.  GI_FLAG_FIXED_SHAPE | GI_FLAG_SHAPE(k), k in 0..7, fixes it instead
- * (every shape gives the same results): bit 2 selects the level-synchronous
- * traversal (grid barriers between the levels) over the work-queue one; bit 1
- * the quad form (one node pair per quad of lanes; level-synchronous: on levels
- * of at most 8 node pairs per warp); bit 0 one block per SM instead of all
- * resident blocks (work queue) or the split form, in which a third of the
- * blocks only filter candidates as the levels publish them (level-synchronous). */
+/* GI_FLAG_FIXED_SHAPE | GI_FLAG_SHAPE(k), k in 0..7, picks a shape of the
+ * traversal other than the library's own choice, for measurements (every shape
+ * gives the same results): bit 0 one block per SM instead of all resident
+ * blocks; bit 1 blocks hand node pairs over earlier (beyond half of what an
+ * iteration takes instead of all of it); bit 2 has no effect. */
 #define GI_FLAG_FIXED_SHAPE 0x100u
 #define GI_FLAG_SHAPE(k) ((((uint32_t)(k)) & 7u) << 9)
 
@@ -136,7 +133,7 @@ typedef struct {
     uint64_t exact_points;            /* constructed points that needed exact division */
     uint64_t pairs;                   /* intersecting pairs */
     uint64_t segments;                /* emitted segments */
-    uint32_t levels;                  /* traversal levels */
+    uint32_t levels;                  /* most expansion iterations of one traversal block */
     uint32_t retries;                 /* capacity retries */
     uint32_t launches;                /* kernels launched by this call */
     uint32_t traverse_shape;          /* traversal shape used (GI_FLAG_SHAPE numbering) */
@@ -149,10 +146,7 @@ typedef struct {
                                          are its phases' own spans (its timestamps) and ms_traverse the
                                          rest of the call, the hand-off between the launches included */
     double ms_total;                  /* device time of the whole call */
-    /* level-synchronous traversal only (else level_times = 0): level_end_ms[l]
-     * is the time from the traversal's start to the end of level l (level 0:
-     * the seeding from the cut pairs; level l > 0 expands the node pairs made
-     * by level l - 1 and filters its leaf pairs), for the first level_times levels */
+    /* kept for the layout: level_times is 0 (the traversal has no common levels) */
     uint32_t level_times;
     uint32_t reserved2;
     double level_end_ms[32];
