@@ -107,7 +107,7 @@ extern "C" gi_status gi_create(const gi_options* opts, gi_ctx** out)
         }
     }
     if (e == cudaSuccess) e = query_launch(c->device, &c->cfg);
-    if (e == cudaSuccess) e = cudaMalloc(&c->d_cnt, sizeof(Counters));
+    if (e == cudaSuccess) e = cudaMalloc(&c->d_cnt, 2 * sizeof(Counters));
     if (e == cudaSuccess) e = cudaMallocHost(&c->h_cnt, sizeof(Counters));
     for (int i = 0; i < 8 && e == cudaSuccess; i++) e = cudaEventCreate(&c->ev[i]);
     if (e != cudaSuccess) {
@@ -127,6 +127,7 @@ extern "C" gi_status gi_destroy(gi_ctx* c)
     for (auto& sg : c->stage) sg.release();
     c->copy_pool.reset();
     if (c->d_cnt) cudaFree(c->d_cnt);
+    if (c->fin_mem) cudaFreeAsync(c->fin_mem, c->st);
     if (c->d_jobs) cudaFree(c->d_jobs);
     void* pooled[] = {c->queue, c->qflag,     c->res,
                       c->esc,   c->segs,      c->nseg,         c->pairs_out, c->job_out,
@@ -614,7 +615,7 @@ static gi_status run_jobs(gi_ctx* c, const std::vector<JobDev>& jobs, const gi_i
         c->cap_jobs = nj;
     }
     memcpy(c->h_jobs, jobs.data(), sizeof(JobDev) * nj);
-    CK(c, cudaMemcpyAsync(c->d_jobs, c->h_jobs, sizeof(JobDev) * nj, cudaMemcpyHostToDevice, c->st), "jobs copy");
+    bool jobs_there = false;  // a single pair's job travels in the kernel parameters where every kernel takes it from there
     const bool tiny = (c->flags & GI_FLAG_TINY_BUFFERS) != 0;
     // pool of handed-over node pairs: a few slots per resident block at every size
     uint32_t need_front = std::max<uint32_t>(c->cap_front, tiny ? 64u : 1u << 21);
@@ -647,8 +648,6 @@ static gi_status run_jobs(gi_ctx* c, const std::vector<JobDev>& jobs, const gi_i
     // into one partition; a refusal keeps the next calls off this path a while)
     bool fin = sort && ba + bb + bj <= 63 && c->pred_pairs <= kFinMax - kFinMax / 4 && c->fin_backoff == 0;
     if (c->fin_backoff) c->fin_backoff--;
-    const int kbits = ba + bb + bj;
-    const int fin_shift = kbits > kFinPartBits ? kbits - kFinPartBits : 0;
     const int shape = c->shape;
     for (;;) {
         CK(c, grow(c->queue, c->cap_front, need_front, c->pool, c->st), "node queue");
@@ -699,12 +698,39 @@ static gi_status run_jobs(gi_ctx* c, const std::vector<JobDev>& jobs, const gi_i
         b.cap_res = c->cap_res;
         b.esc = c->esc;
         b.cap_esc = c->cap_esc;
-        b.cnt = c->d_cnt;
+        b.cnt = c->d_cnt + c->cur;
+        Counters* const next_cnt = c->d_cnt + (c->cur ^ 1);
         b.precision = prec;
         b.two_frame = nj > 1 ? 1 : 0;
         b.keep = 0u;  // set by the launcher
         b.job0 = jobs[0];
-        CK(c, cudaMemsetAsync(c->d_cnt, 0, sizeof(Counters), c->st), "counters");
+        // result block: sized by the previous call's result, with room to grow
+        uint32_t pp = std::min<uint32_t>(cap, (uint32_t)std::min<uint64_t>(c->pred_pairs + c->pred_pairs / 4 + 1024,
+                                                                          0xffffffffu));
+        uint32_t ps = want_segs ? std::min<uint32_t>(3 * cap, c->pred_segs + c->pred_segs / 4 + 1024) : 0u;
+        off_jobs = (sizeof(int32_t) * 2 * (size_t)pp + 15) & ~(size_t)15;
+        off_segs = (off_jobs + (nj > 1 ? sizeof(uint32_t) * (size_t)pp : 0) + 15) & ~(size_t)15;
+        off_segpair = off_segs + sizeof(double) * 6 * (size_t)ps;
+        gi_status s = pinned_for(c, &buf, off_segpair + sizeof(int32_t) * (size_t)ps + 64);
+        if (s != GI_OK) return s;
+        hp = (char*)buf->p;
+        if (!c->fin_mem) {
+            CK(c, pool_alloc(&c->fin_mem, fin_scratch_bytes(), c->pool, c->st), "finish scratch");
+            c->cur_clear = false;
+        }
+        if (!c->cur_clear) {
+            // the last call did not end with the one-launch finish, which clears this set
+            CK(c, cudaMemsetAsync(b.cnt, 0, sizeof(Counters), c->st), "counters");
+            CK(c, cudaMemsetAsync(fin_counts(c->fin_mem, c->cur), 0, sizeof(uint32_t) * 2 * kFinParts, c->st), "finish counts");
+        }
+        c->cur_clear = false;
+        b.fin = make_fin_bufs(c->fin_mem, c->cur, ba, bb, bj);
+        b.fin.on = fin ? 1 : 0;
+        b.fin.segments = want_segs ? 1 : 0;
+        if (!jobs_there && (nj > 1 || !fin)) {
+            CK(c, cudaMemcpyAsync(c->d_jobs, c->h_jobs, sizeof(JobDev) * nj, cudaMemcpyHostToDevice, c->st), "jobs copy");
+            jobs_there = true;
+        }
         CK(c, cudaEventRecord(c->ev[0], c->st), "event");
         CK(c, launch_traverse(b, c->cfg, prec, trav_shape(shape), c->st), "traverse");
         // the finish follows the traversal directly (programmatic dependent
@@ -712,15 +738,22 @@ static gi_status run_jobs(gi_ctx* c, const std::vector<JobDev>& jobs, const gi_i
         if (!fin) CK(c, cudaEventRecord(c->ev[1], c->st), "event");
         if (fin) {
             FinArgs F;
-            F.segs = c->segs;
+            F.h_pairs = (int32_t*)hp;
+            F.h_job = (uint32_t*)(hp + off_jobs);
+            F.h_segs = (double*)(hp + off_segs);
+            F.h_segpair = (int32_t*)(hp + off_segpair);
+            F.host_pairs = pp;
+            F.host_segs = ps;
             F.pairs_out = c->pairs_out;
             F.job_out = c->job_out;
             F.segs_out = c->segs_out;
             F.segpair_out = c->segpair_out;
             F.cap = cap;
             F.want_segments = want_segs ? 1 : 0;
-            F.shift = fin_shift;
-            CK(c, launch_finish(b, O, F, c->cfg, c->st, true), "exact stage, segments and ordering");
+            F.host_cnt = c->h_cnt;
+            F.next_cnt = next_cnt;
+            F.next_count = fin_counts(c->fin_mem, c->cur ^ 1);
+            CK(c, launch_finish(b, F, c->cfg, c->st), "exact stage, segments and ordering");
         } else {
             CK(c, launch_exact(b, c->cfg, c->st), "exact stage");
             CK(c, cudaEventRecord(c->ev[2], c->st), "event");
@@ -751,35 +784,27 @@ static gi_status run_jobs(gi_ctx* c, const std::vector<JobDev>& jobs, const gi_i
             }
         }
         CK(c, cudaEventRecord(c->ev[4], c->st), "event");
-        // speculative copy at the previous call's size
-        uint32_t pp = std::min<uint32_t>(cap, (uint32_t)std::min<uint64_t>(c->pred_pairs + c->pred_pairs / 4 + 1024,
-                                                                          0xffffffffu));
-        uint32_t ps = want_segs ? std::min<uint32_t>(3 * cap, c->pred_segs + c->pred_segs / 4 + 1024) : 0u;
-        off_jobs = sizeof(int32_t) * 2 * (size_t)pp;
-        off_segs = off_jobs + (nj > 1 ? sizeof(uint32_t) * (size_t)pp : 0);
-        off_segs = (off_segs + 15) & ~(size_t)15;
-        off_segpair = off_segs + sizeof(double) * 6 * (size_t)ps;
-        gi_status s = pinned_for(c, &buf, off_segpair + sizeof(int32_t) * (size_t)ps + 64);
-        if (s != GI_OK) return s;
-        hp = (char*)buf->p;
-        CK(c, cudaMemcpyAsync(c->h_cnt, c->d_cnt, sizeof(Counters), cudaMemcpyDeviceToHost, c->st), "counters");
-        CK(c, cudaMemcpyAsync(hp, c->pairs_out, off_jobs, cudaMemcpyDeviceToHost, c->st), "copy pairs");
-        if (nj > 1)
-            CK(c, cudaMemcpyAsync(hp + off_jobs, c->job_out, sizeof(uint32_t) * pp, cudaMemcpyDeviceToHost, c->st),
-               "copy jobs");
-        if (ps) {
-            CK(c, cudaMemcpyAsync(hp + off_segs, c->segs_out, sizeof(double) * 6 * ps, cudaMemcpyDeviceToHost, c->st),
-               "copy segments");
-            CK(c, cudaMemcpyAsync(hp + off_segpair, c->segpair_out, sizeof(int32_t) * ps, cudaMemcpyDeviceToHost,
-                                  c->st),
-               "copy segments");
+        if (!fin) {
+            // speculative copy at the previous call's size
+            CK(c, cudaMemcpyAsync(c->h_cnt, b.cnt, sizeof(Counters), cudaMemcpyDeviceToHost, c->st), "counters");
+            CK(c, cudaMemcpyAsync(hp, c->pairs_out, sizeof(int32_t) * 2 * (size_t)pp, cudaMemcpyDeviceToHost, c->st),
+               "copy pairs");
+            if (nj > 1)
+                CK(c, cudaMemcpyAsync(hp + off_jobs, c->job_out, sizeof(uint32_t) * pp, cudaMemcpyDeviceToHost, c->st),
+                   "copy jobs");
+            if (ps) {
+                CK(c, cudaMemcpyAsync(hp + off_segs, c->segs_out, sizeof(double) * 6 * ps, cudaMemcpyDeviceToHost, c->st),
+                   "copy segments");
+                CK(c, cudaMemcpyAsync(hp + off_segpair, c->segpair_out, sizeof(int32_t) * ps, cudaMemcpyDeviceToHost,
+                                      c->st),
+                   "copy segments");
+            }
         }
         CK(c, cudaStreamSynchronize(c->st), "sync");
-        if (H.err & kErrTimeout) {
-            // a finish launch that gave up may leave partition counts behind
-            if (fin) cudaMemsetAsync(O.fin, 0, sizeof(uint32_t) * 2 * kFinParts, c->st);
-            return set_err(c, GI_ERR_TIMEOUT, "a bounded device wait ran out");
-        }
+        // the finish left the other set clear (after a spent wait nothing is relied on)
+        if (H.err & kErrTimeout) return set_err(c, GI_ERR_TIMEOUT, "a bounded device wait ran out");
+        c->cur ^= 1;
+        c->cur_clear = fin;
         if (H.err & kErrExactCapacity) return set_err(c, GI_ERR_RANGE, "exact arithmetic capacity exceeded");
         if (H.overflow) {
             if (retries >= 12) return set_err(c, GI_ERR_CAPACITY, "intersection buffers stayed too small");
@@ -796,8 +821,6 @@ static gi_status run_jobs(gi_ctx* c, const std::vector<JobDev>& jobs, const gi_i
         }
         if (H.order_redo) {
             if (fin) {
-                // a refusal after the counting leaves the partition counts behind
-                CK(c, cudaMemsetAsync(O.fin, 0, sizeof(uint32_t) * 2 * kFinParts, c->st), "finish counts");
                 fin = false;
                 if (H.order_redo == kRedoCrowded) c->fin_backoff = 64;
                 if (H.res > kOrderSmallMax) small_order = false;
@@ -811,13 +834,15 @@ static gi_status run_jobs(gi_ctx* c, const std::vector<JobDev>& jobs, const gi_i
         nsegs = want_segs ? H.nseg : 0;
         if (nres > pp || nsegs > ps) {
             // the result outgrew the speculative copy: copy it again at its real size
-            off_jobs = sizeof(int32_t) * 2 * (size_t)nres;
+            off_jobs = (sizeof(int32_t) * 2 * (size_t)nres + 15) & ~(size_t)15;
             off_segs = (off_jobs + (nj > 1 ? sizeof(uint32_t) * (size_t)nres : 0) + 15) & ~(size_t)15;
             off_segpair = off_segs + sizeof(double) * 6 * (size_t)nsegs;
             s = pinned_for(c, &buf, off_segpair + sizeof(int32_t) * (size_t)nsegs + 64);
             if (s != GI_OK) return s;
             hp = (char*)buf->p;
-            if (nres) CK(c, cudaMemcpyAsync(hp, c->pairs_out, off_jobs, cudaMemcpyDeviceToHost, c->st), "copy pairs");
+            if (nres)
+                CK(c, cudaMemcpyAsync(hp, c->pairs_out, sizeof(int32_t) * 2 * (size_t)nres, cudaMemcpyDeviceToHost, c->st),
+                   "copy pairs");
             if (nres && nj > 1)
                 CK(c, cudaMemcpyAsync(hp + off_jobs, c->job_out, sizeof(uint32_t) * nres, cudaMemcpyDeviceToHost,
                                       c->st),
@@ -843,12 +868,12 @@ static gi_status run_jobs(gi_ctx* c, const std::vector<JobDev>& jobs, const gi_i
         // and phases from its own timestamps (taken after it waited for the
         // traversal), the traversal the rest of the call
         const double span = H.fin_ns[4] >= H.fin_ns[0] ? 1e-6 * double(H.fin_ns[4] - H.fin_ns[0]) : 0.0;
-        if (H.fin_ns[1] >= H.fin_ns[0] && H.fin_ns[2] >= H.fin_ns[1]) {
-            ms_exact = (float)(1e-6 * double(H.fin_ns[1] - H.fin_ns[0]));
-            ms_seg = (float)(1e-6 * double(H.fin_ns[2] - H.fin_ns[1]));
-        }
         ms_trav = std::max(0.0f, ms_total - (float)span);
-        ms_sort = std::max(0.0f, (float)span - ms_exact - ms_seg);
+        if (H.fin_ns[1] >= H.fin_ns[0] && H.fin_ns[4] >= H.fin_ns[1]) {
+            ms_exact = (float)(1e-6 * double(H.fin_ns[1] - H.fin_ns[0]));
+            ms_sort = H.fin_ns[2] >= H.fin_ns[1] ? (float)(1e-6 * double(H.fin_ns[2] - H.fin_ns[1])) : 0.0f;
+            ms_seg = std::max(0.0f, (float)span - ms_exact - ms_sort);
+        }
     } else {
         cudaEventElapsedTime(&ms_trav, c->ev[0], c->ev[1]);
         cudaEventElapsedTime(&ms_exact, c->ev[1], c->ev[2]);

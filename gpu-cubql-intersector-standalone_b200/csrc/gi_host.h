@@ -278,7 +278,12 @@ struct gi_ctx {
     std::string last_error;
     std::mutex mu;  // serialises device work of this context
 
+    // two sets of counters and partition counts: a call uses set `cur`; the
+    // one-launch finish clears the other one for the next call (other_clear)
     Counters* d_cnt = nullptr;
+    int cur = 0;
+    bool cur_clear = false;     // set `cur` is zero
+    void* fin_mem = nullptr;    // partitions of the one-launch finish (gi::FinBufs)
     Counters* h_cnt = nullptr;  // pinned
     JobDev* d_jobs = nullptr;
     JobDev* h_jobs = nullptr;  // pinned

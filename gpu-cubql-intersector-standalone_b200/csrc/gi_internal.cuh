@@ -116,16 +116,13 @@ struct Counters {
     unsigned long long exact_points;
     unsigned long long tested;  // candidates run through the first filter stage
     // post-traversal launch (k_finish): globaltimer at its start, after the exact
-    // stage, when the last block ended its key phase, after the count scan's
-    // release, and when its last block ended
+    // stage, when block 0 had its run ranked and when it had it written, and when
+    // the last block ended
     unsigned long long fin_ns[5];
     unsigned fin_done;  // blocks of k_finish that have ended
-    unsigned pad11[31];
-    unsigned fbar;      // k_finish: blocks arrived at the barrier after its key phase
-    unsigned pad12[31];
-    unsigned frel;      // k_finish: the last block's release (1), or its refusal (2)
-    unsigned fin_over;  // k_finish: keys put on the overflow list (may exceed its capacity)
-    unsigned pad13[30];
+    unsigned fin_over;  // results whose partition's bucket was full (may exceed the overflow list)
+    unsigned odd;       // 1: some result has other than one segment
+    unsigned pad2;
 };
 
 constexpr unsigned kOvfFrontier = 1u, kOvfRes = 4u, kOvfEsc = 8u;
@@ -133,6 +130,25 @@ constexpr unsigned kErrTimeout = 1u, kErrExactCapacity = 2u;
 // Counters::order_redo: the small-count ordering or the one-launch finish
 // refused; kRedoCrowded: the finish found a key partition over its limit
 constexpr unsigned kRedoCount = 1u, kRedoCrowded = 2u;
+
+// Results by key partition, for the one-launch finish: filled where results are
+// found, read by k_finish.
+constexpr int kFinPartBits = 12;
+constexpr int kFinParts = 1 << kFinPartBits;
+constexpr int kFinBucket = 256;
+constexpr int kFinOverflow = 1 << 14;
+struct FinBufs {
+    uint32_t* count;  // kFinParts key counts (zero when a call begins)
+    uint32_t* extra;  // kFinParts: segments beyond one per key, modulo 2^32 (zero when a call begins)
+    unsigned long long* bkey;  // kFinParts x kFinBucket: each partition's first keys
+    uint32_t* bval;            // ... and their result index | segment count << 30
+    unsigned long long* okey;  // kFinOverflow: the keys beyond a bucket
+    uint2* oval;               // ... their value and their slot in the partition
+    int shift;                 // partition of a key = key >> shift
+    int bits_a, bits_b;
+    int on;                    // 1: results are inserted
+    int segments;              // the call wants segments
+};
 
 // Per-call buffers handed to the kernels.
 struct Bufs {
@@ -150,6 +166,7 @@ struct Bufs {
     int precision;    // 0 FP32 cascade, 1 FP64
     int two_frame;    // also test child boxes in B's own frame (fewer pairs, more work per pair)
     unsigned keep;          // block traversal: node pairs that a block does not hand over
+    FinBufs fin;
     JobDev job0;            // the job of a call with one (njobs == 1), read from the kernel's parameters
 };
 

@@ -1131,6 +1131,43 @@ struct BlockShared {
     unsigned nres, base, hungry, room, ticket, state;
 };
 
+// Segments that a construction code stands for.
+__device__ __forceinline__ uint32_t code_segments(unsigned code)
+{
+    const unsigned kind = code & 3u;
+    return kind == 3u ? 3u : (kind ? 1u : 0u);
+}
+
+// A result's key into its partition (the key's top kFinPartBits bits), for the
+// one-launch finish: into the partition's bucket at the slot that one atomic on
+// its count returns, or beyond the bucket on one overflow list.  ns: its
+// segments (1 unless the exact stage found it).
+__device__ __forceinline__ unsigned long long fin_key(const FinBufs& F, uint32_t job, uint32_t a, uint32_t b)
+{
+    return ((unsigned long long)job << (F.bits_a + F.bits_b)) | ((unsigned long long)a << F.bits_b) | b;
+}
+__device__ __forceinline__ void fin_insert(const Bufs& B, const uint4& r, uint32_t idx, unsigned ns)
+{
+    const FinBufs& F = B.fin;
+    const unsigned long long key = fin_key(F, r.x, r.y, r.z);
+    const unsigned part = (unsigned)(key >> F.shift), slot = atomicAdd(F.count + part, 1u);
+    const uint32_t v = idx | (ns << 30);
+    if (slot < (unsigned)kFinBucket) {
+        F.bkey[part * kFinBucket + slot] = key;
+        F.bval[part * kFinBucket + slot] = v;
+    } else {
+        const unsigned o = atomicAdd(&B.cnt->fin_over, 1u);
+        if (o < (unsigned)kFinOverflow) {
+            F.okey[o] = key;
+            F.oval[o] = make_uint2(v, slot);
+        }
+    }
+    if (ns != 1u) {
+        atomicAdd(F.extra + part, ns - 1u);
+        B.cnt->odd = 1u;
+    }
+}
+
 // Results held by the block to the global list (all threads; nres is uniform).
 template <bool F64, bool MULTI>
 __device__ __forceinline__ void block_flush(const Bufs& B, BlockShared<F64, MULTI>& s, unsigned nres)
@@ -1141,8 +1178,12 @@ __device__ __forceinline__ void block_flush(const Bufs& B, BlockShared<F64, MULT
     __syncthreads();
     const unsigned base = s.base;
     for (unsigned k = threadIdx.x; k < nres; k += kBlkThreads) {
-        if (base + k < B.cap_res) B.res[base + k] = s.res[k];
-        else atomicOr(&B.cnt->overflow, kOvfRes);
+        if (base + k < B.cap_res) {
+            B.res[base + k] = s.res[k];
+            if (B.fin.on) fin_insert(B, s.res[k], base + k, 1u);
+        } else {
+            atomicOr(&B.cnt->overflow, kOvfRes);
+        }
     }
     if (threadIdx.x == 0) s.nres = 0u;
     __syncthreads();
@@ -1586,6 +1627,7 @@ __global__ void __launch_bounds__(kBlkThreads, kBlkPerSm[MULTI ? 1 : 0]) k_trave
 // ===========================================================================
 // Exact stage over the escalated pairs, grid-stride over the threads of the
 // launch (nth a multiple of 32): intersecting pairs are appended to the results.
+template <bool MULTI>
 __device__ __forceinline__ void exact_stage(const Bufs& B, unsigned gtid, unsigned nth)
 {
     Counters* C = B.cnt;
@@ -1602,7 +1644,7 @@ __device__ __forceinline__ void exact_stage(const Bufs& B, unsigned gtid, unsign
         if (have) {
             uint4 c = __ldcg(B.esc + i);
             job = c.x;
-            const JobDev& J = B.jobs[job];
+            const JobDev& J = job_at<MULTI>(B, job);
             double3 pts[6];
             load_tri<false>(J.A, J.pa, c.y, pts, &ta);
             load_tri<false>(J.B, J.pb, c.z, pts + 3, &tb);
@@ -1612,8 +1654,13 @@ __device__ __forceinline__ void exact_stage(const Bufs& B, unsigned gtid, unsign
         }
         unsigned pr = warp_append(yes, &C->res);
         if (yes) {
-            if (pr < B.cap_res) B.res[pr] = make_uint4(job, ta, tb, code);
-            else atomicOr(&C->overflow, kOvfRes);
+            const uint4 r = make_uint4(job, ta, tb, code);
+            if (pr < B.cap_res) {
+                B.res[pr] = r;
+                if (B.fin.on) fin_insert(B, r, pr, B.fin.segments ? code_segments(code) : 1u);
+            } else {
+                atomicOr(&C->overflow, kOvfRes);
+            }
         }
     }
     for (int o = 16; o > 0; o >>= 1) nexact += __shfl_xor_sync(0xffffffffu, nexact, o);
@@ -1622,7 +1669,7 @@ __device__ __forceinline__ void exact_stage(const Bufs& B, unsigned gtid, unsign
 
 __global__ void __launch_bounds__(128) k_exact(Bufs B)
 {
-    exact_stage(B, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    exact_stage<true>(B, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
 __device__ __forceinline__ void load_tri_orig(const MeshDev& M, const DevPose& P, uint32_t tri, double3* out)
@@ -1672,21 +1719,16 @@ __device__ __forceinline__ bool result_point(const double3* P, const double3* Q,
 }
 
 // Segments of one result (up to 3, 6 doubles each, at o) from its construction
-// code: their count, the same in every lane that shares the result.  `per`
-// threads (1 or 2, adjacent lanes) share it, thread `half` constructing the
-// points half, half + per, ..
-__device__ __forceinline__ uint32_t code_segments(unsigned code)
-{
-    const unsigned kind = code & 3u;
-    return kind == 3u ? 3u : (kind ? 1u : 0u);
-}
+// code.  `per` threads (1 or 2, adjacent lanes) share it, thread `half`
+// constructing the points half, half + per, ..
+template <bool MULTI>
 __device__ __forceinline__ void result_segments(const Bufs& B, const uint4& rr, double* o, unsigned half = 0u,
                                                 unsigned per = 1u)
 {
     Counters* C = B.cnt;
     const unsigned kind = rr.w & 3u, drop = (rr.w >> 2) & 3u;
     if (!kind) return;
-    const JobDev& J = B.jobs[B.njobs == 1 ? 0u : rr.x];  // one job: its loads need not wait for rr
+    const JobDev& J = job_at<MULTI>(B, rr.x);
     double3 P[3], Q[3];
     load_tri_orig(J.A, J.pa, rr.y, P);
     load_tri_orig(J.B, J.pb, rr.z, Q);
@@ -1725,7 +1767,7 @@ __global__ void __launch_bounds__(128) k_segments(Bufs B, double* __restrict__ s
     for (unsigned i = gtid; i < nres; i += nth) {
         const uint4 rr = __ldcg(B.res + i);
         nseg[i] = code_segments(rr.w);
-        result_segments(B, rr, segs + 18 * (size_t)i);
+        result_segments<true>(B, rr, segs + 18 * (size_t)i);
     }
 }
 
@@ -1920,8 +1962,8 @@ size_t order_scratch_bytes(uint32_t cap, int passes)
     size_t ntiles = (cap + kOsTile - 1) / kOsTile;
     return 2 * sizeof(unsigned long long) * (size_t)cap + 2 * sizeof(uint32_t) * (size_t)cap +
            sizeof(uint32_t) * ((size_t)(passes + 1) * ntiles * 256 + 2 * kOsMaxPasses * 256 + kOsMaxPasses + 2 +
-                               (size_t)cap / kOsGatherTile + 1 + kOrderSmallBlocks + 5 * kFinParts + 2) +
-           (sizeof(unsigned long long) + sizeof(uint32_t)) * ((size_t)kFinParts * kFinBucket + kFinOverflow) + 8192;
+                               (size_t)cap / kOsGatherTile + 1 + kOrderSmallBlocks) +
+           8192;
 }
 
 OrderBufs make_order_bufs(void* scratch, uint32_t cap, int bits_a, int bits_b, int bits_job)
@@ -1949,12 +1991,6 @@ OrderBufs make_order_bufs(void* scratch, uint32_t cap, int bits_a, int bits_b, i
     O.base = (uint32_t*)take(sizeof(uint32_t) * kOsMaxPasses * 256);
     O.tile_ctr = (uint32_t*)take(sizeof(uint32_t) * (kOsMaxPasses + 2));
     O.tile_tot = (uint32_t*)take(sizeof(uint32_t) * kOrderSmallBlocks);
-    O.fin = (uint32_t*)take(sizeof(uint32_t) * 2 * kFinParts);
-    O.fin_off = (uint32_t*)take(sizeof(uint32_t) * (3 * kFinParts + 2));
-    O.fin_bkey = (unsigned long long*)take(sizeof(unsigned long long) * kFinParts * kFinBucket);
-    O.fin_bval = (uint32_t*)take(sizeof(uint32_t) * kFinParts * kFinBucket);
-    O.fin_okey = (unsigned long long*)take(sizeof(unsigned long long) * kFinOverflow);
-    O.fin_oval = (uint32_t*)take(sizeof(uint32_t) * kFinOverflow);
     return O;
 }
 
@@ -2246,431 +2282,385 @@ cudaError_t launch_order_small_phases(const Bufs& b, const OrderBufs& O, bool so
 }
 
 // ===========================================================================
-// Post-traversal work of a call in one cooperative launch (sorted output, up to
-// kFinMax results, keys of at most 63 bits):
-//   phase 0  the exact stage on the escalated pairs (only when there are any:
-//            the count is final at launch, so every block decides alike);
-//   phase 1  one result per thread, or per two adjacent threads when the grid
-//            has threads enough (each then builds one of the two endpoints),
-//            results spread over all blocks: its key goes into its partition
-//            (the key's top kFinPartBits bits) at the slot one atomic on the
-//            partition's count returns, in a fixed bucket of kFinBucket slots
-//            or, beyond it, one overflow list; then its segments, whose count
-//            the partition's segment count gains;
-//   barrier  the block that arrives last scans the partition counts into key
-//            and segment offsets and lists the partitions over kFinBucket keys
-//            before it releases the others;
-//   phase 2  in a partition of up to kFinBucket keys, each result's thread
-//            ranks its key against the bucket (the keys are unique, so the rank
-//            is the number of smaller keys) and writes its pair, job and
-//            segments at their final positions; a larger partition is one
-//            block's (its bucket and its overflow entries, bitonic sort in
-//            shared memory).
-// Every wait is bounded.  Over kFinMax results (or more results than threads),
-// a partition over kFinBig keys or a full overflow list make the kernel refuse
-// (Counters::order_redo, decided alike in every block).  Launched as a
-// programmatic dependent of the traversal: it waits for the traversal's grid
-// (griddepcontrol.wait) before anything else.
+// Post-traversal work of a call in one launch (sorted output, up to kFinMax
+// results, keys of at most 63 bits).  The traversal has put every result's key
+// into its partition (fin_insert), so the partition counts are complete when
+// the launch begins and no block waits for another:
+//   phase 0  only when pairs were escalated: the exact stage, whose results join
+//            their partitions, and a grid barrier;
+//   phase 1  a block owns a run of consecutive sorted positions.  It scans all
+//            partition counts (16 KB, every block by itself: cheaper than a
+//            barrier), gathers the partitions that meet its run and ranks their
+//            keys (counting the smaller ones; a partition over kFinRank keys is
+//            sorted in shared memory);
+//   phase 2  two adjacent threads construct each result's two endpoints, and the
+//            run's pairs and segments go out in order, as whole lines, straight
+//            into the caller's pinned result block (device memory when the
+//            result outgrew it).  The last block copies the counters there too.
+// It is cooperative for the barrier of phase 0 and a programmatic dependent of
+// the traversal: it waits for that grid (griddepcontrol.wait) before anything
+// else.  The counters and partition counts of the next call are cleared here
+// (each call uses the other one of two sets), so a call needs no memset and no
+// device-to-host copy.  A call over kFinMax results or with a partition over
+// kFinBig keys is refused (Counters::order_redo, decided alike in every block).
+//
+// What bounds it: the FP64 issue of the constructions (about 1,400 instructions
+// an endpoint, one warp per SM sub-partition) and, for larger results, the PCIe
+// writes.  Its predecessor inserted the keys itself (a barrier, one block's scan,
+// a release; partitions over 32 keys searched a common overflow list) and five
+// copies followed it.  Launch to end: 868 results 14.5 -> 10.1 us, 12,245 results
+// clustered in index 33 -> 24 us with their 735 KB written to the host; the whole
+// call of two UV spheres of 1,216 triangles 81 -> 58 us, of two 1.3M-triangle
+// meshes 153 -> 115 us.
 // ===========================================================================
 constexpr int kFinThreads = 256;
-constexpr int kFinWarps = kFinThreads / 32;
-// dynamic shared memory: a big partition's keys and values, or (in the last
-// block of the key phase) the partition counts
-constexpr size_t kFinDyn = (sizeof(unsigned long long) + sizeof(uint32_t)) * kFinBig > 2 * sizeof(uint32_t) * kFinParts
-                               ? (sizeof(unsigned long long) + sizeof(uint32_t)) * kFinBig
-                               : 2 * sizeof(uint32_t) * kFinParts;
-static_assert(kFinParts % (32 * kFinWarps) == 0, "whole rows of 32 partitions per warp");
-static_assert(kFinBucket % 8 == 0, "a bucket is read 8 keys at a time");
+constexpr unsigned kFinRun = 256;   // most positions of a block (kFinMax over the smallest grid)
+constexpr unsigned kFinRank = 256;  // keys of a partition ranked by counting; larger ones are sorted
+constexpr unsigned kFinKeys = kFinRun + 2 * kFinBig;  // a run meets at most two partitions that it does not fill
+static_assert(kFinParts == 16 * kFinThreads, "a thread scans 16 partitions");
+static_assert(kFinRank == (unsigned)kFinBucket, "a partition has keys on the overflow list when, and only when, it is sorted");
 static_assert(kFinMax <= (1u << 30), "a bucket value holds the result index below bit 30");
 
-// One result at its final position: pair and job from the key, its segments
-// copied from the scratch, each segment's pair index set.
-__device__ __forceinline__ void fin_place(const OrderBufs& O, const FinArgs& F, unsigned long long key, unsigned idx,
-                                          unsigned pos, unsigned ns, unsigned so)
-{
-    // (positions stay inside the arrays even after a spent barrier wait)
-    if (pos >= F.cap || (size_t)so + ns > 3 * (size_t)F.cap) return;
-    const unsigned long long ma = (1ull << O.bits_a) - 1ull, mb = (1ull << O.bits_b) - 1ull;
-    F.pairs_out[2 * (size_t)pos] = (int32_t)((key >> O.bits_b) & ma);
-    F.pairs_out[2 * (size_t)pos + 1] = (int32_t)(key & mb);
-    F.job_out[pos] = (uint32_t)(key >> (O.bits_a + O.bits_b));
-    for (unsigned e = 0; e < ns; e++) {
-        const double2* sp = reinterpret_cast<const double2*>(F.segs + 18 * (size_t)idx + 6 * e);
-        double2* dp = reinterpret_cast<double2*>(F.segs_out + 6 * (size_t)(so + e));
-        dp[0] = __ldcg(sp);
-        dp[1] = __ldcg(sp + 1);
-        dp[2] = __ldcg(sp + 2);
-        F.segpair_out[so + e] = (int32_t)pos;
-    }
-}
+struct FinShared {
+    uint32_t koff[kFinParts + 4];  // key offsets of the partitions
+    uint32_t soff[kFinParts + 4];  // segments beyond one per key before them (only with odd results)
+    union {
+        struct {
+            unsigned long long key[kFinKeys];
+            uint32_t val[kFinKeys];
+        } g;                                  // gathered keys
+        double seg[kFinRun * 3 * 6];          // the run's segments, in order
+    } u;
+    unsigned long long skey[kFinRun];  // the run's keys in order, their values and segment offsets
+    uint32_t sval[kFinRun];
+    uint32_t sseg[kFinRun + 1];
+    uint32_t warp[2][kFinThreads / 32];
+    uint32_t big[32];
+    unsigned nbig, ok, last;
+};
 
 __device__ __forceinline__ void fin_stamp(Counters* C, int k)
 {
     if (blockIdx.x == 0 && threadIdx.x == 0) C->fin_ns[k] = globaltimer_ns();
 }
 
-// Block end: the last block to end stamps the launch's end.
-__device__ __forceinline__ void fin_end(Counters* C)
+// Block end: the last block to end stamps the launch's end and copies the
+// counters to the host.
+__device__ __forceinline__ void fin_end(Counters* C, Counters* host, FinShared& s)
 {
     __syncthreads();
-    if (threadIdx.x == 0 && atomicAdd(&C->fin_done, 1u) == gridDim.x - 1u) C->fin_ns[4] = globaltimer_ns();
+    if (threadIdx.x == 0) s.last = arrive_acq_rel(&C->fin_done) == gridDim.x - 1u ? 1u : 0u;
+    __syncthreads();
+    if (!s.last) return;
+    if (threadIdx.x == 0) C->fin_ns[4] = globaltimer_ns();
+    __syncthreads();
+    for (unsigned w = threadIdx.x; w < sizeof(Counters) / 4u; w += kFinThreads)
+        reinterpret_cast<unsigned*>(host)[w] = __ldcg(reinterpret_cast<const unsigned*>(C) + w);
 }
 
-// Layout of O.fin_off: key offsets (kFinParts + 1), segment offsets (kFinParts),
-// the number of big partitions, then their ids.
-constexpr int kFinSoff = kFinParts + 1;
-constexpr int kFinNbig = 2 * kFinParts + 1;
-constexpr int kFinBigIds = 2 * kFinParts + 2;
-
-// Run by the block that arrives last at the phase-1 barrier: the exclusive
-// scans of the partition key and segment counts into O.fin_off (one warp per
-// 512 partitions, 32 at a time, coalesced), the list of partitions over
-// kFinBucket keys, the counts cleared for the next call, and the refusal
-// decided.  Returns the refusal code (0: none).
-__device__ __forceinline__ unsigned fin_scan_counts(const OrderBufs& O, Counters* C, uint32_t* sw, unsigned* s_nbig,
-                                                    uint32_t* sk)
+// Exclusive scan of the partition counts c (16 per thread) into `out`; returns
+// the total.  big: some count is over kFinBig.
+__device__ __forceinline__ uint32_t fin_scan(const uint4 (&c)[4], uint32_t* out, uint32_t* warp)
 {
-    constexpr int kSeg = kFinParts / kFinWarps;  // partitions per warp
-    constexpr int kIt = kSeg / 32;
-    const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    uint32_t* const kcount = O.fin;
-    uint32_t* const scount = O.fin + kFinParts;
-    uint32_t* const koff = O.fin_off;
-    uint32_t* const soff = O.fin_off + kFinSoff;
-    const unsigned over = ld_cg_u32(&C->fin_over);
-    // all counts into shared memory first (every load in flight at once), then
-    // the scan reads them there
-    uint32_t* const ss = sk + kFinParts;
+    const unsigned tid = threadIdx.x, lane = tid & 31u, w = tid >> 5;
+    uint32_t v[16] = {c[0].x, c[0].y, c[0].z, c[0].w, c[1].x, c[1].y, c[1].z, c[1].w,
+                      c[2].x, c[2].y, c[2].z, c[2].w, c[3].x, c[3].y, c[3].z, c[3].w};
+    uint32_t sum = 0;
 #pragma unroll
-    for (int it = 0; it < kFinParts / kFinThreads; it++) {
-        const unsigned q = it * kFinThreads + tid;
-        sk[q] = __ldcg(kcount + q);
-        ss[q] = __ldcg(scount + q);
+    for (int q = 0; q < 16; q++) {
+        const uint32_t t = v[q];
+        v[q] = sum;
+        sum += t;
     }
+    uint32_t inc = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= (unsigned)o) inc += y;
+    }
+    if (lane == 31u) warp[w] = inc;
     __syncthreads();
-    const unsigned w0 = warp * kSeg;
-    uint32_t kc[kIt], sc[kIt];
+    uint32_t before = inc - sum, total = 0;
 #pragma unroll
-    for (int it = 0; it < kIt; it++) {
-        kc[it] = sk[w0 + 32 * it + lane];
-        sc[it] = ss[w0 + 32 * it + lane];
+    for (unsigned q = 0; q < kFinThreads / 32; q++) {
+        if (q < w) before += warp[q];
+        total += warp[q];
     }
-    uint32_t tk = 0, ts = 0;
-    bool too_big = false;
+    uint4* o4 = reinterpret_cast<uint4*>(out + 16 * tid);
 #pragma unroll
-    for (int it = 0; it < kIt; it++) {
-        tk += kc[it];
-        ts += sc[it];
-        too_big |= kc[it] > (uint32_t)kFinBig;
-    }
-    tk = __reduce_add_sync(0xffffffffu, tk);
-    ts = __reduce_add_sync(0xffffffffu, ts);
-    const bool any_big = __any_sync(0xffffffffu, too_big);
-    if (lane == 0) {
-        sw[warp] = tk;
-        sw[kFinWarps + warp] = ts;
-        sw[2 * kFinWarps + warp] = any_big ? 1u : 0u;
-    }
+    for (int q = 0; q < 4; q++)
+        o4[q] = make_uint4(before + v[4 * q], before + v[4 * q + 1], before + v[4 * q + 2], before + v[4 * q + 3]);
+    if (tid == 0) out[kFinParts] = total;
     __syncthreads();
-    unsigned kb = 0, sb = 0, ktot = 0, stot = 0, refuse = 0;
-#pragma unroll
-    for (int w = 0; w < kFinWarps; w++) {
-        const unsigned a = sw[w], b = sw[kFinWarps + w];
-        if ((unsigned)w < warp) {
-            kb += a;
-            sb += b;
-        }
-        ktot += a;
-        stot += b;
-        refuse |= sw[2 * kFinWarps + w];
-    }
-#pragma unroll
-    for (int it = 0; it < kIt; it++) {
-        const unsigned p = w0 + 32 * it + lane;
-        unsigned xk = kc[it], xs = sc[it];
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned yk = __shfl_up_sync(0xffffffffu, xk, o), ys = __shfl_up_sync(0xffffffffu, xs, o);
-            if (lane >= (unsigned)o) {
-                xk += yk;
-                xs += ys;
-            }
-        }
-        koff[p] = kb + xk - kc[it];
-        soff[p] = sb + xs - sc[it];
-        kb += __shfl_sync(0xffffffffu, xk, 31);
-        sb += __shfl_sync(0xffffffffu, xs, 31);
-        kcount[p] = 0u;
-        scount[p] = 0u;
-        if (kc[it] > (uint32_t)kFinBucket) {
-            const unsigned at = atomicAdd(s_nbig, 1u);
-            if (at < (unsigned)kFinParts) O.fin_off[kFinBigIds + at] = p;
-        }
-    }
-    __syncthreads();
-    if (tid == 0) {
-        koff[kFinParts] = ktot;
-        O.fin_off[kFinNbig] = *s_nbig;
-        C->nseg = stot;
-    }
-    if (refuse || over > (unsigned)kFinOverflow) return kRedoCrowded;
-    return 0u;
+    return total;
 }
 
-__global__ void __launch_bounds__(kFinThreads, 2) k_finish(Bufs B, OrderBufs O, FinArgs F)
+// The partition that holds sorted position x (koff[p] <= x < koff[p + 1]).
+__device__ __forceinline__ unsigned fin_part(const uint32_t* koff, unsigned x)
+{
+    unsigned lo = 0, hi = kFinParts;  // koff[lo] <= x < koff[hi]
+#pragma unroll
+    for (int k = 0; k < kFinPartBits; k++) {
+        const unsigned mid = (lo + hi) >> 1;
+        if (koff[mid] <= x) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+
+template <bool MULTI>
+__global__ void __launch_bounds__(kFinThreads, 2) k_finish(const __grid_constant__ Bufs B, const __grid_constant__ FinArgs F)
 {
     wait_prior_grid();  // the traversal's results are complete and visible
-    extern __shared__ unsigned long long fin_dyn[];  // a big partition: kFinBig keys, then kFinBig values
-    __shared__ uint32_t sw[33];
-    __shared__ unsigned s_ok, s_last, s_redo, s_fill, s_nbig;
+    extern __shared__ __align__(16) unsigned char fin_dyn[];
+    FinShared& s = *reinterpret_cast<FinShared*>(fin_dyn);
     Counters* C = B.cnt;
-    const unsigned tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const unsigned tid = threadIdx.x;
     const unsigned gtid = blockIdx.x * kFinThreads + tid, nth = gridDim.x * kFinThreads;
-    if (tid == 0) {
-        s_ok = 1u;
-        s_nbig = 0u;
-    }
+    if (tid == 0) s.ok = 1u;
     fin_stamp(C, 0);
+    // the next call's counters and partition counts
+    for (unsigned w = gtid; w < 2u * kFinParts / 4u; w += nth) reinterpret_cast<uint4*>(F.next_count)[w] = make_uint4(0u, 0u, 0u, 0u);
+    if (gtid < sizeof(Counters) / 8u) reinterpret_cast<unsigned long long*>(F.next_cnt)[gtid] = 0ull;
+    // everything the scan needs, at once; final unless pairs were escalated
+    const uint4* const count4 = reinterpret_cast<const uint4*>(B.fin.count) + 4 * tid;
+    uint4 c4[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) c4[q] = __ldcg(count4 + q);
+    unsigned n = ld_cg_u32(&C->res), over = ld_cg_u32(&C->fin_over);
+    const unsigned esc = ld_cg_u32(&C->esc);
     if (ld_cg_u32(&C->overflow)) {  // final at launch: the call reruns with larger buffers
-        fin_end(C);
+        fin_end(C, F.host_cnt, s);
         return;
     }
+    bool odd = false;
     // ---- phase 0: exact stage ----
-    if (ld_cg_u32(&C->esc)) {
-        exact_stage(B, gtid, nth);
-        grid_barrier(&C->obar, 1u, &C->err, &s_ok);
+    if (esc) {
+        exact_stage<MULTI>(B, gtid, nth);
+        grid_barrier(&C->obar, 1u, &C->err, &s.ok);
         if (ld_cg_u32(&C->overflow)) {  // read after the barrier: alike in every block
-            fin_end(C);
+            fin_end(C, F.host_cnt, s);
             return;
         }
+#pragma unroll
+        for (int q = 0; q < 4; q++) c4[q] = __ldcg(count4 + q);
+        n = ld_cg_u32(&C->res);
+        over = ld_cg_u32(&C->fin_over);
+        odd = ld_cg_u32(&C->odd) != 0u;
     }
     fin_stamp(C, 1);
-    const unsigned n = ld_cg_u32(&C->res);
-    if (n > kFinMax || n > nth) {  // one result per thread at most
+    if (n > kFinMax || n > kFinRun * gridDim.x) {
         if (blockIdx.x == 0 && tid == 0) C->order_redo = kRedoCount;
-        fin_end(C);
+        fin_end(C, F.host_cnt, s);
         return;
     }
-    // ---- phase 1: this thread's result: its key into its partition, its segments ----
-    // thread slots go to the warps of different blocks first (warp w of block b
-    // holds slots 32 (b + w G) ..), so that a small result spreads over every
-    // SM; when there are slots enough, two adjacent slots share a result (its
-    // two endpoints, FP64 work that one warp per SM sub-partition would issue
-    // too slowly), the first of them owning its key
-    const unsigned g = 32u * (blockIdx.x + gridDim.x * warp) + lane;
-    const unsigned per = 2u * n <= nth ? 2u : 1u;
-    const unsigned i = g / per, half = g % per;
-    const bool mine = i < n && half == 0u;
-    unsigned long long key = 0;
-    unsigned p = 0, ns = 0, slot = 0;
-    if (i < n) {
-        const uint4 rr = __ldcg(B.res + i);
-        if (mine) {
-            key = order_key(rr, O);
-            p = (unsigned)(key >> F.shift);
-            slot = atomicAdd(O.fin + p, 1u);  // waited for after the segments
-        }
-        if (F.want_segments) {
-            ns = code_segments(rr.w);
-            result_segments(B, rr, F.segs + 18 * (size_t)i, half, per);
-        }
+    // ---- phase 1: this block's run of sorted positions [lo, hi) ----
+    // runs of at least 16 results (one warp's, two lanes each)
+    const unsigned run = max(16u, (n + gridDim.x - 1u) / gridDim.x);
+    const unsigned lo = blockIdx.x * run, hi = min(n, lo + run);
+    if (lo >= n && blockIdx.x != 0u) {
+        fin_end(C, F.host_cnt, s);
+        return;
     }
-    if (mine) {
-        if (ns) atomicAdd(O.fin + kFinParts + p, ns);
-        const uint32_t v = i | (ns << 30);
+    unsigned most = 0;
+#pragma unroll
+    for (int q = 0; q < 4; q++) most = max(most, max(max(c4[q].x, c4[q].y), max(c4[q].z, c4[q].w)));
+    if (__syncthreads_or(most > (unsigned)kFinBig) || over > (unsigned)kFinOverflow) {
+        if (blockIdx.x == 0 && tid == 0) C->order_redo = kRedoCrowded;
+        fin_end(C, F.host_cnt, s);
+        return;
+    }
+    const uint32_t have = fin_scan(c4, s.koff, s.warp[0]);
+    uint32_t nseg = F.want_segments ? have : 0u;
+    if (odd) {
+        const uint4* const extra4 = reinterpret_cast<const uint4*>(B.fin.extra) + 4 * tid;
+        uint4 e4[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) e4[q] = __ldcg(extra4 + q);
+        nseg += fin_scan(e4, s.soff, s.warp[1]);
+    }
+    // into the caller's block where it fits, else into device memory
+    const bool fits = n <= F.host_pairs && nseg <= F.host_segs;
+    if (blockIdx.x == 0u && tid == 0) C->nseg = nseg;
+    if (lo >= n || have != n || (!fits && n > F.cap)) {  // no result; or (after a spent wait only) inconsistent counts
+        fin_end(C, F.host_cnt, s);
+        return;
+    }
+    const unsigned p0 = fin_part(s.koff, lo), p1 = fin_part(s.koff, hi - 1u) + 1u;
+    const unsigned base = s.koff[p0], m = min(s.koff[p1] - base, kFinKeys);
+    if (tid == 0) s.nbig = 0u;
+    bool spill = false;
+    for (unsigned t = tid; t < m; t += kFinThreads) {
+        const unsigned part = fin_part(s.koff, base + t), slot = base + t - s.koff[part];
         if (slot < (unsigned)kFinBucket) {
-            O.fin_bkey[p * kFinBucket + slot] = key;
-            O.fin_bval[p * kFinBucket + slot] = v;
+            s.u.g.key[t] = __ldcg(B.fin.bkey + part * kFinBucket + slot);
+            s.u.g.val[t] = __ldcg(B.fin.bval + part * kFinBucket + slot);
         } else {
-            const unsigned o = atomicAdd(&C->fin_over, 1u);
-            if (o < (unsigned)kFinOverflow) {
-                O.fin_okey[o] = key;
-                O.fin_oval[o] = v;
-            }
+            spill = true;
         }
     }
-    // ---- barrier: the last block to arrive scans the counts, then releases ----
-    __syncthreads();
-    if (tid == 0) s_last = arrive_acq_rel(&C->fbar) == gridDim.x - 1u ? 1u : 0u;
-    __syncthreads();
-    if (s_last) {
-        if (tid == 0) C->fin_ns[2] = globaltimer_ns();
-        const unsigned r = fin_scan_counts(O, C, sw, &s_nbig, reinterpret_cast<uint32_t*>(fin_dyn));
-        if (tid == 0) {
-            if (r) C->order_redo = r;
-            s_redo = r;
-            __threadfence();
-            st_release_u32(&C->frel, r ? 2u : 1u);
-        }
-    } else if (tid == 0) {
-        unsigned v = ld_acq(&C->frel);
-        unsigned long long spins = 0;
-        while (v == 0u) {
-            if (++spins > kLookbackSpins) {
-                atomicOr(&C->err, kErrTimeout);
-                v = 2u;
-                break;
-            }
-            __nanosleep(32);
-            v = ld_acq(&C->frel);
-        }
-        s_redo = v == 2u ? 1u : 0u;
-    }
-    __syncthreads();
-    if (s_redo) {
-        fin_end(C);
-        return;
-    }
-    fin_stamp(C, 3);
-    // ---- phase 2: each result ranks itself in its partition's bucket ----
-    const uint32_t* const koff = O.fin_off;
-    const uint32_t* const soff = O.fin_off + kFinSoff;
-    if (mine) {
-        // the offsets, the bucket's first 8 keys and the segments, all at once
-        const unsigned base = __ldcg(koff + p), end = __ldcg(koff + p + 1), so = __ldcg(soff + p);
-        const ulonglong2* bk2 = reinterpret_cast<const ulonglong2*>(O.fin_bkey + p * kFinBucket);
-        const uint4* bv4 = reinterpret_cast<const uint4*>(O.fin_bval + p * kFinBucket);
-        ulonglong2 k2[4];
-        uint4 v4[2];
-#pragma unroll
-        for (int q = 0; q < 4; q++) k2[q] = __ldcg(bk2 + q);
-        v4[0] = __ldcg(bv4);
-        v4[1] = __ldcg(bv4 + 1);
-        double2 sg[9];
-#pragma unroll
-        for (int e = 0; e < 9; e++)
-            if (e < 3 * (int)ns) sg[e] = __ldcg(reinterpret_cast<const double2*>(F.segs + 18 * (size_t)i) + e);
-        const unsigned m = end - base;
-        if (m <= (unsigned)kFinBucket) {
-            unsigned rank = 0, pre = 0;
-            const unsigned long long kk[8] = {k2[0].x, k2[0].y, k2[1].x, k2[1].y, k2[2].x, k2[2].y, k2[3].x, k2[3].y};
-            const uint32_t vv[8] = {v4[0].x, v4[0].y, v4[0].z, v4[0].w, v4[1].x, v4[1].y, v4[1].z, v4[1].w};
-#pragma unroll
-            for (int j = 0; j < 8; j++)
-                if ((unsigned)j < m && kk[j] < key) {
-                    rank++;
-                    pre += vv[j] >> 30;
-                }
-            for (unsigned j = 8; j < m; j++) {
-                const unsigned long long kj = __ldcg(O.fin_bkey + p * kFinBucket + j);
-                if (kj < key) {
-                    rank++;
-                    pre += __ldcg(O.fin_bval + p * kFinBucket + j) >> 30;
+    if (__syncthreads_or(spill)) {
+        // keys beyond a bucket: found on the overflow list, their slots with them
+        for (unsigned t = tid; t < over; t += kFinThreads) {
+            const unsigned long long key = __ldcg(B.fin.okey + t);
+            const unsigned part = (unsigned)(key >> B.fin.shift);
+            if (part >= p0 && part < p1) {
+                const uint2 v = __ldcg(B.fin.oval + t);
+                const unsigned at = s.koff[part] - base + v.y;
+                if (at < m) {
+                    s.u.g.key[at] = key;
+                    s.u.g.val[at] = v.x;
                 }
             }
-            const unsigned pos = base + rank, s0 = so + pre;
-            if (pos < F.cap && (size_t)s0 + ns <= 3 * (size_t)F.cap) {
-                const unsigned long long ma = (1ull << O.bits_a) - 1ull, mb = (1ull << O.bits_b) - 1ull;
-                F.pairs_out[2 * (size_t)pos] = (int32_t)((key >> O.bits_b) & ma);
-                F.pairs_out[2 * (size_t)pos + 1] = (int32_t)(key & mb);
-                F.job_out[pos] = (uint32_t)(key >> (O.bits_a + O.bits_b));
-                double2* dp = reinterpret_cast<double2*>(F.segs_out + 6 * (size_t)s0);
-#pragma unroll
-                for (int e = 0; e < 9; e++)
-                    if (e < 3 * (int)ns) dp[e] = sg[e];
-                for (unsigned e = 0; e < ns; e++) F.segpair_out[s0 + e] = (int32_t)pos;
+        }
+        for (unsigned part = p0 + tid; part < p1; part += kFinThreads)
+            if (s.koff[part + 1u] - s.koff[part] > kFinRank) {
+                const unsigned at = atomicAdd(&s.nbig, 1u);
+                if (at < 32u) s.big[at] = part;
             }
-        }
-    }
-    // partitions over kFinBucket keys (listed by the scan): one block each,
-    // whose threads gather its bucket and its overflow entries into shared
-    // memory and sort them there (bitonic)
-    const unsigned nbig = min(__ldcg(O.fin_off + kFinNbig), (unsigned)kFinParts);
-    unsigned long long* bk = fin_dyn;
-    uint32_t* bv = reinterpret_cast<uint32_t*>(fin_dyn + kFinBig);
-    for (unsigned q = blockIdx.x; q < nbig; q += gridDim.x) {
-        const unsigned pb = __ldcg(O.fin_off + kFinBigIds + q);
-        if (pb >= (unsigned)kFinParts) continue;  // block-uniform
-        const unsigned base = __ldcg(koff + pb), m = __ldcg(koff + pb + 1) - base;
-        if (m <= (unsigned)kFinBucket || m > (unsigned)kFinBig) continue;
-        unsigned mp = 2u * kFinBucket;
-        while (mp < m) mp <<= 1;
-        __syncthreads();  // the previous partition's reads are done
-        for (unsigned t = tid; t < mp; t += kFinThreads) {
-            bk[t] = ~0ull;  // padding sorts last
-            bv[t] = 0u;
-        }
-        if (tid == 0) s_fill = kFinBucket;
         __syncthreads();
-        if (tid < (unsigned)kFinBucket) {
-            bk[tid] = __ldcg(O.fin_bkey + pb * kFinBucket + tid);
-            bv[tid] = __ldcg(O.fin_bval + pb * kFinBucket + tid);
-        }
-        const unsigned nover = min(ld_cg_u32(&C->fin_over), (unsigned)kFinOverflow);
-        for (unsigned t = tid; t < nover; t += kFinThreads) {
-            const unsigned long long kt = __ldcg(O.fin_okey + t);
-            if ((unsigned)(kt >> F.shift) == pb) {
-                const unsigned at = atomicAdd(&s_fill, 1u);
-                if (at < mp) {
-                    bk[at] = kt;
-                    bv[at] = __ldcg(O.fin_oval + t);
-                }
-            }
-        }
-        __syncthreads();
-        for (unsigned k = 2; k <= mp; k <<= 1)
-            for (unsigned j = k >> 1; j > 0; j >>= 1) {
-                for (unsigned t = tid; t < mp; t += kFinThreads) {
-                    const unsigned u = t ^ j;
-                    if (u > t) {
-                        const unsigned long long x = bk[t], y = bk[u];
-                        if ((x > y) == ((t & k) == 0u)) {
-                            bk[t] = y;
-                            bk[u] = x;
-                            const uint32_t w = bv[t];
-                            bv[t] = bv[u];
-                            bv[u] = w;
+        const unsigned nbig = min(s.nbig, 32u);
+        for (unsigned q = 0; q < nbig; q++) {
+            // bitonic sort of one partition, every comparison ascending (the first
+            // step of a merge mirrors), so keys past its end need not exist
+            const unsigned part = s.big[q], off = s.koff[part] - base;
+            const unsigned c = min(s.koff[part + 1u] - s.koff[part], m - off);
+            unsigned long long* const kk = s.u.g.key + off;
+            uint32_t* const vv = s.u.g.val + off;
+            unsigned pow = 1;
+            while (pow < c) pow <<= 1;
+            for (unsigned w = 2; w <= pow; w <<= 1)
+                for (unsigned j = w >> 1; j > 0; j >>= 1) {
+                    for (unsigned t = tid; t < pow; t += kFinThreads) {
+                        const unsigned u = j == (w >> 1) ? (t ^ (w - 1u)) : (t ^ j);
+                        if (u > t && u < c && kk[t] > kk[u]) {
+                            const unsigned long long x = kk[t];
+                            kk[t] = kk[u];
+                            kk[u] = x;
+                            const uint32_t y = vv[t];
+                            vv[t] = vv[u];
+                            vv[u] = y;
                         }
                     }
+                    __syncthreads();
                 }
-                __syncthreads();
-            }
-        unsigned run = __ldcg(soff + pb);
-        for (unsigned c0 = 0; c0 < m; c0 += kFinThreads) {
-            const unsigned k = c0 + tid;
-            const bool have = k < m;
-            const uint32_t v = have ? bv[k] : 0u;
-            const unsigned nsk = v >> 30;
-            unsigned idx = v & ((1u << 30) - 1u);
-            if (idx >= n) idx = 0u;
-            unsigned tot;
-            const unsigned ex = block_exclusive_scan(nsk, sw, &tot);
-            if (have) fin_place(O, F, bk[k], idx, base + k, nsk, run + ex);
-            run += tot;
         }
     }
-    fin_end(C);
+    // ranks: the keys of the run to their places
+    for (unsigned t = tid; t < m; t += kFinThreads) {
+        const unsigned part = fin_part(s.koff, base + t), off = s.koff[part] - base;
+        const unsigned c = min(s.koff[part + 1u] - s.koff[part], m - off);
+        const unsigned long long key = s.u.g.key[t];
+        const uint32_t val = s.u.g.val[t];
+        unsigned rank = 0, pre = 0;
+        if (c > kFinRank) {  // sorted above
+            rank = t - off;
+            if (odd)
+                for (unsigned q = 0; q < rank; q++) pre += s.u.g.val[off + q] >> 30;
+        } else if (odd) {
+            for (unsigned q = 0; q < c; q++)
+                if (s.u.g.key[off + q] < key) {
+                    rank++;
+                    pre += s.u.g.val[off + q] >> 30;
+                }
+        } else {
+            for (unsigned q = 0; q < c; q++) rank += s.u.g.key[off + q] < key ? 1u : 0u;
+        }
+        const unsigned pos = base + off + rank;
+        if (pos >= lo && pos < hi) {
+            s.skey[pos - lo] = key;
+            s.sval[pos - lo] = val;
+            s.sseg[pos - lo] = odd ? s.koff[part] + s.soff[part] + pre : pos;
+        }
+    }
+    __syncthreads();  // the gathered keys are done with: their place takes the segments
+    fin_stamp(C, 2);
+    // ---- phase 2: constructions, and the run out in order ----
+    const unsigned cnt = hi - lo, s0 = s.sseg[0];
+    const unsigned idx_mask = (1u << 30) - 1u;
+    int32_t* const pairs = fits ? F.h_pairs : F.pairs_out;
+    {
+        const unsigned long long ma = (1ull << B.fin.bits_a) - 1ull, mb = (1ull << B.fin.bits_b) - 1ull;
+        for (unsigned j = tid; j < cnt; j += kFinThreads) {
+            const unsigned long long key = s.skey[j];
+            reinterpret_cast<int2*>(pairs)[lo + j] = make_int2((int)((key >> B.fin.bits_b) & ma), (int)(key & mb));
+            if constexpr (MULTI) (fits ? F.h_job : F.job_out)[lo + j] = (uint32_t)(key >> (B.fin.bits_a + B.fin.bits_b));
+        }
+    }
+    if (F.want_segments) {
+        int32_t* const segpair = fits ? F.h_segpair : F.segpair_out;
+        for (unsigned j = tid >> 1; j < cnt; j += kFinThreads / 2) {
+            const uint32_t v = s.sval[j], ns = v >> 30;
+            const unsigned so = s.sseg[j];
+            if (!ns) continue;
+            const uint4 rr = __ldcg(B.res + (v & idx_mask));
+            result_segments<MULTI>(B, rr, s.u.seg + 6u * (so - s0), tid & 1u, 2u);
+            for (unsigned e = tid & 1u; e < ns; e += 2u) segpair[so + e] = (int32_t)(lo + j);
+        }
+        __syncthreads();
+        const unsigned s1 = s.sseg[cnt - 1u] + (s.sval[cnt - 1u] >> 30);
+        double2* const out = reinterpret_cast<double2*>((fits ? F.h_segs : F.segs_out) + 6 * (size_t)s0);
+        const double2* const in = reinterpret_cast<const double2*>(s.u.seg);
+        for (unsigned t = tid; t < 3u * (s1 - s0); t += kFinThreads) out[t] = in[t];
+    }
+    fin_stamp(C, 3);
+    fin_end(C, F.host_cnt, s);
 }
 
-cudaError_t launch_finish(const Bufs& b, const OrderBufs& O, const FinArgs& F, const LaunchCfg& cfg, cudaStream_t st,
-                          bool dependent)
+// Layout of the partition memory: two sets of counts (keys, extra segments),
+// then the buckets and the overflow list, which both sets share (a call's are
+// done with when the next begins).
+size_t fin_scratch_bytes()
 {
-    Bufs bb = b;
-    OrderBufs oo = O;
-    FinArgs ff = F;
+    return sizeof(uint32_t) * 4 * kFinParts + (sizeof(unsigned long long) + sizeof(uint32_t)) * (size_t)kFinParts * kFinBucket +
+           (sizeof(unsigned long long) + sizeof(uint2)) * kFinOverflow;
+}
+uint32_t* fin_counts(void* mem, int set)
+{
+    return (uint32_t*)mem + (size_t)set * 2 * kFinParts;
+}
+FinBufs make_fin_bufs(void* mem, int set, int bits_a, int bits_b, int bits_job)
+{
+    FinBufs f;
+    f.count = fin_counts(mem, set);
+    f.extra = f.count + kFinParts;
+    f.bkey = (unsigned long long*)((uint32_t*)mem + 4 * kFinParts);
+    f.okey = f.bkey + (size_t)kFinParts * kFinBucket;
+    f.oval = (uint2*)(f.okey + kFinOverflow);
+    f.bval = (uint32_t*)(f.oval + kFinOverflow);
+    const int bits = bits_a + bits_b + bits_job;
+    f.shift = bits > kFinPartBits ? bits - kFinPartBits : 0;
+    f.bits_a = bits_a;
+    f.bits_b = bits_b;
+    f.on = f.segments = 0;
+    return f;
+}
+
+cudaError_t launch_finish(const Bufs& b, const FinArgs& F, const LaunchCfg& cfg, cudaStream_t st)
+{
     note_launches(1);
-    if (dependent) {
-        // cooperative, and a programmatic dependent of the traversal launched
-        // just before it on the stream: its launch overlaps the traversal's end
-        cudaLaunchConfig_t lc = {};
-        lc.gridDim = dim3(cfg.fin_per_sm * cfg.sms);
-        lc.blockDim = dim3(kFinThreads);
-        lc.dynamicSmemBytes = kFinDyn;
-        lc.stream = st;
-        cudaLaunchAttribute at[2];
-        at[0].id = cudaLaunchAttributeCooperative;
-        at[0].val.cooperative = 1;
-        at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at[1].val.programmaticStreamSerializationAllowed = 1;
-        lc.attrs = at;
-        lc.numAttrs = 2;
-        const cudaError_t e = cudaLaunchKernelEx(&lc, k_finish, bb, oo, ff);
-        if (e == cudaSuccess) return e;
-        (void)cudaGetLastError();  // refused: launch it the plain cooperative way
-    }
-    void* args[] = {&bb, &oo, &ff};
-    return cudaLaunchCooperativeKernel((const void*)k_finish, dim3(cfg.fin_per_sm * cfg.sms), dim3(kFinThreads), args,
-                                      kFinDyn, st);
+    const void* kern = b.njobs > 1 ? (const void*)k_finish<true> : (const void*)k_finish<false>;
+    Bufs bb = b;
+    FinArgs ff = F;
+    void* args[] = {&bb, &ff};
+    // cooperative, and a programmatic dependent of the traversal launched just
+    // before it on the stream: its launch overlaps the traversal's end
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(cfg.fin_per_sm * cfg.sms);
+    lc.blockDim = dim3(kFinThreads);
+    lc.dynamicSmemBytes = sizeof(FinShared);
+    lc.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = at;
+    lc.numAttrs = 2;
+    const cudaError_t e = cudaLaunchKernelExC(&lc, kern, args);
+    if (e == cudaSuccess) return e;
+    (void)cudaGetLastError();  // refused: launch it the plain cooperative way
+    return cudaLaunchCooperativeKernel(kern, lc.gridDim, lc.blockDim, args, lc.dynamicSmemBytes, st);
 }
 
 // ===========================================================================
@@ -2696,8 +2686,12 @@ cudaError_t query_launch(int device, LaunchCfg* cfg)
         }
     for (int a = 0; a < 2; a++)
         for (int m = 0; m < 2; m++) cfg->blocks_per_sm[a][m] = nr[a][m] < 1 ? 1 : nr[a][m];
-    int nf = 0;
-    GI_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nf, k_finish, kFinThreads, kFinDyn));
+    int nf = 0, nm = 0;
+    GI_TRY(cudaFuncSetAttribute(k_finish<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FinShared)));
+    GI_TRY(cudaFuncSetAttribute(k_finish<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FinShared)));
+    GI_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nf, k_finish<false>, kFinThreads, sizeof(FinShared)));
+    GI_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nm, k_finish<true>, kFinThreads, sizeof(FinShared)));
+    nf = nf < nm ? nf : nm;
     cfg->fin_per_sm = nf < 1 ? 1 : (nf > 2 ? 2 : nf);
     return cudaSuccess;
 }

@@ -92,14 +92,6 @@ struct OrderBufs {
     uint32_t* base;      // kOsMaxPasses x 256
     uint32_t* tile_ctr;  // kOsMaxPasses + 2 (per pass, the gather, the histogram blocks)
     uint32_t* tile_tot;  // kOrderSmallBlocks: segment totals per run (small-count path)
-    // one-launch finish (k_finish)
-    uint32_t* fin;       // 2 x kFinParts: keys and segments per partition (zero between calls)
-    uint32_t* fin_off;   // kFinParts + 1 key offsets, kFinParts segment offsets, the number of
-                         // partitions over kFinBucket keys, their ids (kFinParts at most)
-    unsigned long long* fin_bkey;  // kFinParts x kFinBucket: each partition's first keys
-    uint32_t* fin_bval;            // ... and their result index | segment count << 30
-    unsigned long long* fin_okey;  // kFinOverflow: the keys beyond a bucket
-    uint32_t* fin_oval;
     uint32_t ntiles_cap;
     int passes;
     int bits_a, bits_b;
@@ -127,33 +119,38 @@ constexpr unsigned kOrderRank = 1u, kOrderPlace = 2u;
 cudaError_t launch_order_small_phases(const Bufs& b, const OrderBufs& O, bool sort, const double* segs,
                                       const uint32_t* nseg, int32_t* pairs_out, uint32_t* job_out, double* segs_out,
                                       int32_t* segpair_out, bool want_segments, unsigned phases, cudaStream_t st);
-// Everything after the traversal in one cooperative launch, for sorted output
-// of up to kFinMax results with keys of at most 63 bits: the exact stage (when
-// pairs were escalated), the segments, and the ordering by partitions of the
-// key's top kFinPartBits bits (one warp ranks a partition of up to kFinBucket
-// keys, one block a larger one, up to kFinBig).  A call over those limits
-// makes the kernel set only Counters::order_redo; the caller then reruns on
-// the general path (launch_exact, launch_segments, launch_order_gather).
-constexpr int kFinPartBits = 12;
-constexpr int kFinParts = 1 << kFinPartBits;
-constexpr int kFinBucket = 32;
-constexpr int kFinOverflow = 1 << 14;
+// Everything after the traversal in one launch, for sorted output of up to
+// kFinMax results with keys of at most 63 bits: the exact stage (when pairs were
+// escalated), the segments, and the ordering by partitions of the key's top
+// kFinPartBits bits.  A call over those limits, or with a partition over kFinBig
+// keys, makes the kernel set only Counters::order_redo; the caller then reruns
+// on the general path (launch_exact, launch_segments, launch_order_gather).
 constexpr int kFinBig = 2048;
 constexpr uint32_t kFinMax = 1u << 16;
 struct FinArgs {
-    double* segs;       // per result: up to 3 segments (scratch)
+    // results in pinned host memory: for host_pairs pairs and host_segs segments
+    int32_t* h_pairs;
+    uint32_t* h_job;  // batches only
+    double* h_segs;
+    int32_t* h_segpair;
+    uint32_t host_pairs, host_segs;
+    // ... or, when they do not fit, in device memory (cap pairs, 3 segments each)
     int32_t* pairs_out;
     uint32_t* job_out;
     double* segs_out;
     int32_t* segpair_out;
-    uint32_t cap;       // results the output arrays hold (segments: 3 per result)
+    uint32_t cap;
     int want_segments;
-    int shift;          // partition of a key = key >> shift
+    Counters* host_cnt;    // pinned: the counters when the launch ends
+    Counters* next_cnt;    // cleared for the next call
+    uint32_t* next_count;  // 2 x kFinParts, cleared for the next call
 };
-// dependent: launched right after the traversal on the same stream, with no
-// other stream work between them (programmatic dependent launch)
-cudaError_t launch_finish(const Bufs& b, const OrderBufs& O, const FinArgs& F, const LaunchCfg& cfg, cudaStream_t st,
-                          bool dependent = false);
+size_t fin_scratch_bytes();
+uint32_t* fin_counts(void* mem, int set);
+FinBufs make_fin_bufs(void* mem, int set, int bits_a, int bits_b, int bits_job);
+// Launched right after the traversal on the same stream, with no other stream
+// work between them (programmatic dependent launch).
+cudaError_t launch_finish(const Bufs& b, const FinArgs& F, const LaunchCfg& cfg, cudaStream_t st);
 
 // Number of kernels launched by the launchers of this library (monotonic).
 unsigned long long launch_count();

@@ -143,7 +143,8 @@ typedef struct {
     double ms_sort;                   /* device time: output ordering (the part after segment construction
                                          ends; ranking overlaps the segments).  With the one-launch
                                          finish (finish_phases = 4), ms_exact, ms_segments and ms_sort
-                                         are its phases' own spans (its timestamps) and ms_traverse the
+                                         are its phases' own spans (its timestamps; ms_segments includes
+                                         the writing of the results to the host) and ms_traverse the
                                          rest of the call, the hand-off between the launches included */
     double ms_total;                  /* device time of the whole call */
     /* kept for the layout: level_times is 0 (the traversal has no common levels) */
@@ -152,9 +153,8 @@ typedef struct {
     double level_end_ms[32];
     /* one-launch finish after the traversal (sorted output of a small result;
      * else finish_phases = 0): finish_ms[k] is the time from the launch's start
-     * to the end of its exact phase (k = 0), of its key and segment phase (1:
-     * the last block's arrival), of the count scan (2: the release of the
-     * others), and of its last block (3) */
+     * to the end of its exact phase (k = 0), until its first block had its
+     * results ranked (1) and written (2), and to the end of its last block (3) */
     uint32_t finish_phases;
     uint32_t reserved3;
     double finish_ms[4];
