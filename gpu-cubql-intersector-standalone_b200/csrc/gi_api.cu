@@ -109,6 +109,7 @@ extern "C" gi_status gi_create(const gi_options* opts, gi_ctx** out)
     if (e == cudaSuccess) e = query_launch(c->device, &c->cfg);
     if (e == cudaSuccess) e = cudaMalloc(&c->d_cnt, 2 * sizeof(Counters));
     if (e == cudaSuccess) e = cudaMallocHost(&c->h_cnt, sizeof(Counters));
+    if (e == cudaSuccess) e = cudaMallocHost(&c->h_words, 64);
     for (int i = 0; i < 8 && e == cudaSuccess; i++) e = cudaEventCreate(&c->ev[i]);
     if (e != cudaSuccess) {
         gi_destroy(c);
@@ -137,6 +138,7 @@ extern "C" gi_status gi_destroy(gi_ctx* c)
     if (c->st) cudaStreamSynchronize(c->st);
     if (c->pool) cudaMemPoolDestroy(c->pool);
     if (c->h_cnt) cudaFreeHost(c->h_cnt);
+    if (c->h_words) cudaFreeHost(c->h_words);
     if (c->h_jobs) cudaFreeHost(c->h_jobs);
     for (auto& e : c->ev)
         if (e) cudaEventDestroy(e);

@@ -285,6 +285,7 @@ struct gi_ctx {
     bool cur_clear = false;     // set `cur` is zero
     void* fin_mem = nullptr;    // partitions of the one-launch finish (gi::FinBufs)
     Counters* h_cnt = nullptr;  // pinned
+    unsigned* h_words = nullptr;  // pinned: error words of a pair-list call
     JobDev* d_jobs = nullptr;
     JobDev* h_jobs = nullptr;  // pinned
     uint32_t cap_jobs = 0;

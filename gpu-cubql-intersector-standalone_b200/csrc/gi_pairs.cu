@@ -7,6 +7,8 @@
 // gi_classify_pairs does the same job on the device only: the first filter
 // stage decides the general-position pairs, the rest are collected in a
 // scratch list and decided exactly (FP64 filter, then integer arithmetic).
+#include <algorithm>
+
 #include "gi_classify.cuh"
 #include "gi_host.h"
 
@@ -32,16 +34,33 @@ __device__ __forceinline__ void pairs_load_tri(const MeshDev& M, const DevPose& 
     out[2] = world_vertex(M.verts, __ldg(t + 2), P);
 }
 
+// A pair that the FP32 filter escalated, asked of its FP64 form (which leaves the
+// integers only pairs out of general position); out of line, as few need it.
+static __device__ __noinline__ int pairs_again64(const JobDev& J, uint32_t a, uint32_t b)
+{
+    double3 P[3], Q[3];
+    pairs_load_tri(J.A, J.pa, a, P);
+    pairs_load_tri(J.B, J.pb, b, Q);
+    return classify_fast<double>(P, Q);
+}
+
 // scratch layout: [0] escalation count, [1] error bits, [64 ..) escalated pair indices
 constexpr unsigned kPairsScratchHead = 64;
 
+// A candidate pair per thread.  Bound by the gathers' sectors and the FP64 pipe
+// and conversions of the posed vertices together (each near half busy); 64
+// registers (FP32 form) for four blocks per SM.  1.2 M pairs with a few escalated:
+// 59.6 -> 48.4 us a call, since the FP64 filter decides those in place (the exact
+// launch took 10 us for them), the exact launch is a programmatic dependent and
+// the error words need no copy.
 template <bool F64>
-__global__ void __launch_bounds__(256) k_pairs_filter(JobDev J, const int32_t* __restrict__ pairs, uint32_t n,
+__global__ void __launch_bounds__(256, F64 ? 3 : 4) k_pairs_filter(const __grid_constant__ JobDev J, const int32_t* __restrict__ pairs, uint32_t n,
                                                       uint8_t* __restrict__ out, unsigned* __restrict__ scratch)
 {
     const unsigned lane = threadIdx.x & 31;
     const unsigned warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const unsigned nwarps = (gridDim.x * blockDim.x) >> 5;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     for (unsigned base = warp * 32; base < n; base += nwarps * 32) {
         const unsigned i = base + lane;
         int dec = DEC_NO;
@@ -56,6 +75,7 @@ __global__ void __launch_bounds__(256) k_pairs_filter(JobDev J, const int32_t* _
                 pairs_load_tri(J.B, J.pb, (uint32_t)b, Q);
                 if constexpr (F64) dec = classify_fast<double>(P, Q);
                 else dec = classify_fast<float>(P, Q);
+                if (!F64 && dec == DEC_ESC) dec = pairs_again64(J, (uint32_t)a, (uint32_t)b);
                 out[i] = dec == DEC_YES ? 1 : 0;
             }
         }
@@ -65,43 +85,62 @@ __global__ void __launch_bounds__(256) k_pairs_filter(JobDev J, const int32_t* _
     }
 }
 
-__global__ void __launch_bounds__(128) k_pairs_exact(JobDev J, const int32_t* __restrict__ pairs,
+// The pairs that both filters left, exactly.  A programmatic dependent of the
+// filter.  host_err[0] receives the filter's error bits, host_err[1] the exact
+// arithmetic's (pinned host words, zero before the call), so no copy follows.
+__global__ void __launch_bounds__(128) k_pairs_exact(const __grid_constant__ JobDev J, const int32_t* __restrict__ pairs,
                                                      uint8_t* __restrict__ out, unsigned* __restrict__ scratch,
-                                                     bool fp32)
+                                                     volatile unsigned* host_err)
 {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const unsigned gtid = blockIdx.x * blockDim.x + threadIdx.x;
+    if (gtid == 0) host_err[0] = __ldcg(&scratch[1]) & 4u;
     const unsigned nesc = __ldcg(&scratch[0]);
-    for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < nesc; k += gridDim.x * blockDim.x) {
+    for (unsigned k = gtid; k < nesc; k += gridDim.x * blockDim.x) {
         const unsigned i = __ldcg(&scratch[kPairsScratchHead + k]);
         double3 pts[6];
         pairs_load_tri(J.A, J.pa, (uint32_t)pairs[2 * (size_t)i], pts);
         pairs_load_tri(J.B, J.pb, (uint32_t)pairs[2 * (size_t)i + 1], pts + 3);
-        ExactSigns S{&scratch[1], 0ull};
-        unsigned code;
-        out[i] = decide_escalated(pts, fp32, &code, S) ? 1 : 0;
+        unsigned err = 0, code;
+        ExactSigns S{&err, 0ull};
+        out[i] = decide_escalated(pts, false, &code, S) ? 1 : 0;
+        if (err) host_err[1] = err;
     }
 }
 
-// Runs the cascade with `scratch` (kPairsScratchHead + n words, zeroed head)
-// on stream st; returns the error bits through the host copy.
+// Runs the cascade with `scratch` (kPairsScratchHead + n words) on stream st;
+// returns the error bits through two pinned host words.
 static cudaError_t run_pairs(const JobDev& J, const int32_t* d_pairs, uint32_t n, int precision, uint8_t* d_out,
-                             unsigned* scratch, int sms, cudaStream_t st, unsigned* h_err)
+                             unsigned* scratch, int sms, cudaStream_t st, unsigned* pinned, unsigned* h_err)
 {
+    volatile unsigned* const host = pinned;
+    host[0] = host[1] = 0u;
+    *h_err = 0u;
+    if (!n) return cudaStreamSynchronize(st);
     cudaError_t e = cudaMemsetAsync(scratch, 0, sizeof(unsigned) * 2, st);
     if (e != cudaSuccess) return e;
-    if (n) {
-        unsigned blocks = (n + 255) / 256;
-        unsigned maxb = (unsigned)sms * 8;
-        if (blocks > maxb) blocks = maxb;
-        if (precision == GI_PREC_FP64) k_pairs_filter<true><<<blocks, 256, 0, st>>>(J, d_pairs, n, d_out, scratch);
-        else k_pairs_filter<false><<<blocks, 256, 0, st>>>(J, d_pairs, n, d_out, scratch);
-        k_pairs_exact<<<sms * 4, 128, 0, st>>>(J, d_pairs, d_out, scratch, precision != GI_PREC_FP64);
-        note_launches(2);
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-    }
-    e = cudaMemcpyAsync(h_err, scratch + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
+    unsigned blocks = (n + 255) / 256;
+    unsigned maxb = (unsigned)sms * 8;
+    if (blocks > maxb) blocks = maxb;
+    if (precision == GI_PREC_FP64) k_pairs_filter<true><<<blocks, 256, 0, st>>>(J, d_pairs, n, d_out, scratch);
+    else k_pairs_filter<false><<<blocks, 256, 0, st>>>(J, d_pairs, n, d_out, scratch);
+    e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    return cudaStreamSynchronize(st);
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3(std::min((n + 127u) / 128u, (unsigned)sms * 4u));
+    lc.blockDim = dim3(128);
+    lc.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    e = cudaLaunchKernelEx(&lc, k_pairs_exact, J, d_pairs, d_out, scratch, (volatile unsigned*)pinned);
+    if (e != cudaSuccess) return e;
+    note_launches(2);
+    e = cudaStreamSynchronize(st);
+    *h_err = host[0] | host[1];
+    return e;
 }
 
 static gi_status pairs_job(gi_ctx* c, const gi_mesh* A, const gi_pose* pa, const gi_mesh* B, const gi_pose* pb,
@@ -146,7 +185,7 @@ extern "C" gi_status gi_classify_pairs(gi_ctx* c, const gi_mesh* A, const gi_pos
     cudaError_t e = pool_alloc(&scratch, sizeof(unsigned) * (kPairsScratchHead + (size_t)npairs), c->pool, c->st);
     if (e != cudaSuccess) return set_err(c, GI_ERR_OOM, "classify pairs scratch", e);
     unsigned herr = 0;
-    e = run_pairs(J, d_pairs, npairs, precision_mode, d_out, scratch, c->cfg.sms, c->st, &herr);
+    e = run_pairs(J, d_pairs, npairs, precision_mode, d_out, scratch, c->cfg.sms, c->st, c->h_words, &herr);
     cudaFreeAsync(scratch, c->st);
     return pairs_status(c, e, herr);
 }
@@ -217,6 +256,6 @@ extern "C" gi_status gi_classify_pairs_noalloc(gi_ctx* c, const gi_mesh* A, cons
     s = noalloc_scratch(c, &scratch);
     if (s != GI_OK) return s;
     unsigned herr = 0;
-    e = run_pairs(J, d_pairs, npairs, precision_mode, d_out, scratch, c->cfg.sms, c->st, &herr);
+    e = run_pairs(J, d_pairs, npairs, precision_mode, d_out, scratch, c->cfg.sms, c->st, c->h_words, &herr);
     return pairs_status(c, e, herr);
 }
