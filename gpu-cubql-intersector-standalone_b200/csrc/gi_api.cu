@@ -110,6 +110,8 @@ extern "C" gi_status gi_create(const gi_options* opts, gi_ctx** out)
     if (e == cudaSuccess) e = cudaMalloc(&c->d_cnt, 2 * sizeof(Counters));
     if (e == cudaSuccess) e = cudaMallocHost(&c->h_cnt, sizeof(Counters));
     if (e == cudaSuccess) e = cudaMallocHost(&c->h_words, 64);
+    if (e == cudaSuccess) e = cudaMallocHost(&c->h_build, sizeof(unsigned) * 2 * kBuildWords);
+    for (int i = 0; i < 4 && e == cudaSuccess; i++) e = cudaEventCreate(&c->ev_build[i / 2][i % 2]);
     for (int i = 0; i < 8 && e == cudaSuccess; i++) e = cudaEventCreate(&c->ev[i]);
     if (e != cudaSuccess) {
         gi_destroy(c);
@@ -139,6 +141,10 @@ extern "C" gi_status gi_destroy(gi_ctx* c)
     if (c->pool) cudaMemPoolDestroy(c->pool);
     if (c->h_cnt) cudaFreeHost(c->h_cnt);
     if (c->h_words) cudaFreeHost(c->h_words);
+    if (c->h_build) cudaFreeHost(c->h_build);
+    for (auto& e : c->ev_build)
+        for (auto& x : e)
+            if (x) cudaEventDestroy(x);
     if (c->h_jobs) cudaFreeHost(c->h_jobs);
     for (auto& e : c->ev)
         if (e) cudaEventDestroy(e);
@@ -181,39 +187,36 @@ struct UploadSink {
         if (e_ != cudaSuccess) return (sink).cuda(e_, (what)); \
     } while (0)
 
-static gi_status mesh_finish(gi_ctx* c, gi_mesh* m, gi_mesh** out, cudaStream_t st, const UploadSink& sk)
+// Queues the mesh's build on st (one of the context's two streams, which has one
+// build in flight at most); mesh_finish waits for it.
+static gi_status mesh_start(gi_ctx* c, gi_mesh* m, cudaStream_t st, const UploadSink& sk)
 {
     // The validation result is read back with the build's last synchronisation,
     // not before it: the build reads vertex indices clamped to the array, so an
     // invalid mesh costs a wasted build but no out-of-bounds access.
-    unsigned* d_err = nullptr;
-    CKS(sk, pool_alloc(&d_err, sizeof(unsigned), c->pool, st), "alloc");
-    CKS(sk, cudaMemsetAsync(d_err, 0, sizeof(unsigned), st), "memset");
-    // device time of validation + build (the reference's buildRefitMesh*Ms);
-    // events of this call only, as two meshes may build at once on two streams
-    cudaEvent_t eb[2] = {nullptr, nullptr};
-    bool timed = cudaEventCreate(&eb[0]) == cudaSuccess && cudaEventCreate(&eb[1]) == cudaSuccess &&
-                 cudaEventRecord(eb[0], st) == cudaSuccess;
-    cudaError_t e = launch_validate(m->b.verts, m->b.nv, m->b.tris, m->b.nt, d_err, st);
-    if (e == cudaSuccess) e = build_bvh(m->b, false, d_err, c->pool, st);
-    timed = timed && cudaEventRecord(eb[1], st) == cudaSuccess;
-    unsigned herr = 0;
-    // a pageable destination: the copy returns when the stream has reached it (the build is done)
-    cudaError_t es = cudaMemcpyAsync(&herr, d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
-    // on an error the stream may still hold kernels that use the mesh: drain it before freeing
-    const cudaError_t es2 = cudaStreamSynchronize(st);
-    if (es == cudaSuccess) es = es2;
-    if (e == cudaSuccess) e = es;
-    float bms = 0.0f;
-    if (timed && e == cudaSuccess && cudaEventElapsedTime(&bms, eb[0], eb[1]) == cudaSuccess) m->build_ms = bms;
-    for (cudaEvent_t ev : eb)
-        if (ev) cudaEventDestroy(ev);
-    cudaGetLastError();  // a failed event call above is not the build's error
-    cudaFreeAsync(d_err, st);
+    const int s = st == c->st2 ? 1 : 0;
+    // device time of validation + build (the reference's buildRefitMesh*Ms)
+    cudaError_t e = cudaEventRecord(c->ev_build[s][0], st);
+    if (e == cudaSuccess) e = build_bvh(m->b, false, c->h_build + s * kBuildWords, c->pool, st);
+    if (e == cudaSuccess) e = cudaEventRecord(c->ev_build[s][1], st);
+    if (e == cudaSuccess) return GI_OK;
+    // the stream may still hold kernels that use the mesh: drain it before freeing
+    cudaStreamSynchronize(st);
+    mesh_free(c, m, st);
+    return sk.fail(e == cudaErrorMemoryAllocation ? GI_ERR_OOM : GI_ERR_CUDA, "BVH build", e);
+}
+
+static gi_status mesh_finish(gi_ctx* c, gi_mesh* m, gi_mesh** out, cudaStream_t st, const UploadSink& sk)
+{
+    const int s = st == c->st2 ? 1 : 0;
+    const cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) {
         mesh_free(c, m, st);
         return sk.fail(e == cudaErrorMemoryAllocation ? GI_ERR_OOM : GI_ERR_CUDA, "BVH build", e);
     }
+    float bms = 0.0f;
+    if (cudaEventElapsedTime(&bms, c->ev_build[s][0], c->ev_build[s][1]) == cudaSuccess) m->build_ms = bms;
+    const unsigned herr = build_result(m->b, false, c->h_build + s * kBuildWords);
     if (herr) {
         mesh_free(c, m, st);
         if (herr & 1u) return sk.fail(GI_ERR_INVALID_ARG, "triangle index out of range");
@@ -237,20 +240,17 @@ static gi_status mesh_alloc(gi_ctx* c, uint32_t nv, uint32_t nt, gi_mesh** pm, c
     m->ctx = c;
     m->b.nv = nv;
     m->b.nt = nt;
-    // 16 bytes past the last vertex: the kernels read a vertex as the two
-    // aligned 16-byte vectors that hold it (load_vertex)
-    size_t vb = sizeof(double) * 3 * (size_t)(nv ? nv : 1) + 16, tb = sizeof(uint32_t) * 3 * (size_t)(nt ? nt : 1);
+    const size_t vb = sizeof(double) * 3 * (size_t)(nv ? nv : 1) + 16, tb = sizeof(uint32_t) * 3 * (size_t)(nt ? nt : 1);
     if (c->budget && c->mesh_bytes + vb + tb > c->budget) {
         delete m;
         return sk.fail(GI_ERR_OOM, "HBM budget exceeded by mesh upload");
     }
-    cudaError_t e = pool_alloc(&m->b.verts, vb, c->pool, st);
-    if (e == cudaSuccess) e = pool_alloc(&m->b.tris, tb, c->pool, st);
+    const cudaError_t e = pool_alloc(&m->b.arena, mesh_arena_bytes(nv, nt), c->pool, st);
     if (e != cudaSuccess) {
-        if (m->b.verts) cudaFreeAsync(m->b.verts, st);
         delete m;
         return sk.fail(GI_ERR_OOM, "mesh allocation", e);
     }
+    mesh_arena(m->b, m->b.arena);
     m->b.bytes = vb + tb;
     *pm = m;
     return GI_OK;
@@ -295,9 +295,10 @@ static cudaError_t h2d(gi_ctx* c, void* dst, const void* src, size_t bytes, cuda
     return cudaSuccess;
 }
 
-// Host arrays -> device mesh with its BVH, on stream st (the caller holds c->mu).
-static gi_status mesh_upload_on(gi_ctx* c, const double* verts, uint32_t nv, const uint32_t* tris, uint32_t nt,
-                                gi_mesh** out, cudaStream_t st, const UploadSink& sk)
+// Host arrays -> device mesh with its BVH, on stream st (the caller holds c->mu):
+// queued by the first function, waited for by mesh_finish.
+static gi_status mesh_upload_start(gi_ctx* c, const double* verts, uint32_t nv, const uint32_t* tris, uint32_t nt,
+                                   gi_mesh** pm, cudaStream_t st, const UploadSink& sk)
 {
     gi_mesh* m = nullptr;
     gi_status s = mesh_alloc(c, nv, nt, &m, st, sk);
@@ -310,7 +311,16 @@ static gi_status mesh_upload_on(gi_ctx* c, const double* verts, uint32_t nv, con
         mesh_free(c, m, st);
         return sk.cuda(e, "upload mesh");
     }
-    return mesh_finish(c, m, out, st, sk);
+    s = mesh_start(c, m, st, sk);
+    if (s == GI_OK) *pm = m;
+    return s;
+}
+static gi_status mesh_upload_on(gi_ctx* c, const double* verts, uint32_t nv, const uint32_t* tris, uint32_t nt,
+                                gi_mesh** out, cudaStream_t st, const UploadSink& sk)
+{
+    gi_mesh* m = nullptr;
+    const gi_status s = mesh_upload_start(c, verts, nv, tris, nt, &m, st, sk);
+    return s == GI_OK ? mesh_finish(c, m, out, st, sk) : s;
 }
 
 extern "C" gi_status gi_mesh_upload(gi_ctx* c, const double* verts, uint32_t nv, const uint32_t* tris, uint32_t nt,
@@ -349,7 +359,8 @@ extern "C" gi_status gi_mesh_upload_device(gi_ctx* c, const double* d_verts, uin
                                   c->st), "copy vertices");
     if (nt) CK(c, cudaMemcpyAsync(m->b.tris, d_tris, sizeof(uint32_t) * 3 * (size_t)nt, cudaMemcpyDeviceToDevice,
                                   c->st), "copy triangles");
-    return mesh_finish(c, m, out, c->st, sk);
+    s = mesh_start(c, m, c->st, sk);
+    return s == GI_OK ? mesh_finish(c, m, out, c->st, sk) : s;
 }
 
 // Frees a mesh's buffers in order on stream st (the caller holds c->mu).
@@ -357,8 +368,7 @@ static void mesh_free(gi_ctx* c, gi_mesh* m, cudaStream_t st)
 {
     cudaSetDevice(c->device);
     // stream-ordered: work already queued on st still sees the mesh
-    void* p[] = {m->b.verts,   m->b.tris,   m->b.leafTri, m->b.leafBox,  m->b.nodes,   m->b.leafBox64,
-                 m->b.nodes64, m->b.cutRef, m->b.cutBox,  m->b.cutBox64, m->b.ncuts};
+    void* p[] = {m->b.arena, m->b.nodes, m->b.leafBox64, m->b.nodes64, m->b.cutBox64, m->b.cutRef64};
     for (void* q : p)
         if (q) cudaFreeAsync(q, st);
     if (m->b.bytes <= c->mesh_bytes) c->mesh_bytes -= m->b.bytes;
@@ -527,6 +537,7 @@ MeshDev mesh_dev(const gi_mesh* m)
     d.nodes = m->b.nodes;
     d.nodes64 = m->b.nodes64;
     d.cutRef = m->b.cutRef;
+    d.cutRef64 = m->b.cutRef64;
     d.cutBox = m->b.cutBox;
     d.cutBox64 = m->b.cutBox64;
     d.ncuts = m->b.ncuts;
@@ -560,18 +571,11 @@ static gi_status ensure_fp64(gi_ctx* c, gi_mesh* m)
         m->has64 = true;
         return GI_OK;
     }
-    unsigned* d_err = nullptr;
-    cudaError_t e = pool_alloc(&d_err, sizeof(unsigned), c->pool, c->st);
-    if (e != cudaSuccess) return set_err(c, GI_ERR_OOM, "FP64 BVH build", e);
-    unsigned herr = 0;
-    e = cudaMemsetAsync(d_err, 0, sizeof(unsigned), c->st);
-    if (e == cudaSuccess) e = build_bvh(m->b, true, d_err, c->pool, c->st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&herr, d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, c->st);
+    cudaError_t e = build_bvh(m->b, true, c->h_build, c->pool, c->st);
     const cudaError_t es = cudaStreamSynchronize(c->st);
     if (e == cudaSuccess) e = es;
-    cudaFreeAsync(d_err, c->st);
     if (e != cudaSuccess) return set_err(c, GI_ERR_CUDA, "FP64 BVH build", e);
-    if (herr) return set_err(c, GI_ERR_CUDA, "FP64 BVH build: inconsistent wide-node collapse");
+    if (build_result(m->b, true, c->h_build)) return set_err(c, GI_ERR_CUDA, "FP64 BVH build: inconsistent wide-node collapse");
     m->has64 = true;
     return GI_OK;
 }
@@ -1017,19 +1021,29 @@ extern "C" gi_status gi_intersect_oneshot(gi_ctx* c, const double* vA, uint32_t 
     gi_mesh *A = nullptr, *B = nullptr;
     gi_status s;
     {
-        // B is copied and built on the second stream by a helper thread while A
-        // is on the context's stream: B's copy overlaps A's build and the two
-        // builds overlap each other
+        // B is copied and built on the second stream while A is on the context's
+        // stream: B's copy overlaps A's build and the two builds overlap each
+        // other.  Builds that are queued in one go (and copies that are not
+        // staged) need no second host thread: starting and joining one took 40 us.
         std::lock_guard<std::mutex> lk(c->mu);
         cudaSetDevice(c->device);
         gi_status sb = GI_OK;
         std::string msg_b;
-        std::thread tb([&] {
-            cudaSetDevice(c->device);
-            sb = mesh_upload_on(c, vB, nvB, tB, ntB, &B, c->st2, UploadSink{c, &msg_b});
-        });
-        s = mesh_upload_on(c, vA, nvA, tA, ntA, &A, c->st, UploadSink{c, nullptr});
-        tb.join();
+        const UploadSink ka{c, nullptr}, kb{c, &msg_b};
+        if (!build_needs_host(ntA) && !build_needs_host(ntB)) {
+            gi_mesh *ma = nullptr, *mb = nullptr;
+            s = mesh_upload_start(c, vA, nvA, tA, ntA, &ma, c->st, ka);
+            sb = mesh_upload_start(c, vB, nvB, tB, ntB, &mb, c->st2, kb);
+            if (s == GI_OK) s = mesh_finish(c, ma, &A, c->st, ka);
+            if (sb == GI_OK) sb = mesh_finish(c, mb, &B, c->st2, kb);
+        } else {
+            std::thread tb([&] {
+                cudaSetDevice(c->device);
+                sb = mesh_upload_on(c, vB, nvB, tB, ntB, &B, c->st2, kb);
+            });
+            s = mesh_upload_on(c, vA, nvA, tA, ntA, &A, c->st, ka);
+            tb.join();
+        }
         if (s == GI_OK && sb != GI_OK) {
             s = sb;
             c->last_error = msg_b;

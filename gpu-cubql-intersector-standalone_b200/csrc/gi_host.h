@@ -270,6 +270,8 @@ struct gi_ctx {
     std::unique_ptr<CopyPool> copy_pool;  // created with the first staged upload
     std::once_flag copy_pool_once;
     Staging stage[2];                     // per upload stream (st, st2)
+    unsigned* h_build = nullptr;          // pinned: header words of the builds on st and st2
+    cudaEvent_t ev_build[2][2] = {};      // start and end of the builds on st and st2
     cudaMemPool_t pool = nullptr;  // stream-ordered allocations of this context
     gi::LaunchCfg cfg;
     uint64_t budget = 0;

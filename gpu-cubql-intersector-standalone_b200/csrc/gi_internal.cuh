@@ -76,6 +76,7 @@ struct MeshDev {
     // cuts: node / leaf refs whose subtrees cover all leaves, the depth-3 cut in
     // entries [0, kCutMax) and the depth-4 cut in [kCutMax, kCutMax + kCut4Max)
     const uint32_t* cutRef;
+    const uint32_t* cutRef64;  // the same for nodes64 (the two trees number their nodes apart)
     const float* cutBox;     // their boxes (6 floats each)
     const double* cutBox64;  // FP64 boxes of the same cuts (FP64 form)
     uint32_t root;  // wide node index, or kLeaf | leaf position when nt == 1

@@ -3,10 +3,10 @@
 // Build (once per mesh, replaces the reference's level-cut / forest builders,
 // include/third-party/cubql/level_cut_builder.h:278-364 and forest_builder.h:405-517,
 // which loop on the host with a device sync per tree level):
-//   k_validate -> k_tri_boxes -> k_morton_hist -> radix sort -> k_karras_leaves (leaves + binary tree)
-//   -> k_state_tables -> k_wide_flags -> scan -> k_collapse (size-greedy 4-wide nodes,
+//   k_tri_boxes (and validation) -> k_morton_hist -> radix sort -> k_karras_leaves (leaves + binary tree)
+//   -> k_state_tables -> k_wide_flags -> k_collapse (size-greedy 4-wide nodes,
 //   topology) -> k_refit_wide (bottom-up over the wide tree, atomic arrival counters)
-// One host round trip, for the wide-node count (the node array's size).
+// Large meshes: one host round trip, for the wide-node count (the node array's size).
 //
 // Intersect (replaces crossCheck.cu, DualTreeStep.cu, rapidDescendKernel.cu and the
 // chunk loop of SingleTreeBatchIntersector.cu:170-455 in the reference):
@@ -17,6 +17,7 @@
 //   k_exact     FP64 filter + exact integer signs for the escalated pairs.
 //   k_segments  intersection sets and correctly rounded endpoints.
 //   ordering    radix sort by (job, a, b) and gathers.
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 
@@ -39,20 +40,6 @@ unsigned long long launch_count()
 // ===========================================================================
 // Build
 // ===========================================================================
-__global__ void k_validate(const double* __restrict__ V, uint32_t nv, const uint32_t* __restrict__ T, uint32_t nt,
-                           unsigned* err)
-{
-    size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t k = i; k < 3ull * nv; k += stride) {
-        double x = V[k];
-        double a = fabs(x);
-        if (!(a <= 0x1p100) || (x != 0.0 && a < 0x1p-100)) atomicOr(err, 2u);
-    }
-    for (size_t k = i; k < 3ull * nt; k += stride)
-        if (T[k] >= nv) atomicOr(err, 1u);
-}
-
 __device__ __forceinline__ unsigned f2ord(float f)
 {
     unsigned u = __float_as_uint(f);
@@ -112,14 +99,25 @@ __device__ __forceinline__ void store_kid(WKid64* kd, const double b[6], uint32_
 // FP32 boxes rounded outward (so every exact triangle lies inside its box) and
 // centroid bounds.  The reference rounds to nearest (src/common/utils.cu:639),
 // which can drop true pairs; outward rounding keeps the candidate set a superset.
+// The same launch checks every vertex coordinate against the supported domain
+// and every index against the vertex array (the boxes clamp it meanwhile), in
+// the loads it needs anyway; a launch of its own took 4 to 11 us.
+//
+// Words of a build's header on the device, zero before the build.
+enum { kHdrErr = 0, kHdrMin = 1, kHdrMax = 4, kHdrWide = 7, kHdrWords = 8 };
 constexpr int kTriBoxThreads = 256;
 __global__ void __launch_bounds__(kTriBoxThreads, 4) k_tri_boxes(const double* __restrict__ V, uint32_t nv,
                                                               const uint32_t* __restrict__ T, uint32_t nt,
                                                               float* __restrict__ box, double* __restrict__ box64,
-                                                              unsigned* __restrict__ cb)
+                                                              unsigned* __restrict__ hdr)
 {
     pdl_enter();
     float cmin[3] = {INFINITY, INFINITY, INFINITY}, cmax[3] = {-INFINITY, -INFINITY, -INFINITY};
+    unsigned bad = 0;
+    for (size_t c = blockIdx.x * (size_t)blockDim.x + threadIdx.x; c < 3ull * nv; c += (size_t)gridDim.x * blockDim.x) {
+        const double x = V[c], ax = fabs(x);
+        if (!(ax <= 0x1p100) || (x != 0.0 && ax < 0x1p-100)) bad |= 2u;
+    }
     // two triangles per iteration, all their loads issued before any use
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nt; t += 2 * stride) {
@@ -129,7 +127,11 @@ __global__ void __launch_bounds__(kTriBoxThreads, 4) k_tri_boxes(const double* _
 #pragma unroll
         for (int q = 0; q < 2; q++)
 #pragma unroll
-            for (int j = 0; j < 3; j++) ix[q][j] = min(T[3 * (size_t)tt[q] + j], nv - 1u);  // validated later
+            for (int j = 0; j < 3; j++) {
+                const uint32_t x = T[3 * (size_t)tt[q] + j];
+                if (x >= nv) bad |= 1u;
+                ix[q][j] = min(x, nv - 1u);
+            }
 #pragma unroll
         for (int q = 0; q < 2; q++)
 #pragma unroll
@@ -181,9 +183,10 @@ __global__ void __launch_bounds__(kTriBoxThreads, 4) k_tri_boxes(const double* _
         const int k = threadIdx.x;
         float v = red[0][k];
         for (int q = 1; q < kTriBoxThreads / 32; q++) v = k < 3 ? fminf(v, red[q][k]) : fmaxf(v, red[q][k]);
-        if (k < 3) atomicMin(&cb[k], f2ord(v));
-        else atomicMax(&cb[k], f2ord(v));
+        // the minima as maxima of the complement: a header of zeros is neutral
+        atomicMax(&hdr[kHdrMin + k], k < 3 ? ~f2ord(v) : f2ord(v));
     }
+    if (bad) atomicOr(&hdr[kHdrErr], bad);
 }
 
 __device__ __forceinline__ uint32_t spread10(uint32_t x)
@@ -205,14 +208,13 @@ __device__ __forceinline__ uint32_t morton_axis(float c, float lo, float ext)
 }
 
 // 30-bit Morton keys of the triangles (their box centres quantised to 10 bits
-// per axis over the centroid bounds cb: ordered-float min x, y, z, max x, y,
-// z) with identity values, kRsTile triangles per block, and each block's counts
+// per axis over the centroid bounds of the header) with identity values, a tile's triangles per block, and each block's counts
 // of the first radix digit in the layout of k_rs_hist (digit-major, one column
 // per block), so the sort's first pass needs no histogram launch.  All of a
 // thread's box loads are issued before its first shared-memory atomic.
-template <int BITS>
+template <int BITS, int ITEMS>
 __global__ void __launch_bounds__(kRsThreads) k_morton_hist(const float* __restrict__ box, uint32_t nt,
-                                                            const unsigned* __restrict__ cb,
+                                                            const unsigned* __restrict__ hdr,
                                                             uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
                                                             uint32_t* __restrict__ counts, uint32_t ntiles)
 {
@@ -223,13 +225,13 @@ __global__ void __launch_bounds__(kRsThreads) k_morton_hist(const float* __restr
     float lo[3], ext[3];
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        lo[k] = ord2f(cb[k]);
-        ext[k] = ord2f(cb[3 + k]) - lo[k];
+        lo[k] = ord2f(~hdr[kHdrMin + k]);
+        ext[k] = ord2f(hdr[kHdrMax + k]) - lo[k];
     }
-    const uint32_t base = blockIdx.x * kRsTile;
-    uint32_t kk[kRsItems];
+    const uint32_t base = blockIdx.x * (kRsThreads * ITEMS);
+    uint32_t kk[ITEMS];
 #pragma unroll
-    for (int it = 0; it < kRsItems; it++) {
+    for (int it = 0; it < ITEMS; it++) {
         const uint32_t t = base + it * kRsThreads + threadIdx.x;
         kk[it] = 0;
         if (t < nt) {
@@ -243,7 +245,7 @@ __global__ void __launch_bounds__(kRsThreads) k_morton_hist(const float* __restr
     }
     __syncthreads();  // the histogram is cleared
 #pragma unroll
-    for (int it = 0; it < kRsItems; it++) {
+    for (int it = 0; it < ITEMS; it++) {
         const uint32_t t = base + it * kRsThreads + threadIdx.x;
         if (t < nt) {
             keys[t] = kk[it];
@@ -394,28 +396,45 @@ __global__ void k_state_tables(int n, const uint4* __restrict__ child, const int
     tab[y] = (uint8_t)(sW | (sO2 << 2) | (kStW << 4));
 }
 
-// wide[i] = 1 iff binary node i becomes a wide node.
-__global__ void k_wide_flags(int n, const int* __restrict__ parent, const uint8_t* __restrict__ tab,
-                             uint32_t* __restrict__ wide)
+// widx[i]: the wide node that binary node i becomes, or kEmpty.  The root is wide
+// node 0; a block's others take consecutive places from one atomic on the
+// header's count (the order of the blocks' runs varies from build to build and
+// shows in no result; a scan of the flags kept it, for three launches more).
+__global__ void __launch_bounds__(256) k_wide_flags(int n, const int* __restrict__ parent, const uint8_t* __restrict__ tab,
+                                                    uint32_t* __restrict__ widx, unsigned* __restrict__ hdr)
 {
     pdl_enter();
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n - 1) return;
-    if (i == 0) {
-        wide[0] = 1u;
-        return;
+    __shared__ unsigned s_warp[8], s_base;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    bool wide = false;
+    if (i > 0 && i < n - 1) {
+        unsigned f = tab[i];  // state of i as a function of the state of the node above the chain
+        int x = parent[i];
+        for (int guard = 0; x > 0 && guard < n; guard++) {
+            const unsigned f0 = f & 3u, f1 = (f >> 2) & 3u, f2 = (f >> 4) & 3u;
+            if (f0 == f1 && f1 == f2) break;
+            const unsigned t = __ldg(tab + x);
+            f = ((f >> (2u * (t & 3u))) & 3u) | (((f >> (2u * ((t >> 2) & 3u))) & 3u) << 2) |
+                (((f >> (2u * ((t >> 4) & 3u))) & 3u) << 4);
+            x = parent[x];
+        }
+        wide = (f & 3u) == kStW;  // the root is a wide node
     }
-    unsigned f = tab[i];  // state of i as a function of the state of the node above the chain
-    int x = parent[i];
-    for (int guard = 0; x > 0 && guard < n; guard++) {
-        const unsigned f0 = f & 3u, f1 = (f >> 2) & 3u, f2 = (f >> 4) & 3u;
-        if (f0 == f1 && f1 == f2) break;
-        const unsigned t = __ldg(tab + x);
-        f = ((f >> (2u * (t & 3u))) & 3u) | (((f >> (2u * ((t >> 2) & 3u))) & 3u) << 2) |
-            (((f >> (2u * ((t >> 4) & 3u))) & 3u) << 4);
-        x = parent[x];
+    const unsigned lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+    const unsigned m = __ballot_sync(0xffffffffu, wide);
+    if (lane == 0) s_warp[w] = __popc(m);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned tot = 0;
+        for (unsigned q = 0; q < 8u; q++) {
+            const unsigned t = s_warp[q];
+            s_warp[q] = tot;
+            tot += t;
+        }
+        s_base = tot ? atomicAdd(&hdr[kHdrWide], tot) : 0u;
     }
-    wide[i] = (f & 3u) == kStW ? 1u : 0u;  // the root is a wide node
+    __syncthreads();
+    if (i < n - 1) widx[i] = i == 0 ? 0u : (wide ? 1u + s_base + s_warp[w] + __popc(m & ((1u << lane) - 1u)) : kEmpty);
 }
 
 // Writes wide node widx[i] from binary node i: the size-greedy expansion of i
@@ -428,15 +447,15 @@ __global__ void k_wide_flags(int n, const int* __restrict__ parent, const uint8_
 // index is out of range, cannot arise; it is written as an empty slot and
 // flagged in *bad rather than followed.
 template <class S, class NodeT>
-__global__ void k_collapse(int n, const uint4* __restrict__ child, const uint32_t* __restrict__ wide,
-                           const uint32_t* __restrict__ widx, uint32_t nw, const S* __restrict__ leafBox,
+__global__ void k_collapse(int n, const uint4* __restrict__ child, const uint32_t* __restrict__ widx, uint32_t nw, const S* __restrict__ leafBox,
                            NodeT* __restrict__ nodes, uint2* __restrict__ nodeUp, uint32_t* __restrict__ nkids,
                            unsigned* __restrict__ arrive, unsigned* __restrict__ bad)
 {
     pdl_enter();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n - 1 || !wide[i]) return;
+    if (i >= n - 1) return;
     const uint32_t wi = widx[i];
+    if (wi == kEmpty) return;
     if (wi >= nw) {
         atomicOr(bad, kErrBuild);
         return;
@@ -467,7 +486,7 @@ __global__ void k_collapse(int n, const uint4* __restrict__ child, const uint32_
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         uint32_t r = k < ns ? slot[k] : kEmpty;
-        if (r != kEmpty && !(r & kLeaf) && (!wide[r] || widx[r] >= nw)) {
+        if (r != kEmpty && !(r & kLeaf) && widx[r] >= nw) {
             atomicOr(bad, kErrBuild);
             r = kEmpty;
         }
@@ -534,10 +553,11 @@ __device__ __forceinline__ void node_union_cg(const WNode64* nd, double b[6])
 // level costs the slot stores, the arrival atomic and one read of the node's
 // six box fields; the wide tree has about half the levels of the binary one.
 template <class S, class NodeT>
-__global__ void k_refit_wide(uint32_t nw, const uint2* __restrict__ nodeUp, const uint32_t* __restrict__ nkids,
-                             NodeT* nodes, unsigned* arrive, unsigned* bad)
+__global__ void k_refit_wide(uint32_t cap, unsigned* hdr, const uint2* __restrict__ nodeUp, const uint32_t* __restrict__ nkids,
+                             NodeT* nodes, unsigned* arrive)
 {
     pdl_enter();
+    const uint32_t nw = min(1u + __ldcg(&hdr[kHdrWide]), cap);
     const uint32_t w0 = blockIdx.x * blockDim.x + threadIdx.x;
     if (w0 >= nw) return;
     const uint32_t k0 = nkids[w0];
@@ -550,7 +570,7 @@ __global__ void k_refit_wide(uint32_t nw, const uint2* __restrict__ nodeUp, cons
         if (up.x == kEmpty) return;  // the root is complete
         const uint32_t w = up.x, k = up.y & 3u;
         if (w >= nw) {
-            atomicOr(bad, kErrBuild);
+            atomicOr(&hdr[kHdrErr], kErrBuild);
             return;
         }
         NodeT* nd = nodes + w;
@@ -643,77 +663,121 @@ __global__ void __launch_bounds__(kCutThreads) k_cut(const NodeT* __restrict__ n
     }
 }
 
-cudaError_t launch_validate(const double* verts, uint32_t nv, const uint32_t* tris, uint32_t nt, unsigned* d_err,
-                            cudaStream_t st)
-{
-    k_validate<<<1024, 256, 0, st>>>(verts, nv, tris, nt, d_err);
-    note_launches(1);
-    return cudaGetLastError();
-}
-
 #define GI_TRY(x)                                \
     do {                                         \
         cudaError_t e_ = (x);                    \
         if (e_ != cudaSuccess) return e_;        \
     } while (0)
 
-cudaError_t build_bvh(MeshBuffers& m, bool fp64, unsigned* d_err, cudaMemPool_t pool, cudaStream_t st)
+// One piece of device memory handed out in aligned parts.
+struct Carve {
+    char* p;
+    template <class T>
+    T* take(size_t n)
+    {
+        T* q = (T*)p;
+        p += (sizeof(T) * n + 255) & ~(size_t)255;
+        return q;
+    }
+};
+
+// Wide nodes of n triangles at most.  A node has four children unless it holds
+// only two or three leaves; with a, b, c nodes of four, three and two children,
+// 3a + 2b + c = n - 1 and 3b + 2c <= n, so a + b + c <= 2n / 3.
+static uint32_t wide_bound(uint32_t n)
+{
+    return 2u * (n / 3u) + 2u;
+}
+
+// Above this many triangles the node array has its exact size, for a host round
+// trip in the middle of the build (15 us of an idle GPU); below, the size of the
+// bound (a third more nodes, 12 MB at most), and the build is queued in one go.
+constexpr uint32_t kExactNodesAbove = 1u << 19;
+// Radix tiles of 1,024 keys up to this many triangles, else 3,072: the sort's
+// kernels have a block per tile, and 3,072 leave most SMs idle (20 k triangles
+// made seven blocks, 11-13 us a kernel; 300 k ninety-nine).
+constexpr uint32_t kSmallTilesUpTo = 1u << 19;
+
+bool build_needs_host(uint32_t nt)
+{
+    return nt > kExactNodesAbove;
+}
+
+cudaError_t build_bvh(MeshBuffers& m, bool fp64, unsigned* h_words, cudaMemPool_t pool, cudaStream_t st)
 {
     const uint32_t n = m.nt;
-    if (n == 0) {
-        m.root = kEmpty;
-        m.nnodes = 0;
-        return cudaSuccess;
-    }
-    // scratch
-    float* box = nullptr;
-    double* box64 = nullptr;
-    unsigned* cb = nullptr;
-    uint32_t *k0 = nullptr, *v0 = nullptr, *k1 = nullptr, *v1 = nullptr, *counts = nullptr, *stemp = nullptr;
-    uint4* child = nullptr;
-    int* parent = nullptr;
-    unsigned* arrive = nullptr;
-    uint2* nodeUp = nullptr;
-    uint32_t* nkids = nullptr;
-    uint32_t *wide = nullptr, *widx = nullptr;
-    uint8_t* tab = nullptr;
     constexpr int kMortonDigit = 10;  // 30-bit keys: three passes
-    size_t cw = radix_counts_words<kMortonDigit>(n);
-    size_t sw = scan_temp_words(cw > n ? cw : n);
-    GI_TRY(pool_alloc(&box, sizeof(float) * 6 * n, pool, st));
-    if (fp64) GI_TRY(pool_alloc(&box64, sizeof(double) * 6 * n, pool, st));
-    GI_TRY(pool_alloc(&cb, sizeof(unsigned) * 8, pool, st));
-    GI_TRY(pool_alloc(&k0, sizeof(uint32_t) * n, pool, st));
-    GI_TRY(pool_alloc(&v0, sizeof(uint32_t) * n, pool, st));
-    GI_TRY(pool_alloc(&k1, sizeof(uint32_t) * n, pool, st));
-    GI_TRY(pool_alloc(&v1, sizeof(uint32_t) * n, pool, st));
-    GI_TRY(pool_alloc(&counts, sizeof(uint32_t) * cw, pool, st));
-    GI_TRY(pool_alloc(&stemp, sizeof(uint32_t) * sw, pool, st));
-    unsigned cbinit[8] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u, 0u, 0u};
-    GI_TRY(cudaMemcpyAsync(cb, cbinit, sizeof(cbinit), cudaMemcpyHostToDevice, st));
-    int tb = 256;
-    int gb = (int)((n + tb - 1) / tb);
+    constexpr uint32_t kDig = 1u << kMortonDigit;
+    const bool small = n <= kSmallTilesUpTo;
+    const uint32_t tile = kRsThreads * (small ? kRsItemsSmall : kRsItems), ntiles = (n + tile - 1) / tile;
+    const uint32_t bound = n > 1 ? wide_bound(n) : 0u;
+    // scratch in one allocation
+    char* mem = nullptr;
+    unsigned* hdr;
+    float* box;
+    double* box64;
+    uint32_t *k0, *v0, *k1, *v1, *counts, *totals, *widx, *nkids;
+    uint4* child;
+    int* parent;
+    uint8_t* tab;
+    uint2* nodeUp;
+    unsigned* arrive;
+    for (;;) {
+        Carve c{mem};
+        hdr = c.take<unsigned>(kHdrWords);
+        box = c.take<float>(6 * (size_t)n);
+        box64 = fp64 ? c.take<double>(6 * (size_t)n) : nullptr;
+        k0 = c.take<uint32_t>(n);
+        v0 = c.take<uint32_t>(n);
+        k1 = c.take<uint32_t>(n);
+        v1 = c.take<uint32_t>(n);
+        counts = c.take<uint32_t>((size_t)kDig * ntiles);
+        totals = c.take<uint32_t>(kDig);
+        child = c.take<uint4>(n);
+        parent = c.take<int>(n);
+        tab = c.take<uint8_t>(n);
+        widx = c.take<uint32_t>(n);
+        nodeUp = c.take<uint2>(bound);
+        nkids = c.take<uint32_t>(bound);
+        arrive = c.take<unsigned>(bound);
+        if (mem) break;
+        GI_TRY(pool_alloc(&mem, (size_t)(c.p - mem) + 256, pool, st));
+    }
+    struct Free {
+        void* p;
+        cudaStream_t st;
+        ~Free() { cudaFreeAsync(p, st); }
+    } free_{mem, st};
+    GI_TRY(cudaMemsetAsync(hdr, 0, sizeof(unsigned) * kHdrWords, st));
+    const int tb = 256;
+    const int gb = (int)((n + tb - 1) / tb);
     // Kernels that follow another kernel in the stream are launched as its
     // programmatic dependents (launch_dep): each waits for its predecessor at
     // its first statement, so only the next launch's latency overlaps the tail
     // of the current kernel (0.474 -> 0.446 ms per 1.3M-triangle build on
-    // B200).  The two kernels that follow a copy (k_tri_boxes after the bounds'
-    // initial values, k_collapse after the wide-node count) are plain launches.
+    // B200).  A kernel that follows a copy or a memset is a plain launch.
     // four resident blocks per SM, each looping: the centroid bounds take one set of atomics per block
-    const int gboxes = (int)((n + 2 * kTriBoxThreads - 1) / (2 * kTriBoxThreads));
-    k_tri_boxes<<<gboxes < 592 ? gboxes : 592, kTriBoxThreads, 0, st>>>(m.verts, m.nv, m.tris, n, box, box64, cb);
-    const uint32_t ntiles = (n + kRsTile - 1) / kRsTile;
-    launch_dep(k_morton_hist<kMortonDigit>, ntiles, kRsThreads, st, (const float*)box, n, (const unsigned*)cb, k0, v0,
-               counts, ntiles);
-    radix_sort<uint32_t, kMortonDigit>(k0, v0, k1, v1, n, 30, counts, stemp, st, true);
-    if (n > 1) {
-        GI_TRY(pool_alloc(&child, sizeof(uint4) * (n - 1), pool, st));
-        GI_TRY(pool_alloc(&parent, sizeof(int) * (n - 1), pool, st));
+    const uint32_t work = std::max(n, m.nv);
+    const int gboxes = (int)((work + 2 * kTriBoxThreads - 1) / (2 * kTriBoxThreads));
+    k_tri_boxes<<<gboxes < 1 ? 1 : (gboxes < 592 ? gboxes : 592), kTriBoxThreads, 0, st>>>(m.verts, m.nv, m.tris, n, box, box64, hdr);
+    note_launches(1);
+    m.root = kEmpty;
+    m.nnodes = 0;
+    if (n == 0) {
+        GI_TRY(cudaGetLastError());
+        return cudaMemcpyAsync(h_words, hdr, sizeof(unsigned) * kHdrWords, cudaMemcpyDeviceToHost, st);
+    }
+    if (small) {
+        launch_dep(k_morton_hist<kMortonDigit, kRsItemsSmall>, ntiles, kRsThreads, st, (const float*)box, n,
+                   (const unsigned*)hdr, k0, v0, counts, ntiles);
+        radix_sort<uint32_t, kMortonDigit, kRsItemsSmall>(k0, v0, k1, v1, n, 30, counts, totals, st);
+    } else {
+        launch_dep(k_morton_hist<kMortonDigit, kRsItems>, ntiles, kRsThreads, st, (const float*)box, n,
+                   (const unsigned*)hdr, k0, v0, counts, ntiles);
+        radix_sort<uint32_t, kMortonDigit, kRsItems>(k0, v0, k1, v1, n, 30, counts, totals, st);
     }
     // leaves in sorted order, and the binary radix tree
     if (!fp64) {
-        GI_TRY(pool_alloc(&m.leafBox, sizeof(float) * 6 * n, pool, st));
-        GI_TRY(pool_alloc(&m.leafTri, sizeof(uint4) * n, pool, st));
         launch_dep(k_karras_leaves<float>, gb, tb, st, (const uint32_t*)k0, (const uint32_t*)v0, (int)n,
                    (const uint32_t*)m.tris, (const float*)box, m.leafBox, m.leafTri, child, parent);
     } else {
@@ -723,80 +787,88 @@ cudaError_t build_bvh(MeshBuffers& m, bool fp64, unsigned* d_err, cudaMemPool_t 
     }
     if (n == 1) {
         m.root = kLeaf | 0u;
-        m.nnodes = 0;
     } else {
-        GI_TRY(pool_alloc(&wide, sizeof(uint32_t) * (n - 1), pool, st));
-        GI_TRY(pool_alloc(&tab, sizeof(uint8_t) * (n - 1), pool, st));
-        GI_TRY(pool_alloc(&widx, sizeof(uint32_t) * (n - 1), pool, st));
-        int gi_ = (int)((n - 1 + tb - 1) / tb);
+        const int gi_ = (int)((n - 1 + tb - 1) / tb);
         launch_dep(k_state_tables, gi_, tb, st, (int)n, (const uint4*)child, (const int*)parent, tab);
-        launch_dep(k_wide_flags, gi_, tb, st, (int)n, (const int*)parent, (const uint8_t*)tab, wide);
-        scan_exclusive(wide, widx, n - 1, stemp, st);
-        // number of wide nodes = widx[n-2] + wide[n-2]
-        uint32_t last[2];
-        GI_TRY(cudaMemcpyAsync(&last[0], widx + (n - 2), sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-        GI_TRY(cudaMemcpyAsync(&last[1], wide + (n - 2), sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-        GI_TRY(cudaStreamSynchronize(st));
-        uint32_t nw = last[0] + last[1];
-        GI_TRY(pool_alloc(&nodeUp, sizeof(uint2) * (size_t)nw, pool, st));
-        GI_TRY(pool_alloc(&nkids, sizeof(uint32_t) * (size_t)nw, pool, st));
-        GI_TRY(pool_alloc(&arrive, sizeof(unsigned) * (size_t)nw, pool, st));
-        const int gw = (int)((nw + tb - 1) / tb);
-        if (!fp64) {
-            GI_TRY(pool_alloc(&m.nodes, sizeof(WNode) * (size_t)nw, pool, st));
-            k_collapse<float, WNode><<<gi_, tb, 0, st>>>((int)n, child, wide, widx, nw, m.leafBox, m.nodes,
-                                                         nodeUp, nkids, arrive, d_err);
-            launch_dep(k_refit_wide<float, WNode>, gw, tb, st, nw, (const uint2*)nodeUp, (const uint32_t*)nkids, m.nodes,
-                       arrive, d_err);
-        } else {
-            GI_TRY(pool_alloc(&m.nodes64, sizeof(WNode64) * (size_t)nw, pool, st));
-            k_collapse<double, WNode64><<<gi_, tb, 0, st>>>((int)n, child, wide, widx, nw, m.leafBox64,
-                                                            m.nodes64, nodeUp, nkids, arrive, d_err);
-            launch_dep(k_refit_wide<double, WNode64>, gw, tb, st, nw, (const uint2*)nodeUp, (const uint32_t*)nkids,
-                       m.nodes64, arrive, d_err);
+        launch_dep(k_wide_flags, gi_, tb, st, (int)n, (const int*)parent, (const uint8_t*)tab, widx, hdr);
+        uint32_t cap = bound;
+        const bool exact = build_needs_host(n);
+        if (exact) {
+            GI_TRY(cudaMemcpyAsync(h_words, hdr, sizeof(unsigned) * kHdrWords, cudaMemcpyDeviceToHost, st));
+            GI_TRY(cudaStreamSynchronize(st));
+            cap = std::min(bound, 1u + h_words[kHdrWide]);
         }
-        m.nnodes = nw;
+        const int gw = (int)((cap + tb - 1) / tb);
+        // (a plain launch after the host round trip, a dependent one otherwise)
+        auto collapse = [&](auto kern, auto... args) {
+            if (exact) kern<<<gi_, tb, 0, st>>>(args...);
+            else launch_dep(kern, gi_, tb, st, args...);
+        };
+        if (!fp64) {
+            GI_TRY(pool_alloc(&m.nodes, sizeof(WNode) * (size_t)cap, pool, st));
+            collapse(k_collapse<float, WNode>, (int)n, (const uint4*)child, (const uint32_t*)widx, cap,
+                     (const float*)m.leafBox, m.nodes, nodeUp, nkids, arrive, hdr + kHdrErr);
+            launch_dep(k_refit_wide<float, WNode>, gw, tb, st, cap, hdr, (const uint2*)nodeUp, (const uint32_t*)nkids,
+                       m.nodes, arrive);
+        } else {
+            GI_TRY(pool_alloc(&m.nodes64, sizeof(WNode64) * (size_t)cap, pool, st));
+            collapse(k_collapse<double, WNode64>, (int)n, (const uint4*)child, (const uint32_t*)widx, cap,
+                     (const double*)m.leafBox64, m.nodes64, nodeUp, nkids, arrive, hdr + kHdrErr);
+            launch_dep(k_refit_wide<double, WNode64>, gw, tb, st, cap, hdr, (const uint2*)nodeUp,
+                       (const uint32_t*)nkids, m.nodes64, arrive);
+        }
         m.root = 0;
+        note_launches(4);
     }
-    // depth-3 and depth-4 cuts (refs and sizes shared by both precisions; boxes per
-    // precision); the sizes stay on the device, where the seeding reads them
-    {
-        if (!m.ncuts) GI_TRY(pool_alloc(&m.ncuts, sizeof(uint32_t) * 2, pool, st));
-        uint32_t* d_n = m.ncuts;
-        if (!m.cutRef) GI_TRY(pool_alloc(&m.cutRef, sizeof(uint32_t) * kCutCap, pool, st));
-        if (!fp64) {
-            GI_TRY(pool_alloc(&m.cutBox, sizeof(float) * 6 * kCutCap, pool, st));
-            launch_dep(k_cut<float, WNode>, 1, kCutThreads, st, (const WNode*)m.nodes, (const float*)m.leafBox, m.root,
-                       m.cutRef, m.cutBox, d_n);
-        } else {
-            GI_TRY(pool_alloc(&m.cutBox64, sizeof(double) * 6 * kCutCap, pool, st));
-            launch_dep(k_cut<double, WNode64>, 1, kCutThreads, st, (const WNode64*)m.nodes64,
-                       (const double*)m.leafBox64, m.root, m.cutRef, m.cutBox64, d_n);
-        }
+    // depth-3 and depth-4 cuts, per precision (their sizes are the same); the sizes
+    // stay on the device, where the seeding reads them
+    if (!fp64) {
+        launch_dep(k_cut<float, WNode>, 1, kCutThreads, st, (const WNode*)m.nodes, (const float*)m.leafBox, m.root,
+                   m.cutRef, m.cutBox, m.ncuts);
+    } else {
+        GI_TRY(pool_alloc(&m.cutBox64, sizeof(double) * 6 * kCutCap, pool, st));
+        GI_TRY(pool_alloc(&m.cutRef64, sizeof(uint32_t) * kCutCap, pool, st));
+        launch_dep(k_cut<double, WNode64>, 1, kCutThreads, st, (const WNode64*)m.nodes64, (const double*)m.leafBox64,
+                   m.root, m.cutRef64, m.cutBox64, m.ncuts);
     }
+    note_launches(3);
     GI_TRY(cudaGetLastError());
-    cudaFreeAsync(box, st);
-    if (box64) cudaFreeAsync(box64, st);
-    cudaFreeAsync(cb, st);
-    cudaFreeAsync(k0, st);
-    cudaFreeAsync(v0, st);
-    cudaFreeAsync(k1, st);
-    cudaFreeAsync(v1, st);
-    cudaFreeAsync(counts, st);
-    cudaFreeAsync(stemp, st);
-    if (child) cudaFreeAsync(child, st);
-    if (parent) cudaFreeAsync(parent, st);
-    if (arrive) cudaFreeAsync(arrive, st);
-    if (nodeUp) cudaFreeAsync(nodeUp, st);
-    if (nkids) cudaFreeAsync(nkids, st);
-    if (wide) cudaFreeAsync(wide, st);
-    if (tab) cudaFreeAsync(tab, st);
-    if (widx) cudaFreeAsync(widx, st);
+    return cudaMemcpyAsync(h_words, hdr, sizeof(unsigned) * kHdrWords, cudaMemcpyDeviceToHost, st);
+}
+
+unsigned build_result(MeshBuffers& m, bool fp64, const unsigned* h_words)
+{
+    const uint32_t n = m.nt;
+    if (n > 1) m.nnodes = 1u + h_words[kHdrWide];
     if (!fp64)
         m.bytes += sizeof(float) * 6 * (size_t)n + sizeof(uint4) * (size_t)n + sizeof(WNode) * (size_t)m.nnodes;
     else
         m.bytes += sizeof(double) * 6 * (size_t)n + sizeof(WNode64) * (size_t)m.nnodes;
-    return cudaGetLastError();
+    return h_words[kHdrErr];
+}
+
+size_t mesh_arena_bytes(uint32_t nv, uint32_t nt)
+{
+    MeshBuffers m;
+    m.nv = nv;
+    m.nt = nt;
+    return mesh_arena(m, nullptr);
+}
+size_t mesh_arena(MeshBuffers& m, void* mem)
+{
+    Carve c{(char*)mem};
+    // 16 bytes past the last vertex: the kernels read a vertex as the two
+    // aligned 16-byte vectors that hold it (load_vertex)
+    m.verts = c.take<double>(3 * (size_t)(m.nv ? m.nv : 1) + 2);
+    m.tris = c.take<uint32_t>(3 * (size_t)(m.nt ? m.nt : 1));
+    if (m.nt) {
+        m.leafTri = c.take<uint4>(m.nt);
+        m.leafBox = c.take<float>(6 * (size_t)m.nt);
+        m.cutBox = c.take<float>(6 * kCutCap);
+        m.cutRef = c.take<uint32_t>(kCutCap);
+        m.ncuts = c.take<uint32_t>(2);
+    }
+    return (size_t)(c.p - (char*)mem);
 }
 
 // ===========================================================================
@@ -1266,7 +1338,7 @@ __device__ __forceinline__ bool seed_test(const Bufs& B, unsigned t, unsigned nA
         bb.lo[k] = __ldg(bb_ + 6 * j + k);
         bb.hi[k] = __ldg(bb_ + 6 * j + 3 + k);
     }
-    ab = make_uint2(__ldg(J.A.cutRef + i), __ldg(J.B.cutRef + j));
+    ab = make_uint2(__ldg((F64 ? J.A.cutRef64 : J.A.cutRef) + i), __ldg((F64 ? J.B.cutRef64 : J.B.cutRef) + j));
     if (!J.pa.identity) world_box(J.pa, ba);
     if (!J.pb.identity) world_box(J.pb, bb);
     return overlap(ba, bb);

@@ -9,6 +9,7 @@ namespace gi {
 
 // Device arrays owned by one resident mesh.
 struct MeshBuffers {
+    void* arena = nullptr;  // holds verts, tris, leafTri, leafBox, cutRef, cutBox, ncuts
     double* verts = nullptr;
     uint32_t* tris = nullptr;
     uint4* leafTri = nullptr;
@@ -20,6 +21,7 @@ struct MeshBuffers {
     uint32_t* ncuts = nullptr;  // device: sizes of the depth-3 and depth-4 cuts
     float* cutBox = nullptr;
     double* cutBox64 = nullptr;
+    uint32_t* cutRef64 = nullptr;
     uint32_t nv = 0, nt = 0, nnodes = 0, root = 0;
     size_t bytes = 0;
 };
@@ -36,14 +38,22 @@ inline cudaError_t pool_alloc(T** p, size_t bytes, cudaMemPool_t pool, cudaStrea
     return pool_alloc(reinterpret_cast<void**>(p), bytes, pool, st);
 }
 
-// Validates indices / coordinate domain (err bit 1: bad index, 2: out of domain).
-cudaError_t launch_validate(const double* verts, uint32_t nv, const uint32_t* tris, uint32_t nt, unsigned* d_err,
-                            cudaStream_t st);
+// A mesh's arrays of known size (all but the nodes) in one piece of device
+// memory: sets their pointers and returns the bytes used.
+size_t mesh_arena(MeshBuffers& m, void* mem);
+size_t mesh_arena_bytes(uint32_t nv, uint32_t nt);
 
-// Builds the 4-wide BVH (FP32 boxes) or, with fp64 = true, the FP64 node copy.
-// d_err: a device word (required); bit 2 (4u) is set if the wide tree came out
-// inconsistent (not expected; the kernels then skip the bad links).
-cudaError_t build_bvh(MeshBuffers& m, bool fp64, unsigned* d_err, cudaMemPool_t pool, cudaStream_t st);
+// Validates the input (error bit 1: bad index, 2: out of domain) and builds the
+// 4-wide BVH (FP32 boxes) or, with fp64 = true, the FP64 node copy.  Queues
+// everything on st, the copy of the build's header to h_words (kBuildWords
+// pinned words) last; with build_needs_host the call waits once in between.
+// After the stream has been synchronised, build_result reads the header: the
+// node count and the error bits (4: the wide tree came out inconsistent, not
+// expected; the kernels then skip the bad links).
+constexpr int kBuildWords = 8;
+bool build_needs_host(uint32_t nt);
+cudaError_t build_bvh(MeshBuffers& m, bool fp64, unsigned* h_words, cudaMemPool_t pool, cudaStream_t st);
+unsigned build_result(MeshBuffers& m, bool fp64, const unsigned* h_words);
 
 // Intersect launch configuration.
 struct LaunchCfg {

@@ -1,4 +1,4 @@
-// gi_sort.cuh -- device scan and LSD radix sort (8- or 10-bit digits, stable).
+// gi_sort.cuh -- block scan, decoupled look-back and LSD radix sort (10-bit digits, stable).
 //
 // Used by the BVH build (30-bit Morton keys, replaces the reference's CUB
 // DeviceRadixSort in include/third-party/cubql/level_cut_builder.h:345-347)
@@ -50,10 +50,6 @@ inline void launch_dep(void (*k)(KArgs...), unsigned grid, unsigned block, cudaS
     }
 }
 
-constexpr int kScanThreads = 1024;
-constexpr int kScanItems = 4;
-constexpr int kScanTile = kScanThreads * kScanItems;
-
 // block-wide exclusive scan of per-thread sums; returns the block total
 __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* smem_warp, uint32_t* total)
 {
@@ -82,82 +78,6 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* s
     *total = smem_warp[32];
     __syncthreads();
     return r;
-}
-
-__global__ void k_scan_tiles(const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* tile_sums)
-{
-    pdl_enter();
-    __shared__ uint32_t sw[33];
-    uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-    uint32_t v[kScanItems];
-    uint32_t s = 0;
-#pragma unroll
-    for (int k = 0; k < kScanItems; k++) {
-        v[k] = (base + k < n) ? in[base + k] : 0u;
-        s += v[k];
-    }
-    uint32_t tot;
-    uint32_t ex = block_exclusive_scan(s, sw, &tot);
-#pragma unroll
-    for (int k = 0; k < kScanItems; k++) {
-        if (base + k < n) out[base + k] = ex;
-        ex += v[k];
-    }
-    if (threadIdx.x == 0 && tile_sums) tile_sums[blockIdx.x] = tot;
-}
-
-__global__ void k_scan_add(uint32_t* out, uint32_t n, const uint32_t* tile_offsets)
-{
-    pdl_enter();
-    uint32_t add = tile_offsets[blockIdx.x];
-    uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-#pragma unroll
-    for (int k = 0; k < kScanItems; k++)
-        if (base + k < n) out[base + k] += add;
-}
-
-// exclusive scan of n uint32 (in and out may alias); temp needs scan_temp_words(n)
-inline size_t scan_temp_words(size_t n)
-{
-    size_t t = 0;
-    while (n > (size_t)kScanTile) {
-        n = (n + kScanTile - 1) / kScanTile;
-        t += n + 1;
-    }
-    return t + 1;
-}
-inline void scan_exclusive(const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* temp, cudaStream_t st)
-{
-    if (n == 0) return;
-    uint32_t tiles = (n + kScanTile - 1) / kScanTile;
-    if (tiles == 1) {
-        launch_dep(k_scan_tiles, 1, kScanThreads, st, in, out, n, (uint32_t*)nullptr);
-        note_launches(1);
-        return;
-    }
-    uint32_t* sums = temp;
-    launch_dep(k_scan_tiles, tiles, kScanThreads, st, in, out, n, sums);
-    scan_exclusive(sums, sums, tiles, temp + tiles + 1, st);
-    launch_dep(k_scan_add, tiles, kScanThreads, st, out, n, (const uint32_t*)sums);
-    note_launches(2);
-}
-
-// Exclusive scan left in two parts: out[] holds the scan within each tile of
-// kScanTile words and *sums (nullptr for a single tile) the scanned tile
-// totals, so that the full scan at j is out[j] + sums[j / kScanTile].  A
-// consumer that adds the tile offset itself saves the add pass.
-inline void scan_exclusive_split(const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* temp, const uint32_t** sums,
-                                 cudaStream_t st)
-{
-    *sums = nullptr;
-    if (n == 0) return;
-    uint32_t tiles = (n + kScanTile - 1) / kScanTile;
-    launch_dep(k_scan_tiles, tiles, kScanThreads, st, in, out, n, tiles > 1 ? temp : (uint32_t*)nullptr);
-    note_launches(1);
-    if (tiles > 1) {
-        scan_exclusive(temp, temp, tiles, temp + tiles + 1, st);
-        *sums = temp;
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -205,16 +125,17 @@ __device__ __forceinline__ bool lookback(unsigned* status, unsigned tile, unsign
 // ---------------------------------------------------------------------------
 // Radix sort
 // ---------------------------------------------------------------------------
-// 12 keys per thread: 427 tiles of 3,072 keys for a 1.3M-triangle mesh, which
-// keeps more scatter warps resident per SM than 4,096-key tiles (build 0.435 ->
-// 0.418 ms on B200; 10 and 14 keys per thread gave 0.427 and 0.426 ms, 8 keys
-// 0.436 ms: smaller tiles pay more per-tile overhead)
+// Keys per thread of a tile.  Large sorts: 12, 427 tiles of 3,072 keys for a
+// 1.3M-triangle mesh, which keeps more scatter warps resident per SM than
+// 4,096-key tiles (build 0.435 -> 0.418 ms on B200; 10 and 14 keys per thread
+// gave 0.427 and 0.426 ms, 8 keys 0.436 ms: smaller tiles pay more per-tile
+// overhead).  Small sorts: 4, so that they have blocks enough for the SMs.
 constexpr int kRsThreads = 256;
 constexpr int kRsItems = 12;
-constexpr int kRsTile = kRsThreads * kRsItems;  // 3072
+constexpr int kRsItemsSmall = 4;
 constexpr int kRsWarps = kRsThreads / 32;
 
-template <class K, int BITS>
+template <class K, int BITS, int ITEMS>
 __global__ void __launch_bounds__(kRsThreads) k_rs_hist(const K* __restrict__ keys, uint32_t n, int shift,
                                                         uint32_t* __restrict__ counts, uint32_t ntiles)
 {
@@ -225,15 +146,15 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_hist(const K* __restrict__ ke
     __syncthreads();
     // every load of the tile is issued before the first shared-memory atomic
     // (one round trip to memory per thread instead of one per few keys)
-    uint32_t base = blockIdx.x * kRsTile;
-    K kk[kRsItems];
+    uint32_t base = blockIdx.x * (kRsThreads * ITEMS);
+    K kk[ITEMS];
 #pragma unroll
-    for (int k = 0; k < kRsItems; k++) {
+    for (int k = 0; k < ITEMS; k++) {
         const uint32_t i = base + k * kRsThreads + threadIdx.x;
         kk[k] = i < n ? keys[i] : (K)0;
     }
 #pragma unroll
-    for (int k = 0; k < kRsItems; k++) {
+    for (int k = 0; k < ITEMS; k++) {
         const uint32_t i = base + k * kRsThreads + threadIdx.x;
         if (i < n) atomicAdd(&h[(uint32_t)(kk[k] >> shift) & (kDig - 1u)], 1u);
     }
@@ -241,11 +162,45 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_hist(const K* __restrict__ ke
     for (uint32_t d = threadIdx.x; d < kDig; d += kRsThreads) counts[d * ntiles + blockIdx.x] = h[d];
 }
 
-template <class K, int BITS>
+// Exclusive scan of every digit's tile counts, a warp per digit, in place; the
+// digit's total to totals[d].  (The counts of all digits as one sequence took
+// two launches: tiles of 4,096 counts and their sums.)
+template <int BITS>
+__global__ void __launch_bounds__(256) k_rs_scan(uint32_t* __restrict__ counts, uint32_t* __restrict__ totals, uint32_t ntiles)
+{
+    pdl_enter();
+    const uint32_t d = blockIdx.x * 8u + (threadIdx.x >> 5), lane = threadIdx.x & 31u;
+    uint32_t* const c = counts + (size_t)d * ntiles;
+    uint32_t run = 0;
+    constexpr int kAhead = 4;  // chunks of 32 counts in flight
+    for (uint32_t t0 = 0; t0 < ntiles; t0 += 32u * kAhead) {
+        uint32_t v[kAhead];
+#pragma unroll
+        for (int q = 0; q < kAhead; q++) {
+            const uint32_t t = t0 + 32u * q + lane;
+            v[q] = t < ntiles ? c[t] : 0u;
+        }
+#pragma unroll
+        for (int q = 0; q < kAhead; q++) {
+            uint32_t x = v[q];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= (uint32_t)o) x += y;
+            }
+            const uint32_t t = t0 + 32u * q + lane;
+            if (t < ntiles) c[t] = run + x - v[q];
+            run += __shfl_sync(0xffffffffu, x, 31);
+        }
+    }
+    if (lane == 0) totals[d] = run;
+}
+
+template <class K, int BITS, int ITEMS>
 __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const K* __restrict__ kin, const uint32_t* __restrict__ vin,
                                                            K* __restrict__ kout, uint32_t* __restrict__ vout, uint32_t n,
                                                            int shift, const uint32_t* __restrict__ offsets,
-                                                           const uint32_t* __restrict__ tile_sums, uint32_t ntiles)
+                                                           const uint32_t* __restrict__ totals, uint32_t ntiles)
 {
     pdl_enter();
     constexpr uint32_t kDig = 1u << BITS;
@@ -253,19 +208,32 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const K* __restrict__
     __shared__ uint32_t tile_off[kDig];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     for (uint32_t d = lane; d < kDig; d += 32) wc[w][d] = 0;
-    for (uint32_t d = threadIdx.x; d < kDig; d += kRsThreads) {
-        const uint32_t j = d * ntiles + blockIdx.x;
-        tile_off[d] = offsets[j] + (tile_sums ? tile_sums[j / kScanTile] : 0u);
+    {
+        // a digit's place: the digits before it (a scan of the totals, four per
+        // thread) and its keys in the tiles before this one
+        static_assert(kDig == 4u * kRsThreads, "four digits per thread");
+        __shared__ uint32_t sw[33];
+        const uint4 t4 = __ldg(reinterpret_cast<const uint4*>(totals) + threadIdx.x);
+        const uint32_t d = 4u * threadIdx.x;
+        uint32_t o4[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) o4[q] = offsets[(size_t)(d + q) * ntiles + blockIdx.x];
+        uint32_t tot;
+        const uint32_t base = block_exclusive_scan(t4.x + t4.y + t4.z + t4.w, sw, &tot);
+        tile_off[d] = base + o4[0];
+        tile_off[d + 1] = base + t4.x + o4[1];
+        tile_off[d + 2] = base + t4.x + t4.y + o4[2];
+        tile_off[d + 3] = base + t4.x + t4.y + t4.z + o4[3];
     }
     __syncwarp();
-    const uint32_t seg = blockIdx.x * kRsTile + w * 32 * kRsItems;
-    K key[kRsItems];
-    uint32_t val[kRsItems];
-    uint32_t rank[kRsItems];
-    uint32_t dig[kRsItems];
+    const uint32_t seg = blockIdx.x * (kRsThreads * ITEMS) + w * 32 * ITEMS;
+    K key[ITEMS];
+    uint32_t val[ITEMS];
+    uint32_t rank[ITEMS];
+    uint32_t dig[ITEMS];
     const unsigned lt = (1u << lane) - 1u;
 #pragma unroll
-    for (int c = 0; c < kRsItems; c++) {
+    for (int c = 0; c < ITEMS; c++) {
         uint32_t i = seg + c * 32 + lane;
         bool ok = i < n;
         key[c] = ok ? kin[i] : (K)0;
@@ -292,7 +260,7 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const K* __restrict__
     }
     __syncthreads();
 #pragma unroll
-    for (int c = 0; c < kRsItems; c++) {
+    for (int c = 0; c < ITEMS; c++) {
         uint32_t d = dig[c];
         if (d < kDig) {
             uint32_t pos = tile_off[d] + wc[w][d] + rank[c];
@@ -305,31 +273,30 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const K* __restrict__
 // Sorts (keys, vals) by the low `bits` bits of the key in passes of BITS-bit
 // digits.  The passes alternate between the two buffer pairs; on return
 // (k0, v0) point to the pair that holds the result and (k1, v1) to the other
-// (swapped after an odd number of passes, nothing copied).  Scratch: counts
-// radix_counts_words<BITS>(n) words, scan temp.  hist0_done: the producer of the
-// keys already wrote the first pass's per-tile digit counts into `counts`
-// (layout of k_rs_hist: digit-major, one column per kRsTile keys).
-template <class K, int BITS = 8>
-void radix_sort(K*& k0, uint32_t*& v0, K*& k1, uint32_t*& v1, uint32_t n, int bits, uint32_t* counts, uint32_t* temp,
-                cudaStream_t st, bool hist0_done = false)
+// (swapped after an odd number of passes, nothing copied).  Scratch: 2^BITS
+// counts per tile of 256 x ITEMS keys, 2^BITS totals.  The producer of the keys
+// has already written the first pass's per-tile digit counts into `counts`
+// (layout of k_rs_hist: digit-major, one column per tile).
+template <class K, int BITS, int ITEMS>
+void radix_sort(K*& k0, uint32_t*& v0, K*& k1, uint32_t*& v1, uint32_t n, int bits, uint32_t* counts, uint32_t* totals,
+                cudaStream_t st)
 {
     if (n <= 1) return;
-    uint32_t ntiles = (n + kRsTile - 1) / kRsTile;
+    const uint32_t tile = kRsThreads * ITEMS, ntiles = (n + tile - 1) / tile;
     int passes = (bits + BITS - 1) / BITS;
     K* ks = k0;
     uint32_t* vs = v0;
     K* kd = k1;
     uint32_t* vd = v1;
     for (int p = 0; p < passes; p++) {
-        if (p > 0 || !hist0_done) {
-            launch_dep(k_rs_hist<K, BITS>, ntiles, kRsThreads, st, (const K*)ks, n, BITS * p, counts, ntiles);
+        if (p > 0) {
+            launch_dep(k_rs_hist<K, BITS, ITEMS>, ntiles, kRsThreads, st, (const K*)ks, n, BITS * p, counts, ntiles);
             note_launches(1);
         }
-        const uint32_t* sums = nullptr;
-        scan_exclusive_split(counts, counts, (1u << BITS) * ntiles, temp, &sums, st);
-        launch_dep(k_rs_scatter<K, BITS>, ntiles, kRsThreads, st, (const K*)ks, (const uint32_t*)vs, kd, vd, n,
-                   BITS * p, (const uint32_t*)counts, sums, ntiles);
-        note_launches(1);
+        launch_dep(k_rs_scan<BITS>, (1u << BITS) / 8u, 256, st, counts, totals, ntiles);
+        launch_dep(k_rs_scatter<K, BITS, ITEMS>, ntiles, kRsThreads, st, (const K*)ks, (const uint32_t*)vs, kd, vd, n,
+                   BITS * p, (const uint32_t*)counts, (const uint32_t*)totals, ntiles);
+        note_launches(2);
         K* tk = ks;
         ks = kd;
         kd = tk;
@@ -341,12 +308,6 @@ void radix_sort(K*& k0, uint32_t*& v0, K*& k1, uint32_t*& v1, uint32_t n, int bi
     v1 = vd;
     k0 = ks;
     v0 = vs;
-}
-
-template <int BITS = 8>
-inline size_t radix_counts_words(uint32_t n)
-{
-    return (1ull << BITS) * ((n + kRsTile - 1) / kRsTile);
 }
 
 }  // namespace gi
