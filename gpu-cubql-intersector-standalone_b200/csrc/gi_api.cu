@@ -594,15 +594,17 @@ static gi_status pinned_for(gi_ctx* c, PinnedBuf** buf, size_t need)
 // One host synchronisation per call: every kernel takes its sizes from the
 // device counters, and the results are copied back speculatively at the size
 // of the previous call (a second copy follows only when the result grew).
-static gi_status run_jobs(gi_ctx* c, const std::vector<JobDev>& jobs, const gi_intersect_opts& o,
+static gi_status run_jobs(gi_ctx* c, std::vector<JobDev>& jobs, const gi_intersect_opts& o,
                           std::vector<gi_result*>& outs)
 {
     const uint32_t nj = (uint32_t)jobs.size();
     const int prec = o.precision_mode == GI_PREC_FP64 ? 1 : 0;
     const bool want_segs = o.want_segments != 0;
     const bool sort = o.sort_output != 0;
-    uint64_t maxA = 1, maxB = 1, sumT = 0;
-    for (const auto& j : jobs) {
+    uint64_t maxA = 1, maxB = 1, sumA = 0, sumT = 0;
+    for (auto& j : jobs) {
+        j.a0 = sumA;
+        sumA += j.A.nt;
         maxA = std::max<uint64_t>(maxA, j.A.nt);
         maxB = std::max<uint64_t>(maxB, j.B.nt);
         sumT += j.A.nt + j.B.nt;
@@ -652,7 +654,7 @@ static gi_status run_jobs(gi_ctx* c, const std::vector<JobDev>& jobs, const gi_i
     // the previous call's count says is small enough (the kernel refuses, and
     // this loop reruns on the general path, if it is not, or if its keys crowd
     // into one partition; a refusal keeps the next calls off this path a while)
-    bool fin = sort && ba + bb + bj <= 63 && c->pred_pairs <= kFinMax - kFinMax / 4 && c->fin_backoff == 0;
+    bool fin = sort && ba + bb + bj <= 63 && c->pred_pairs + c->pred_pairs / 16 <= kFinMax && c->fin_backoff == 0;
     if (c->fin_backoff) c->fin_backoff--;
     const int shape = c->shape;
     for (;;) {
@@ -720,8 +722,12 @@ static gi_status run_jobs(gi_ctx* c, const std::vector<JobDev>& jobs, const gi_i
         gi_status s = pinned_for(c, &buf, off_segpair + sizeof(int32_t) * (size_t)ps + 64);
         if (s != GI_OK) return s;
         hp = (char*)buf->p;
-        if (!c->fin_mem) {
-            CK(c, pool_alloc(&c->fin_mem, fin_scratch_bytes(), c->pool, c->st), "finish scratch");
+        const int bucket = c->pred_pairs <= 65536 ? kFinBucketSmall : kFinBucketLarge;
+        if (!c->fin_mem || c->fin_bucket < bucket) {
+            if (c->fin_mem) cudaFreeAsync(c->fin_mem, c->st);
+            c->fin_mem = nullptr;
+            CK(c, pool_alloc(&c->fin_mem, fin_scratch_bytes(bucket), c->pool, c->st), "finish scratch");
+            c->fin_bucket = bucket;
             c->cur_clear = false;
         }
         if (!c->cur_clear) {
@@ -730,7 +736,7 @@ static gi_status run_jobs(gi_ctx* c, const std::vector<JobDev>& jobs, const gi_i
             CK(c, cudaMemsetAsync(fin_counts(c->fin_mem, c->cur), 0, sizeof(uint32_t) * 2 * kFinParts, c->st), "finish counts");
         }
         c->cur_clear = false;
-        b.fin = make_fin_bufs(c->fin_mem, c->cur, ba, bb, bj);
+        b.fin = make_fin_bufs(c->fin_mem, c->fin_bucket, c->cur, ba, bb, sumA, maxB);
         b.fin.on = fin ? 1 : 0;
         b.fin.segments = want_segs ? 1 : 0;
         if (!jobs_there && (nj > 1 || !fin)) {

@@ -286,6 +286,7 @@ struct gi_ctx {
     int cur = 0;
     bool cur_clear = false;     // set `cur` is zero
     void* fin_mem = nullptr;    // partitions of the one-launch finish (gi::FinBufs)
+    int fin_bucket = 0;         // ... keys per bucket it was made for
     Counters* h_cnt = nullptr;  // pinned
     unsigned* h_words = nullptr;  // pinned: error words of a pair-list call
     JobDev* d_jobs = nullptr;

@@ -88,8 +88,10 @@ constexpr int kCutMax = 64;    // 4^3
 constexpr int kCut4Max = 256;  // 4^4
 constexpr int kCutCap = kCutMax + kCut4Max;
 
-struct JobDev {
+struct __align__(16) JobDev {
     MeshDev A, B;
+    unsigned long long a0;  // triangles of A in the jobs before this one
+    unsigned long long pad_;
     DevPose pa, pb;
 };
 
@@ -136,17 +138,22 @@ constexpr unsigned kRedoCount = 1u, kRedoCrowded = 2u;
 // found, read by k_finish.
 constexpr int kFinPartBits = 12;
 constexpr int kFinParts = 1 << kFinPartBits;
-constexpr int kFinBucket = 256;
-constexpr int kFinOverflow = 1 << 14;
+constexpr int kFinOverflow = 1 << 16;
+// keys of a partition's bucket: up to 65,536 expected results, and beyond (a
+// partition then holds 16 to 64 keys on average, but results cluster in index)
+constexpr int kFinBucketSmall = 256, kFinBucketLarge = 1024;
 struct FinBufs {
     uint32_t* count;  // kFinParts key counts (zero when a call begins)
     uint32_t* extra;  // kFinParts: segments beyond one per key, modulo 2^32 (zero when a call begins)
-    unsigned long long* bkey;  // kFinParts x kFinBucket: each partition's first keys
+    unsigned long long* bkey;  // kFinParts x bucket: each partition's first keys
     uint32_t* bval;            // ... and their result index | segment count << 30
     unsigned long long* okey;  // kFinOverflow: the keys beyond a bucket
-    uint2* oval;               // ... their value and their slot in the partition
-    int shift;                 // partition of a key = key >> shift
+    uint2* oval;               // ... their value, and their slot in the partition | partition << 20
+    int bucket;
     int bits_a, bits_b;
+    // partition of a result: its rank among all conceivable pairs, ((A triangles of
+    // the earlier jobs + a) * stride + b), times scale / 2^64
+    unsigned long long stride, scale;
     int on;                    // 1: results are inserted
     int segments;              // the call wants segments
 };

@@ -1210,28 +1210,33 @@ __device__ __forceinline__ uint32_t code_segments(unsigned code)
     return kind == 3u ? 3u : (kind ? 1u : 0u);
 }
 
-// A result's key into its partition (the key's top kFinPartBits bits), for the
-// one-launch finish: into the partition's bucket at the slot that one atomic on
-// its count returns, or beyond the bucket on one overflow list.  ns: its
-// segments (1 unless the exact stage found it).
+// A result's key into its partition, for the one-launch finish: into the
+// partition's bucket at the slot that one atomic on its count returns, or beyond
+// the bucket on one overflow list.  The partitions divide the conceivable pairs
+// evenly, in order (by the key's top bits, a job with a small mesh A had all its
+// results in one partition).  ns: the result's segments (1 unless the exact
+// stage found it).
 __device__ __forceinline__ unsigned long long fin_key(const FinBufs& F, uint32_t job, uint32_t a, uint32_t b)
 {
     return ((unsigned long long)job << (F.bits_a + F.bits_b)) | ((unsigned long long)a << F.bits_b) | b;
 }
+template <bool MULTI>
 __device__ __forceinline__ void fin_insert(const Bufs& B, const uint4& r, uint32_t idx, unsigned ns)
 {
     const FinBufs& F = B.fin;
     const unsigned long long key = fin_key(F, r.x, r.y, r.z);
-    const unsigned part = (unsigned)(key >> F.shift), slot = atomicAdd(F.count + part, 1u);
+    const unsigned long long rank = (job_at<MULTI>(B, r.x).a0 + r.y) * F.stride + r.z;
+    const unsigned part = min((unsigned)__umul64hi(rank, F.scale), (unsigned)kFinParts - 1u);
+    const unsigned slot = atomicAdd(F.count + part, 1u);
     const uint32_t v = idx | (ns << 30);
-    if (slot < (unsigned)kFinBucket) {
-        F.bkey[part * kFinBucket + slot] = key;
-        F.bval[part * kFinBucket + slot] = v;
+    if (slot < (unsigned)F.bucket) {
+        F.bkey[(size_t)part * F.bucket + slot] = key;
+        F.bval[(size_t)part * F.bucket + slot] = v;
     } else {
         const unsigned o = atomicAdd(&B.cnt->fin_over, 1u);
         if (o < (unsigned)kFinOverflow) {
             F.okey[o] = key;
-            F.oval[o] = make_uint2(v, slot);
+            F.oval[o] = make_uint2(v, slot | (part << 20));
         }
     }
     if (ns != 1u) {
@@ -1252,7 +1257,7 @@ __device__ __forceinline__ void block_flush(const Bufs& B, BlockShared<F64, MULT
     for (unsigned k = threadIdx.x; k < nres; k += kBlkThreads) {
         if (base + k < B.cap_res) {
             B.res[base + k] = s.res[k];
-            if (B.fin.on) fin_insert(B, s.res[k], base + k, 1u);
+            if (B.fin.on) fin_insert<MULTI>(B, s.res[k], base + k, 1u);
         } else {
             atomicOr(&B.cnt->overflow, kOvfRes);
         }
@@ -1729,7 +1734,7 @@ __device__ __forceinline__ void exact_stage(const Bufs& B, unsigned gtid, unsign
             const uint4 r = make_uint4(job, ta, tb, code);
             if (pr < B.cap_res) {
                 B.res[pr] = r;
-                if (B.fin.on) fin_insert(B, r, pr, B.fin.segments ? code_segments(code) : 1u);
+                if (B.fin.on) fin_insert<MULTI>(B, r, pr, B.fin.segments ? code_segments(code) : 1u);
             } else {
                 atomicOr(&C->overflow, kOvfRes);
             }
@@ -2386,11 +2391,12 @@ cudaError_t launch_order_small_phases(const Bufs& b, const OrderBufs& O, bool so
 // meshes 153 -> 115 us.
 // ===========================================================================
 constexpr int kFinThreads = 256;
-constexpr unsigned kFinRun = 256;   // most positions of a block (kFinMax over the smallest grid)
+constexpr unsigned kFinRun = 1024;  // most positions of a block (two blocks per SM fit with it)
+constexpr unsigned kFinPart = 256;  // results constructed and written at a time
 constexpr unsigned kFinRank = 256;  // keys of a partition ranked by counting; larger ones are sorted
 constexpr unsigned kFinKeys = kFinRun + 2 * kFinBig;  // a run meets at most two partitions that it does not fill
 static_assert(kFinParts == 16 * kFinThreads, "a thread scans 16 partitions");
-static_assert(kFinRank == (unsigned)kFinBucket, "a partition has keys on the overflow list when, and only when, it is sorted");
+static_assert(kFinMax <= (1u << 20) && kFinParts <= (1 << 12), "slot and partition share a word");
 static_assert(kFinMax <= (1u << 30), "a bucket value holds the result index below bit 30");
 
 struct FinShared {
@@ -2401,11 +2407,11 @@ struct FinShared {
             unsigned long long key[kFinKeys];
             uint32_t val[kFinKeys];
         } g;                                  // gathered keys
-        double seg[kFinRun * 3 * 6];          // the run's segments, in order
+        double seg[kFinPart * 3 * 6];         // segments on their way out, in order
     } u;
     unsigned long long skey[kFinRun];  // the run's keys in order, their values and segment offsets
     uint32_t sval[kFinRun];
-    uint32_t sseg[kFinRun + 1];
+    uint32_t sseg[kFinRun];
     uint32_t warp[2][kFinThreads / 32];
     uint32_t big[32];
     unsigned nbig, ok, last;
@@ -2489,7 +2495,10 @@ __global__ void __launch_bounds__(kFinThreads, 2) k_finish(const __grid_constant
     Counters* C = B.cnt;
     const unsigned tid = threadIdx.x;
     const unsigned gtid = blockIdx.x * kFinThreads + tid, nth = gridDim.x * kFinThreads;
-    if (tid == 0) s.ok = 1u;
+    if (tid == 0) {
+        s.ok = 1u;
+        s.nbig = 0u;
+    }
     fin_stamp(C, 0);
     // the next call's counters and partition counts
     for (unsigned w = gtid; w < 2u * kFinParts / 4u; w += nth) reinterpret_cast<uint4*>(F.next_count)[w] = make_uint4(0u, 0u, 0u, 0u);
@@ -2560,37 +2569,37 @@ __global__ void __launch_bounds__(kFinThreads, 2) k_finish(const __grid_constant
     }
     const unsigned p0 = fin_part(s.koff, lo), p1 = fin_part(s.koff, hi - 1u) + 1u;
     const unsigned base = s.koff[p0], m = min(s.koff[p1] - base, kFinKeys);
-    if (tid == 0) s.nbig = 0u;
     bool spill = false;
     for (unsigned t = tid; t < m; t += kFinThreads) {
         const unsigned part = fin_part(s.koff, base + t), slot = base + t - s.koff[part];
-        if (slot < (unsigned)kFinBucket) {
-            s.u.g.key[t] = __ldcg(B.fin.bkey + part * kFinBucket + slot);
-            s.u.g.val[t] = __ldcg(B.fin.bval + part * kFinBucket + slot);
+        if (slot < (unsigned)B.fin.bucket) {
+            s.u.g.key[t] = __ldcg(B.fin.bkey + (size_t)part * B.fin.bucket + slot);
+            s.u.g.val[t] = __ldcg(B.fin.bval + (size_t)part * B.fin.bucket + slot);
         } else {
             spill = true;
+        }
+        if (slot == kFinRank) {  // one of its keys lists a partition that is sorted
+            const unsigned at = atomicAdd(&s.nbig, 1u);
+            if (at < 32u) s.big[at] = part;
         }
     }
     if (__syncthreads_or(spill)) {
         // keys beyond a bucket: found on the overflow list, their slots with them
         for (unsigned t = tid; t < over; t += kFinThreads) {
             const unsigned long long key = __ldcg(B.fin.okey + t);
-            const unsigned part = (unsigned)(key >> B.fin.shift);
+            const uint2 v = __ldcg(B.fin.oval + t);
+            const unsigned part = v.y >> 20;
             if (part >= p0 && part < p1) {
-                const uint2 v = __ldcg(B.fin.oval + t);
-                const unsigned at = s.koff[part] - base + v.y;
+                const unsigned at = s.koff[part] - base + (v.y & 0xfffffu);
                 if (at < m) {
                     s.u.g.key[at] = key;
                     s.u.g.val[at] = v.x;
                 }
             }
         }
-        for (unsigned part = p0 + tid; part < p1; part += kFinThreads)
-            if (s.koff[part + 1u] - s.koff[part] > kFinRank) {
-                const unsigned at = atomicAdd(&s.nbig, 1u);
-                if (at < 32u) s.big[at] = part;
-            }
         __syncthreads();
+    }
+    if (s.nbig) {
         const unsigned nbig = min(s.nbig, 32u);
         for (unsigned q = 0; q < nbig; q++) {
             // bitonic sort of one partition, every comparison ascending (the first
@@ -2648,7 +2657,7 @@ __global__ void __launch_bounds__(kFinThreads, 2) k_finish(const __grid_constant
     __syncthreads();  // the gathered keys are done with: their place takes the segments
     fin_stamp(C, 2);
     // ---- phase 2: constructions, and the run out in order ----
-    const unsigned cnt = hi - lo, s0 = s.sseg[0];
+    const unsigned cnt = hi - lo;
     const unsigned idx_mask = (1u << 30) - 1u;
     int32_t* const pairs = fits ? F.h_pairs : F.pairs_out;
     {
@@ -2661,19 +2670,23 @@ __global__ void __launch_bounds__(kFinThreads, 2) k_finish(const __grid_constant
     }
     if (F.want_segments) {
         int32_t* const segpair = fits ? F.h_segpair : F.segpair_out;
-        for (unsigned j = tid >> 1; j < cnt; j += kFinThreads / 2) {
-            const uint32_t v = s.sval[j], ns = v >> 30;
-            const unsigned so = s.sseg[j];
-            if (!ns) continue;
-            const uint4 rr = __ldcg(B.res + (v & idx_mask));
-            result_segments<MULTI>(B, rr, s.u.seg + 6u * (so - s0), tid & 1u, 2u);
-            for (unsigned e = tid & 1u; e < ns; e += 2u) segpair[so + e] = (int32_t)(lo + j);
+        for (unsigned q = 0; q < cnt; q += kFinPart) {
+            const unsigned end = min(cnt, q + kFinPart), s0 = s.sseg[q];
+            for (unsigned j = q + (tid >> 1); j < end; j += kFinThreads / 2) {
+                const uint32_t v = s.sval[j], ns = v >> 30;
+                const unsigned so = s.sseg[j];
+                if (!ns) continue;
+                const uint4 rr = __ldcg(B.res + (v & idx_mask));
+                result_segments<MULTI>(B, rr, s.u.seg + 6u * (so - s0), tid & 1u, 2u);
+                for (unsigned e = tid & 1u; e < ns; e += 2u) segpair[so + e] = (int32_t)(lo + j);
+            }
+            __syncthreads();
+            const unsigned s1 = s.sseg[end - 1u] + (s.sval[end - 1u] >> 30);
+            double2* const out = reinterpret_cast<double2*>((fits ? F.h_segs : F.segs_out) + 6 * (size_t)s0);
+            const double2* const in = reinterpret_cast<const double2*>(s.u.seg);
+            for (unsigned t = tid; t < 3u * (s1 - s0); t += kFinThreads) out[t] = in[t];
+            __syncthreads();  // read before the next part's segments take its place
         }
-        __syncthreads();
-        const unsigned s1 = s.sseg[cnt - 1u] + (s.sval[cnt - 1u] >> 30);
-        double2* const out = reinterpret_cast<double2*>((fits ? F.h_segs : F.segs_out) + 6 * (size_t)s0);
-        const double2* const in = reinterpret_cast<const double2*>(s.u.seg);
-        for (unsigned t = tid; t < 3u * (s1 - s0); t += kFinThreads) out[t] = in[t];
     }
     fin_stamp(C, 3);
     fin_end(C, F.host_cnt, s);
@@ -2682,28 +2695,30 @@ __global__ void __launch_bounds__(kFinThreads, 2) k_finish(const __grid_constant
 // Layout of the partition memory: two sets of counts (keys, extra segments),
 // then the buckets and the overflow list, which both sets share (a call's are
 // done with when the next begins).
-size_t fin_scratch_bytes()
+size_t fin_scratch_bytes(int bucket)
 {
-    return sizeof(uint32_t) * 4 * kFinParts + (sizeof(unsigned long long) + sizeof(uint32_t)) * (size_t)kFinParts * kFinBucket +
+    return sizeof(uint32_t) * 4 * kFinParts + (sizeof(unsigned long long) + sizeof(uint32_t)) * (size_t)kFinParts * bucket +
            (sizeof(unsigned long long) + sizeof(uint2)) * kFinOverflow;
 }
 uint32_t* fin_counts(void* mem, int set)
 {
     return (uint32_t*)mem + (size_t)set * 2 * kFinParts;
 }
-FinBufs make_fin_bufs(void* mem, int set, int bits_a, int bits_b, int bits_job)
+FinBufs make_fin_bufs(void* mem, int bucket, int set, int bits_a, int bits_b, uint64_t sum_a, uint64_t max_b)
 {
     FinBufs f;
     f.count = fin_counts(mem, set);
     f.extra = f.count + kFinParts;
     f.bkey = (unsigned long long*)((uint32_t*)mem + 4 * kFinParts);
-    f.okey = f.bkey + (size_t)kFinParts * kFinBucket;
+    f.okey = f.bkey + (size_t)kFinParts * bucket;
     f.oval = (uint2*)(f.okey + kFinOverflow);
     f.bval = (uint32_t*)(f.oval + kFinOverflow);
-    const int bits = bits_a + bits_b + bits_job;
-    f.shift = bits > kFinPartBits ? bits - kFinPartBits : 0;
+    f.bucket = bucket;
     f.bits_a = bits_a;
     f.bits_b = bits_b;
+    // rank * scale / 2^64 < kFinParts for every rank < sum_a * max_b (< 2^63: the keys' bits)
+    f.stride = max_b;
+    f.scale = (unsigned long long)(((unsigned __int128)kFinParts << 64) / std::max<unsigned __int128>((unsigned __int128)sum_a * max_b, kFinParts + 1));
     f.on = f.segments = 0;
     return f;
 }

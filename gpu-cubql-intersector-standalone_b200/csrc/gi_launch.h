@@ -136,7 +136,7 @@ cudaError_t launch_order_small_phases(const Bufs& b, const OrderBufs& O, bool so
 // keys, makes the kernel set only Counters::order_redo; the caller then reruns
 // on the general path (launch_exact, launch_segments, launch_order_gather).
 constexpr int kFinBig = 2048;
-constexpr uint32_t kFinMax = 1u << 16;
+constexpr uint32_t kFinMax = 1u << 18;
 struct FinArgs {
     // results in pinned host memory: for host_pairs pairs and host_segs segments
     int32_t* h_pairs;
@@ -155,9 +155,9 @@ struct FinArgs {
     Counters* next_cnt;    // cleared for the next call
     uint32_t* next_count;  // 2 x kFinParts, cleared for the next call
 };
-size_t fin_scratch_bytes();
+size_t fin_scratch_bytes(int bucket);
 uint32_t* fin_counts(void* mem, int set);
-FinBufs make_fin_bufs(void* mem, int set, int bits_a, int bits_b, int bits_job);
+FinBufs make_fin_bufs(void* mem, int bucket, int set, int bits_a, int bits_b, uint64_t sum_a, uint64_t max_b);
 // Launched right after the traversal on the same stream, with no other stream
 // work between them (programmatic dependent launch).
 cudaError_t launch_finish(const Bufs& b, const FinArgs& F, const LaunchCfg& cfg, cudaStream_t st);

@@ -56,3 +56,28 @@ def test_finish_partition_edges(gi, oc, k, odd):
                 _same(r, ref)
         A.release()
         B.release()
+
+
+def test_finish_large_and_uneven_batch(gi, oc):
+    """Over 65,536 results (the larger buckets, from the second call on), with
+    none to three segments each, alone and in a batch with a small job between
+    two large ones."""
+    from gpuintersector import meshgen as mg
+
+    grid, small = mg.config3(n=128, seed=9), mg.config1(seed=4)
+    refs = [oc.intersect_meshes(d["vA"], d["tA"], oc.pose_identity(), d["vB"], d["tB"], oc.pose_identity(),
+                                want_segments=True) for d in (grid, small)]
+    assert 65536 < len(refs[0]["pairs"]) < 120000
+    with gi.Context(0) as c:
+        G = (c.upload(grid["vA"], grid["tA"]), c.upload(grid["vB"], grid["tB"]))
+        S = (c.upload(small["vA"], small["tA"]), c.upload(small["vB"], small["tB"]))
+        for _ in range(3):
+            r = c.intersect(*G)
+            _same(r, refs[0])
+        assert r.stats["launches"] == 2
+        for _ in range(2):
+            rs = c.intersect_batch([(G[0], None, G[1], None), (S[0], None, S[1], None), (G[0], None, G[1], None)])
+            for r, ref in zip(rs, (refs[0], refs[1], refs[0])):
+                _same(r, ref)
+        for m in G + S:
+            m.release()
