@@ -594,8 +594,9 @@ static gi_status pinned_for(gi_ctx* c, PinnedBuf** buf, size_t need)
 // One host synchronisation per call: every kernel takes its sizes from the
 // device counters, and the results are copied back speculatively at the size
 // of the previous call (a second copy follows only when the result grew).
+// flat_offsets: not null for one result over all jobs (outs[0]), its offsets here.
 static gi_status run_jobs(gi_ctx* c, std::vector<JobDev>& jobs, const gi_intersect_opts& o,
-                          std::vector<gi_result*>& outs)
+                          std::vector<gi_result*>& outs, int64_t* flat_offsets)
 {
     const uint32_t nj = (uint32_t)jobs.size();
     const int prec = o.precision_mode == GI_PREC_FP64 ? 1 : 0;
@@ -635,6 +636,7 @@ static gi_status run_jobs(gi_ctx* c, std::vector<JobDev>& jobs, const gi_interse
     int retries = 0;
     uint32_t nres = 0, nsegs = 0;
     char* hp = nullptr;
+    bool segpair64 = false;  // the block's pair indices have 64 bits
     size_t off_jobs = 0, off_segs = 0, off_segpair = 0;
     // pinned block the results land in; returned to the pool on every early exit
     PinnedBuf* buf = nullptr;
@@ -719,7 +721,7 @@ static gi_status run_jobs(gi_ctx* c, std::vector<JobDev>& jobs, const gi_interse
         off_jobs = (sizeof(int32_t) * 2 * (size_t)pp + 15) & ~(size_t)15;
         off_segs = (off_jobs + (nj > 1 ? sizeof(uint32_t) * (size_t)pp : 0) + 15) & ~(size_t)15;
         off_segpair = off_segs + sizeof(double) * 6 * (size_t)ps;
-        gi_status s = pinned_for(c, &buf, off_segpair + sizeof(int32_t) * (size_t)ps + 64);
+        gi_status s = pinned_for(c, &buf, off_segpair + (flat_offsets ? sizeof(int64_t) : sizeof(int32_t)) * (size_t)ps + 64);
         if (s != GI_OK) return s;
         hp = (char*)buf->p;
         const int bucket = c->pred_pairs <= 65536 ? kFinBucketSmall : kFinBucketLarge;
@@ -754,6 +756,7 @@ static gi_status run_jobs(gi_ctx* c, std::vector<JobDev>& jobs, const gi_interse
             F.h_job = (uint32_t*)(hp + off_jobs);
             F.h_segs = (double*)(hp + off_segs);
             F.h_segpair = (int32_t*)(hp + off_segpair);
+            F.h_segpair64 = flat_offsets ? (int64_t*)(hp + off_segpair) : nullptr;
             F.host_pairs = pp;
             F.host_segs = ps;
             F.pairs_out = c->pairs_out;
@@ -844,7 +847,9 @@ static gi_status run_jobs(gi_ctx* c, std::vector<JobDev>& jobs, const gi_interse
         }
         nres = H.res;
         nsegs = want_segs ? H.nseg : 0;
+        segpair64 = fin && flat_offsets;
         if (nres > pp || nsegs > ps) {
+            segpair64 = false;
             // the result outgrew the speculative copy: copy it again at its real size
             off_jobs = (sizeof(int32_t) * 2 * (size_t)nres + 15) & ~(size_t)15;
             off_segs = (off_jobs + (nj > 1 ? sizeof(uint32_t) * (size_t)nres : 0) + 15) & ~(size_t)15;
@@ -892,56 +897,14 @@ static gi_status run_jobs(gi_ctx* c, std::vector<JobDev>& jobs, const gi_interse
         cudaEventElapsedTime(&ms_seg, c->ev[2], c->ev[3]);
         cudaEventElapsedTime(&ms_sort, c->ev[3], c->ev[4]);
     }
-    // split per job (sorted by job first)
-    std::vector<uint32_t> job_start(nj + 1, 0);
-    if (nj == 1) {
-        job_start[1] = nres;
-    } else {
-        const uint32_t* hj = (const uint32_t*)(hp + off_jobs);
-        for (uint32_t k = 0; k < nres; k++) job_start[hj[k] + 1]++;
-        for (uint32_t j = 0; j < nj; j++) job_start[j + 1] += job_start[j];
-    }
-    // results are views into the pinned block (no further copy); a batch's
-    // segment pair indices are rebased to each job in place
-    const int32_t* hpairs = (const int32_t*)hp;
-    const double* hsegs = (const double*)(hp + off_segs);
-    int32_t* hsegpair = (int32_t*)(hp + off_segpair);
-    for (uint32_t j = 0; j < nj; j++) {
-        outs[j] = new (std::nothrow) gi_result();
-        if (!outs[j]) {
-            for (uint32_t k = 0; k < j; k++) {
-                delete outs[k];
-                outs[k] = nullptr;
-            }
-            return set_err(c, GI_ERR_OOM, "result");
-        }
-    }
-    buf->refs.store((int)nj);
-    buf->home = c->pinned;
-    size_t sp = 0;
-    for (uint32_t j = 0; j < nj; j++) {
-        gi_result* r = outs[j];
-        r->buf = buf;
-        uint32_t a = job_start[j], e = job_start[j + 1];
-        r->pairs = hpairs + 2 * (size_t)a;
-        r->npairs = e - a;
-        size_t s0 = sp;
-        if (nj == 1) sp = nsegs;  // one job: all segments are its own
-        else
-            while (sp < nsegs && (uint32_t)hsegpair[sp] < e) sp++;
-        r->segs = hsegs + 6 * s0;
-        r->seg_pair = hsegpair + s0;
-        r->nsegs = sp - s0;
-        if (a)
-            for (size_t q = s0; q < sp; q++) hsegpair[q] -= (int32_t)a;
-        gi_stats& s2 = r->stats;
+    auto fill_stats = [&](gi_stats& s2, uint32_t j, uint64_t npairs, uint64_t njsegs) {
         memset(&s2, 0, sizeof s2);
         s2.tris_a = jobs[j].A.nt;
         s2.tris_b = jobs[j].B.nt;
         s2.nodes_a = jobs[j].A.nnodes;
         s2.nodes_b = jobs[j].B.nnodes;
-        s2.pairs = e - a;
-        s2.segments = r->nsegs;
+        s2.pairs = npairs;
+        s2.segments = njsegs;
         // launch-wide counters (shared by all jobs of a batch)
         s2.node_pairs = H.node_pairs;
         s2.candidates = H.tested;
@@ -963,6 +926,92 @@ static gi_status run_jobs(gi_ctx* c, std::vector<JobDev>& jobs, const gi_interse
                 s2.finish_ms[k] = H.fin_ns[k + 1] >= H.fin_ns[0] ? 1e-6 * double(H.fin_ns[k + 1] - H.fin_ns[0]) : 0.0;
             s2.finish_phases = 4;
         }
+    };
+    const int32_t* hpairs = (const int32_t*)hp;
+    const double* hsegs = (const double*)(hp + off_segs);
+    int32_t* hsegpair = (int32_t*)(hp + off_segpair);
+    const uint32_t* hj = nj > 1 ? (const uint32_t*)(hp + off_jobs) : nullptr;
+    if (flat_offsets) {
+        // the arrays stay as they came, ordered by job
+        gi_result* r = outs[0] = new (std::nothrow) gi_result();
+        if (!r) return set_err(c, GI_ERR_OOM, "result");
+        r->flat = true;
+        r->pairs = hpairs;
+        r->npairs = nres;
+        r->segs = hsegs;
+        r->nsegs = nsegs;
+        if (hj) {
+            r->job = hj;
+            std::fill(flat_offsets, flat_offsets + nj + 1, (int64_t)0);
+            if (sort) {
+                for (uint32_t j = 0; j < nj; j++)
+                    flat_offsets[j + 1] = std::upper_bound(hj + flat_offsets[j], hj + nres, j) - hj;
+            } else {
+                for (uint32_t k = 0; k < nres; k++) flat_offsets[hj[k] + 1]++;
+                for (uint32_t j = 0; j < nj; j++) flat_offsets[j + 1] += flat_offsets[j];
+            }
+        } else {
+            r->job_own.assign(nres, 0u);
+            r->job = r->job_own.data();
+            flat_offsets[0] = 0;
+            flat_offsets[1] = nres;
+        }
+        if (segpair64) {
+            r->seg_pair64 = (const int64_t*)(hp + off_segpair);
+        } else {
+            r->seg_pair_own.assign(hsegpair, hsegpair + nsegs);
+            r->seg_pair64 = r->seg_pair_own.data();
+        }
+        const int64_t* const sp64 = r->seg_pair64;
+        fill_stats(r->stats, 0, (uint64_t)flat_offsets[1],
+                   (uint64_t)(std::lower_bound(sp64, sp64 + nsegs, flat_offsets[1]) - sp64));
+        buf->refs.store(1);
+        buf->home = c->pinned;
+        c->pinned->held += buf->bytes;
+        r->buf = buf;
+        buf = nullptr;  // now held by the result
+        return GI_OK;
+    }
+    // split per job (sorted by job first)
+    std::vector<uint32_t> job_start(nj + 1, 0);
+    if (nj == 1) {
+        job_start[1] = nres;
+    } else {
+        for (uint32_t k = 0; k < nres; k++) job_start[hj[k] + 1]++;
+        for (uint32_t j = 0; j < nj; j++) job_start[j + 1] += job_start[j];
+    }
+    // results are views into the pinned block (no further copy); a batch's
+    // segment pair indices are rebased to each job in place
+    for (uint32_t j = 0; j < nj; j++) {
+        outs[j] = new (std::nothrow) gi_result();
+        if (!outs[j]) {
+            for (uint32_t k = 0; k < j; k++) {
+                delete outs[k];
+                outs[k] = nullptr;
+            }
+            return set_err(c, GI_ERR_OOM, "result");
+        }
+    }
+    buf->refs.store((int)nj);
+    buf->home = c->pinned;
+    c->pinned->held += buf->bytes;
+    size_t sp = 0;
+    for (uint32_t j = 0; j < nj; j++) {
+        gi_result* r = outs[j];
+        r->buf = buf;
+        uint32_t a = job_start[j], e = job_start[j + 1];
+        r->pairs = hpairs + 2 * (size_t)a;
+        r->npairs = e - a;
+        size_t s0 = sp;
+        if (nj == 1) sp = nsegs;  // one job: all segments are its own
+        else
+            while (sp < nsegs && (uint32_t)hsegpair[sp] < e) sp++;
+        r->segs = hsegs + 6 * s0;
+        r->seg_pair = hsegpair + s0;
+        r->nsegs = sp - s0;
+        if (a)
+            for (size_t q = s0; q < sp; q++) hsegpair[q] -= (int32_t)a;
+        fill_stats(r->stats, j, e - a, r->nsegs);
     }
     buf = nullptr;  // now held by the results
     return GI_OK;
@@ -982,8 +1031,8 @@ extern "C" gi_status gi_intersect(gi_ctx* c, const gi_mesh* A, const gi_pose* pa
     return gi_intersect_batch(c, &j, 1, opts, out);
 }
 
-extern "C" gi_status gi_intersect_batch(gi_ctx* c, const gi_pair_job* jobs, uint32_t nj, const gi_intersect_opts* opts,
-                                        gi_result** out)
+static gi_status batch_call(gi_ctx* c, const gi_pair_job* jobs, uint32_t nj, const gi_intersect_opts* opts,
+                            gi_result** out, int64_t* flat_offsets)
 {
     if (!c || !jobs || !out || nj == 0) return GI_ERR_INVALID_ARG;
     gi_intersect_opts o;
@@ -1007,13 +1056,26 @@ extern "C" gi_status gi_intersect_batch(gi_ctx* c, const gi_pair_job* jobs, uint
         jd[i].pb = make_dev_pose(j.pose_b);
     }
     std::vector<gi_result*> outs(nj, nullptr);
-    gi_status s = run_jobs(c, jd, o, outs);
+    gi_status s = run_jobs(c, jd, o, outs, flat_offsets);
     if (s != GI_OK) {
         for (auto* r : outs) delete r;
         return s;
     }
-    for (uint32_t i = 0; i < nj; i++) out[i] = outs[i];
+    for (uint32_t i = 0; i < (flat_offsets ? 1u : nj); i++) out[i] = outs[i];
     return GI_OK;
+}
+
+extern "C" gi_status gi_intersect_batch(gi_ctx* c, const gi_pair_job* jobs, uint32_t nj, const gi_intersect_opts* opts,
+                                        gi_result** out)
+{
+    return batch_call(c, jobs, nj, opts, out, nullptr);
+}
+
+extern "C" gi_status gi_intersect_batch_flat(gi_ctx* c, const gi_pair_job* jobs, uint32_t nj,
+                                             const gi_intersect_opts* opts, int64_t* offsets, gi_result** out)
+{
+    if (!offsets) return GI_ERR_INVALID_ARG;
+    return batch_call(c, jobs, nj, opts, out, offsets);
 }
 
 extern "C" gi_status gi_intersect_oneshot(gi_ctx* c, const double* vA, uint32_t nvA, const uint32_t* tA, uint32_t ntA,
@@ -1071,14 +1133,14 @@ extern "C" gi_status gi_intersect_oneshot(gi_ctx* c, const double* vA, uint32_t 
 // ---------------------------------------------------------------------------
 extern "C" gi_status gi_result_pairs(const gi_result* r, const int32_t** p, uint64_t* n)
 {
-    if (!r || !p || !n) return GI_ERR_INVALID_ARG;
+    if (!r || !p || !n || r->flat) return GI_ERR_INVALID_ARG;
     *p = r->pairs;
     *n = r->npairs;
     return GI_OK;
 }
 extern "C" gi_status gi_result_segments(const gi_result* r, const double** s, const int32_t** sp, uint64_t* n)
 {
-    if (!r || !s || !n) return GI_ERR_INVALID_ARG;
+    if (!r || !s || !n || r->flat) return GI_ERR_INVALID_ARG;
     *s = r->segs;
     if (sp) *sp = r->seg_pair;
     *n = r->nsegs;
@@ -1088,6 +1150,19 @@ extern "C" gi_status gi_result_stats(const gi_result* r, gi_stats* out)
 {
     if (!r || !out) return GI_ERR_INVALID_ARG;
     *out = r->stats;
+    return GI_OK;
+}
+extern "C" gi_status gi_result_view(const gi_result* r, gi_result_arrays* out)
+{
+    if (!r || !out) return GI_ERR_INVALID_ARG;
+    out->pairs_ab = r->pairs;
+    out->job = r->job;
+    out->npairs = r->npairs;
+    out->seg6 = r->segs;
+    out->seg_pair = r->seg_pair;
+    out->seg_pair64 = r->seg_pair64;
+    out->nsegs = r->nsegs;
+    out->held_bytes = r->buf && r->buf->home ? r->buf->home->held.load() : 0;
     return GI_OK;
 }
 extern "C" gi_status gi_result_free(gi_result* r)

@@ -176,6 +176,7 @@ struct PinnedPool {
     std::mutex mu;
     std::vector<PinnedBuf*> free_list;
     size_t free_bytes = 0;
+    std::atomic<size_t> held{0};  // bytes of the blocks that results hold
     // free blocks kept for reuse up to this many bytes; beyond it the smallest
     // are released.  Pinning and unpinning cost milliseconds and cudaFreeHost
     // waits for the device, so a serving loop whose round sizes vary must not
@@ -246,8 +247,10 @@ inline void pinned_release(PinnedBuf* b)
 {
     if (!b || b->refs.fetch_sub(1) != 1) return;
     std::shared_ptr<PinnedPool> pool = std::move(b->home);
-    if (pool) pool->put(b);
-    else {
+    if (pool) {
+        pool->held -= b->bytes;
+        pool->put(b);
+    } else {
         cudaFreeHost(b->p);
         delete b;
     }
@@ -260,6 +263,13 @@ struct gi_result {
     const double* segs = nullptr;
     const int32_t* seg_pair = nullptr;
     uint64_t nsegs = 0;
+    // whole-batch results: the job of each pair, 64-bit pair indices (in the block,
+    // or here when the block holds other forms)
+    bool flat = false;
+    const uint32_t* job = nullptr;
+    const int64_t* seg_pair64 = nullptr;
+    std::vector<uint32_t> job_own;
+    std::vector<int64_t> seg_pair_own;
     gi_stats stats;
 };
 

@@ -2678,7 +2678,10 @@ __global__ void __launch_bounds__(kFinThreads, 2) k_finish(const __grid_constant
                 if (!ns) continue;
                 const uint4 rr = __ldcg(B.res + (v & idx_mask));
                 result_segments<MULTI>(B, rr, s.u.seg + 6u * (so - s0), tid & 1u, 2u);
-                for (unsigned e = tid & 1u; e < ns; e += 2u) segpair[so + e] = (int32_t)(lo + j);
+                for (unsigned e = tid & 1u; e < ns; e += 2u) {
+                    if (fits && F.h_segpair64) F.h_segpair64[so + e] = (int64_t)(lo + j);
+                    else segpair[so + e] = (int32_t)(lo + j);
+                }
             }
             __syncthreads();
             const unsigned s1 = s.sseg[end - 1u] + (s.sval[end - 1u] >> 30);

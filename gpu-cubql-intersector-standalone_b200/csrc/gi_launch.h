@@ -143,6 +143,7 @@ struct FinArgs {
     uint32_t* h_job;  // batches only
     double* h_segs;
     int32_t* h_segpair;
+    int64_t* h_segpair64;  // not null: pair indices in this form instead
     uint32_t host_pairs, host_segs;
     // ... or, when they do not fit, in device memory (cap pairs, 3 segments each)
     int32_t* pairs_out;

@@ -172,16 +172,21 @@ class Context:
         self.check(rc, "gi_intersect")
         return Result(r)
 
+    @staticmethod
+    def _jobs(jobs):
+        arr = (_abi.PairJob * len(jobs))()
+        ident = pose_identity()
+        for j, (A, pa, B, pb) in zip(arr, jobs):
+            j.A = A.handle
+            j.B = B.handle
+            j.pose_a = pa if pa is not None else ident
+            j.pose_b = pb if pb is not None else ident
+        return arr
+
     def intersect_batch(self, jobs, want_segments=True, precision=GI_PREC_FP32_CASCADE, sort_output=True):
         """jobs: list of (A, pose_a, B, pose_b); returns a list of Result."""
         n = len(jobs)
-        arr = (_abi.PairJob * n)()
-        ident = pose_identity()
-        for i, (A, pa, B, pb) in enumerate(jobs):
-            arr[i].A = A.handle
-            arr[i].B = B.handle
-            arr[i].pose_a = pa if pa is not None else ident
-            arr[i].pose_b = pb if pb is not None else ident
+        arr = self._jobs(jobs)
         outs = (ctypes.c_void_p * n)()
         o = self._opts(want_segments, precision, sort_output)
         rc = self._lib.gi_intersect_batch(self.handle, arr, n, ctypes.byref(o), outs)
@@ -198,21 +203,17 @@ class Context:
           segments (M, 6) float64, seg_pair (M,) int64: index into pairs,
           stats: the launch-wide statistics of the call.
 
-        pairs and segments are views of the library's pinned result block
-        (all jobs' results lie in it back to back; copies are made otherwise)."""
+        The arrays are views of the library's pinned result block, which they
+        keep alive."""
         n = len(jobs)
-        arr = (_abi.PairJob * n)()
-        ident = pose_identity()
-        for i, (A, pa, B, pb) in enumerate(jobs):
-            arr[i].A = A.handle
-            arr[i].B = B.handle
-            arr[i].pose_a = pa if pa is not None else ident
-            arr[i].pose_b = pb if pb is not None else ident
-        outs = (ctypes.c_void_p * n)()
+        arr = self._jobs(jobs)
+        offsets = np.empty(n + 1, dtype=np.int64)
+        h = ctypes.c_void_p()
         o = self._opts(want_segments, precision, sort_output)
-        rc = self._lib.gi_intersect_batch(self.handle, arr, n, ctypes.byref(o), outs)
+        rc = self._lib.gi_intersect_batch_flat(self.handle, arr, n, ctypes.byref(o),
+                                               offsets.ctypes.data_as(ctypes.POINTER(ctypes.c_int64)), ctypes.byref(h))
         self.check(rc, "gi_intersect_batch")
-        return BatchResult([_ResultOwner(ctypes.c_void_p(outs[i])) for i in range(n)])
+        return BatchResult(h, offsets)
 
     def intersect_oneshot(self, vA, tA, vB, tB, pose_a=None, pose_b=None, want_segments=True,
                           precision=GI_PREC_FP32_CASCADE, sort_output=True):
@@ -420,21 +421,34 @@ class _View:
 
     __slots__ = ("__array_interface__", "owner")
 
-    def __init__(self, owner, addr, shape, dtype):
+    def __init__(self, owner, addr, shape, typestr):
         self.owner = owner
-        self.__array_interface__ = {"shape": shape, "typestr": np.dtype(dtype).str, "data": (addr, False),
-                                    "version": 3}
+        self.__array_interface__ = {"shape": shape, "typestr": typestr, "data": (addr, False), "version": 3}
+
+
+_I4, _U4, _I8, _F8 = (np.dtype(t).str for t in (np.int32, np.uint32, np.int64, np.float64))
+
+
+def _array(owner, addr, shape, typestr, view=True):
+    """Library memory as a numpy array: a view that keeps its owner, or a copy."""
+    if not shape[0]:
+        return np.zeros(shape, dtype=typestr)
+    a = np.asarray(_View(owner, addr, shape, typestr))
+    return a if view else a.copy()
 
 
 class Result:
     """Pairs (n, 2) int32 sorted by (a, b); segments (m, 6) float64; seg_pair (m,).
 
-    Results up to ZERO_COPY_BYTES are numpy views of the library's pinned result
-    block (no copy; the block is released when the last view is dropped);
-    larger ones are copied out and the block is released at once, so holding
-    many large results pins no host memory."""
+    The arrays are numpy views of the library's pinned result block (no copy; the
+    block is released when the last view is dropped) while the results of the
+    context hold at most ZERO_COPY_HELD bytes of pinned memory, and always up to
+    ZERO_COPY_BYTES; beyond that they are copied out and the block is released at
+    once, so holding many large results pins a bounded amount of memory.  (Copying
+    two coplanar 512 x 512 grids' 105 MB out took 18 ms of a 26 ms call.)"""
 
     ZERO_COPY_BYTES = 4 << 20
+    ZERO_COPY_HELD = 1 << 30
 
     __slots__ = ("_owner", "_stats", "_npairs", "_pairs", "_segments", "_seg_pair")
 
@@ -459,34 +473,19 @@ class Result:
     def _load(self):
         if self._pairs is not None:
             return
-        L = lib()
-        handle = self._owner.handle
-        p = ctypes.POINTER(ctypes.c_int32)()
-        n = ctypes.c_uint64()
-        L.gi_result_pairs(handle, ctypes.byref(p), ctypes.byref(n))
-        sp = ctypes.POINTER(ctypes.c_double)()
-        spp = ctypes.POINTER(ctypes.c_int32)()
-        m = ctypes.c_uint64()
-        L.gi_result_segments(handle, ctypes.byref(sp), ctypes.byref(spp), ctypes.byref(m))
-        npairs, nsegs = n.value, m.value
         owner = self._owner
-        zero_copy = 8 * npairs + 52 * nsegs <= self.ZERO_COPY_BYTES
+        v = _abi.ResultArrays()
+        lib().gi_result_view(owner.handle, ctypes.byref(v))
+        npairs, nsegs = v.npairs, v.nsegs
+        zero_copy = 8 * npairs + 52 * nsegs <= self.ZERO_COPY_BYTES or v.held_bytes <= self.ZERO_COPY_HELD
         if not zero_copy:
             self.stats  # read now: the handle is released once the arrays are copied
-
-        def arr(ptr, shape, dtype, count):
-            if count == 0:
-                return np.zeros(shape, dtype=dtype)
-            a = np.asarray(_View(owner, ctypes.cast(ptr, ctypes.c_void_p).value, shape, dtype))
-            return a if zero_copy else a.copy()
-
         self._npairs = npairs
-        self._segments = arr(sp, (nsegs, 6), np.float64, nsegs)
-        self._seg_pair = arr(spp, (nsegs,), np.int32, nsegs)
-        self._pairs = arr(p, (npairs, 2), np.int32, npairs)
+        self._segments = _array(owner, v.seg6, (nsegs, 6), _F8, zero_copy)
+        self._seg_pair = _array(owner, v.seg_pair, (nsegs,), _I4, zero_copy)
+        self._pairs = _array(owner, v.pairs_ab, (npairs, 2), _I4, zero_copy)
         if not zero_copy:
             self._owner = None  # freed here: every array was copied
-        del owner
 
     @property
     def npairs(self):
@@ -549,9 +548,7 @@ def curves_of_jobs(segments, seg_pair, pair_offsets, drop_coplanar_interior=True
     addr = lambda ptr: ctypes.cast(ptr, ctypes.c_void_p).value or 0
 
     def view(ptr, shape, dtype):
-        if int(np.prod(shape)) == 0:
-            return np.zeros(shape, dtype=dtype)
-        return np.asarray(_View(owner, addr(ptr), shape, dtype))
+        return _array(owner, addr(ptr), shape, np.dtype(dtype).str)
 
     vp = ctypes.POINTER(ctypes.c_double)()
     nv = ctypes.c_uint64()
@@ -571,62 +568,21 @@ def curves_of_jobs(segments, seg_pair, pair_offsets, drop_coplanar_interior=True
                 job_curves=view(jo, (nj.value + 1,), np.uint64))
 
 
-class _BatchOwner:
-    """Keeps every result handle of a batch alive while views of their shared block exist."""
-
-    __slots__ = ("owners",)
-
-    def __init__(self, owners):
-        self.owners = owners
-
-
 class BatchResult:
-    """Whole-batch arrays of one gi_intersect_batch call (see Context.intersect_batch_flat)."""
+    """Whole-batch arrays of one gi_intersect_batch_flat call (see Context.intersect_batch_flat)."""
 
-    def __init__(self, owners):
-        L = lib()
-        n = len(owners)
-        p = ctypes.POINTER(ctypes.c_int32)()
-        cnt = ctypes.c_uint64()
-        sp = ctypes.POINTER(ctypes.c_double)()
-        spp = ctypes.POINTER(ctypes.c_int32)()
-        m = ctypes.c_uint64()
-        pa, sa, qa = np.zeros(n, np.uint64), np.zeros(n, np.uint64), np.zeros(n, np.uint64)
-        npairs, nsegs = np.zeros(n, np.int64), np.zeros(n, np.int64)
-        for i, ow in enumerate(owners):
-            L.gi_result_pairs(ow.handle, ctypes.byref(p), ctypes.byref(cnt))
-            L.gi_result_segments(ow.handle, ctypes.byref(sp), ctypes.byref(spp), ctypes.byref(m))
-            pa[i] = ctypes.cast(p, ctypes.c_void_p).value or 0
-            sa[i] = ctypes.cast(sp, ctypes.c_void_p).value or 0
-            qa[i] = ctypes.cast(spp, ctypes.c_void_p).value or 0
-            npairs[i], nsegs[i] = cnt.value, m.value
-        self.offsets = np.concatenate([[0], np.cumsum(npairs)]).astype(np.int64)
-        soff = np.concatenate([[0], np.cumsum(nsegs)]).astype(np.int64)
+    def __init__(self, handle, offsets):
+        owner = _ResultOwner(handle)
+        v = _abi.ResultArrays()
+        lib().gi_result_view(handle, ctypes.byref(v))
         st = _abi.Stats()
-        if n:
-            L.gi_result_stats(owners[0].handle, ctypes.byref(st))
+        lib().gi_result_stats(handle, ctypes.byref(st))
         self.stats = st.as_dict()
-        holder = _BatchOwner(owners)
-
-        def whole(addr, counts, starts, width, dtype):
-            total = int(starts[-1])
-            item = np.dtype(dtype).itemsize * width
-            nz = np.nonzero(counts)[0]
-            if total == 0:
-                return np.zeros((0, width) if width > 1 else (0,), dtype=dtype)
-            shape = (total, width) if width > 1 else (total,)
-            first = int(nz[0])
-            base = int(addr[first]) - item * int(starts[first])
-            if np.all(addr[nz].astype(np.int64) == base + item * starts[nz]):  # back to back in one block
-                return np.asarray(_View(holder, base + item * int(starts[0]), shape, dtype))
-            parts = [np.asarray(_View(holder, int(addr[i]), (int(counts[i]),) + shape[1:], dtype)) for i in nz]
-            return np.concatenate(parts)
-
-        self.pairs = whole(pa, npairs, self.offsets, 2, np.int32)
-        self.segments = whole(sa, nsegs, soff, 6, np.float64)
-        local = whole(qa, nsegs, soff, 1, np.int32)  # per job, relative to the job's first pair
-        self.seg_pair = local.astype(np.int64) + np.repeat(self.offsets[:-1], nsegs)
-        self.job = np.repeat(np.arange(n, dtype=np.uint32), npairs)
+        self.offsets = offsets
+        self.pairs = _array(owner, v.pairs_ab, (v.npairs, 2), _I4)
+        self.job = _array(owner, v.job, (v.npairs,), _U4)
+        self.segments = _array(owner, v.seg6, (v.nsegs, 6), _F8)
+        self.seg_pair = _array(owner, v.seg_pair64, (v.nsegs,), _I8)
 
     def curves(self, drop_coplanar_interior=True):
         """Every job's curves in one call (see curves_of_jobs)."""

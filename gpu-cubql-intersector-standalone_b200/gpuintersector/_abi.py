@@ -43,12 +43,13 @@ EXPORTED = [
     "gi_mesh_upload", "gi_mesh_upload_device", "gi_mesh_release", "gi_mesh_info", "gi_mesh_build_ms",
     "gi_pose_identity", "gi_pose_from_euler_deg", "gi_pose_apply",
     "gi_intersect_opts_default", "gi_intersect", "gi_intersect_oneshot", "gi_intersect_batch",
+    "gi_intersect_batch_flat",
     "gi_classify_pairs", "gi_classify_pairs_noalloc", "gi_predicate_signs",
     "gi_off_load", "gi_off_arrays", "gi_off_free", "gi_scene_load", "gi_mesh_download",
     "gi_curves_build", "gi_result_curves", "gi_curves_vertices", "gi_curves_polylines", "gi_curves_free",
     "gi_curves_build_jobs", "gi_curves_job_offsets",
     "gi_records_write_csv", "gi_pairs_diff", "gi_sweep_poses",
-    "gi_result_pairs", "gi_result_segments", "gi_result_stats", "gi_result_free",
+    "gi_result_pairs", "gi_result_segments", "gi_result_stats", "gi_result_view", "gi_result_free",
     "gi_server_start", "gi_server_submit", "gi_server_poll", "gi_server_wait", "gi_server_stop",
 ]
 
@@ -112,6 +113,12 @@ class Stats(ctypes.Structure):
         return d
 
 
+class ResultArrays(ctypes.Structure):
+    _fields_ = [("pairs_ab", ctypes.c_void_p), ("job", ctypes.c_void_p), ("npairs", ctypes.c_uint64),
+                ("seg6", ctypes.c_void_p), ("seg_pair", ctypes.c_void_p), ("seg_pair64", ctypes.c_void_p),
+                ("nsegs", ctypes.c_uint64), ("held_bytes", ctypes.c_uint64)]
+
+
 class PairJob(ctypes.Structure):
     _fields_ = [("A", ctypes.c_void_p), ("B", ctypes.c_void_p), ("pose_a", Pose), ("pose_b", Pose)]
 
@@ -159,6 +166,8 @@ def load(path=None):
                                   ctypes.POINTER(IntersectOpts), ctypes.POINTER(vp)], st),
         "gi_intersect_batch": ([vp, ctypes.POINTER(PairJob), ctypes.c_uint32, ctypes.POINTER(IntersectOpts),
                                 ctypes.POINTER(vp)], st),
+        "gi_intersect_batch_flat": ([vp, ctypes.POINTER(PairJob), ctypes.c_uint32, ctypes.POINTER(IntersectOpts),
+                                     ctypes.POINTER(ctypes.c_int64), ctypes.POINTER(vp)], st),
         "gi_classify_pairs": ([vp, vp, ctypes.POINTER(Pose), vp, ctypes.POINTER(Pose), vp, ctypes.c_uint32,
                                ctypes.c_int32, vp], st),
         "gi_classify_pairs_noalloc": ([vp, vp, ctypes.POINTER(Pose), vp, ctypes.POINTER(Pose), vp, ctypes.c_uint32,
@@ -196,6 +205,7 @@ def load(path=None):
         "gi_result_segments": ([vp, ctypes.POINTER(dp), ctypes.POINTER(ctypes.POINTER(ctypes.c_int32)),
                                 ctypes.POINTER(ctypes.c_uint64)], st),
         "gi_result_stats": ([vp, ctypes.POINTER(Stats)], st),
+        "gi_result_view": ([vp, ctypes.POINTER(ResultArrays)], st),
         "gi_result_free": ([vp], st),
         "gi_server_start": ([vp, ctypes.POINTER(ServerOpts), ctypes.POINTER(vp)], st),
         "gi_server_submit": ([vp, vp, ctypes.POINTER(Pose), vp, ctypes.POINTER(Pose),

@@ -225,6 +225,15 @@ gi_status gi_intersect_oneshot(gi_ctx* ctx, const double* vA, uint32_t nvA, cons
 gi_status gi_intersect_batch(gi_ctx* ctx, const gi_pair_job* jobs, uint32_t njobs, const gi_intersect_opts* opts,
                              gi_result** out);
 
+/* gi_intersect_batch with one result for the whole batch instead of one per job
+ * (no counterpart in the reference): gi_result_view gives its arrays, ordered by
+ * job, and offsets[njobs + 1] receives job j's range of pairs, offsets[j] ..
+ * offsets[j + 1].  gi_result_stats gives the first job's statistics (the
+ * launch-wide counters are shared); gi_result_pairs and gi_result_segments are
+ * not for this result (GI_ERR_INVALID_ARG). */
+gi_status gi_intersect_batch_flat(gi_ctx* ctx, const gi_pair_job* jobs, uint32_t njobs, const gi_intersect_opts* opts,
+                                  int64_t* offsets, gi_result** out);
+
 /* Exact closed-triangle test over an explicit candidate list: d_out[i] = 1 iff
  * A[d_pairs[2i]] and B[d_pairs[2i+1]] intersect under the poses.  Replaces the
  * reference's predicate kernels over a pair list plus its CPU fallback
@@ -403,6 +412,22 @@ gi_status gi_result_pairs(const gi_result* r, const int32_t** pairs_ab, uint64_t
 /* seg6: 6 doubles per segment (p0 xyz, p1 xyz); seg_pair: pair index per segment. */
 gi_status gi_result_segments(const gi_result* r, const double** seg6, const int32_t** seg_pair, uint64_t* n);
 gi_status gi_result_stats(const gi_result* r, gi_stats* out);
+/* Everything of a result in one call; the pointers are valid until
+ * gi_result_free.  Of gi_intersect_batch_flat: job (the job of each pair) and
+ * seg_pair64 (batch-wide pair index of each segment) are set and seg_pair is
+ * null; of the other calls the other way round.  held_bytes: pinned memory that
+ * the results of this result's context hold at the moment, this one included. */
+typedef struct {
+    const int32_t* pairs_ab;
+    const uint32_t* job;
+    uint64_t npairs;
+    const double* seg6;
+    const int32_t* seg_pair;
+    const int64_t* seg_pair64;
+    uint64_t nsegs;
+    uint64_t held_bytes;
+} gi_result_arrays;
+gi_status gi_result_view(const gi_result* r, gi_result_arrays* out);
 gi_status gi_result_free(gi_result* r);
 
 /* ---- serving: pose-update loop with continuous batching ------------------ */
