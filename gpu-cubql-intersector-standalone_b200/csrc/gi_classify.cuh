@@ -1105,18 +1105,272 @@ __device__ __forceinline__ unsigned result_code(const TTRes& r)
     return c | (drop << 2);
 }
 
+// ---------------------------------------------------------------------------
+// Exact classification of pairs whose eighteen coordinates lie on a common grid
+// of few bits: all multiples of one power of two, and within 2^14 of them of the
+// first vertex.  CAD-like input does (integer grids, binary fractions), and it is
+// such input that is coplanar and touching in earnest.  Relative to the first
+// vertex the coordinates are then integers below 2^14 in magnitude, 2x2 minors
+// of their differences fit in 32 bits and orient3d in 64, so every sign is exact
+// integer arithmetic in registers: no filter, no common-grid search, no local
+// memory.  The steps and the order of the result's points are classify_exact's.
+//
+// Bound by instruction issue.  Two coplanar 512 x 512 grids (2.4 M escalated
+// pairs): 0.20 ms, 3.5 ms with the general form alone, whose out-of-line code
+// stalls on instruction fetches (4 warps waited for them per issue).
+// ---------------------------------------------------------------------------
+struct I3 {
+    int x, y, z;
+};
+// (modulo 2^32: the low words of grid coordinates differ by little)
+__device__ __forceinline__ I3 isub(const I3& a, const I3& b)
+{
+    return {(int)((unsigned)a.x - (unsigned)b.x), (int)((unsigned)a.y - (unsigned)b.y),
+            (int)((unsigned)a.z - (unsigned)b.z)};
+}
+__device__ __forceinline__ I3 icross(const I3& a, const I3& b)
+{
+    return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
+}
+__device__ __forceinline__ int idot_sign(const I3& a, const I3& n)
+{
+    const long long v = (long long)a.x * n.x + (long long)a.y * n.y + (long long)a.z * n.z;
+    return v > 0 ? 1 : (v < 0 ? -1 : 0);
+}
+__device__ __forceinline__ I3 isel3(int i, const I3& a, const I3& b, const I3& c)
+{
+    return {i == 0 ? a.x : (i == 1 ? b.x : c.x), i == 0 ? a.y : (i == 1 ? b.y : c.y),
+            i == 0 ? a.z : (i == 1 ? b.z : c.z)};
+}
+// sign of orient2d(a, b, c) on projected points
+__device__ __forceinline__ int io2(const int2& a, const int2& b, const int2& c)
+{
+    const int v = (a.x - c.x) * (b.y - c.y) - (a.y - c.y) * (b.x - c.x);
+    return v > 0 ? 1 : (v < 0 ? -1 : 0);
+}
+
+// One interval of two triangles in general or touching position (build_interval):
+// its one or two ends, each with its point code and the vertices (cn, cp) of the
+// edge that represents it, side(cn) <= 0 <= side(cp).
+struct SmallEnds {
+    int n, cn[2], cp[2];
+    unsigned code[2];
+};
+__device__ __forceinline__ SmallEnds small_ends(int s0, int s1, int s2, unsigned base)
+{
+    SmallEnds e;
+    const int z = (s0 == 0) + (s1 == 0) + (s2 == 0);
+    const unsigned plane = kCodePlane + 2u * base;  // edges 0-2 of P, 3-5 of Q
+    if (z == 1) {
+        const int u = s0 == 0 ? 0 : (s1 == 0 ? 1 : 2), x = u == 2 ? 0 : u + 1, y = u == 0 ? 2 : u - 1;
+        const int sx = u == 0 ? s1 : (u == 1 ? s2 : s0), sy = u == 0 ? s2 : (u == 1 ? s0 : s1);
+        e.n = sx * sy > 0 ? 1 : 2;
+        e.code[0] = base + u;
+        e.cn[0] = sx < 0 ? x : u;
+        e.cp[0] = sx < 0 ? u : x;
+        e.code[1] = plane + edge_code(x, y);
+        e.cn[1] = sx < 0 ? x : y;
+        e.cp[1] = sx < 0 ? y : x;
+        return e;
+    }
+    const int o = z == 2 ? (s0 != 0 ? 0 : (s1 != 0 ? 1 : 2)) : lone3(s0, s1, s2);
+    const bool neg = (o == 0 ? s0 : (o == 1 ? s1 : s2)) < 0;
+    e.n = 2;
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const int i = k == 0 ? (o == 0 ? 1 : 0) : (o == 2 ? 1 : 2);
+        e.code[k] = z == 2 ? base + i : plane + edge_code(o, i);
+        e.cn[k] = neg ? o : i;
+        e.cp[k] = neg ? i : o;
+    }
+    return e;
+}
+
+// DEC_NO / DEC_YES (with *code), or DEC_ESC when the coordinates are not of this
+// kind or a triangle is degenerate.  *signs: orientation signs evaluated.
+__device__ __forceinline__ int classify_small(const double3* pts, unsigned* code, unsigned* signs)
+{
+    // scale s: the largest difference from the first vertex gets below 2^14
+    double far = 0.0, big = fmax(fmax(fabs(pts[0].x), fabs(pts[0].y)), fabs(pts[0].z));
+#pragma unroll
+    for (int i = 1; i < 6; i++) {
+        far = fmax(far, fmax(fmax(fabs(__dsub_rn(pts[i].x, pts[0].x)), fabs(__dsub_rn(pts[i].y, pts[0].y))),
+                             fabs(__dsub_rn(pts[i].z, pts[0].z))));
+        big = fmax(big, fmax(fmax(fabs(pts[i].x), fabs(pts[i].y)), fabs(pts[i].z)));
+    }
+    // (for coordinates that pass the test below the differences are exact, so far is)
+    const int e = (int)((unsigned)__double2hiint(far) >> 20);  // its biased exponent
+    if (e <= 13 || e > 2000) return DEC_ESC;
+    const double s = __hiloint2double((2046 + 13 - e) << 20, 0);  // 2^(13 - (e - 1023))
+    if (!(big * s < 0x1p50)) return DEC_ESC;
+    // x * s integer for every coordinate: then all differences are exact integers.
+    // Adding 1.5 * 2^52 leaves the integer in the low word.
+    const double magic = 0x1.8p52;
+    I3 v[6];
+    bool whole = true;
+#pragma unroll
+    for (int i = 0; i < 6; i++) {
+        const double x = pts[i].x * s, y = pts[i].y * s, z = pts[i].z * s;
+        const double rx = __dadd_rn(x, magic), ry = __dadd_rn(y, magic), rz = __dadd_rn(z, magic);
+        whole = whole & (__dsub_rn(rx, magic) == x) & (__dsub_rn(ry, magic) == y) & (__dsub_rn(rz, magic) == z);
+        v[i] = {__double2loint(rx), __double2loint(ry), __double2loint(rz)};
+    }
+    if (!whole) return DEC_ESC;
+    const I3 O = v[0];
+    const I3 P0 = {0, 0, 0}, P1 = isub(v[1], O), P2 = isub(v[2], O), Q0 = isub(v[3], O), Q1 = isub(v[4], O),
+             Q2 = isub(v[5], O);
+    const I3 nP = icross(P1, P2), nQ = icross(isub(Q1, Q0), isub(Q2, Q0));
+    if ((nP.x | nP.y | nP.z) == 0 || (nQ.x | nQ.y | nQ.z) == 0) return DEC_ESC;
+    // orient3d(P0, P1, P2, X) = (P0 - X) . nP
+    const int s20 = -idot_sign(Q0, nP), s21 = -idot_sign(Q1, nP), s22 = -idot_sign(Q2, nP);
+    *signs += 3u;
+    if ((s20 > 0 && s21 > 0 && s22 > 0) || (s20 < 0 && s21 < 0 && s22 < 0)) return DEC_NO;
+    if (s20 == 0 && s21 == 0 && s22 == 0) {
+        // coplanar: 2D tests in the projection that drops the normal's largest axis
+        *signs += 20u;
+        const int ax = abs(nP.x), ay = abs(nP.y), az = abs(nP.z);
+        const unsigned drop = ay > ax ? (az > ay ? 2u : 1u) : (az > ax ? 2u : 0u);
+        auto pr = [&](const I3& q) {
+            return drop == 0u ? make_int2(q.y, q.z) : (drop == 1u ? make_int2(q.z, q.x) : make_int2(q.x, q.y));
+        };
+        const int2 p[3] = {pr(P0), pr(P1), pr(P2)}, q[3] = {pr(Q0), pr(Q1), pr(Q2)};
+        const int g1 = io2(p[0], p[1], p[2]), g2 = io2(q[0], q[1], q[2]);
+        int E2[3][3], E1[3][3];
+#pragma unroll
+        for (int j = 0; j < 3; j++)
+#pragma unroll
+            for (int i = 0; i < 3; i++) {
+                E2[j][i] = g2 * io2(q[j], q[(j + 1) % 3], p[i]);
+                E1[i][j] = g1 * io2(p[i], p[(i + 1) % 3], q[j]);
+            }
+        unsigned in = 0;  // bit i: vertex i lies in the other triangle (0-2 of P, 3-5 of Q)
+        bool sep = false;
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+            if (E2[0][i] >= 0 && E2[1][i] >= 0 && E2[2][i] >= 0) in |= 1u << i;
+            if (E1[0][i] >= 0 && E1[1][i] >= 0 && E1[2][i] >= 0) in |= 8u << i;
+            sep |= E2[i][0] <= 0 && E2[i][1] <= 0 && E2[i][2] <= 0;
+            sep |= E1[i][0] <= 0 && E1[i][1] <= 0 && E1[i][2] <= 0;
+        }
+        unsigned cross = 0;  // bit 3i + j: P's edge i and Q's edge j cross properly
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+#pragma unroll
+            for (int j = 0; j < 3; j++)
+                if (E2[j][i] * E2[j][(i + 1) % 3] < 0 && E1[i][j] * E1[i][(j + 1) % 3] < 0) cross |= 1u << (3 * i + j);
+        if (!(in | cross)) return DEC_NO;
+        // a vertex of Q equal to a listed one of P is the same point
+        const I3 P[3] = {P0, P1, P2}, Q[3] = {Q0, Q1, Q2};
+#pragma unroll
+        for (int j = 0; j < 3; j++)
+#pragma unroll
+            for (int i = 0; i < 3; i++)
+                if (((in >> i) & 1u) && P[i].x == Q[j].x && P[i].y == Q[j].y && P[i].z == Q[j].z) in &= ~(8u << j);
+        const int nv = __popc(in);
+        if (!sep) {
+            if (nv + __popc(cross) != 3) {
+                *code = 0u;  // a polygon with more corners: no segment
+                return DEC_YES;
+            }
+            unsigned pt[3] = {0u, 0u, 0u};
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                if (in) {
+                    pt[k] = __ffs(in) - 1;
+                    in &= in - 1u;
+                } else {
+                    pt[k] = kCodeLine + 4u * (__ffs(cross) - 1);
+                    cross &= cross - 1u;
+                }
+            }
+            *code = make_code(3u, drop, pt[0], pt[1], pt[2]);
+            return DEC_YES;
+        }
+        if (nv == 0) return DEC_ESC;  // cannot arise
+        if (nv == 1) {
+            const unsigned w = __ffs(in) - 1;
+            *code = make_code(1u, 0u, w, 0u, 0u);
+            return DEC_YES;
+        }
+        // touching along a segment: the extreme vertices on the first axis that tells them apart
+        auto axis = [&](int m, unsigned w) {
+            const I3 t = w < 3u ? isel3((int)w, P0, P1, P2) : isel3((int)w - 3, Q0, Q1, Q2);
+            return m == 0 ? t.x : (m == 1 ? t.y : t.z);
+        };
+        const unsigned first = __ffs(in) - 1;
+        unsigned lo = first, hi = first;
+        for (int m = 0; m < 3 && lo == hi; m++) {
+            int vl = axis(m, first), vh = vl;
+            for (unsigned rest = in & (in - 1u); rest; rest &= rest - 1u) {
+                const unsigned w = __ffs(rest) - 1;
+                const int x = axis(m, w);
+                if (x < vl) {
+                    vl = x;
+                    lo = w;
+                }
+                if (x > vh) {
+                    vh = x;
+                    hi = w;
+                }
+            }
+        }
+        *code = make_code(2u, 0u, lo, hi, 0u);
+        return DEC_YES;
+    }
+    const int s10 = idot_sign(isub(Q0, P0), nQ), s11 = idot_sign(isub(Q0, P1), nQ), s12 = idot_sign(isub(Q0, P2), nQ);
+    *signs += 3u;
+    if ((s10 > 0 && s11 > 0 && s12 > 0) || (s10 < 0 && s11 < 0 && s12 < 0)) return DEC_NO;
+    const SmallEnds X = small_ends(s10, s11, s12, 0u), Y = small_ends(s20, s21, s22, 3u);
+    int c[2][2] = {{0, 0}, {0, 0}};
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            if (i >= X.n || j >= Y.n) continue;
+            const I3 d = isel3(Y.cp[j], Q0, Q1, Q2);
+            c[i][j] = idot_sign(isub(isel3(X.cn[i], P0, P1, P2), d),
+                                icross(isub(isel3(X.cp[i], P0, P1, P2), d), isub(isel3(Y.cn[j], Q0, Q1, Q2), d)));
+        }
+    *signs += (unsigned)(X.n * Y.n);
+    bool xin[2], yin[2];
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        xin[k] = k < X.n && (Y.n == 1 ? c[k][0] == 0 : c[k][0] * c[k][1] <= 0);
+        yin[k] = k < Y.n && (X.n == 1 ? c[0][k] == 0 : c[0][k] * c[1][k] <= 0);
+    }
+    unsigned kind = 0, pt[2] = {0u, 0u};
+    auto put = [&](unsigned q) {
+        if (kind == 0u) pt[0] = q;
+        else if (kind == 1u) pt[1] = q;
+        kind = kind < 2u ? kind + 1u : 2u;
+    };
+    if (xin[0]) put(X.code[0]);
+    if (xin[1]) put(X.code[1]);
+#pragma unroll
+    for (int j = 0; j < 2; j++)
+        if (yin[j] && !(xin[0] && c[0][j] == 0) && !(xin[1] && c[1][j] == 0)) put(Y.code[j]);
+    if (!kind) return DEC_NO;
+    *code = make_code(kind, 0u, pt[0], pt[1], 0u);
+    return DEC_YES;
+}
+
 // Decides a pair that the first stage escalated; *code receives the construction
-// code of an intersecting one.  After the FP32 form (fp32) the FP64 form of the
-// same filter is asked first: its bound is 2^29 times tighter, so of pairs in
-// general position it leaves none to the integers, whose out-of-line code and
-// local memory take 8 us for a single pair (two 1.3M-triangle meshes with 3
-// escalated pairs: exact phase of the finish 9.0 -> 4.8 us; 1.2 M pairs
-// classified, a few escalated: 59.8 -> 58.9 us).  Pairs that are not in general
-// position pay for it: 2.4 M on coplanar grids, 3.2 -> 3.5 ms.
+// code of an intersecting one.  Small-grid coordinates first.  Then, after the
+// FP32 form (fp32), the FP64 form of the same filter: its bound is 2^29 times
+// tighter, so of pairs in general position it leaves none to the general
+// integers, whose out-of-line code and local memory take 8 us for a single pair
+// (two 1.3M-triangle meshes with 3 escalated pairs: exact phase of the finish
+// 9.0 -> 4.8 us).
 __device__ __forceinline__ bool decide_escalated(const double3* pts, bool fp32, unsigned* code, ExactSigns& S)
 {
+    unsigned signs = 0;
+    int dec = classify_small(pts, code, &signs);
+    if (dec != DEC_ESC) {
+        S.nexact += signs;
+        return dec == DEC_YES;
+    }
     if (fp32) {
-        const int dec = classify_fast<double>(pts, pts + 3, code);
+        dec = classify_fast<double>(pts, pts + 3, code);
         if (dec != DEC_ESC) return dec == DEC_YES;
     }
     TTRes r;
