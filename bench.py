@@ -44,8 +44,7 @@ METRIC = "ms/intersect at 2×1.3M tris & tri-pair tests/s; pose-update p50/p99 v
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one traversal
 # launch on the level-8 pose workload with L2 flushed, from the ncu captures
 # summarised in profiles/k_traverse_config2.md, per traversal shape captured
-# (shape 7 with a quarter of the blocks filtering candidates)
-TRAVERSE_DRAM_BYTES = {0: 11.373824e6 + 512.0, 7: 13.270784e6 + 256.0}
+TRAVERSE_DRAM_BYTES = {}
 
 
 def parse():
@@ -70,7 +69,7 @@ def parse():
     ap.add_argument("--pose-samples", type=int, default=1000,
                     help="pose-update latency: wall-clock samples of gi_intersect after the timed steps")
     ap.add_argument("--shape", type=int, default=-1,
-                    help="pin the traversal shape (0..7) instead of autotuning it (for profiling runs)")
+                    help="another traversal shape (0..7) than the library's own (for measurements)")
     return ap.parse_args()
 
 
@@ -233,7 +232,8 @@ def run_batch(args, gi, world, rank, dist):
     from gpuintersector import shard
 
     npairs = args.pairs or 4096
-    ctx = gi.Context(int(os.environ.get("LOCAL_RANK", "0")))
+    # device times from CUDA events around the calls
+    ctx = gi.Context(int(os.environ.get("LOCAL_RANK", "0")), flags=gi._abi.GI_FLAG_EVENT_TIMES)
     costs = [shard.job_cost(a, b) for a, b in mg.config4_sizes(seed=4, pairs=npairs)]
     mine = shard.assign(costs, world)[rank]
     jobs, meshes, tris = [], [], 0
@@ -245,7 +245,7 @@ def run_batch(args, gi, world, rank, dist):
         R, C, T = j["poseB"]
         jobs.append((A, None, B, gi.pose_raw(R, C, T)))
     upload_s = time.perf_counter() - t_up
-    for k in range(2 * gi._abi.GI_TRAVERSE_SHAPES + args.warmup):  # autotuning, then warm-up (untimed)
+    for k in range(4 + args.warmup):  # buffers grow on the first calls, then warm-up (untimed)
         rs = ctx.intersect_batch(jobs, want_segments=True)
     flush = torch.empty(256 << 20, dtype=torch.uint8, device="cuda")
     dev, wall, st = [], [], None
@@ -279,7 +279,7 @@ def run_batch(args, gi, world, rank, dist):
         "config": {"workload": "batch of %d mesh pairs" % npairs, "pairs_this_rank": len(jobs),
                    "tris_this_rank": tris, "l2": "flushed (256 MB write) before each step",
                    "parallelism": "pairs sharded by cost" if world > 1 else "single",
-                   "traverse_shape": int(st["traverse_shape"]), "autotuned": True},
+                   "traverse_shape": int(st["traverse_shape"]), "autotuned": False},
         "mesh_pairs_per_s": npairs / (ms * 1e-3), "intersecting_pairs": found,
         "node_pairs": int(st["node_pairs"]), "candidates": int(st["candidates"]),
         "tri_pair_tests_per_s": float(st["candidates"]) / (float(np.mean([st["ms_traverse"]])) * 1e-3),
@@ -550,7 +550,9 @@ def main():
     # is drawn pose by pose, so the first warmup + steps poses do not depend on it)
     poses = step_poses(cfg, rng, args.warmup + args.steps + args.pose_samples)
     flags = 0 if args.shape < 0 else (gi._abi.GI_FLAG_FIXED_SHAPE | gi._abi.GI_FLAG_SHAPE(args.shape))
-    ctx = gi.Context(local, flags=flags)
+    # device times from CUDA events around the calls (the steps below; the wall-clock
+    # parts after them use a context as a program has it, without events)
+    ctx = gi.Context(local, flags=flags | gi._abi.GI_FLAG_EVENT_TIMES)
     A = ctx.upload(cfg["vA"], cfg["tA"])
     B = ctx.upload(cfg["vB"], cfg["tB"])
     flush = torch.empty(256 << 20, dtype=torch.uint8, device="cuda")
@@ -559,10 +561,8 @@ def main():
         R, C, T = pose
         return ctx.intersect(A, B, None, gi.pose_raw(R, C, T), want_segments=True, precision=precision)
 
-    # autotuning: the library times each traversal shape (expansion form x
-    # blocks per SM) twice per workload class on its own calls, then keeps the
-    # fastest; these calls precede the warm-up and are not timed
-    for k in range(2 * gi._abi.GI_TRAVERSE_SHAPES if args.shape < 0 else 0):
+    # the first calls of a context size its buffers; they precede the warm-up
+    for k in range(4):
         one(poses[0])
         one(poses[0], precision=1)
     for k in range(args.warmup):
@@ -602,6 +602,14 @@ def main():
         r64 = one(poses[args.warmup + k], precision=1)
         fp64_ms.append(r64.stats["ms_total"])
         assert np.array_equal(r64.pairs, r.pairs) or k != args.steps - 1
+
+    event_ctx, event_meshes = ctx, (A, B)
+    ctx = gi.Context(local, flags=flags)
+    A, B = ctx.upload(cfg["vA"], cfg["tA"]), ctx.upload(cfg["vB"], cfg["tB"])
+    for k in range(4 + args.warmup):
+        one(poses[k % args.warmup if args.warmup else 0])
+    for m in event_meshes:
+        m.release()
 
     # pose-update latency (the serving loop's steady state): resident meshes, a
     # new pose in, the pairs and segments usable on the host; no L2 flush.
@@ -733,7 +741,7 @@ def main():
         "config": pose_config(args.level, cfg),
         "parallelism": "replicas" if world > 1 else "single",
         "impl_config": {"l2": "flushed (256 MB write) before each step", "precision": "fp32 filter -> fp64 filter -> exact",
-                        "traverse_shape": int(st["traverse_shape"]), "autotuned": args.shape < 0},
+                        "traverse_shape": int(st["traverse_shape"]), "autotuned": False},
         "pairs": int(st["pairs"]), "segments": int(st["segments"]), "candidates": int(cand),
         "tri_pair_tests_per_s": tests_per_s,
         "filter_decided_frac": float(st["filter_decided"] / max(1, st["candidates"])),
@@ -758,7 +766,7 @@ def main():
                      "traffic_source": "dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture of the "
                                        "traversal on this workload with the same shape (null: shape not captured); "
                                        "profiles/k_traverse_config2.md",
-                     "kernel": "k_traverse", "peak_source": peak_src,
+                     "kernel": "k_traverse_blocks", "peak_source": peak_src,
                      "alg_bytes_per_launch": float(alg_bytes),
                      "note": "output-sensitive traversal: bytes = node pairs x 2 nodes x 128 B + leaf pairs x "
                              "2 x (16 B record + 3 x 24 B vertices) + results x 16 B"},

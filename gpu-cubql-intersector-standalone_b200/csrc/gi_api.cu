@@ -637,6 +637,7 @@ static gi_status run_jobs(gi_ctx* c, std::vector<JobDev>& jobs, const gi_interse
     uint32_t nres = 0, nsegs = 0;
     char* hp = nullptr;
     bool segpair64 = false;  // the block's pair indices have 64 bits
+    bool events = true;      // the call's times come from CUDA events
     size_t off_jobs = 0, off_segs = 0, off_segpair = 0;
     // pinned block the results land in; returned to the pool on every early exit
     PinnedBuf* buf = nullptr;
@@ -745,7 +746,9 @@ static gi_status run_jobs(gi_ctx* c, std::vector<JobDev>& jobs, const gi_interse
             CK(c, cudaMemcpyAsync(c->d_jobs, c->h_jobs, sizeof(JobDev) * nj, cudaMemcpyHostToDevice, c->st), "jobs copy");
             jobs_there = true;
         }
-        CK(c, cudaEventRecord(c->ev[0], c->st), "event");
+        // (the finish stamps its own times; two events cost 4.5 us a call)
+        events = !fin || (c->flags & GI_FLAG_EVENT_TIMES);
+        if (events) CK(c, cudaEventRecord(c->ev[0], c->st), "event");
         CK(c, launch_traverse(b, c->cfg, prec, trav_shape(shape), c->st), "traverse");
         // the finish follows the traversal directly (programmatic dependent
         // launch): no event between them; the general path keeps its events
@@ -798,7 +801,7 @@ static gi_status run_jobs(gi_ctx* c, std::vector<JobDev>& jobs, const gi_interse
                        "ordering");
             }
         }
-        CK(c, cudaEventRecord(c->ev[4], c->st), "event");
+        if (events) CK(c, cudaEventRecord(c->ev[4], c->st), "event");
         if (!fin) {
             // speculative copy at the previous call's size
             CK(c, cudaMemcpyAsync(c->h_cnt, b.cnt, sizeof(Counters), cudaMemcpyDeviceToHost, c->st), "counters");
@@ -879,7 +882,8 @@ static gi_status run_jobs(gi_ctx* c, std::vector<JobDev>& jobs, const gi_interse
     c->pred_pairs = nres;
     c->pred_segs = nsegs;
     float ms_trav = 0, ms_exact = 0, ms_seg = 0, ms_sort = 0, ms_total = 0;
-    cudaEventElapsedTime(&ms_total, c->ev[0], c->ev[4]);
+    if (events) cudaEventElapsedTime(&ms_total, c->ev[0], c->ev[4]);
+    else if (H.t_start && H.fin_ns[4] >= H.t_start) ms_total = (float)(1e-6 * double(H.fin_ns[4] - H.t_start));
     if (fin) {
         // the finish follows the traversal with no event between them: its span
         // and phases from its own timestamps (taken after it waited for the

@@ -122,6 +122,7 @@ struct Counters {
     // stage, when block 0 had its run ranked and when it had it written, and when
     // the last block ended
     unsigned long long fin_ns[5];
+    unsigned long long t_start;  // globaltimer when the traversal's first block began
     unsigned fin_done;  // blocks of k_finish that have ended
     unsigned fin_over;  // results whose partition's bucket was full (may exceed the overflow list)
     unsigned odd;       // 1: some result has other than one segment

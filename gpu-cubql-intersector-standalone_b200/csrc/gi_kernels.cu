@@ -1509,6 +1509,7 @@ __global__ void __launch_bounds__(kBlkThreads, kBlkPerSm[MULTI ? 1 : 0]) k_trave
     const unsigned nslots = B.cap_queue / kBlkUnits;
     const unsigned lt = (1u << lane) - 1u;
     allow_dependent_launch();
+    if (b == 0 && tid == 0) C->t_start = globaltimer_ns();
     if (tid == 0) {
         s.push[0] = s.push[1] = 0u;
         s.nres = 0u;

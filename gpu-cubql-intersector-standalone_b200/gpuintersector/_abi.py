@@ -16,6 +16,7 @@ GI_ERR_NOT_READY = 7
 GI_ERR_NO_DEVICE = 8
 
 GI_FLAG_TINY_BUFFERS = 1
+GI_FLAG_EVENT_TIMES = 2
 GI_FLAG_FIXED_SHAPE = 0x100
 
 

@@ -87,6 +87,10 @@ typedef struct gi_server gi_server;
 /* gi_options.flags */
 #define GI_FLAG_TINY_BUFFERS 1u /* start every intersect buffer at 64 entries: exercises the
                                    capacity-overflow / retry path (host-side fault injection) */
+#define GI_FLAG_EVENT_TIMES 2u  /* the times in gi_stats come from CUDA events recorded around every call's
+                                   launches (launch latencies included); without it, calls that end with
+                                   the one-launch finish take them from the kernels' own timestamps, first
+                                   block's start to last block's end (the two events cost 4.5 us a call) */
 /* GI_FLAG_FIXED_SHAPE | GI_FLAG_SHAPE(k), k in 0..7, picks a shape of the
  * traversal other than the library's own choice, for measurements (every shape
  * gives the same results): bit 0 one block per SM instead of all resident
