@@ -5,7 +5,7 @@
 // which loop on the host with a device sync per tree level):
 //   k_tri_boxes (and validation) -> k_morton_hist -> radix sort -> k_karras_leaves (leaves + binary tree)
 //   -> k_state_tables -> k_wide_flags -> k_collapse (size-greedy 4-wide nodes,
-//   topology) -> k_refit_wide (bottom-up over the wide tree, atomic arrival counters)
+//   their boxes from a pyramid of the sorted leaves' boxes) -> k_cut
 // Large meshes: one host round trip, for the wide-node count (the node array's size).
 //
 // Intersect (replaces crossCheck.cu, DualTreeStep.cu, rapidDescendKernel.cu and the
@@ -295,6 +295,135 @@ __device__ __forceinline__ void karras_node(int i, const uint32_t* __restrict__ 
     if (i == 0) parent[0] = -1;
 }
 
+// Unions of the sorted leaves' boxes over aligned runs of 2^L leaves (level L,
+// entry e: leaves [e 2^L, (e + 1) 2^L)), L = 1 .. levels.  Every node of the
+// radix tree covers consecutive leaves, so its box is the union of a few entries
+// (range_box), read by whoever needs it, without a bottom-up pass over the tree.
+// k_state_tables writes the levels that a block completes from its own leaves and
+// one block of k_wide_flags the rest, beside work of the same latency.  (A
+// bottom-up refit, an atomic arrival per node and level, took 61 us of a 1.3M-
+// triangle build and 26 of a 300k one; the pyramid adds 14 us to k_state_tables
+// and 15 to k_collapse at 1.3M, 2.5 and 0.5 at 300k.)
+constexpr int kPyrLevels = 32;
+constexpr int kPyrBlock = 8;  // levels that a block completes from its own leaves
+constexpr int kPyrThreads = 1 << kPyrBlock;
+template <class S>
+struct Pyramid {
+    S* box;                    // 6 values an entry
+    uint32_t off[kPyrLevels];  // first entry of level L (L >= 1)
+    int levels;
+};
+
+template <class S>
+__device__ __forceinline__ void box_union(S (&b)[6], const S (&o)[6])
+{
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        b[k] = min(b[k], o[k]);
+        b[3 + k] = max(b[3 + k], o[3 + k]);
+    }
+}
+
+// Levels 1 .. kPyrBlock of the pyramid over the block's leaves (thread = leaf):
+// shuffles within a warp, shared memory within the block.  Every thread calls.
+template <class S>
+__device__ __forceinline__ void pyramid_block(const S* __restrict__ leafBox, int n, const Pyramid<S>& pyr)
+{
+    __shared__ S s_box[kPyrThreads / 32][6];
+    const unsigned p = blockIdx.x * (unsigned)kPyrThreads + threadIdx.x;
+    S b[6] = {(S)INFINITY, (S)INFINITY, (S)INFINITY, (S)-INFINITY, (S)-INFINITY, (S)-INFINITY};
+    if (p < (unsigned)n) load_box_cg(leafBox + 6 * (size_t)p, b);
+    const unsigned lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int L = 1; L <= 5; L++) {
+        S o[6];
+#pragma unroll
+        for (int q = 0; q < 6; q++) o[q] = __shfl_xor_sync(0xffffffffu, b[q], 1 << (L - 1));
+        box_union(b, o);
+        if (L <= pyr.levels && (lane & ((1u << L) - 1u)) == 0u && p < (unsigned)n)
+            store_box(pyr.box + 6 * ((size_t)pyr.off[L] + (p >> L)), b);
+    }
+    if (lane == 0)
+#pragma unroll
+        for (int q = 0; q < 6; q++) s_box[w][q] = b[q];
+    __syncthreads();
+    // thread t of each level: its entry's warps t << (L - 5) ...
+    for (int L = 6; L <= kPyrBlock && L <= pyr.levels; L++) {
+        const unsigned width = 1u << (L - 5), x0 = threadIdx.x * width;
+        const size_t first = (size_t)blockIdx.x * kPyrThreads + ((size_t)threadIdx.x << L);
+        if (threadIdx.x < (unsigned)(kPyrThreads >> L) && first < (size_t)n) {
+            S u[6], v[6];
+#pragma unroll
+            for (int q = 0; q < 6; q++) u[q] = s_box[x0][q];
+            for (unsigned x = 1; x < width; x++) {
+#pragma unroll
+                for (int q = 0; q < 6; q++) v[q] = s_box[x0 + x][q];
+                box_union(u, v);
+            }
+            store_box(pyr.box + 6 * ((size_t)pyr.off[L] + (first >> L)), u);
+        }
+    }
+}
+
+// The levels above a block's, by one block.
+template <class S>
+__device__ __forceinline__ void pyramid_top(int n, const Pyramid<S>& pyr)
+{
+    for (int L = kPyrBlock + 1; L <= pyr.levels; L++) {
+        const uint32_t below = (uint32_t)(((unsigned long long)n + (1ull << (L - 1)) - 1u) >> (L - 1));
+        const uint32_t here = (below + 1u) / 2u;
+#pragma unroll 4
+        for (uint32_t e = threadIdx.x; e < here; e += kPyrThreads) {
+            S u[6], v[6];
+            const S* const src = pyr.box + 6 * ((size_t)pyr.off[L - 1] + 2u * (size_t)e);
+            const S* const src2 = 2u * e + 1u < below ? src + 6 : src;
+            load_box_cg(src, u);
+            load_box_cg(src2, v);
+            box_union(u, v);
+            store_box(pyr.box + 6 * ((size_t)pyr.off[L] + e), u);
+        }
+        __syncthreads();
+    }
+}
+
+// Union of the boxes of the leaves [a, e): at most two entries a level, and the
+// loads of two levels in flight at once (their addresses depend on a and e
+// alone).  k_collapse at 300k / 1.3M triangles: 18 / 65 us with one level, 13 / 60
+// with two, 13 / 63 with three, 15 / 67 with four (registers).
+template <class S>
+__device__ __forceinline__ void range_box(const S* __restrict__ leafBox, const Pyramid<S>& pyr, uint32_t a, uint32_t e, S (&b)[6])
+{
+    constexpr int kAhead = 2;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        b[k] = (S)INFINITY;
+        b[3 + k] = (S)-INFINITY;
+    }
+    for (int L = 0; a < e; L += kAhead) {
+        S o[2 * kAhead][6];
+#pragma unroll
+        for (int s = 0; s < kAhead; s++) {
+            const S* const level = L + s == 0 || a >= e ? leafBox : pyr.box + 6 * (size_t)pyr.off[L + s];
+            const bool ua = a < e && (a & 1u);
+            const S* const pa = level + 6 * (size_t)a;
+            a += ua ? 1u : 0u;
+            const bool ue = a < e && (e & 1u);
+            e -= ue ? 1u : 0u;
+            const S* const pe = level + 6 * (size_t)e;
+#pragma unroll
+            for (int k = 0; k < 6; k++) o[2 * s][k] = o[2 * s + 1][k] = k < 3 ? (S)INFINITY : (S)-INFINITY;
+            if (ua) load_box_cg(pa, o[2 * s]);
+            if (ue) load_box_cg(pe, o[2 * s + 1]);
+            if (a < e) {
+                a >>= 1;
+                e >>= 1;
+            }
+        }
+#pragma unroll
+        for (int s = 0; s < 2 * kAhead; s++) box_union(b, o[s]);
+    }
+}
+
 // Leaves in sorted order (position p < n: the box and the vertex indices of
 // triangle vals[p]) and the radix tree's internal node p (p < n - 1), in one
 // launch: both are gathers or searches bound by latency, so each thread has
@@ -361,10 +490,13 @@ __device__ __forceinline__ unsigned first_max3(uint32_t a, uint32_t b, uint32_t 
 
 // tab[y] bits 2s..2s+1: the state of internal node y (y >= 1) when its parent
 // is in state s (s = W, O2; a child of an O3 node is always W).
-__global__ void k_state_tables(int n, const uint4* __restrict__ child, const int* __restrict__ parent,
-                               uint8_t* __restrict__ tab)
+template <class S>
+__global__ void __launch_bounds__(kPyrThreads) k_state_tables(int n, const uint4* __restrict__ child, const int* __restrict__ parent,
+                               uint8_t* __restrict__ tab, const S* __restrict__ leafBox,
+                               const __grid_constant__ Pyramid<S> pyr)
 {
     pdl_enter();
+    pyramid_block(leafBox, n, pyr);
     int y = blockIdx.x * blockDim.x + threadIdx.x;
     if (y < 1 || y >= n - 1) return;
     const int p = parent[y];
@@ -400,10 +532,13 @@ __global__ void k_state_tables(int n, const uint4* __restrict__ child, const int
 // node 0; a block's others take consecutive places from one atomic on the
 // header's count (the order of the blocks' runs varies from build to build and
 // shows in no result; a scan of the flags kept it, for three launches more).
-__global__ void __launch_bounds__(256) k_wide_flags(int n, const int* __restrict__ parent, const uint8_t* __restrict__ tab,
-                                                    uint32_t* __restrict__ widx, unsigned* __restrict__ hdr)
+template <class S>
+__global__ void __launch_bounds__(kPyrThreads) k_wide_flags(int n, const int* __restrict__ parent, const uint8_t* __restrict__ tab,
+                                                    uint32_t* __restrict__ widx, unsigned* __restrict__ hdr,
+                                                    const __grid_constant__ Pyramid<S> pyr)
 {
     pdl_enter();
+    if (blockIdx.x == 0) pyramid_top(n, pyr);
     __shared__ unsigned s_warp[8], s_base;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     bool wide = false;
@@ -438,150 +573,86 @@ __global__ void __launch_bounds__(256) k_wide_flags(int n, const int* __restrict
 }
 
 // Writes wide node widx[i] from binary node i: the size-greedy expansion of i
-// (the same choices as k_state_tables), with the boxes of its leaf children
-// (consecutive leaves: the loads of neighbouring threads share lines); the
-// boxes of wide children are filled by k_refit_wide.  For each wide child it
-// writes the (wide node, slot) it sits in (nodeUp; the root's is kEmpty),
-// and per node kids | leaf kids << 8 (nkids) and the arrival count so far,
-// its leaf kids (arrive).  An internal part that is not a wide node, or whose
-// index is out of range, cannot arise; it is written as an empty slot and
-// flagged in *bad rather than followed.
+// (the same choices as k_state_tables), each child with the box of the leaves it
+// covers (a left child's leaves end at its own index, a right child's begin
+// there).  An internal part that is not a wide node, or whose index is out of
+// range, cannot arise; it is written as an empty slot and flagged in *bad rather
+// than followed.
+//
+// A block finds the children of its 256 binary nodes' wide nodes first, one
+// thread a node, and then fills the child slots, one thread a slot: two nodes in
+// five are wide, and a child with many leaves costs only its own thread the
+// longer union.
+constexpr int kColThreads = 256;
 template <class S, class NodeT>
-__global__ void k_collapse(int n, const uint4* __restrict__ child, const uint32_t* __restrict__ widx, uint32_t nw, const S* __restrict__ leafBox,
-                           NodeT* __restrict__ nodes, uint2* __restrict__ nodeUp, uint32_t* __restrict__ nkids,
-                           unsigned* __restrict__ arrive, unsigned* __restrict__ bad)
+__global__ void __launch_bounds__(kColThreads) k_collapse(int n, const uint4* __restrict__ child, const uint32_t* __restrict__ widx,
+                           uint32_t nw, const S* __restrict__ leafBox, const __grid_constant__ Pyramid<S> pyr,
+                           NodeT* __restrict__ nodes, unsigned* __restrict__ bad)
 {
     pdl_enter();
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n - 1) return;
-    const uint32_t wi = widx[i];
-    if (wi == kEmpty) return;
-    if (wi >= nw) {
+    __shared__ unsigned s_n;
+    __shared__ uint32_t s_wi[kColThreads];
+    __shared__ uint32_t s_ref[kColThreads * 4], s_lo[kColThreads * 4], s_num[kColThreads * 4];
+    if (threadIdx.x == 0) s_n = 0u;
+    __syncthreads();
+    const int i = blockIdx.x * kColThreads + threadIdx.x;
+    uint32_t wi = i < n - 1 ? widx[i] : kEmpty;
+    if (wi != kEmpty && wi >= nw) {
         atomicOr(bad, kErrBuild);
-        return;
+        wi = kEmpty;
     }
-    if (wi == 0u) nodeUp[0] = make_uint2(kEmpty, 0u);
-    const uint4 c = child[i];
-    uint32_t slot[4] = {c.x, c.y, kEmpty, kEmpty};
-    uint32_t num[4] = {c.z, c.w, 0u, 0u};
-    int ns = 2;
+    if (wi != kEmpty) {
+        const uint4 c = child[i];
+        uint32_t slot[4] = {c.x, c.y, kEmpty, kEmpty};
+        uint32_t num[4] = {c.z, c.w, 0u, 0u};
+        uint32_t right = 2u;  // bit k: part k is a right child
+        int ns = 2;
 #pragma unroll
-    for (int step = 0; step < 2; step++) {
-        int b = 0;
-        for (int k = 1; k < ns; k++)
-            if (num[k] > num[b]) b = k;
-        if (num[b] < 2u) break;
-        const uint4 g = child[slot[b]];
-        for (int k = ns; k > b + 1; k--) {
-            slot[k] = slot[k - 1];
-            num[k] = num[k - 1];
+        for (int step = 0; step < 2; step++) {
+            int b = 0;
+#pragma unroll
+            for (int k = 1; k < 2 + step; k++)
+                if (k < ns && num[k] > num[b]) b = k;
+            if (num[b] < 2u) break;
+            const uint4 g = child[slot[b]];
+#pragma unroll
+            for (int k = 3; k > 0; k--)
+                if (k <= ns && k > b + 1) {
+                    slot[k] = slot[k - 1];
+                    num[k] = num[k - 1];
+                }
+            right = (right & ((1u << b) - 1u)) | (2u << b) | ((right >> (b + 1)) << (b + 2));
+            slot[b] = g.x;
+            slot[b + 1] = g.y;
+            num[b] = g.z;
+            num[b + 1] = g.w;
+            ns++;
         }
-        slot[b] = g.x;
-        slot[b + 1] = g.y;
-        num[b] = g.z;
-        num[b + 1] = g.w;
-        ns++;
-    }
-    uint32_t kids = 0, leaves = 0;
+        const unsigned at = atomicAdd(&s_n, 1u);
+        s_wi[at] = wi;
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        uint32_t r = k < ns ? slot[k] : kEmpty;
-        if (r != kEmpty && !(r & kLeaf) && widx[r] >= nw) {
-            atomicOr(bad, kErrBuild);
-            r = kEmpty;
+        for (int k = 0; k < 4; k++) {
+            const uint32_t r = k < ns ? slot[k] : kEmpty, leaf = r & ~kLeaf;
+            s_ref[4 * at + k] = r;
+            s_num[4 * at + k] = num[k];
+            s_lo[4 * at + k] = ((right >> k) & 1u) ? leaf : leaf - (num[k] - 1u);
+        }
+    }
+    __syncthreads();
+    for (unsigned t = threadIdx.x; t < 4u * s_n; t += kColThreads) {
+        uint32_t r = s_ref[t], ref = kEmpty;
+        if (r != kEmpty && !(r & kLeaf)) {
+            ref = widx[r];
+            if (ref >= nw) {
+                atomicOr(bad, kErrBuild);
+                r = ref = kEmpty;
+            }
+        } else {
+            ref = r;
         }
         S bx[6] = {(S)INFINITY, (S)INFINITY, (S)INFINITY, (S)-INFINITY, (S)-INFINITY, (S)-INFINITY};
-        uint32_t ref = kEmpty;
-        if (r == kEmpty) {
-        } else if (r & kLeaf) {
-            load_box_cg(leafBox + 6 * (size_t)(r & ~kLeaf), bx);
-            ref = r;
-            kids++;
-            leaves++;
-        } else {
-            ref = widx[r];
-            nodeUp[ref] = make_uint2(wi, (uint32_t)k);
-            kids++;
-        }
-        store_kid(&nodes[wi].kid[k], bx, ref);
-    }
-    nkids[wi] = kids | (leaves << 8);
-    arrive[wi] = leaves;
-}
-
-// The child boxes of a wide node, read through L2 (other threads of the same
-// launch wrote them): the union of its slots (empty slots hold +inf / -inf and
-// change nothing).
-__device__ __forceinline__ void node_union_cg(const WNode* nd, float b[6])
-{
-    const float4* q = reinterpret_cast<const float4*>(nd);
-    float4 lo[4], hi[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        lo[k] = __ldcg(q + 2 * k);
-        hi[k] = __ldcg(q + 2 * k + 1);
-    }
-    b[0] = fminf(fminf(lo[0].x, lo[1].x), fminf(lo[2].x, lo[3].x));
-    b[1] = fminf(fminf(lo[0].y, lo[1].y), fminf(lo[2].y, lo[3].y));
-    b[2] = fminf(fminf(lo[0].z, lo[1].z), fminf(lo[2].z, lo[3].z));
-    b[3] = fmaxf(fmaxf(hi[0].x, hi[1].x), fmaxf(hi[2].x, hi[3].x));
-    b[4] = fmaxf(fmaxf(hi[0].y, hi[1].y), fmaxf(hi[2].y, hi[3].y));
-    b[5] = fmaxf(fmaxf(hi[0].z, hi[1].z), fmaxf(hi[2].z, hi[3].z));
-}
-__device__ __forceinline__ void node_union_cg(const WNode64* nd, double b[6])
-{
-    for (int f = 0; f < 6; f++) b[f] = f < 3 ? (double)INFINITY : (double)-INFINITY;
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const double2* q = reinterpret_cast<const double2*>(&nd->kid[k]);
-        const double2 u = __ldcg(q), v = __ldcg(q + 1), w = __ldcg(q + 2);
-        b[0] = fmin(b[0], u.x);
-        b[1] = fmin(b[1], u.y);
-        b[2] = fmin(b[2], v.x);
-        b[3] = fmax(b[3], v.y);
-        b[4] = fmax(b[4], w.x);
-        b[5] = fmax(b[5], w.y);
-    }
-}
-
-// Bottom-up refit of the wide tree, one thread per wide node.  A node whose
-// children are all leaves is complete after k_collapse: its thread takes the
-// union of its slots, stores it into its slot of the node above and arrives
-// there; the thread that arrives last (after the node's other children) takes
-// that node's union and climbs on.  Nodes with a wide child return at once.
-// The links of the node above are loaded while the arrival is in flight, so a
-// level costs the slot stores, the arrival atomic and one read of the node's
-// six box fields; the wide tree has about half the levels of the binary one.
-template <class S, class NodeT>
-__global__ void k_refit_wide(uint32_t cap, unsigned* hdr, const uint2* __restrict__ nodeUp, const uint32_t* __restrict__ nkids,
-                             NodeT* nodes, unsigned* arrive)
-{
-    pdl_enter();
-    const uint32_t nw = min(1u + __ldcg(&hdr[kHdrWide]), cap);
-    const uint32_t w0 = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w0 >= nw) return;
-    const uint32_t k0 = nkids[w0];
-    if ((k0 & 0xffu) != (k0 >> 8)) return;  // a wide child completes this node
-    S b[6];
-    node_union_cg(nodes + w0, b);
-    uint2 up = nodeUp[w0];
-    uint32_t self = w0;  // the slot holds this node
-    for (uint32_t guard = 0; guard < nw; guard++) {
-        if (up.x == kEmpty) return;  // the root is complete
-        const uint32_t w = up.x, k = up.y & 3u;
-        if (w >= nw) {
-            atomicOr(&hdr[kHdrErr], kErrBuild);
-            return;
-        }
-        NodeT* nd = nodes + w;
-        store_kid(&nd->kid[k], b, self);
-        const uint2 upn = nodeUp[w];
-        const uint32_t need = nkids[w] & 0xffu;
-        // release: this slot's stores before the arrival; acquire: the other slots' after it
-        if (arrive_acq_rel(&arrive[w]) + 1u != need) return;
-        node_union_cg(nd, b);
-        up = upn;
-        self = w;
+        if (r != kEmpty) range_box(leafBox, pyr, s_lo[t], s_lo[t] + s_num[t], bx);
+        store_kid(&nodes[s_wi[t >> 2]].kid[t & 3u], bx, ref);
     }
 }
 
@@ -716,12 +787,20 @@ cudaError_t build_bvh(MeshBuffers& m, bool fp64, unsigned* h_words, cudaMemPool_
     unsigned* hdr;
     float* box;
     double* box64;
-    uint32_t *k0, *v0, *k1, *v1, *counts, *totals, *widx, *nkids;
+    uint32_t *k0, *v0, *k1, *v1, *counts, *totals, *widx;
     uint4* child;
     int* parent;
     uint8_t* tab;
-    uint2* nodeUp;
-    unsigned* arrive;
+    Pyramid<float> py = {};
+    Pyramid<double> py64 = {};
+    // levels until one entry covers everything
+    uint32_t off[kPyrLevels] = {}, entries = 0;
+    int levels = 0;
+    for (uint32_t m_ = n; m_ > 1;) {
+        m_ = (m_ + 1u) / 2u;
+        off[++levels] = entries;
+        entries += m_;
+    }
     for (;;) {
         Carve c{mem};
         hdr = c.take<unsigned>(kHdrWords);
@@ -737,9 +816,8 @@ cudaError_t build_bvh(MeshBuffers& m, bool fp64, unsigned* h_words, cudaMemPool_
         parent = c.take<int>(n);
         tab = c.take<uint8_t>(n);
         widx = c.take<uint32_t>(n);
-        nodeUp = c.take<uint2>(bound);
-        nkids = c.take<uint32_t>(bound);
-        arrive = c.take<unsigned>(bound);
+        if (fp64) py64.box = c.take<double>(6 * (size_t)entries);
+        else py.box = c.take<float>(6 * (size_t)entries);
         if (mem) break;
         GI_TRY(pool_alloc(&mem, (size_t)(c.p - mem) + 256, pool, st));
     }
@@ -748,8 +826,11 @@ cudaError_t build_bvh(MeshBuffers& m, bool fp64, unsigned* h_words, cudaMemPool_
         cudaStream_t st;
         ~Free() { cudaFreeAsync(p, st); }
     } free_{mem, st};
+    py.levels = py64.levels = levels;
+    for (int L = 0; L < kPyrLevels; L++) py.off[L] = py64.off[L] = off[L];
     GI_TRY(cudaMemsetAsync(hdr, 0, sizeof(unsigned) * kHdrWords, st));
-    const int tb = 256;
+    constexpr int tb = 256;
+    static_assert(kPyrThreads == tb && kColThreads == tb, "one block count serves all");
     const int gb = (int)((n + tb - 1) / tb);
     // Kernels that follow another kernel in the stream are launched as its
     // programmatic dependents (launch_dep): each waits for its predecessor at
@@ -789,8 +870,15 @@ cudaError_t build_bvh(MeshBuffers& m, bool fp64, unsigned* h_words, cudaMemPool_
         m.root = kLeaf | 0u;
     } else {
         const int gi_ = (int)((n - 1 + tb - 1) / tb);
-        launch_dep(k_state_tables, gi_, tb, st, (int)n, (const uint4*)child, (const int*)parent, tab);
-        launch_dep(k_wide_flags, gi_, tb, st, (int)n, (const int*)parent, (const uint8_t*)tab, widx, hdr);
+        if (!fp64) {
+            launch_dep(k_state_tables<float>, gb, kPyrThreads, st, (int)n, (const uint4*)child, (const int*)parent, tab,
+                       (const float*)m.leafBox, py);
+            launch_dep(k_wide_flags<float>, gi_, kPyrThreads, st, (int)n, (const int*)parent, (const uint8_t*)tab, widx, hdr, py);
+        } else {
+            launch_dep(k_state_tables<double>, gb, kPyrThreads, st, (int)n, (const uint4*)child, (const int*)parent, tab,
+                       (const double*)m.leafBox64, py64);
+            launch_dep(k_wide_flags<double>, gi_, kPyrThreads, st, (int)n, (const int*)parent, (const uint8_t*)tab, widx, hdr, py64);
+        }
         uint32_t cap = bound;
         const bool exact = build_needs_host(n);
         if (exact) {
@@ -798,27 +886,22 @@ cudaError_t build_bvh(MeshBuffers& m, bool fp64, unsigned* h_words, cudaMemPool_
             GI_TRY(cudaStreamSynchronize(st));
             cap = std::min(bound, 1u + h_words[kHdrWide]);
         }
-        const int gw = (int)((cap + tb - 1) / tb);
         // (a plain launch after the host round trip, a dependent one otherwise)
         auto collapse = [&](auto kern, auto... args) {
-            if (exact) kern<<<gi_, tb, 0, st>>>(args...);
-            else launch_dep(kern, gi_, tb, st, args...);
+            if (exact) kern<<<gi_, kColThreads, 0, st>>>(args...);
+            else launch_dep(kern, gi_, kColThreads, st, args...);
         };
         if (!fp64) {
             GI_TRY(pool_alloc(&m.nodes, sizeof(WNode) * (size_t)cap, pool, st));
             collapse(k_collapse<float, WNode>, (int)n, (const uint4*)child, (const uint32_t*)widx, cap,
-                     (const float*)m.leafBox, m.nodes, nodeUp, nkids, arrive, hdr + kHdrErr);
-            launch_dep(k_refit_wide<float, WNode>, gw, tb, st, cap, hdr, (const uint2*)nodeUp, (const uint32_t*)nkids,
-                       m.nodes, arrive);
+                     (const float*)m.leafBox, py, m.nodes, hdr + kHdrErr);
         } else {
             GI_TRY(pool_alloc(&m.nodes64, sizeof(WNode64) * (size_t)cap, pool, st));
             collapse(k_collapse<double, WNode64>, (int)n, (const uint4*)child, (const uint32_t*)widx, cap,
-                     (const double*)m.leafBox64, m.nodes64, nodeUp, nkids, arrive, hdr + kHdrErr);
-            launch_dep(k_refit_wide<double, WNode64>, gw, tb, st, cap, hdr, (const uint2*)nodeUp,
-                       (const uint32_t*)nkids, m.nodes64, arrive);
+                     (const double*)m.leafBox64, py64, m.nodes64, hdr + kHdrErr);
         }
         m.root = 0;
-        note_launches(4);
+        note_launches(3);
     }
     // depth-3 and depth-4 cuts, per precision (their sizes are the same); the sizes
     // stay on the device, where the seeding reads them
