@@ -215,8 +215,8 @@ __device__ __forceinline__ uint32_t morton_axis(float c, float lo, float ext)
 template <int BITS, int ITEMS>
 __global__ void __launch_bounds__(kRsThreads) k_morton_hist(const float* __restrict__ box, uint32_t nt,
                                                             const unsigned* __restrict__ hdr,
-                                                            uint32_t* __restrict__ keys, uint32_t* __restrict__ vals,
-                                                            uint32_t* __restrict__ counts, uint32_t ntiles)
+                                                            RsElem* __restrict__ out, uint32_t* __restrict__ counts,
+                                                            uint32_t ntiles)
 {
     pdl_enter();
     constexpr uint32_t kDig = 1u << BITS;
@@ -248,8 +248,7 @@ __global__ void __launch_bounds__(kRsThreads) k_morton_hist(const float* __restr
     for (int it = 0; it < ITEMS; it++) {
         const uint32_t t = base + it * kRsThreads + threadIdx.x;
         if (t < nt) {
-            keys[t] = kk[it];
-            vals[t] = t;
+            out[t] = (RsElem)kk[it] << 32 | t;
             atomicAdd(&h[kk[it] & (kDig - 1u)], 1u);
         }
     }
@@ -787,7 +786,8 @@ cudaError_t build_bvh(MeshBuffers& m, bool fp64, unsigned* h_words, cudaMemPool_
     unsigned* hdr;
     float* box;
     double* box64;
-    uint32_t *k0, *v0, *k1, *v1, *counts, *totals, *widx;
+    RsElem *e0, *e1;
+    uint32_t *k0, *v0, *counts, *totals, *widx;
     uint4* child;
     int* parent;
     uint8_t* tab;
@@ -806,10 +806,10 @@ cudaError_t build_bvh(MeshBuffers& m, bool fp64, unsigned* h_words, cudaMemPool_
         hdr = c.take<unsigned>(kHdrWords);
         box = c.take<float>(6 * (size_t)n);
         box64 = fp64 ? c.take<double>(6 * (size_t)n) : nullptr;
+        e0 = c.take<RsElem>(n);
+        e1 = c.take<RsElem>(n);
         k0 = c.take<uint32_t>(n);
         v0 = c.take<uint32_t>(n);
-        k1 = c.take<uint32_t>(n);
-        v1 = c.take<uint32_t>(n);
         counts = c.take<uint32_t>((size_t)kDig * ntiles);
         totals = c.take<uint32_t>(kDig);
         child = c.take<uint4>(n);
@@ -850,12 +850,12 @@ cudaError_t build_bvh(MeshBuffers& m, bool fp64, unsigned* h_words, cudaMemPool_
     }
     if (small) {
         launch_dep(k_morton_hist<kMortonDigit, kRsItemsSmall>, ntiles, kRsThreads, st, (const float*)box, n,
-                   (const unsigned*)hdr, k0, v0, counts, ntiles);
-        radix_sort<uint32_t, kMortonDigit, kRsItemsSmall>(k0, v0, k1, v1, n, 30, counts, totals, st);
+                   (const unsigned*)hdr, e0, counts, ntiles);
+        radix_sort<kMortonDigit, kRsItemsSmall>(e0, e1, k0, v0, n, 30, counts, totals, st);
     } else {
         launch_dep(k_morton_hist<kMortonDigit, kRsItems>, ntiles, kRsThreads, st, (const float*)box, n,
-                   (const unsigned*)hdr, k0, v0, counts, ntiles);
-        radix_sort<uint32_t, kMortonDigit, kRsItems>(k0, v0, k1, v1, n, 30, counts, totals, st);
+                   (const unsigned*)hdr, e0, counts, ntiles);
+        radix_sort<kMortonDigit, kRsItems>(e0, e1, k0, v0, n, 30, counts, totals, st);
     }
     // leaves in sorted order, and the binary radix tree
     if (!fp64) {
