@@ -795,16 +795,21 @@ static gi_status run_jobs(gi_ctx* c, std::vector<JobDev>& jobs, const gi_interse
                     CK(c, launch_order_small(b, O, sort, c->segs, c->nseg, c->pairs_out, c->job_out, c->segs_out,
                                              c->segpair_out, want_segs, c->st),
                        "ordering");
-                else
+                else {
+                    const HostOut host{(int32_t*)hp, nj > 1 ? (uint32_t*)(hp + off_jobs) : nullptr, (double*)(hp + off_segs),
+                                       (int32_t*)(hp + off_segpair), pp, ps};
                     CK(c, launch_order_gather(b, O, sort, c->segs, c->nseg, c->pairs_out, c->job_out, c->segs_out,
-                                              c->segpair_out, want_segs, c->cfg, c->st),
+                                              c->segpair_out, host, want_segs, c->cfg, c->st),
                        "ordering");
+                }
             }
         }
         if (events) CK(c, cudaEventRecord(c->ev[4], c->st), "event");
         if (!fin) {
-            // speculative copy at the previous call's size
             CK(c, cudaMemcpyAsync(c->h_cnt, b.cnt, sizeof(Counters), cudaMemcpyDeviceToHost, c->st), "counters");
+        }
+        if (!fin && small_order) {
+            // speculative copy at the previous call's size
             CK(c, cudaMemcpyAsync(hp, c->pairs_out, sizeof(int32_t) * 2 * (size_t)pp, cudaMemcpyDeviceToHost, c->st),
                "copy pairs");
             if (nj > 1)

@@ -2075,21 +2075,27 @@ __global__ void __launch_bounds__(kOsThreads) k_os_scatter(Bufs B, OrderBufs O, 
 
 // sorted position k -> pairs_out[k], job_out[k]; the segments of the pair go
 // to the prefix sum of the segment counts (tile look-back).  One item per
-// thread, so every load of a thread is issued at once.
+// thread, so every load of a thread is issued at once.  A tile's segments are
+// one run of the output: it is written 16 bytes a lane from a list of their
+// sources.  What fits into the host's arrays goes there as well, at the link's
+// rate and at the result's own size (the copies that did this afterwards moved
+// the size guessed before the call, a quarter more than the last result).
 __global__ void __launch_bounds__(kOsGatherTile) k_os_gather(Bufs B, OrderBufs O, const double* __restrict__ segs,
                                                              const uint32_t* __restrict__ nseg, int32_t* pairs_out,
                                                              uint32_t* job_out, double* segs_out,
-                                                             int32_t* segpair_out, int want_segments, int sorted)
+                                                             int32_t* segpair_out, HostOut H, int want_segments, int sorted)
 {
     __shared__ uint32_t sw[33];
     __shared__ unsigned s_tile, s_base;
+    __shared__ uint32_t s_src[3 * kOsGatherTile];  // a segment's pair, its place in the results
+    __shared__ uint16_t s_at[3 * kOsGatherTile];   // ... and its place in the tile, 4 x that + the segment's number
     const unsigned n = res_count(B);
     const unsigned ntiles = (n + kOsGatherTile - 1) / kOsGatherTile;
     if (threadIdx.x == 0) s_tile = atomicAdd(&O.tile_ctr[O.passes], 1u);
     __syncthreads();
     const unsigned tile = s_tile;
     if (tile >= ntiles) return;
-    const unsigned k = tile * kOsGatherTile + threadIdx.x;
+    const unsigned k0 = tile * kOsGatherTile, k = k0 + threadIdx.x;
     const bool ok = k < n;
     const unsigned src = ok ? (sorted ? __ldcg(O.vals[O.passes & 1] + k) : k) : 0u;
     const unsigned c = (ok && want_segments) ? __ldcg(nseg + src) : 0u;
@@ -2102,19 +2108,32 @@ __global__ void __launch_bounds__(kOsGatherTile) k_os_gather(Bufs B, OrderBufs O
         s_base = excl;
         if (tile == ntiles - 1) B.cnt->nseg = excl + tot;
     }
+    for (unsigned q = 0; q < c; q++) {  // c <= 3
+        s_src[ex + q] = src;
+        s_at[ex + q] = (uint16_t)(4u * threadIdx.x + q);
+    }
     __syncthreads();
-    if (!ok) return;
-    pairs_out[2 * (size_t)k] = (int32_t)r.y;
-    pairs_out[2 * (size_t)k + 1] = (int32_t)r.z;
-    job_out[k] = r.x;
-    const unsigned off = s_base + ex;
-    for (unsigned q = 0; q < c; q++) {
-        const double2* sp = reinterpret_cast<const double2*>(segs + 18 * (size_t)src + 6 * q);
-        double2* dp = reinterpret_cast<double2*>(segs_out + 6 * (size_t)(off + q));
-        dp[0] = __ldcg(sp);
-        dp[1] = __ldcg(sp + 1);
-        dp[2] = __ldcg(sp + 2);
-        segpair_out[off + q] = (int32_t)k;
+    if (ok) {
+        const int2 p = make_int2((int32_t)r.y, (int32_t)r.z);
+        reinterpret_cast<int2*>(pairs_out)[k] = p;
+        job_out[k] = r.x;
+        if (k < H.pairs_cap) {
+            reinterpret_cast<int2*>(H.pairs)[k] = p;
+            if (H.job) H.job[k] = r.x;
+        }
+    }
+    const size_t base = s_base;
+#pragma unroll 3
+    for (unsigned j = threadIdx.x; j < 3u * tot; j += kOsGatherTile) {
+        const unsigned s = j / 3u, part = j - 3u * s;
+        const double2 v = __ldcg(reinterpret_cast<const double2*>(segs + 18 * (size_t)s_src[s] + 6 * (s_at[s] & 3u)) + part);
+        reinterpret_cast<double2*>(segs_out)[3 * base + j] = v;
+        if (base + s < H.segs_cap) reinterpret_cast<double2*>(H.segs)[3 * base + j] = v;
+    }
+    for (unsigned s = threadIdx.x; s < tot; s += kOsGatherTile) {
+        const int32_t at = (int32_t)(k0 + (s_at[s] >> 2));
+        segpair_out[base + s] = at;
+        if (base + s < H.segs_cap) H.segpair[base + s] = at;
     }
 }
 
@@ -2157,7 +2176,8 @@ OrderBufs make_order_bufs(void* scratch, uint32_t cap, int bits_a, int bits_b, i
 
 cudaError_t launch_order_gather(const Bufs& b, const OrderBufs& O, bool sort, const double* segs,
                                 const uint32_t* nseg, int32_t* pairs_out, uint32_t* job_out, double* segs_out,
-                                int32_t* segpair_out, bool want_segments, const LaunchCfg& cfg, cudaStream_t st)
+                                int32_t* segpair_out, const HostOut& host, bool want_segments, const LaunchCfg& cfg,
+                                cudaStream_t st)
 {
     const unsigned tiles = O.ntiles_cap ? O.ntiles_cap : 1u;
     OrderBufs o = O;
@@ -2172,7 +2192,7 @@ cudaError_t launch_order_gather(const Bufs& b, const OrderBufs& O, bool sort, co
     }
     const unsigned gtiles = O.ntiles_cap * (kOsTile / kOsGatherTile);
     k_os_gather<<<gtiles, kOsGatherTile, 0, st>>>(b, o, segs, nseg, pairs_out, job_out, segs_out, segpair_out,
-                                                  want_segments ? 1 : 0, sort ? 1 : 0);
+                                                  host, want_segments ? 1 : 0, sort ? 1 : 0);
     note_launches(1);
     return cudaGetLastError();
 }

@@ -108,9 +108,19 @@ struct OrderBufs {
 };
 size_t order_scratch_bytes(uint32_t cap, int passes);
 OrderBufs make_order_bufs(void* scratch, uint32_t cap, int bits_a, int bits_b, int bits_job);
+// Pinned host arrays for the first pairs_cap pairs and segs_cap segments of the
+// ordered result (job null: not wanted); the device arrays get all of it.
+struct HostOut {
+    int32_t* pairs;
+    uint32_t* job;
+    double* segs;
+    int32_t* segpair;
+    uint32_t pairs_cap, segs_cap;
+};
 cudaError_t launch_order_gather(const Bufs& b, const OrderBufs& O, bool sort, const double* segs,
                                 const uint32_t* nseg, int32_t* pairs_out, uint32_t* job_out, double* segs_out,
-                                int32_t* segpair_out, bool want_segments, const LaunchCfg& cfg, cudaStream_t st);
+                                int32_t* segpair_out, const HostOut& host, bool want_segments, const LaunchCfg& cfg,
+                                cudaStream_t st);
 // Small-count ordering: a cooperative launch of kOrderSmallBlocks blocks,
 // each sorting a run of kOrderSmallRun keys, for up to kOrderSmallMax results.
 // If the call produced more, the kernel only sets Counters::order_redo and the
