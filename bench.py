@@ -44,7 +44,7 @@ METRIC = "ms/intersect at 2×1.3M tris & tri-pair tests/s; pose-update p50/p99 v
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one traversal
 # launch on the level-8 pose workload with L2 flushed, from the ncu captures
 # summarised in profiles/k_traverse_config2.md, per traversal shape captured
-TRAVERSE_DRAM_BYTES = {}
+TRAVERSE_DRAM_BYTES = {4: 12.177e6}
 
 
 def parse():

@@ -4,9 +4,11 @@
 // src/GPUIntersector/KernelBVHController.cu:603-699 in the reference, whose chunk
 // loop syncs and copies to the host several times per chunk and calls CGAL on
 // the CPU for undecided pairs):
-//   counters reset -> k_traverse_blocks (cooperative) -> k_exact
-//   -> one counters read-back (capacity check; buffers grow x4 and the call is
-//      re-run on overflow) -> k_segments -> ordering -> copies to the host.
+//   k_traverse_blocks (cooperative) -> k_finish (exact stage, ordering, segments,
+//   results and counters written to pinned host memory) -> one synchronisation
+//   (capacity check; buffers grow x4 and the call is re-run on overflow).
+// Results past the finish's limits, and unsorted ones: k_exact -> k_segments ->
+// ordering kernels instead of k_finish.
 // No CPU fallback exists: every pair is decided on the device.
 #include <algorithm>
 #include <atomic>

@@ -21,7 +21,7 @@ constexpr uint32_t kEmpty = 0xFFFFFFFFu;  // unused child slot
 // 4-wide BVH node: a child's box and reference lie together, so that lane k of a
 // quad reads child k with two 16-byte loads (field by field it took seven
 // 4-byte ones, each of which touched the lines of all eight quads of a warp)
-// and the refit writes it with two stores.
+// and the collapse writes it with two stores.
 struct __align__(32) WKid {
     float lo[3];
     uint32_t ref;

@@ -14,9 +14,11 @@
 //               BVH4 traversal in the blocks' shared memory (16 child pairs per
 //               node pair), a pool through which loaded blocks hand node pairs to
 //               idle ones, and the first filter stage on the leaf pairs.
-//   k_exact     FP64 filter + exact integer signs for the escalated pairs.
-//   k_segments  intersection sets and correctly rounded endpoints.
-//   ordering    radix sort by (job, a, b) and gathers.
+//   k_finish    sorted output of up to kFinMax results: the exact stage for the
+//               escalated pairs, ordering, correctly rounded endpoints, and the
+//               write to the host, in one launch.
+//   k_exact, k_segments, ordering kernels  the same in separate launches, for
+//               larger or unsorted results.
 #include <algorithm>
 #include <atomic>
 #include <cstdio>

@@ -145,7 +145,8 @@ typedef struct {
     double ms_exact;                  /* device time: FP64 / exact stage */
     double ms_segments;               /* device time: segment construction */
     double ms_sort;                   /* device time: output ordering (the part after segment construction
-                                         ends; ranking overlaps the segments).  With the one-launch
+                                         ends; ranking overlaps the segments;
+                                         for large results the write to the host too).  With the one-launch
                                          finish (finish_phases = 4), ms_exact, ms_segments and ms_sort
                                          are its phases' own spans (its timestamps; ms_segments includes
                                          the writing of the results to the host) and ms_traverse the
