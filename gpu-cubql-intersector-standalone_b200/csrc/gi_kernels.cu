@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdio>
+#include <type_traits>
 
 #include "gi_classify.cuh"
 #include "gi_launch.h"
@@ -211,10 +212,9 @@ __device__ __forceinline__ uint32_t morton_axis(float c, float lo, float ext)
 
 // 30-bit Morton keys of the triangles (their box centres quantised to 10 bits
 // per axis over the centroid bounds of the header) with identity values, a tile's triangles per block, and each block's counts
-// of the first radix digit in the layout of k_rs_hist (digit-major, one column
-// per block), so the sort's first pass needs no histogram launch.  All of a
+// of the first radix digit where k_rs_hist would write them, so the sort's first pass needs no histogram launch.  All of a
 // thread's box loads are issued before its first shared-memory atomic.
-template <int BITS, int ITEMS>
+template <int BITS, int ITEMS, bool FEW>
 __global__ void __launch_bounds__(kRsThreads) k_morton_hist(const float* __restrict__ box, uint32_t nt,
                                                             const unsigned* __restrict__ hdr,
                                                             RsElem* __restrict__ out, uint32_t* __restrict__ counts,
@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(kRsThreads) k_morton_hist(const float* __restr
         }
     }
     __syncthreads();
-    for (uint32_t d = threadIdx.x; d < kDig; d += kRsThreads) counts[d * ntiles + blockIdx.x] = h[d];
+    for (uint32_t d = threadIdx.x; d < kDig; d += kRsThreads) counts[rs_count_at<BITS, FEW>(d, blockIdx.x, ntiles)] = h[d];
 }
 
 __device__ __forceinline__ int kdelta(const uint32_t* __restrict__ keys, int n, int i, int j)
@@ -850,15 +850,16 @@ cudaError_t build_bvh(MeshBuffers& m, bool fp64, unsigned* h_words, cudaMemPool_
         GI_TRY(cudaGetLastError());
         return cudaMemcpyAsync(h_words, hdr, sizeof(unsigned) * kHdrWords, cudaMemcpyDeviceToHost, st);
     }
-    if (small) {
-        launch_dep(k_morton_hist<kMortonDigit, kRsItemsSmall>, ntiles, kRsThreads, st, (const float*)box, n,
+    auto sort = [&](auto items, auto few) {
+        constexpr int kItems = decltype(items)::value;
+        constexpr bool kFew = decltype(few)::value;
+        launch_dep(k_morton_hist<kMortonDigit, kItems, kFew>, ntiles, kRsThreads, st, (const float*)box, n,
                    (const unsigned*)hdr, e0, counts, ntiles);
-        radix_sort<kMortonDigit, kRsItemsSmall>(e0, e1, k0, v0, n, 30, counts, totals, st);
-    } else {
-        launch_dep(k_morton_hist<kMortonDigit, kRsItems>, ntiles, kRsThreads, st, (const float*)box, n,
-                   (const unsigned*)hdr, e0, counts, ntiles);
-        radix_sort<kMortonDigit, kRsItems>(e0, e1, k0, v0, n, 30, counts, totals, st);
-    }
+        radix_sort<kMortonDigit, kItems, kFew>(e0, e1, k0, v0, n, 30, counts, totals, st);
+    };
+    if (!small) sort(std::integral_constant<int, kRsItems>(), std::false_type());
+    else if (ntiles <= kRsFew) sort(std::integral_constant<int, kRsItemsSmall>(), std::true_type());
+    else sort(std::integral_constant<int, kRsItemsSmall>(), std::false_type());
     // leaves in sorted order, and the binary radix tree
     if (!fp64) {
         launch_dep(k_karras_leaves<float>, gb, tb, st, (const uint32_t*)k0, (const uint32_t*)v0, (int)n,

@@ -1,6 +1,6 @@
 """Mesh builds on the GPU at the sizes where their kernels change: the smallest
 trees, the edges of the box pyramid (32 and 256 leaves) and of the radix tiles
-(1,024 and 3,072 keys) and both sides of the
+(1,024 and 3,072 keys), 20 and 21 small tiles, and both sides of the
 limit for small tiles and the bounded node array (2^19 triangles); each mesh is
 intersected in FP32, FP64 and FP32 form again (the two trees number their nodes
 apart) and compared with the exact oracle.  Invalid input at both sizes."""
@@ -21,7 +21,7 @@ def _strip(n, rng):
     return v, t[rng.permutation(len(t))[:n]].astype(np.uint32)
 
 
-@pytest.mark.parametrize("n", [1, 2, 3, 4, 5, 7, 31, 32, 33, 255, 256, 257, 511, 513, 1023, 1024, 1025, 3072, 3073, 20000, 524288, 524289])
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 5, 7, 31, 32, 33, 255, 256, 257, 511, 513, 1023, 1024, 1025, 3072, 3073, 20000, 20480, 20481, 524288, 524289])
 def test_build_sizes(ctx, gi, oc, n):
     rng = np.random.default_rng(n)
     vA, tA = _strip(n, rng)
