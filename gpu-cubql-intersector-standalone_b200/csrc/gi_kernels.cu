@@ -211,9 +211,10 @@ __device__ __forceinline__ uint32_t morton_axis(float c, float lo, float ext)
 }
 
 // 30-bit Morton keys of the triangles (their box centres quantised to 10 bits
-// per axis over the centroid bounds of the header) with identity values, a tile's triangles per block, and each block's counts
-// of the first radix digit where k_rs_hist would write them, so the sort's first pass needs no histogram launch.  All of a
-// thread's box loads are issued before its first shared-memory atomic.
+// per axis over the centroid bounds of the header) with identity values, a tile's
+// triangles per block, and each block's counts of the first radix digit where
+// k_rs_hist would write them, so the sort's first pass needs no histogram launch.
+// All of a thread's box loads are issued before its first shared-memory atomic.
 template <int BITS, int ITEMS, bool FEW>
 __global__ void __launch_bounds__(kRsThreads) k_morton_hist(const float* __restrict__ box, uint32_t nt,
                                                             const unsigned* __restrict__ hdr,
