@@ -603,7 +603,9 @@ static gi_status run_jobs(gi_ctx* c, std::vector<JobDev>& jobs, const gi_interse
     const uint32_t nj = (uint32_t)jobs.size();
     const int prec = o.precision_mode == GI_PREC_FP64 ? 1 : 0;
     const bool want_segs = o.want_segments != 0;
-    const bool sort = o.sort_output != 0;
+    // a batch's results are split into its jobs, which takes an order by job: only
+    // one pair's can stay as they were found
+    const bool sort = o.sort_output != 0 || nj > 1;
     uint64_t maxA = 1, maxB = 1, sumA = 0, sumT = 0;
     for (auto& j : jobs) {
         j.a0 = sumA;
@@ -953,14 +955,9 @@ static gi_status run_jobs(gi_ctx* c, std::vector<JobDev>& jobs, const gi_interse
         r->nsegs = nsegs;
         if (hj) {
             r->job = hj;
-            std::fill(flat_offsets, flat_offsets + nj + 1, (int64_t)0);
-            if (sort) {
-                for (uint32_t j = 0; j < nj; j++)
-                    flat_offsets[j + 1] = std::upper_bound(hj + flat_offsets[j], hj + nres, j) - hj;
-            } else {
-                for (uint32_t k = 0; k < nres; k++) flat_offsets[hj[k] + 1]++;
-                for (uint32_t j = 0; j < nj; j++) flat_offsets[j + 1] += flat_offsets[j];
-            }
+            flat_offsets[0] = 0;
+            for (uint32_t j = 0; j < nj; j++)
+                flat_offsets[j + 1] = std::upper_bound(hj + flat_offsets[j], hj + nres, j) - hj;
         } else {
             r->job_own.assign(nres, 0u);
             r->job = r->job_own.data();
@@ -983,7 +980,7 @@ static gi_status run_jobs(gi_ctx* c, std::vector<JobDev>& jobs, const gi_interse
         buf = nullptr;  // now held by the result
         return GI_OK;
     }
-    // split per job (sorted by job first)
+    // split per job (the results are ordered by job)
     std::vector<uint32_t> job_start(nj + 1, 0);
     if (nj == 1) {
         job_start[1] = nres;

@@ -121,7 +121,8 @@ typedef struct {
 typedef struct {
     int32_t want_segments;  /* 1: emit intersection segments */
     int32_t precision_mode; /* GI_PREC_* */
-    int32_t sort_output;    /* 1: pairs sorted by (a, b) (default 1) */
+    int32_t sort_output;    /* 1: pairs sorted by (a, b) (default 1); 0: one pair's in any order (the
+                               results of a batch are always sorted, by job first) */
     int32_t reserved;
 } gi_intersect_opts;
 
