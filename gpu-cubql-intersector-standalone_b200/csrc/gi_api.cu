@@ -842,7 +842,7 @@ static gi_status run_jobs(gi_ctx* c, std::vector<JobDev>& jobs, const gi_interse
             };
             // (a pool that was too small starves the later stages: they may grow too)
             if (H.overflow & kOvfFrontier) need_front = g4(c->cap_front, (uint32_t)std::min<uint64_t>((H.pool & 0xffffffffull) * 64, 0x7fffffffu));
-            if (H.overflow & kOvfRes) need_res = g4(c->cap_res, H.res);
+            if (H.overflow & (kOvfRes | kOvfResExact)) need_res = g4(c->cap_res, H.res);
             if (H.overflow & kOvfEsc) need_esc = g4(c->cap_esc, H.esc);
             continue;
         }

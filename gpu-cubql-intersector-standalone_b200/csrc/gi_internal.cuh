@@ -129,7 +129,9 @@ struct Counters {
     unsigned pad2;
 };
 
-constexpr unsigned kOvfFrontier = 1u, kOvfRes = 4u, kOvfEsc = 8u;
+// (kOvfResExact: the exact stage's results did not fit; a bit of its own, because
+// the traversal's are final when k_finish begins and this one is not)
+constexpr unsigned kOvfFrontier = 1u, kOvfRes = 4u, kOvfEsc = 8u, kOvfResExact = 16u;
 constexpr unsigned kErrTimeout = 1u, kErrExactCapacity = 2u;
 // Counters::order_redo: the small-count ordering or the one-launch finish
 // refused; kRedoCrowded: the finish found a key partition over its limit

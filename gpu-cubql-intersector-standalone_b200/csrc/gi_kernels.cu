@@ -1824,7 +1824,7 @@ __device__ __forceinline__ void exact_stage(const Bufs& B, unsigned gtid, unsign
                 B.res[pr] = r;
                 if (B.fin.on) fin_insert<MULTI>(B, r, pr, B.fin.segments ? code_segments(code) : 1u);
             } else {
-                atomicOr(&C->overflow, kOvfRes);
+                atomicOr(&C->overflow, kOvfResExact);
             }
         }
     }
@@ -2618,7 +2618,10 @@ __global__ void __launch_bounds__(kFinThreads, 2) k_finish(const __grid_constant
     for (int q = 0; q < 4; q++) c4[q] = __ldcg(count4 + q);
     unsigned n = ld_cg_u32(&C->res), over = ld_cg_u32(&C->fin_over);
     const unsigned esc = ld_cg_u32(&C->esc);
-    if (ld_cg_u32(&C->overflow)) {  // final at launch: the call reruns with larger buffers
+    // the traversal's overflows, final at launch: the call reruns with larger buffers.
+    // (Not the exact stage's: a block that began late would see another block's,
+    // leave here and be missed at the barrier below.)
+    if (ld_cg_u32(&C->overflow) & ~kOvfResExact) {
         fin_end(C, F.host_cnt, s);
         return;
     }
