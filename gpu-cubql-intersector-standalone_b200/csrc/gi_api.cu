@@ -592,6 +592,10 @@ static gi_status pinned_for(gi_ctx* c, PinnedBuf** buf, size_t need)
     return *buf ? GI_OK : set_err(c, GI_ERR_OOM, "pinned result staging");
 }
 
+// Node pairs of the hand-over pool: to begin with, and where growing after a call
+// that ran short ends (an overflow in a call still grows it further).
+constexpr uint32_t kPoolMin = 1u << 21, kPoolMax = 1u << 26;
+
 // Core: runs the job list on the device and fills per-job results.
 // One host synchronisation per call: every kernel takes its sizes from the
 // device counters, and the results are copied back speculatively at the size
@@ -630,8 +634,28 @@ static gi_status run_jobs(gi_ctx* c, std::vector<JobDev>& jobs, const gi_interse
     memcpy(c->h_jobs, jobs.data(), sizeof(JobDev) * nj);
     bool jobs_there = false;  // a single pair's job travels in the kernel parameters where every kernel takes it from there
     const bool tiny = (c->flags & GI_FLAG_TINY_BUFFERS) != 0;
-    // pool of handed-over node pairs: a few slots per resident block at every size
-    uint32_t need_front = std::max<uint32_t>(c->cap_front, tiny ? 64u : 1u << 21);
+    // pool of handed-over node pairs (a call's slots of 64 are given out once): two
+    // meshes of 1.3 M triangles use 1,200 slots, coincident ones 5,100, a batch of
+    // 256 pairs of 1 k to 200 k 3,300; kPoolMin has 32,768, larger batches more
+    uint32_t need_front =
+        std::max<uint32_t>(c->cap_front, tiny ? 64u : (uint32_t)std::min<uint64_t>(std::max<uint64_t>(kPoolMin, sumT), kPoolMax));
+    if (c->want_front > need_front) {
+        // the last call ran short of slots near its end.  It ran all the same, so a
+        // larger pool that cannot be had is no error.
+        uint4* q = nullptr;
+        unsigned* f = nullptr;
+        if (pool_alloc(&q, sizeof(uint4) * (size_t)c->want_front, c->pool, c->st) == cudaSuccess &&
+            pool_alloc(&f, sizeof(unsigned) * (size_t)c->want_front, c->pool, c->st) == cudaSuccess &&
+            cudaMemsetAsync(f, 0, sizeof(unsigned) * (size_t)c->want_front, c->st) == cudaSuccess) {
+            std::swap(q, c->queue);
+            std::swap(f, c->qflag);
+            c->cap_front = c->cap_qflag = need_front = c->want_front;
+        }
+        if (q) cudaFreeAsync(q, c->st);
+        if (f) cudaFreeAsync(f, c->st);
+        cudaGetLastError();
+        c->want_front = 0;
+    }
     const uint32_t guess = (uint32_t)std::min<uint64_t>(sumT * 2 + 4096, 1u << 22);
     uint32_t need_res = std::max<uint32_t>(c->cap_res, tiny ? 64u : std::max<uint32_t>(guess / 4, 1u << 16));
     uint32_t need_esc = std::max<uint32_t>(c->cap_esc, tiny ? 64u : std::max<uint32_t>(guess / 4, 1u << 16));
@@ -832,6 +856,7 @@ static gi_status run_jobs(gi_ctx* c, std::vector<JobDev>& jobs, const gi_interse
         if (H.err & kErrTimeout) return set_err(c, GI_ERR_TIMEOUT, "a bounded device wait ran out");
         c->cur ^= 1;
         c->cur_clear = fin;
+        if (H.starved) c->want_front = (uint32_t)std::min<uint64_t>((uint64_t)c->cap_front * 4, kPoolMax);
         if (H.err & kErrExactCapacity) return set_err(c, GI_ERR_RANGE, "exact arithmetic capacity exceeded");
         if (H.overflow) {
             if (retries >= 12) return set_err(c, GI_ERR_CAPACITY, "intersection buffers stayed too small");
@@ -929,6 +954,7 @@ static gi_status run_jobs(gi_ctx* c, std::vector<JobDev>& jobs, const gi_interse
         s2.retries = (uint32_t)retries;
         s2.launches = (uint32_t)(launch_count() - launches0);
         s2.traverse_shape = (uint32_t)shape;
+        s2.pool_slots = (uint32_t)H.pool;
         s2.ms_traverse = ms_trav;
         s2.ms_exact = ms_exact;
         s2.ms_segments = ms_seg;

@@ -305,6 +305,7 @@ struct gi_ctx {
     uint4* queue = nullptr;
     unsigned* qflag = nullptr;
     uint32_t cap_front = 0, cap_qflag = 0;
+    uint32_t want_front = 0;  // not 0: a call ran short of pool slots, the next one tries this size
     unsigned tag = 0;
     uint4* res = nullptr;
     uint32_t cap_res = 0;

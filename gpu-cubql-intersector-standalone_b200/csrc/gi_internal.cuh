@@ -112,7 +112,7 @@ struct Counters {
     unsigned int nseg;      // total segments after ordering
     unsigned int obar;      // grid barrier of the small-count ordering kernel
     unsigned int order_redo;  // small-count ordering refused (too many results): rerun on the radix path
-    unsigned int pad5;
+    unsigned int starved;   // iterations that kept node pairs others waited for, the pool being nearly used up
     unsigned long long node_pairs;
     unsigned long long filter_decided;
     unsigned long long exact_signs;

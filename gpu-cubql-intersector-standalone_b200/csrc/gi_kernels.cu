@@ -1143,7 +1143,9 @@ __device__ __forceinline__ void load_kid(const MeshDev& M, uint32_t ref, unsigne
 }
 
 constexpr unsigned kBlkThreads = 256, kBlkWarps = kBlkThreads / 32;
-constexpr unsigned kIdleSpins = 1u << 22;     // consecutive idle polls of one warp (~1 s)
+// consecutive idle polls of a block (a second or more), and how often they begin
+// again because other blocks, with node pairs that they cannot share out, still work
+constexpr unsigned kIdleSpins = 1u << 22, kIdleRounds = 64u;
 
 __device__ __forceinline__ unsigned ld_vol(const unsigned* p)
 {
@@ -1230,12 +1232,17 @@ __device__ __forceinline__ void block_stats(Counters* C, unsigned long long visi
 // published by the call's tag in their flag word (release; a poll acquires it),
 // so nothing is cleared between calls.
 //
+// A call's slots are given out once.  Near the pool's end blocks keep what they
+// have (only one that would exceed its ring still gives, and past the end the call
+// reruns with a larger pool); the host is told (`starved`) and takes a larger
+// pool for the context's next call.
+//
 // Termination: the high half of `pool` counts blocks that work plus slots given
 // out and not yet taken, less the grid's blocks.  A hand-over raises it in the
 // same atomic that reserves its slots, a block lowers it when it runs out, and
 // a taken slot's count becomes its taker's; so it reaches -blocks when, and
-// only when, no node pair is left.  Every wait is bounded; a spent wait sets
-// kErrTimeout and the block ends.
+// only when, no node pair is left.  Every wait is bounded (longer while `starved`
+// counts on); a spent wait sets kErrTimeout and the block ends.
 //
 // What bounds it is latency: an iteration is a chain of a shared-memory pop, a
 // node load, a box transform, the tests and two block barriers, 1.2-2 us with
@@ -1674,9 +1681,9 @@ __global__ void __launch_bounds__(kBlkThreads, kBlkPerSm[MULTI ? 1 : 0]) k_trave
             unsigned state = 0;
             for (;;) {
                 if (tid == 0) {
-                    const unsigned t = s.ticket, patience = cn ? 1u : kIdleSpins;
-                    unsigned st = 0;
-                    for (unsigned spins = 0; spins < patience; spins++) {
+                    const unsigned t = s.ticket;
+                    unsigned st = 0, seen = 0, rounds = 0;
+                    for (unsigned spins = 0;;) {
                         if (t < nslots && ld_acq(B.qflag + t) == B.tag) {
                             st = 1u;
                             break;
@@ -1685,7 +1692,13 @@ __global__ void __launch_bounds__(kBlkThreads, kBlkPerSm[MULTI ? 1 : 0]) k_trave
                             st = 2u;
                             break;
                         }
+                        if (cn) break;  // candidates first
                         if (spins) __nanosleep(64);
+                        if (++spins < kIdleSpins) continue;
+                        const unsigned now = ld_vol(&C->starved);
+                        if (now == seen || ++rounds > kIdleRounds) break;
+                        seen = now;
+                        spins = 0;
                     }
                     if (!st && !cn) {
                         atomicOr(&C->err, kErrTimeout);
@@ -1768,7 +1781,9 @@ __global__ void __launch_bounds__(kBlkThreads, kBlkPerSm[MULTI ? 1 : 0]) k_trave
         }
         if (tid == 0) {
             // tickets waiting; none where the pool is nearly full (every block may give 16 slots at once)
-            s.hungry = tail + 16u * G < nslots && (int)(head - tail) > 0 ? head - tail : 0u;
+            const bool room = tail + 16u * G < nslots;
+            s.hungry = room && (int)(head - tail) > 0 ? head - tail : 0u;
+            if (!room && (int)(head - tail) > 0) atomicAdd(&C->starved, 1u);
         }
         __syncthreads();
         const unsigned p = s.push[it & 1u], hungry = s.hungry;

@@ -155,7 +155,7 @@ typedef struct {
     double ms_total;                  /* device time of the whole call */
     /* kept for the layout: level_times is 0 (the traversal has no common levels) */
     uint32_t level_times;
-    uint32_t reserved2;
+    uint32_t pool_slots;              /* slots (of up to 64 node pairs) that traversal blocks handed to others */
     double level_end_ms[32];
     /* one-launch finish after the traversal (sorted output of a small result;
      * else finish_phases = 0): finish_ms[k] is the time from the launch's start
