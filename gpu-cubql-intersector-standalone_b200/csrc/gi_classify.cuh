@@ -1204,15 +1204,18 @@ __device__ __forceinline__ int classify_small(const double3* pts, unsigned* code
     const double s = __hiloint2double((2046 + 13 - e) << 20, 0);  // 2^(13 - (e - 1023))
     if (!(big * s < 0x1p50)) return DEC_ESC;
     // x * s integer for every coordinate: then all differences are exact integers.
-    // Adding 1.5 * 2^52 leaves the integer in the low word.
-    const double magic = 0x1.8p52;
+    // Adding 1.5 * 2^52 leaves the integer in the low word.  The integer scaled back
+    // must be x itself: x * s alone may underflow to 0 (coordinates near 2^100
+    // beside one of 2^-1000 that a pose made).
+    const double magic = 0x1.8p52, back = __hiloint2double((e - 13) << 20, 0);  // 1 / s
     I3 v[6];
     bool whole = true;
 #pragma unroll
     for (int i = 0; i < 6; i++) {
-        const double x = pts[i].x * s, y = pts[i].y * s, z = pts[i].z * s;
-        const double rx = __dadd_rn(x, magic), ry = __dadd_rn(y, magic), rz = __dadd_rn(z, magic);
-        whole = whole & (__dsub_rn(rx, magic) == x) & (__dsub_rn(ry, magic) == y) & (__dsub_rn(rz, magic) == z);
+        const double3 p = pts[i];
+        const double rx = __fma_rn(p.x, s, magic), ry = __fma_rn(p.y, s, magic), rz = __fma_rn(p.z, s, magic);
+        whole = whole & (__dsub_rn(rx, magic) * back == p.x) & (__dsub_rn(ry, magic) * back == p.y) &
+                (__dsub_rn(rz, magic) * back == p.z);
         v[i] = {__double2loint(rx), __double2loint(ry), __double2loint(rz)};
     }
     if (!whole) return DEC_ESC;
