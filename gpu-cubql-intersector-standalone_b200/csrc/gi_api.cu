@@ -225,7 +225,8 @@ static gi_status mesh_finish(gi_ctx* c, gi_mesh* m, gi_mesh** out, cudaStream_t 
         if (herr & 2u) return sk.fail(GI_ERR_RANGE, "vertex coordinate outside the supported domain");
         return sk.fail(GI_ERR_CUDA, "BVH build: inconsistent wide-node collapse");
     }
-    c->mesh_bytes += m->b.bytes;
+    m->counted = m->b.bytes;
+    c->mesh_bytes += m->counted;
     if (c->budget && c->mesh_bytes > c->budget) {
         mesh_free(c, m, st);
         return sk.fail(GI_ERR_OOM, "HBM budget exceeded by mesh upload");
@@ -373,7 +374,7 @@ static void mesh_free(gi_ctx* c, gi_mesh* m, cudaStream_t st)
     void* p[] = {m->b.arena, m->b.nodes, m->b.leafBox64, m->b.nodes64, m->b.cutBox64, m->b.cutRef64};
     for (void* q : p)
         if (q) cudaFreeAsync(q, st);
-    if (m->b.bytes <= c->mesh_bytes) c->mesh_bytes -= m->b.bytes;
+    c->mesh_bytes -= m->counted;  // (nothing of a mesh whose upload failed; without a later FP64 copy)
     delete m;
 }
 

@@ -24,6 +24,7 @@ struct gi_mesh {
     gi_ctx* ctx = nullptr;
     gi::MeshBuffers b;
     bool has64 = false;
+    size_t counted = 0;     // bytes that the context's mesh_bytes holds for this mesh
     double build_ms = 0.0;  // device time of validation + BVH build (CUDA events on the build stream)
 };
 
