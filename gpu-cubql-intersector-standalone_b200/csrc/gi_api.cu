@@ -189,6 +189,13 @@ struct UploadSink {
         if (e_ != cudaSuccess) return (sink).cuda(e_, (what)); \
     } while (0)
 
+// Under a budget every node array has its exact size, so that a mesh is admitted
+// by what its tree takes and not by the bound that spares small builds a wait.
+static bool exact_nodes(const gi_ctx* c)
+{
+    return c->budget != 0;
+}
+
 // Queues the mesh's build on st (one of the context's two streams, which has one
 // build in flight at most); mesh_finish waits for it.
 static gi_status mesh_start(gi_ctx* c, gi_mesh* m, cudaStream_t st, const UploadSink& sk)
@@ -199,7 +206,7 @@ static gi_status mesh_start(gi_ctx* c, gi_mesh* m, cudaStream_t st, const Upload
     const int s = st == c->st2 ? 1 : 0;
     // device time of validation + build (the reference's buildRefitMesh*Ms)
     cudaError_t e = cudaEventRecord(c->ev_build[s][0], st);
-    if (e == cudaSuccess) e = build_bvh(m->b, false, c->h_build + s * kBuildWords, c->pool, st);
+    if (e == cudaSuccess) e = build_bvh(m->b, false, exact_nodes(c), c->h_build + s * kBuildWords, c->pool, st);
     if (e == cudaSuccess) e = cudaEventRecord(c->ev_build[s][1], st);
     if (e == cudaSuccess) return GI_OK;
     // the stream may still hold kernels that use the mesh: drain it before freeing
@@ -574,7 +581,7 @@ static gi_status ensure_fp64(gi_ctx* c, gi_mesh* m)
         m->has64 = true;
         return GI_OK;
     }
-    cudaError_t e = build_bvh(m->b, true, c->h_build, c->pool, c->st);
+    cudaError_t e = build_bvh(m->b, true, exact_nodes(c), c->h_build, c->pool, c->st);
     const cudaError_t es = cudaStreamSynchronize(c->st);
     if (e == cudaSuccess) e = es;
     if (e != cudaSuccess) return set_err(c, GI_ERR_CUDA, "FP64 BVH build", e);
@@ -1133,7 +1140,7 @@ extern "C" gi_status gi_intersect_oneshot(gi_ctx* c, const double* vA, uint32_t 
         gi_status sb = GI_OK;
         std::string msg_b;
         const UploadSink ka{c, nullptr}, kb{c, &msg_b};
-        if (!build_needs_host(ntA) && !build_needs_host(ntB)) {
+        if (!exact_nodes(c) && !build_wants_exact(ntA) && !build_wants_exact(ntB)) {
             gi_mesh *ma = nullptr, *mb = nullptr;
             s = mesh_upload_start(c, vA, nvA, tA, ntA, &ma, c->st, ka);
             sb = mesh_upload_start(c, vB, nvB, tB, ntB, &mb, c->st2, kb);

@@ -764,19 +764,22 @@ static uint32_t wide_bound(uint32_t n)
 
 // Above this many triangles the node array has its exact size, for a host round
 // trip in the middle of the build (15 us of an idle GPU); below, the size of the
-// bound (a third more nodes, 12 MB at most), and the build is queued in one go.
+// bound, and the build is queued in one go.  (At 2^19 triangles the bound is 45 MB;
+// a surface's tree takes about 33 MB of it, any tree 22 at least; twice that in
+// FP64.  MeshBuffers::bytes counts the tree, and a budgeted context, which admits
+// by it, has exact arrays at every size.)
 constexpr uint32_t kExactNodesAbove = 1u << 19;
 // Radix tiles of 1,024 keys up to this many triangles, else 3,072: the sort's
 // kernels have a block per tile, and 3,072 leave most SMs idle (20 k triangles
 // made seven blocks, 11-13 us a kernel; 300 k ninety-nine).
 constexpr uint32_t kSmallTilesUpTo = 1u << 19;
 
-bool build_needs_host(uint32_t nt)
+bool build_wants_exact(uint32_t nt)
 {
     return nt > kExactNodesAbove;
 }
 
-cudaError_t build_bvh(MeshBuffers& m, bool fp64, unsigned* h_words, cudaMemPool_t pool, cudaStream_t st)
+cudaError_t build_bvh(MeshBuffers& m, bool fp64, bool exact_nodes, unsigned* h_words, cudaMemPool_t pool, cudaStream_t st)
 {
     const uint32_t n = m.nt;
     constexpr int kMortonDigit = 10;  // 30-bit keys: three passes
@@ -884,7 +887,7 @@ cudaError_t build_bvh(MeshBuffers& m, bool fp64, unsigned* h_words, cudaMemPool_
             launch_dep(k_wide_flags<double>, gi_, kPyrThreads, st, (int)n, (const int*)parent, (const uint8_t*)tab, widx, hdr, py64);
         }
         uint32_t cap = bound;
-        const bool exact = build_needs_host(n);
+        const bool exact = exact_nodes || build_wants_exact(n);
         if (exact) {
             GI_TRY(cudaMemcpyAsync(h_words, hdr, sizeof(unsigned) * kHdrWords, cudaMemcpyDeviceToHost, st));
             GI_TRY(cudaStreamSynchronize(st));

@@ -46,13 +46,14 @@ size_t mesh_arena_bytes(uint32_t nv, uint32_t nt);
 // Validates the input (error bit 1: bad index, 2: out of domain) and builds the
 // 4-wide BVH (FP32 boxes) or, with fp64 = true, the FP64 node copy.  Queues
 // everything on st, the copy of the build's header to h_words (kBuildWords
-// pinned words) last; with build_needs_host the call waits once in between.
+// pinned words) last.  With exact_nodes the node array has its exact size, for
+// which the call waits once in between.
 // After the stream has been synchronised, build_result reads the header: the
 // node count and the error bits (4: the wide tree came out inconsistent, not
 // expected; the kernels then skip the bad links).
 constexpr int kBuildWords = 8;
-bool build_needs_host(uint32_t nt);
-cudaError_t build_bvh(MeshBuffers& m, bool fp64, unsigned* h_words, cudaMemPool_t pool, cudaStream_t st);
+bool build_wants_exact(uint32_t nt);  // true: a mesh of this size is built so in any case
+cudaError_t build_bvh(MeshBuffers& m, bool fp64, bool exact_nodes, unsigned* h_words, cudaMemPool_t pool, cudaStream_t st);
 unsigned build_result(MeshBuffers& m, bool fp64, const unsigned* h_words);
 
 // Intersect launch configuration.

@@ -203,6 +203,9 @@ gi_status gi_mesh_upload(gi_ctx* ctx, const double* verts_xyz, uint32_t nv, cons
 gi_status gi_mesh_upload_device(gi_ctx* ctx, const double* d_verts_xyz, uint32_t nv, const uint32_t* d_tris,
                                 uint32_t nt, gi_mesh** out);
 gi_status gi_mesh_release(gi_ctx* ctx, gi_mesh* mesh);
+/* device_bytes: what a budget counts for the mesh, vertices, indices, leaves and
+ * the tree's nodes.  (Without a budget the node array of a mesh of up to 2^19
+ * triangles has room for 2/3 node per triangle, which no tree exceeds.) */
 gi_status gi_mesh_info(const gi_mesh* mesh, uint32_t* nv, uint32_t* nt, uint64_t* nodes, uint64_t* device_bytes);
 /* Device time in ms of the mesh's validation and BVH build (CUDA events around
  * the build kernels on the build stream; the upload's copies are not in it):
