@@ -266,6 +266,18 @@ static gi_status mesh_alloc(gi_ctx* c, uint32_t nv, uint32_t nt, gi_mesh** pm, c
     return GI_OK;
 }
 
+// A host array that h2d copies through the context's staging buffers.
+static bool staged_copy(const void* src, size_t bytes)
+{
+    if (bytes < 2 * Staging::kChunk) return false;
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, src) != cudaSuccess) {
+        cudaGetLastError();  // an unknown pointer is ordinary host memory
+        a.type = cudaMemoryTypeUnregistered;
+    }
+    return a.type == cudaMemoryTypeUnregistered;
+}
+
 // Host -> device copy on stream st.  Pinned sources go straight to the DMA
 // engine.  A large pageable source would be staged by the CUDA driver on the
 // calling thread at about a third of the link rate; instead the context's
@@ -273,14 +285,7 @@ static gi_status mesh_alloc(gi_ctx* c, uint32_t nv, uint32_t nt, gi_mesh** pm, c
 // Returns when the source may be reused (like a pageable cudaMemcpyAsync).
 static cudaError_t h2d(gi_ctx* c, void* dst, const void* src, size_t bytes, cudaStream_t st)
 {
-    if (bytes < 2 * Staging::kChunk) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
-    cudaPointerAttributes a{};
-    if (cudaPointerGetAttributes(&a, src) != cudaSuccess) {
-        cudaGetLastError();  // an unknown pointer is ordinary host memory
-        a.type = cudaMemoryTypeUnregistered;
-    }
-    if (a.type != cudaMemoryTypeUnregistered)
-        return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+    if (!staged_copy(src, bytes)) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
     Staging& sg = c->stage[st == c->st2 ? 1 : 0];
     cudaError_t e = sg.init();
     if (e != cudaSuccess) {
@@ -1133,27 +1138,33 @@ extern "C" gi_status gi_intersect_oneshot(gi_ctx* c, const double* vA, uint32_t 
     {
         // B is copied and built on the second stream while A is on the context's
         // stream: B's copy overlaps A's build and the two builds overlap each
-        // other.  Builds that are queued in one go (and copies that are not
-        // staged) need no second host thread: starting and joining one took 40 us.
+        // other.  A helper thread queues B's part where A's holds up the calling
+        // thread: a build that waits in between, or arrays that are staged (two
+        // meshes of a million pageable vertices and 10 k triangles: 1.7-2.6 ms a call
+        // in thirteen runs; without the thread 1.8-2.5 in ten, 3.6-5.5 in six).  Its start
+        // and join take 40 us.  Pageable arrays that are not staged do not repay
+        // them: meshes of 5 k, 41 k, 82 k, 162 k, 328 k, 512 k triangles 362, 391,
+        // 640, 891, 1208, 1813 us a call with it and 406, 415, 656, 893, 1200, 1652
+        // without.
         std::lock_guard<std::mutex> lk(c->mu);
         cudaSetDevice(c->device);
         gi_status sb = GI_OK;
         std::string msg_b;
         const UploadSink ka{c, nullptr}, kb{c, &msg_b};
-        if (!exact_nodes(c) && !build_wants_exact(ntA) && !build_wants_exact(ntB)) {
-            gi_mesh *ma = nullptr, *mb = nullptr;
-            s = mesh_upload_start(c, vA, nvA, tA, ntA, &ma, c->st, ka);
-            sb = mesh_upload_start(c, vB, nvB, tB, ntB, &mb, c->st2, kb);
-            if (s == GI_OK) s = mesh_finish(c, ma, &A, c->st, ka);
-            if (sb == GI_OK) sb = mesh_finish(c, mb, &B, c->st2, kb);
-        } else {
-            std::thread tb([&] {
+        gi_mesh *ma = nullptr, *mb = nullptr;
+        const bool waits = exact_nodes(c) || build_wants_exact(ntA) || build_wants_exact(ntB);
+        auto start_b = [&] { sb = mesh_upload_start(c, vB, nvB, tB, ntB, &mb, c->st2, kb); };
+        std::thread tb;
+        if (waits || staged_copy(vA, sizeof(double) * 3 * (size_t)nvA) || staged_copy(tA, sizeof(uint32_t) * 3 * (size_t)ntA))
+            tb = std::thread([&] {
                 cudaSetDevice(c->device);
-                sb = mesh_upload_on(c, vB, nvB, tB, ntB, &B, c->st2, kb);
+                start_b();
             });
-            s = mesh_upload_on(c, vA, nvA, tA, ntA, &A, c->st, ka);
-            tb.join();
-        }
+        s = mesh_upload_start(c, vA, nvA, tA, ntA, &ma, c->st, ka);
+        if (tb.joinable()) tb.join();
+        else start_b();
+        if (s == GI_OK) s = mesh_finish(c, ma, &A, c->st, ka);
+        if (sb == GI_OK) sb = mesh_finish(c, mb, &B, c->st2, kb);
         if (s == GI_OK && sb != GI_OK) {
             s = sb;
             c->last_error = msg_b;
