@@ -887,7 +887,10 @@ static gi_status run_jobs(gi_ctx* c, std::vector<JobDev>& jobs, const gi_interse
         if (H.order_redo) {
             if (fin) {
                 fin = false;
-                if (H.order_redo == kRedoCrowded) c->fin_backoff = 64;
+                // (keys spill past small buckets only at more than 65,536 results, after
+                // which the next call has large ones)
+                if (H.order_redo == kRedoCrowded || (H.order_redo == kRedoSpilled && c->fin_bucket == kFinBucketLarge))
+                    c->fin_backoff = 64;
                 if (H.res > kOrderSmallMax) small_order = false;
                 continue;
             }

@@ -134,8 +134,9 @@ struct Counters {
 constexpr unsigned kOvfFrontier = 1u, kOvfRes = 4u, kOvfEsc = 8u, kOvfResExact = 16u;
 constexpr unsigned kErrTimeout = 1u, kErrExactCapacity = 2u;
 // Counters::order_redo: the small-count ordering or the one-launch finish
-// refused; kRedoCrowded: the finish found a key partition over its limit
-constexpr unsigned kRedoCount = 1u, kRedoCrowded = 2u;
+// refused; the finish because of a key partition over its limit (kRedoCrowded) or
+// of more keys beyond their buckets than the overflow list holds (kRedoSpilled)
+constexpr unsigned kRedoCount = 1u, kRedoCrowded = 2u, kRedoSpilled = 3u;
 
 // Results by key partition, for the one-launch finish: filled where results are
 // found, read by k_finish.

@@ -2675,8 +2675,9 @@ __global__ void __launch_bounds__(kFinThreads, 2) k_finish(const __grid_constant
     unsigned most = 0;
 #pragma unroll
     for (int q = 0; q < 4; q++) most = max(most, max(max(c4[q].x, c4[q].y), max(c4[q].z, c4[q].w)));
-    if (__syncthreads_or(most > (unsigned)kFinBig) || over > (unsigned)kFinOverflow) {
-        if (blockIdx.x == 0 && tid == 0) C->order_redo = kRedoCrowded;
+    const bool crowded = __syncthreads_or(most > (unsigned)kFinBig);
+    if (crowded || over > (unsigned)kFinOverflow) {
+        if (blockIdx.x == 0 && tid == 0) C->order_redo = crowded ? kRedoCrowded : kRedoSpilled;
         fin_end(C, F.host_cnt, s);
         return;
     }
