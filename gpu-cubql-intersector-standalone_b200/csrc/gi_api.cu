@@ -1361,7 +1361,7 @@ extern "C" gi_status gi_server_stop(gi_server* s)
     }
     s->cv.notify_all();
     if (s->worker.joinable()) s->worker.join();
-    for (auto& kv : s->done) delete kv.second;
+    for (auto& kv : s->done) gi_result_free(kv.second);  // never fetched: their blocks go back too
     delete s;
     return GI_OK;
 }
