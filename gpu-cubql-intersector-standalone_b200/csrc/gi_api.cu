@@ -609,6 +609,8 @@ static gi_status pinned_for(gi_ctx* c, PinnedBuf** buf, size_t need)
 // that ran short ends (an overflow in a call still grows it further).
 constexpr uint32_t kPoolMin = 1u << 21, kPoolMax = 1u << 26;
 
+constexpr uint32_t kMaxJobs = 1u << 19;  // (a batch's seed tests, 4,096 a job, are numbered in 32 bits)
+
 // Core: runs the job list on the device and fills per-job results.
 // One host synchronisation per call: every kernel takes its sizes from the
 // device counters, and the results are copied back speculatively at the size
@@ -633,7 +635,6 @@ static gi_status run_jobs(gi_ctx* c, std::vector<JobDev>& jobs, const gi_interse
     }
     int ba = bits_for(maxA), bb = bits_for(maxB), bj = nj > 1 ? bits_for(nj) : 0;
     if (ba + bb + bj > 64) return set_err(c, GI_ERR_INVALID_ARG, "batch too large for 64-bit ordering keys");
-    if (nj > (1u << 19)) return set_err(c, GI_ERR_INVALID_ARG, "at most 2^19 jobs per batch");
     if (nj > c->cap_jobs) {
         if (c->d_jobs) cudaFree(c->d_jobs);
         if (c->h_jobs) cudaFreeHost(c->h_jobs);
@@ -1089,24 +1090,32 @@ static gi_status batch_call(gi_ctx* c, const gi_pair_job* jobs, uint32_t nj, con
     if (opts) o = *opts;
     else gi_intersect_opts_default(&o);
     std::lock_guard<std::mutex> lk(c->mu);
+    if (nj > kMaxJobs) return set_err(c, GI_ERR_INVALID_ARG, "at most 2^19 jobs per batch");
     cudaSetDevice(c->device);
-    std::vector<JobDev> jd(nj);
-    for (uint32_t i = 0; i < nj; i++) {
-        const gi_pair_job& j = jobs[i];
-        if (!j.A || !j.B || j.A->ctx != c || j.B->ctx != c) return GI_ERR_INVALID_ARG;
-        if (!pose_ok(j.pose_a) || !pose_ok(j.pose_b)) return set_err(c, GI_ERR_RANGE, "pose outside the supported domain");
-        if (o.precision_mode == GI_PREC_FP64) {
-            gi_status s = ensure_fp64(c, const_cast<gi_mesh*>(j.A));
-            if (s == GI_OK) s = ensure_fp64(c, const_cast<gi_mesh*>(j.B));
-            if (s != GI_OK) return s;
+    std::vector<gi_result*> outs;
+    gi_status s = GI_OK;
+    try {
+        outs.assign(nj, nullptr);
+        std::vector<JobDev> jd(nj);
+        for (uint32_t i = 0; i < nj; i++) {
+            const gi_pair_job& j = jobs[i];
+            if (!j.A || !j.B || j.A->ctx != c || j.B->ctx != c) return GI_ERR_INVALID_ARG;
+            if (!pose_ok(j.pose_a) || !pose_ok(j.pose_b))
+                return set_err(c, GI_ERR_RANGE, "pose outside the supported domain");
+            if (o.precision_mode == GI_PREC_FP64) {
+                s = ensure_fp64(c, const_cast<gi_mesh*>(j.A));
+                if (s == GI_OK) s = ensure_fp64(c, const_cast<gi_mesh*>(j.B));
+                if (s != GI_OK) return s;
+            }
+            jd[i].A = mesh_dev(j.A);
+            jd[i].B = mesh_dev(j.B);
+            jd[i].pa = make_dev_pose(j.pose_a);
+            jd[i].pb = make_dev_pose(j.pose_b);
         }
-        jd[i].A = mesh_dev(j.A);
-        jd[i].B = mesh_dev(j.B);
-        jd[i].pa = make_dev_pose(j.pose_a);
-        jd[i].pb = make_dev_pose(j.pose_b);
+        s = run_jobs(c, jd, o, outs, flat_offsets);
+    } catch (const std::bad_alloc&) {
+        s = set_err(c, GI_ERR_OOM, "host memory");
     }
-    std::vector<gi_result*> outs(nj, nullptr);
-    gi_status s = run_jobs(c, jd, o, outs, flat_offsets);
     if (s != GI_OK) {
         for (auto* r : outs) delete r;
         return s;
