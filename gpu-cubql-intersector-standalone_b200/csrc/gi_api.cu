@@ -586,11 +586,23 @@ static gi_status ensure_fp64(gi_ctx* c, gi_mesh* m)
         m->has64 = true;
         return GI_OK;
     }
+    const size_t bytes = m->b.bytes;
     cudaError_t e = build_bvh(m->b, true, exact_nodes(c), c->h_build, c->pool, c->st);
     const cudaError_t es = cudaStreamSynchronize(c->st);
     if (e == cudaSuccess) e = es;
-    if (e != cudaSuccess) return set_err(c, GI_ERR_CUDA, "FP64 BVH build", e);
-    if (build_result(m->b, true, c->h_build)) return set_err(c, GI_ERR_CUDA, "FP64 BVH build: inconsistent wide-node collapse");
+    const unsigned herr = e == cudaSuccess ? build_result(m->b, true, c->h_build) : 0u;
+    if (e != cudaSuccess || herr) {
+        // what it has of the copy goes back: the next call builds it anew
+        void* p[] = {m->b.leafBox64, m->b.nodes64, m->b.cutBox64, m->b.cutRef64};
+        for (void* q : p)
+            if (q) cudaFreeAsync(q, c->st);
+        m->b.leafBox64 = m->b.cutBox64 = nullptr;
+        m->b.nodes64 = nullptr;
+        m->b.cutRef64 = nullptr;
+        m->b.bytes = bytes;
+        if (e == cudaSuccess) return set_err(c, GI_ERR_CUDA, "FP64 BVH build: inconsistent wide-node collapse");
+        return set_err(c, GI_ERR_CUDA, "FP64 BVH build", e);
+    }
     m->has64 = true;
     return GI_OK;
 }

@@ -848,8 +848,10 @@ cudaError_t build_bvh(MeshBuffers& m, bool fp64, bool exact_nodes, unsigned* h_w
     const int gboxes = (int)((work + 2 * kTriBoxThreads - 1) / (2 * kTriBoxThreads));
     k_tri_boxes<<<gboxes < 1 ? 1 : (gboxes < 592 ? gboxes : 592), kTriBoxThreads, 0, st>>>(m.verts, m.nv, m.tris, n, box, box64, hdr);
     note_launches(1);
-    m.root = kEmpty;
-    m.nnodes = 0;
+    if (!fp64) {  // (both trees have the same; a failed FP64 build leaves the FP32 one's)
+        m.root = kEmpty;
+        m.nnodes = 0;
+    }
     if (n == 0) {
         GI_TRY(cudaGetLastError());
         return cudaMemcpyAsync(h_words, hdr, sizeof(unsigned) * kHdrWords, cudaMemcpyDeviceToHost, st);
