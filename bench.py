@@ -43,7 +43,7 @@ sys.path.insert(0, PKG)
 METRIC = "ms/intersect at 2×1.3M tris & tri-pair tests/s; pose-update p50/p99 vs FP64 path"
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one traversal
 # launch on the level-8 pose workload with L2 flushed, from the ncu captures
-# summarised in profiles/k_traverse_config2.md, per traversal shape captured
+# of the traversal (committed with the profiles), per traversal shape captured
 TRAVERSE_DRAM_BYTES = {4: 12.177e6}
 
 
@@ -703,10 +703,10 @@ def main():
     st = stats[-1]
     # BVH build roofline: the algorithmic bytes of one build of a T-triangle,
     # V-vertex mesh (read the mesh 24V + 12T, a 32-bit key sort 64T, write 2T-1
-    # nodes of 32 B and T ids, read the nodes once to refit) over the device time
-    # of the build kernels (gi_mesh_build_ms), averaged over the builds above
+    # nodes of 32 B and T ids) over the device time of the build kernels
+    # (gi_mesh_build_ms), averaged over the builds above
     T, V = int(cfg["tA"].shape[0]), int(cfg["vA"].shape[0])
-    build_bytes = 24 * V + 12 * T + 64 * T + 32 * (2 * T - 1) + 4 * T + 32 * (2 * T - 1)
+    build_bytes = 24 * V + 12 * T + 64 * T + 32 * (2 * T - 1) + 4 * T
     # warm builds only (the first launches of a process also load the kernels)
     build_ms = []
     for k in range(5):
@@ -764,8 +764,7 @@ def main():
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": TRAVERSE_DRAM_BYTES.get(int(st["traverse_shape"])) if args.level == 8 else None,
                      "traffic_source": "dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture of the "
-                                       "traversal on this workload with the same shape (null: shape not captured); "
-                                       "profiles/k_traverse_config2.md",
+                                       "traversal on this workload with the same shape (null: shape not captured)",
                      "kernel": "k_traverse_blocks", "peak_source": peak_src,
                      "alg_bytes_per_launch": float(alg_bytes),
                      "note": "output-sensitive traversal: bytes = node pairs x 2 nodes x 128 B + leaf pairs x "
@@ -776,8 +775,8 @@ def main():
                            "what": "mean of 4 warm builds of mesh A from pinned host arrays (gi_mesh_build_ms: "
                                    "CUDA events around validation + build, the mid-build host round trip included)",
                            "alg_bytes_per_mesh": build_bytes, "peak_source": peak_src,
-                           "note": "24V + 12T (mesh) + 64T (32-bit key sort) + 32(2T-1) + 4T (nodes, ids) + "
-                                   "32(2T-1) (refit read) over the device time of validation + build kernels"},
+                           "note": "24V + 12T (mesh) + 64T (32-bit key sort) + 32(2T-1) + 4T (nodes, ids) over the "
+                                   "device time of validation + build kernels"},
         "clocks": clk.summary(),
     }
     if rank == 0 and world == 1 and not args.no_cpu_baseline:

@@ -625,8 +625,10 @@ constexpr uint32_t kMaxJobs = 1u << 19;  // (a batch's seed tests, 4,096 a job, 
 
 // Core: runs the job list on the device and fills per-job results.
 // One host synchronisation per call: every kernel takes its sizes from the
-// device counters, and the results are copied back speculatively at the size
-// of the previous call (a second copy follows only when the result grew).
+// device counters.  The result block is sized by the previous call's result; the
+// finish and the large results' gather write into it themselves, the small-count
+// ordering's results are copied at that size.  A result that outgrew the block is
+// copied from device memory afterwards.
 // flat_offsets: not null for one result over all jobs (outs[0]), its offsets here.
 static gi_status run_jobs(gi_ctx* c, std::vector<JobDev>& jobs, const gi_intersect_opts& o,
                           std::vector<gi_result*>& outs, int64_t* flat_offsets)
@@ -916,7 +918,7 @@ static gi_status run_jobs(gi_ctx* c, std::vector<JobDev>& jobs, const gi_interse
         segpair64 = fin && flat_offsets;
         if (nres > pp || nsegs > ps) {
             segpair64 = false;
-            // the result outgrew the speculative copy: copy it again at its real size
+            // the result outgrew the block: copied at its real size from device memory
             off_jobs = (sizeof(int32_t) * 2 * (size_t)nres + 15) & ~(size_t)15;
             off_segs = (off_jobs + (nj > 1 ? sizeof(uint32_t) * (size_t)nres : 0) + 15) & ~(size_t)15;
             off_segpair = off_segs + sizeof(double) * 6 * (size_t)nsegs;

@@ -1115,9 +1115,14 @@ __device__ __forceinline__ unsigned result_code(const TTRes& r)
 // integer arithmetic in registers: no filter, no common-grid search, no local
 // memory.  The steps and the order of the result's points are classify_exact's.
 //
-// Bound by instruction issue.  Two coplanar 512 x 512 grids (2.4 M escalated
-// pairs): 0.20 ms, 3.5 ms with the general form alone, whose out-of-line code
-// stalls on instruction fetches (4 warps waited for them per issue).
+// Bound by the latency of the gathers and of the integer chains at 16 warps per SM
+// (124 registers): issue slots 42 % busy, of 8.6 cycles per issued instruction and
+// warp 3.3 wait for memory and 2.1 for a result.  Two coplanar 512 x 512 grids
+// (2.4 M escalated pairs): 0.20 ms, 3.5 ms with the general form alone, whose
+// out-of-line code stalls on instruction fetches (4 warps waited for them per issue).
+// Coordinates of other grids pay for the attempt and for the FP64 filter after it:
+// on the same grids with a spacing of 0.1 (multi-limb signs) k_exact takes 16.5 ms
+// where the general form alone takes 15.0, 1.35 for 0.95 on 128 x 128.
 // ---------------------------------------------------------------------------
 struct I3 {
     int x, y, z;

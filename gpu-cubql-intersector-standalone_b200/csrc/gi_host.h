@@ -292,7 +292,7 @@ struct gi_ctx {
     std::mutex mu;  // serialises device work of this context
 
     // two sets of counters and partition counts: a call uses set `cur`; the
-    // one-launch finish clears the other one for the next call (other_clear)
+    // one-launch finish clears the other one for the next call
     Counters* d_cnt = nullptr;
     int cur = 0;
     bool cur_clear = false;     // set `cur` is zero

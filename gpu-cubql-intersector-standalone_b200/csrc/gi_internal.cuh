@@ -95,7 +95,8 @@ struct __align__(16) JobDev {
     DevPose pa, pb;
 };
 
-// Device counters of one intersect launch sequence (zeroed by the host).
+// Device counters of one intersect launch sequence: zero when it begins (the
+// one-launch finish clears the next call's, the host's memset does otherwise).
 struct Counters {
     // hot counters, each on its own 128-byte line (polled and updated by every block)
     // pool of the traversal: slots given out (low half), and blocks at work plus

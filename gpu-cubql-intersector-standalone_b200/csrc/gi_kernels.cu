@@ -582,8 +582,8 @@ __global__ void __launch_bounds__(kPyrThreads) k_wide_flags(int n, const int* __
 // than followed.
 //
 // A block finds the children of its 256 binary nodes' wide nodes first, one
-// thread a node, and then fills the child slots, one thread a slot: two nodes in
-// five are wide, and a child with many leaves costs only its own thread the
+// thread a node, and then fills the child slots, one thread a slot: one node in
+// two is wide, and a child with many leaves costs only its own thread the
 // longer union.
 constexpr int kColThreads = 256;
 template <class S, class NodeT>
@@ -1157,9 +1157,7 @@ __device__ __forceinline__ unsigned ld_vol(const unsigned* p)
     return *(const volatile unsigned*)p;
 }
 
-// Release / acquire fence at GPU scope: orders entry stores before the tag
-// stores that follow, and an observed tag before the entry loads that follow.
-// acquire load: the loads after it see what the writer published before its
+// Acquire load: the loads after it see what the writer published before its
 // release (fence + tag store), without waiting for this thread's own stores
 __device__ __forceinline__ unsigned ld_acq(const unsigned* p)
 {
@@ -1231,7 +1229,7 @@ __device__ __forceinline__ void block_stats(Counters* C, unsigned long long visi
 //
 // Sharing out: a block without node pairs takes a ticket (q_head) and polls
 // that slot of the pool.  Every iteration a block looks, with loads that its
-// node loads hide, how many tickets are ahead of the slots given out (q_tail);
+// node loads hide, how many tickets are ahead of the slots given out (pool's low half);
 // if some are, what it holds beyond one iteration's 64 node pairs goes to them
 // from the oldest end (the largest subtrees), up to 64 a slot.  Slots are
 // published by the call's tag in their flag word (release; a poll acquires it),
@@ -1274,7 +1272,9 @@ __device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v)
 
 // resident blocks per SM that the registers are cut for, [batch].  A single pair
 // is bound by latency: a fourth block's tighter registers cost small meshes 1 us;
-// a batch is bound by work (256 pairs: 564 us of traversal with three, 519 with four).
+// a batch is bound by work (256 pairs: 564 us of traversal with three, 519 with
+// four, although its 64 registers spill: 220 bytes of stores in the FP32 form, 464
+// in FP64; a single pair's 80 do not in FP32, 68 bytes in FP64).
 constexpr int kBlkPerSm[2] = {3, 4};
 constexpr unsigned kBlkUnits = kBlkThreads / 4;  // node pairs per iteration, and per slot of the pool
 constexpr unsigned kBlkRing = 32 * kBlkUnits;               // node pairs a block holds (an iteration pushes at most 16 per unit)
@@ -2509,9 +2509,10 @@ cudaError_t launch_order_small_phases(const Bufs& b, const OrderBufs& O, bool so
 // device-to-host copy.  A call over kFinMax results or with a partition over
 // kFinBig keys is refused (Counters::order_redo, decided alike in every block).
 //
-// What bounds it: the FP64 issue of the constructions (about 1,400 instructions
-// an endpoint, one warp per SM sub-partition) and, for larger results, the PCIe
-// writes.  Its predecessor inserted the keys itself (a barrier, one block's scan,
+// What bounds it: latency, the chain of one block's scan, gather, ranking and one
+// result's construction (about 1,400 instructions an endpoint) with barriers
+// between (at 12 k results 23 stalled warps per issue at barriers, issue 9 % and
+// FP64 pipe 5 % busy), and, for larger results, the PCIe writes.  Its predecessor inserted the keys itself (a barrier, one block's scan,
 // a release; partitions over 32 keys searched a common overflow list) and five
 // copies followed it.  Launch to end: 868 results 14.5 -> 10.1 us, 12,245 results
 // clustered in index 33 -> 24 us with their 735 KB written to the host; the whole
@@ -2565,7 +2566,7 @@ __device__ __forceinline__ void fin_end(Counters* C, Counters* host, FinShared& 
 }
 
 // Exclusive scan of the partition counts c (16 per thread) into `out`; returns
-// the total.  big: some count is over kFinBig.
+// the total.
 __device__ __forceinline__ uint32_t fin_scan(const uint4 (&c)[4], uint32_t* out, uint32_t* warp)
 {
     const unsigned tid = threadIdx.x, lane = tid & 31u, w = tid >> 5;

@@ -69,7 +69,8 @@ struct LaunchCfg {
 // they hold beyond half an iteration's node pairs instead of beyond a whole
 // one's.  The default has neither: the other forms measured slower or equal at
 // every size (two 1.3 M-triangle meshes: 55 us of traversal against 60 with
-// bit 1 and 78 with bit 0).
+// bit 1 and 78 with bit 0).  Bit 2 has no effect; the default has it set because
+// gi_stats.traverse_shape has named the default so.
 struct TravShape {
     bool one_per_sm = false;
     bool give_half = false;
@@ -142,9 +143,9 @@ cudaError_t launch_order_small_phases(const Bufs& b, const OrderBufs& O, bool so
                                       int32_t* segpair_out, bool want_segments, unsigned phases, cudaStream_t st);
 // Everything after the traversal in one launch, for sorted output of up to
 // kFinMax results with keys of at most 63 bits: the exact stage (when pairs were
-// escalated), the segments, and the ordering by partitions of the key's top
-// kFinPartBits bits.  A call over those limits, or with a partition over kFinBig
-// keys, makes the kernel set only Counters::order_redo; the caller then reruns
+// escalated), the segments, and the ordering by the kFinParts partitions that
+// the results were put into as they were found (FinBufs).  A call over those
+// limits, or with a partition over kFinBig keys, makes the kernel set only Counters::order_redo; the caller then reruns
 // on the general path (launch_exact, launch_segments, launch_order_gather).
 constexpr int kFinBig = 2048;
 constexpr uint32_t kFinMax = 1u << 18;

@@ -134,8 +134,10 @@ constexpr int kRsItemsSmall = 4;
 constexpr int kRsWarps = kRsThreads / 32;
 // FEW: up to kRsFew small tiles, every scatter block adds up the tiles' digit
 // counts itself, kept a row per tile, instead of a scan launch before each pass.
-// Builds of 1,000 / 4,000 / 20,000 triangles: 67 / 70 / 81 us with the scans, 58 /
-// 66 / 78 without; of 32,768 triangles (32 tiles) 81 with and 87 without.
+// Builds of 1 / 4 / 16 / 20 tiles: 67.5 / 75.0 / 81.2 / 82.8 us with the scans, 59.6 /
+// 69.3 / 77.0 / 80.2 without.  Beyond, nothing is to be had: of 22 / 24 / 28 / 32
+// tiles 84.1 / 84.8 / 90.9 / 92.8 with and 82.4 / 89.6 / 90.4 / 92.2 without (two
+// spheres' build of 32 tiles: 81 and 87).
 constexpr uint32_t kRsFew = 20;
 // Place of a tile's count of digit d (2^BITS digits).
 template <int BITS, bool FEW>

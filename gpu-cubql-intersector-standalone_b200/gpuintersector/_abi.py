@@ -20,9 +20,6 @@ GI_FLAG_EVENT_TIMES = 2
 GI_FLAG_FIXED_SHAPE = 0x100
 
 
-GI_TRAVERSE_SHAPES = 8
-
-
 def GI_FLAG_SHAPE(k):
     return (int(k) & 7) << 9
 
