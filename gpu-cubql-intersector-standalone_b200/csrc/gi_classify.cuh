@@ -1208,19 +1208,28 @@ __device__ __forceinline__ int classify_small(const double3* pts, unsigned* code
     if (e <= 13 || e > 2000) return DEC_ESC;
     const double s = __hiloint2double((2046 + 13 - e) << 20, 0);  // 2^(13 - (e - 1023))
     if (!(big * s < 0x1p50)) return DEC_ESC;
+    // (a coordinate of 1e-300 that a pose made, beside ones of 2^99, scales to 0; with
+    // s >= 1 none can.  Looked at apart: comparing every integer, scaled back, with
+    // its coordinate keeps both alive, for 84 bytes more of spills in k_finish and
+    // 3 us more of a 59 us call on 56 x 56 grids.)
+    if (s < 1.0) {
+        bool lost = false;
+#pragma unroll
+        for (int i = 0; i < 6; i++)
+            lost = lost | (pts[i].x != 0.0 & pts[i].x * s == 0.0) | (pts[i].y != 0.0 & pts[i].y * s == 0.0) |
+                   (pts[i].z != 0.0 & pts[i].z * s == 0.0);
+        if (lost) return DEC_ESC;
+    }
     // x * s integer for every coordinate: then all differences are exact integers.
-    // Adding 1.5 * 2^52 leaves the integer in the low word.  The integer scaled back
-    // must be x itself: x * s alone may underflow to 0 (coordinates near 2^100
-    // beside one of 2^-1000 that a pose made).
-    const double magic = 0x1.8p52, back = __hiloint2double((e - 13) << 20, 0);  // 1 / s
+    // Adding 1.5 * 2^52 leaves the integer in the low word.
+    const double magic = 0x1.8p52;
     I3 v[6];
     bool whole = true;
 #pragma unroll
     for (int i = 0; i < 6; i++) {
-        const double3 p = pts[i];
-        const double rx = __fma_rn(p.x, s, magic), ry = __fma_rn(p.y, s, magic), rz = __fma_rn(p.z, s, magic);
-        whole = whole & (__dsub_rn(rx, magic) * back == p.x) & (__dsub_rn(ry, magic) * back == p.y) &
-                (__dsub_rn(rz, magic) * back == p.z);
+        const double x = pts[i].x * s, y = pts[i].y * s, z = pts[i].z * s;
+        const double rx = __dadd_rn(x, magic), ry = __dadd_rn(y, magic), rz = __dadd_rn(z, magic);
+        whole = whole & (__dsub_rn(rx, magic) == x) & (__dsub_rn(ry, magic) == y) & (__dsub_rn(rz, magic) == z);
         v[i] = {__double2loint(rx), __double2loint(ry), __double2loint(rz)};
     }
     if (!whole) return DEC_ESC;
