@@ -1116,8 +1116,8 @@ __device__ __forceinline__ unsigned result_code(const TTRes& r)
 // memory.  The steps and the order of the result's points are classify_exact's.
 //
 // Bound by the latency of the gathers and of the integer chains at 16 warps per SM
-// (124 registers): issue slots 42 % busy, of 8.6 cycles per issued instruction and
-// warp 3.3 wait for memory and 2.1 for a result.  Two coplanar 512 x 512 grids
+// (128 registers): issue slots 42 % busy, of 8.8 cycles per issued instruction and
+// warp 3.4 wait for memory and 2.0 for a result.  Two coplanar 512 x 512 grids
 // (2.4 M escalated pairs): 0.20 ms, 3.5 ms with the general form alone, whose
 // out-of-line code stalls on instruction fetches (4 warps waited for them per issue).
 // Coordinates of other grids pay for the attempt and for the FP64 filter after it:
